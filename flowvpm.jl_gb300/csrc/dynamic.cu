@@ -53,7 +53,7 @@ __device__ __forceinline__ void dyn_stage(SrcMixed* d, const SrcMixed* g)
 template <int N>
 __device__ __forceinline__ void dyn_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
 
-// dJ of every target (Morton order) from every source of the pack (same
+// dJ of every target (curve order) from every source of the pack (same
 // order), accumulated into dJ[idx*9 + k].  Pair math as above; dx as a
 // double-float (x_hi, x_lo).  Each warp streams the sources on its own, 32 per
 // tile, double-buffered with cp.async, over the tiles whose pack box is within
@@ -184,14 +184,18 @@ uj_filter_diff_kernel(int64_t nt, const TgtPos* __restrict__ tgt, int64_t ns_pad
     for (int k = 0; k < 9; k++) dJ[9 * (int64_t)idx + k] += acc[k] + (double)f[k];
 }
 
+// Sources in the targets' curve order, so that the 32-source tiles are compact whatever the
+// caller's order and the walk over those in reach skips the others.
 template <int K>
 __global__ void pack_src_dyn(int64_t ns, int64_t ns_pad, const double* __restrict__ xs, const double* __restrict__ gs,
-                             const double* __restrict__ sgs, SrcMixed* __restrict__ out, float4* __restrict__ box)
+                             const double* __restrict__ sgs, const TgtPos* __restrict__ order,
+                             SrcMixed* __restrict__ out, float4* __restrict__ box)
 {
-    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i >= ns_pad) return;   // whole warps: ns_pad is a multiple of 32
+    const int64_t o = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (o >= ns_pad) return;   // whole warps: ns_pad is a multiple of 32
     SrcMixed p;
-    if (i < ns) {
+    if (o < ns) {
+        const int64_t i = order[o].idx;
         const double px = xs[3 * i], py = xs[3 * i + 1], pz = xs[3 * i + 2];
         const float xh = (float)px, yh = (float)py, zh = (float)pz;
         const double sig = (K == K_SING) ? 1.0 : sgs[i];
@@ -204,8 +208,8 @@ __global__ void pack_src_dyn(int64_t ns, int64_t ns_pad, const double* __restric
         p.b = make_float4(0.f, 0.f, 0.f, 1.f);
         p.gam = make_float4(0.f, 0.f, 0.f, 0.f);
     }
-    out[i] = p;
-    estr_tile_box(i, ns, p.a.x, p.a.y, p.a.z, p.b.w * p.b.w, box);
+    out[o] = p;
+    estr_tile_box(o, ns, p.a.x, p.a.y, p.a.z, p.b.w * p.b.w, box);
 }
 
 // the records, then two float4 per 32-source tile (estr_tile_box)
@@ -227,7 +231,7 @@ static cudaError_t launch_uj_filter_diff_k(int64_t n, const double* x, const dou
     if (w.src_pack_bytes < dyn_src_pack_bytes(n)) return cudaErrorInvalidValue;
     SrcMixed* src = (SrcMixed*)w.src_pack;
     float4* box = (float4*)(src + ns_pad);
-    pack_src_dyn<K><<<(unsigned)((ns_pad + 255) / 256), 256, 0, st>>>(n, ns_pad, x, gam, sig, src, box);
+    pack_src_dyn<K><<<(unsigned)((ns_pad + 255) / 256), 256, 0, st>>>(n, ns_pad, x, gam, sig, tgt, src, box);
     const unsigned grid = (unsigned)((n + DYN_THREADS - 1) / DYN_THREADS);
     const double ha = 1.0 / alpha - 1.0;
     const int m = filter_panels(ha);

@@ -9,7 +9,7 @@
 // costs about 25 flop.  The self pair, which the reference includes but which
 // contributes exactly zero there, is excluded by index (in the factored form
 // its two terms would only cancel to rounding).  Static sources are packed with
-// zero strength; static targets are left untouched.  Targets run in Morton
+// zero strength; static targets are left untouched.  Targets run in curve
 // order (order.cu) like the UJ kernels.  The FP64 kernel keeps the reference's
 // zeta formula; the mixed kernel uses FP32 pair math on per-warp FP32 offsets
 // (see uj.cu) and FP64 accumulation of FP32 blocks, and skips every pair at
@@ -67,7 +67,7 @@ __global__ void pack_estr_mixed(int64_t ns, int64_t ns_pad, const double* __rest
                                 const TgtPos* __restrict__ order, SrcEstrDF* __restrict__ out,
                                 float4* __restrict__ box)
 {
-    // with `order` (sources = targets) the pack follows the targets' Morton order
+    // with `order` (sources = targets) the pack follows the targets' curve order
     const int64_t o = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (o >= ns_pad) return;   // whole warps: ns_pad is a multiple of 32
     SrcEstrDF p;
@@ -240,7 +240,7 @@ template <int K, bool ZETA, bool DZ = false>
 __global__ void __launch_bounds__(UJ_THREADS)
 estr_mixed_kernel(int64_t nt, const TgtPos* __restrict__ tgt, const double* __restrict__ Jt, int64_t ldJt,
                   const uint8_t* __restrict__ static_t, int64_t ns_pad, const SrcEstrDF* __restrict__ src,
-                  const float4* __restrict__ box, int64_t per_split, bool self, bool transposed, double* SFS,
+                  const float4* __restrict__ box, bool self, bool transposed, double* SFS,
                   int64_t ldS, double* partial, int64_t nt_pad, float3 fd = make_float3(0.f, 0.f, 0.f))
 {
     __shared__ SrcEstrDF stage[UJ_WARPS][2][EWT];
@@ -296,14 +296,11 @@ estr_mixed_kernel(int64_t nt, const TgtPos* __restrict__ tgt, const double* __re
     }
     double zg[3] = {0.0, 0.0, 0.0}, zv[3] = {0.0, 0.0, 0.0};
     float sg[3] = {0.f, 0.f, 0.f}, cg[3] = {0.f, 0.f, 0.f}, sv[3] = {0.f, 0.f, 0.f}, cv[3] = {0.f, 0.f, 0.f};
-    const int64_t s0 = (int64_t)blockIdx.y * per_split;
-    const int64_t s1 = min(s0 + per_split, ns_pad);
-    const int ntiles = (int)((s1 - s0) / EWT);
-    const SrcEstrDF* wsrc = src + s0 + lane;
+    const SrcEstrDF* wsrc = src + lane;
     // the split's tiles within reach of the warp's targets, 32 tiles per ballot
     TileWalk walk;
-    walk.init(ntiles);
-    int cur = walk.next<K>(box + 2 * (s0 / EWT), wbox[warp][2], wbox[warp][3], lane);
+    walk.init((int)(ns_pad / EWT), blockIdx.y, gridDim.y);
+    int cur = walk.next<K>(box, wbox[warp][2], wbox[warp][3], lane);
     if (cur >= 0) {
         SrcEstrDF* d = &stage[warp][0][lane];
         const SrcEstrDF* gp = wsrc + (int64_t)cur * EWT;
@@ -313,7 +310,7 @@ estr_mixed_kernel(int64_t nt, const TgtPos* __restrict__ tgt, const double* __re
     }
     int in_flush = 0, buf = 0;
     while (cur >= 0) {
-        const int nxt = walk.next<K>(box + 2 * (s0 / EWT), wbox[warp][2], wbox[warp][3], lane);
+        const int nxt = walk.next<K>(box, wbox[warp][2], wbox[warp][3], lane);
         if (nxt >= 0) {
             const SrcEstrDF* gp = wsrc + (int64_t)nxt * EWT;
             SrcEstrDF* d = &stage[warp][buf ^ 1][lane];
@@ -444,18 +441,18 @@ static cudaError_t launch_estr_k(const EstrArgs& a, const Workspace& w, int num_
                                                   static_s, a.transposed, a.self ? tgt : nullptr, src, box);
         if (a.zeta)
             estr_mixed_kernel<K, true><<<grid, UJ_THREADS, 0, st>>>(a.nt, tgt, a.Jt, a.ldJt, static_t, ns_pad, src,
-                                                                    box, per_split, a.self, a.transposed, a.SFS,
+                                                                    box, a.self, a.transposed, a.SFS,
                                                                     a.ldS, partial, nt_pad);
         else if (a.dz_alpha > 0.0) {
             const double al = a.dz_alpha;
             const float3 fd = make_float3((float)(1.0 / (al * al * al) - 1.0), (float)(1.0 / (al * al * al)),
                                           (float)(1.0 / (al * al) - 1.0));
             estr_mixed_kernel<K, false, true><<<grid, UJ_THREADS, 0, st>>>(a.nt, tgt, a.Jt, a.ldJt, static_t, ns_pad,
-                                                                           src, box, per_split, a.self, a.transposed,
+                                                                           src, box, a.self, a.transposed,
                                                                            a.SFS, a.ldS, partial, nt_pad, fd);
         } else
             estr_mixed_kernel<K, false><<<grid, UJ_THREADS, 0, st>>>(a.nt, tgt, a.Jt, a.ldJt, static_t, ns_pad, src,
-                                                                     box, per_split, a.self, a.transposed, a.SFS,
+                                                                     box, a.self, a.transposed, a.SFS,
                                                                      a.ldS, partial, nt_pad);
     }
     *launches += 2;

@@ -24,7 +24,7 @@
 // so the results are deterministic: pass 1 with the targets in the lanes
 // (Zg_t and the x_t sum), pass 2 with the sources in the lanes (the ten
 // source-side sums; z_ts depends on sigma_s only, so every 1/sigma_s factor is a
-// lane constant applied once at the end).  Particles run in Morton order
+// lane constant applied once at the end).  Particles run in curve order
 // (order.cu) in both roles; sums go to FP64 partial arrays per source split,
 // and an epilogue kernel per pass adds the splits in order and forms the
 // outputs.  FP64 follows the formulas above pair by pair, coincident pairs
@@ -88,7 +88,7 @@ __device__ __forceinline__ float kappa_f32(float s)
 }
 
 // ------------------------------------------------------------------- packing
-// Sources (pass 1) and targets (pass 2) in the targets' Morton order; static
+// Sources (pass 1) and targets (pass 2) in the targets' curve order; static
 // particles carry zero Gamma, v, a and Sbar (they take no part in Estr).
 template <int K>
 __global__ void ea_pack(int64_t n, int64_t n_pad, const TgtPos* __restrict__ order, const double* __restrict__ x,
@@ -144,7 +144,7 @@ __device__ __forceinline__ void write_partial(double* partial, int nacc, int64_t
 }
 
 // ------------------------------------------------------------------ FP64 passes
-// Pass 1: lanes are targets t (Morton position), the tile holds sources.
+// Pass 1: lanes are targets t (curve position), the tile holds sources.
 template <int K>
 __global__ void __launch_bounds__(UJ_THREADS)
 ea1_f64(int64_t n, const TgtPos* __restrict__ tgt, const EA2F64* __restrict__ self, int64_t n_pad,
@@ -176,7 +176,7 @@ ea1_f64(int64_t n, const TgtPos* __restrict__ tgt, const EA2F64* __restrict__ se
     if (t < n) write_partial(partial, NACC1, n_pad, t, acc);
 }
 
-// Pass 2: lanes are sources s (Morton position), the tile holds targets.
+// Pass 2: lanes are sources s (curve position), the tile holds targets.
 template <int K>
 __global__ void __launch_bounds__(UJ_THREADS)
 ea2_f64(int64_t n, const EA1F64* __restrict__ self, int64_t n_pad, const EA2F64* __restrict__ src,
@@ -297,11 +297,11 @@ struct EaFrame {
     }
 };
 
-// Pass 1: lanes are targets t (Morton position), the tiles hold sources.
+// Pass 1: lanes are targets t (curve position), the tiles hold sources.
 template <int K>
 __global__ void __launch_bounds__(UJ_THREADS)
 ea1_mx(int64_t n, const TgtPos* __restrict__ tgt, const EA2Mx* __restrict__ self, int64_t n_pad,
-       const EA1Mx* __restrict__ src, const float4* __restrict__ box, int64_t per_split, double* __restrict__ partial)
+       const EA1Mx* __restrict__ src, const float4* __restrict__ box, double* __restrict__ partial)
 {
     __shared__ EA1Mx stage[UJ_WARPS][2][EA_WT];
     __shared__ float4 offs[UJ_WARPS][2][EA_WT];
@@ -316,17 +316,14 @@ ea1_mx(int64_t n, const TgtPos* __restrict__ tgt, const EA2Mx* __restrict__ self
     float sm[NACC1], cm[NACC1];
 #pragma unroll
     for (int k = 0; k < NACC1; k++) { sm[k] = 0.f; cm[k] = 0.f; }
-    const int64_t s0 = (int64_t)blockIdx.y * per_split, s1 = min(s0 + per_split, n_pad);
-    const int ntiles = (int)((s1 - s0) / EA_WT);
-    const EA1Mx* wsrc = src + s0 + lane;
-    const float4* tbox = box + 2 * (s0 / EA_WT);
+    const EA1Mx* wsrc = src + lane;
     TileWalk walk;
-    walk.init(ntiles);
-    int cur = walk.next<K>(tbox, wbox[warp][0], wbox[warp][1], lane);
+    walk.init((int)(n_pad / EA_WT), blockIdx.y, gridDim.y);
+    int cur = walk.next<K>(box, wbox[warp][0], wbox[warp][1], lane);
     if (cur >= 0) ea_stage(&stage[warp][0][lane], wsrc + (int64_t)cur * EA_WT);
     int in_flush = 0, buf = 0;
     while (cur >= 0) {
-        const int nxt = walk.next<K>(tbox, wbox[warp][0], wbox[warp][1], lane);
+        const int nxt = walk.next<K>(box, wbox[warp][0], wbox[warp][1], lane);
         if (nxt >= 0) {
             ea_stage(&stage[warp][buf ^ 1][lane], wsrc + (int64_t)nxt * EA_WT);
             ea_wait<1>();
@@ -389,12 +386,12 @@ ea1_mx(int64_t n, const TgtPos* __restrict__ tgt, const EA2Mx* __restrict__ self
     if (t < n) write_partial(partial, NACC1, n_pad, t, acc);
 }
 
-// Pass 2: lanes are sources s (Morton position), the tiles hold targets.
+// Pass 2: lanes are sources s (curve position), the tiles hold targets.
 template <int K>
 __global__ void __launch_bounds__(UJ_THREADS)
 ea2_mx(int64_t n, const EA1Mx* __restrict__ self, const double* __restrict__ gam, const TgtPos* __restrict__ tgt,
        const double* __restrict__ J, const uint8_t* __restrict__ st, bool transposed, int64_t n_pad,
-       const EA2Mx* __restrict__ src, const float4* __restrict__ box, int64_t per_split, double* __restrict__ partial)
+       const EA2Mx* __restrict__ src, const float4* __restrict__ box, double* __restrict__ partial)
 {
     __shared__ EA2Mx stage[UJ_WARPS][2][EA_WT];
     __shared__ float4 offs[UJ_WARPS][2][EA_WT];
@@ -425,17 +422,14 @@ ea2_mx(int64_t n, const EA1Mx* __restrict__ self, const double* __restrict__ gam
     float sm[NACC2], cm[NACC2];
 #pragma unroll
     for (int k = 0; k < NACC2; k++) { acc[k] = 0.0; sm[k] = 0.f; cm[k] = 0.f; }
-    const int64_t s0 = (int64_t)blockIdx.y * per_split, s1 = min(s0 + per_split, n_pad);
-    const int ntiles = (int)((s1 - s0) / EA_WT);
-    const EA2Mx* wsrc = src + s0 + lane;
-    const float4* tbox = box + 2 * (s0 / EA_WT);
+    const EA2Mx* wsrc = src + lane;
     TileWalk walk;   // target tiles, tested at the lanes' largest sigma
-    walk.init(ntiles);
-    int cur = walk.next<K>(tbox, wbox[warp][0], wbox[warp][1], lane, i2min);
+    walk.init((int)(n_pad / EA_WT), blockIdx.y, gridDim.y);
+    int cur = walk.next<K>(box, wbox[warp][0], wbox[warp][1], lane, i2min);
     if (cur >= 0) ea_stage(&stage[warp][0][lane], wsrc + (int64_t)cur * EA_WT);
     int in_flush = 0, buf = 0;
     while (cur >= 0) {
-        const int nxt = walk.next<K>(tbox, wbox[warp][0], wbox[warp][1], lane, i2min);
+        const int nxt = walk.next<K>(box, wbox[warp][0], wbox[warp][1], lane, i2min);
         if (nxt >= 0) {
             ea_stage(&stage[warp][buf ^ 1][lane], wsrc + (int64_t)nxt * EA_WT);
             ea_wait<1>();
@@ -504,7 +498,7 @@ ea2_mx(int64_t n, const EA1Mx* __restrict__ self, const double* __restrict__ gam
 }
 
 // ---------------------------------------------------------------- epilogues
-// Pass 1: x_t and J_t of every non-static target (Morton position t).
+// Pass 1: x_t and J_t of every non-static target (curve position t).
 __global__ void ea1_epilogue(int64_t n, int nsplit, const double* __restrict__ partial, int64_t n_pad,
                              const TgtPos* __restrict__ tgt, const uint8_t* __restrict__ st,
                              const double* __restrict__ Sbar, bool transposed, double* xbar, double* Jbar)
@@ -526,7 +520,7 @@ __global__ void ea1_epilogue(int64_t n, int nsplit, const double* __restrict__ p
             Jbar[9 * i + p + 3 * q] += transposed ? a[p] * sb[q] : sb[p] * a[q];
 }
 
-// Pass 2: x_s, Gamma_s, sigma_s and J_s of every non-static source (Morton position s);
+// Pass 2: x_s, Gamma_s, sigma_s and J_s of every non-static source (curve position s);
 // `scale` = (ZNORM/sigma^3, ZNORM/sigma^5, -ZNORM/sigma^4) applied to (A, B), X, Sg (FP64:
 // A, B, Sg, X hold zeta itself, with ZNORM; mixed: zeta / ZNORM).
 template <int K>
@@ -590,12 +584,11 @@ cudaError_t launch_k(const EstrAdjArgs& a, const EstrAdjWork& w, int num_sms, cu
                                                 w.partial);
     } else {
         ea1_mx<K><<<grid, UJ_THREADS, 0, st>>>(n, tgt, (const EA2Mx*)w.pack2, n_pad, (const EA1Mx*)w.pack1, box,
-                                               per_split, w.partial);
+                                               w.partial);
         ea1_epilogue<<<eg, pb, 0, st>>>(n, nsplit, w.partial, n_pad, tgt, a.static_flags, a.Sbar, a.transposed,
                                         a.xbar, a.Jbar);
         ea2_mx<K><<<grid, UJ_THREADS, 0, st>>>(n, (const EA1Mx*)w.pack1, a.gam, tgt, a.J, a.static_flags,
-                                               a.transposed, n_pad, (const EA2Mx*)w.pack2, box, per_split,
-                                               w.partial);
+                                               a.transposed, n_pad, (const EA2Mx*)w.pack2, box, w.partial);
     }
     ea2_epilogue<K><<<eg, pb, 0, st>>>(n, nsplit, w.partial, n_pad, tgt, a.static_flags, a.gam, a.sig, a.J,
                                        a.transposed, mixed, a.xbar, a.gbar, a.sbar, a.Jbar);

@@ -34,8 +34,9 @@ __device__ __forceinline__ void estr_tile_box(int64_t o, int64_t ns, float xh, f
     }
 }
 
-// The tiles of a warp's source range that can be within reach of its targets, in order:
-// lane l tests tile 32 c + l of chunk c against the targets' FP32 box (lo, hi) with the
+// The tiles of a warp's share (every step-th of ntiles from `first`: a target's tiles in reach
+// are its neighbours on the curve, so contiguous shares would leave them all to one split) that
+// can be within reach of its targets, in order: lane l tests tile 32 c + l of chunk c against the targets' FP32 box (lo, hi) with the
 // tile's box from the pack (estr_tile_box), a ballot gives the chunk's tiles in reach, and
 // next() pops them.  A tile is out of reach when its box is farther than zeta_skip_s
 // sigma^2 from the target box at the tile's largest sigma (every pair then has
@@ -46,9 +47,16 @@ __device__ __forceinline__ void estr_tile_box(int64_t o, int64_t ns, float xh, f
 // reach skip_s explicitly (the filter differences' dyn_skip_s); skip_s <= 0 or >= 1e37 (a
 // kernel without a reach) takes every tile.  All 32 lanes call it, with the same values.
 struct TileWalk {
-    int n, c;
+    int n, c, first, step;
     unsigned mask;
-    __device__ __forceinline__ void init(int ntiles) { n = ntiles; c = -1; mask = 0u; }
+    __device__ __forceinline__ void init(int ntiles, int first_ = 0, int step_ = 1)
+    {
+        n = (ntiles - first_ + step_ - 1) / step_;
+        first = first_;
+        step = step_;
+        c = -1;
+        mask = 0u;
+    }
     template <int K>
     __device__ __forceinline__ int next(const float4* __restrict__ box, const float4 lo, const float4 hi, int lane,
                                         float wfix = 0.0f)
@@ -61,8 +69,8 @@ struct TileWalk {
         while (mask == 0u) {
             if ((c + 1) * 32 >= n) return -1;
             ++c;
-            const int i = c * 32 + lane;
-            bool in = i < n;
+            const int i = first + (c * 32 + lane) * step;
+            bool in = c * 32 + lane < n;
             if (skip_s > 0.0f && skip_s < 1.0e37f && in) {
                 const float4 bl = box[2 * i], bh = box[2 * i + 1];
                 const float ex = fmaxf(fmaxf(lo.x - bh.x, bl.x - hi.x), 0.0f);
@@ -74,7 +82,7 @@ struct TileWalk {
         }
         const int b = __ffs(mask) - 1;
         mask &= mask - 1u;
-        return c * 32 + b;
+        return first + (c * 32 + b) * step;
     }
 };
 
