@@ -71,7 +71,7 @@ struct vpm_ctx {
     PinBuf hin, hout;
     DevBuf din, dout;
     // packing and split-K scratch
-    DevBuf src_pack, order, partial, flag;
+    DevBuf src_pack, order, partial, flag, tiles;
     // near-field: packed particles, and the lists (built on the device or uploaded)
     DevBuf leaf;
     NearScratch near;
@@ -324,6 +324,21 @@ int ensure_work(vpm_ctx* c, int64_t nt, int64_t ns, int precision, bool estr, Wo
     return VPM_OK;
 }
 
+// Scratch of the tensor pass of a self-induced FP32-comp UJ; without room for it the call
+// takes the plain kernel.
+void ensure_tiles(vpm_ctx* c, const UJArgs& a, Workspace* w)
+{
+    if (!uj_takes_tiles(a)) return;
+    if (c->tiles.grow(uj_tc_bytes(a.ns)) != cudaSuccess ||
+        c->partial.grow(uj_partial_bytes(a.nt, uj_tc_splits(a.nt, c->num_sms))) != cudaSuccess) {
+        cudaGetLastError();
+        return;
+    }
+    w->tiles = c->tiles.p;
+    w->partial = (double*)c->partial.p;
+    w->partial_bytes = c->partial.cap;
+}
+
 int grow(vpm_ctx* c, DevBuf& b, size_t bytes, const char* what)
 {
     if (b.grow(bytes) != cudaSuccess) {
@@ -419,7 +434,7 @@ int vpm_ctx_destroy(vpm_ctx* c)
         DeviceGuard dg(c->device);
         if (!c->broken) cudaStreamSynchronize(c->stream);
         for (DevBuf* b : {&c->mat, &c->mat2, &c->x, &c->g, &c->s, &c->st, &c->xt, &c->src_pack, &c->order,
-                          &c->partial, &c->flag, &c->leaf})
+                          &c->partial, &c->flag, &c->tiles, &c->leaf})
             b->release();
         c->near.release_all();
         for (DevBuf* b : {&c->din, &c->dout}) b->release();
@@ -557,6 +572,7 @@ static int uj_full_matrix(vpm_ctx* c, double* particles, int64_t np, int kernel,
     a.nt = np; a.ns = np; a.xt = x; a.xs = x; a.gs = g; a.sgs = s;
     a.U = mat + R_U; a.ldU = VPM_NFIELDS; a.J = mat + R_J; a.ldJ = VPM_NFIELDS;
     a.kernel = kernel; a.precision = precision; a.self = true;
+    ensure_tiles(c, a, &w);
     CK(launch_uj(a, w, c->num_sms, st, &c->launches), "UJ kernels");
     if (sfs) {
         EstrArgs e;
@@ -643,6 +659,7 @@ static int uj_staged(vpm_ctx* c, double* particles, int64_t np, int kernel, int 
     a.nt = np; a.ns = np; a.xt = x; a.xs = x; a.gs = g; a.sgs = s;
     a.U = dU; a.ldU = 3; a.J = dJ; a.ldJ = 9;
     a.kernel = kernel; a.precision = precision; a.self = true;
+    ensure_tiles(c, a, &w);
     CK(launch_uj(a, w, c->num_sms, st, &c->launches), "UJ kernels");
     if (sfs) {
         EstrArgs e;
@@ -742,6 +759,7 @@ int vpm_uj_cross(vpm_ctx* c, const double* src, int64_t ld_src, int64_t ns, doub
     a.nt = nt; a.ns = ns; a.xt = (double*)c->xt.p; a.xs = (double*)c->x.p; a.gs = (double*)c->g.p;
     a.sgs = (double*)c->s.p; a.U = mt + R_U; a.ldU = VPM_NFIELDS; a.J = mt + R_J; a.ldJ = VPM_NFIELDS;
     a.kernel = kernel; a.precision = precision; a.self = false;
+    ensure_tiles(c, a, &w);
     CK(launch_uj(a, w, c->num_sms, st, &c->launches), "UJ kernels");
     RC(bounded_wait(c));
     const size_t pitch = VPM_NFIELDS * sizeof(double);
@@ -773,6 +791,7 @@ int vpm_uj_dev(vpm_ctx* c, int64_t nt, const double* xt, int64_t ns, const doubl
     UJArgs a;
     a.nt = nt; a.ns = ns; a.xt = xt; a.xs = xs; a.gs = gs; a.sgs = sgs;
     a.U = U; a.ldU = 3; a.J = J; a.ldJ = 9; a.kernel = kernel; a.precision = precision; a.self = self;
+    ensure_tiles(c, a, &w);
     CK(launch_uj(a, w, c->num_sms, c->stream, &c->launches), "UJ kernels");
     return bounded_wait(c);
 }
@@ -1362,7 +1381,7 @@ int vpm_estr_adjoint_dev(vpm_ctx* c, int64_t n, const double* x, const double* g
         !is_device_ptr(Jbar) || (static_flags && !is_device_ptr(static_flags)))
         return fail(c, VPM_ERR_ARG, "%s: every array must be a device pointer", fn);
     const EstrAdjSizes z = estr_adjoint_sizes(n, c->num_sms);
-    RC(grow(c, c->order, order_bytes(n), "Morton ordering"));
+    RC(grow(c, c->order, order_bytes(n), "curve ordering"));
     RC(grow(c, c->src_pack, 2 * z.pack, "adjoint packs"));
     RC(grow(c, c->partial, z.partial, "adjoint partial sums"));
     EstrAdjWork w;

@@ -14,7 +14,7 @@
 // with q'' (hence the kernels' g'') in B'.  x_t gets +dphi/d(dx), x_s gets
 // -dphi/d(dx).
 //
-// Layout: one target per thread (Morton order, as in uj.cu), sources staged in
+// Layout: one target per thread (curve order, as in uj.cu), sources staged in
 // shared memory.  Target-side sums stay in registers; each source's 7 sums
 // (x, Gamma, sigma) are reduce-scattered across the warp with shuffles, four
 // sources at a time (adj_reduce4), summed across the
@@ -257,7 +257,7 @@ __global__ void pack_src_adj(int64_t ns, int64_t ns_pad, const double* __restric
 
 // ------------------------------------------------------------- FP32-comp adjoint
 // The same pair derivatives in FP32 with the forward mixed kernel's layout:
-// targets and sources in Morton order, FP32 offsets from the warp's first
+// targets and sources in curve order, FP32 offsets from the warp's first
 // target, four-source votes between the singular form (every lane's pairs
 // beyond s_far and twice the warp radius) and the full form on the
 // double-float displacement.  With s = r^2/sigma^2 and e = e^{-s/2}, the

@@ -17,7 +17,7 @@ struct TraceRange {
     TraceRange& operator=(const TraceRange&) = delete;
 };
 
-// A target in Morton order: FP64 position and its index in the caller's arrays.
+// A target in curve order: FP64 position and its index in the caller's arrays.
 struct __align__(16) TgtPos { double x, y, z; int32_t idx, pad; };
 
 // Packed source of the mixed (FP32-comp) UJ kernel, 48 B:
@@ -93,7 +93,7 @@ struct EstrAdjArgs {
     bool transposed;
 };
 struct EstrAdjWork {
-    void* order; size_t order_bytes;          // Morton ordering of the particles
+    void* order; size_t order_bytes;          // curve ordering of the particles
     void* pack1; void* pack2;                 // EstrAdjSizes::pack bytes each
     double* partial;                          // EstrAdjSizes::partial bytes
 };
@@ -116,8 +116,9 @@ struct LeafArgs {
 // Scratch and packing buffers supplied by the caller (the context).
 struct Workspace {
     void* src_pack; size_t src_pack_bytes;
-    void* order; size_t order_bytes;          // Morton ordering of the targets
+    void* order; size_t order_bytes;          // curve ordering of the targets
     double* partial; size_t partial_bytes;    // split-source partial sums
+    void* tiles = nullptr;                    // uj_tc_bytes: the tensor pass's tiles (null: not taken)
 };
 
 size_t uj_src_pack_bytes(int64_t ns, int precision);
@@ -125,8 +126,14 @@ size_t estr_src_pack_bytes(int64_t ns, int precision);
 size_t order_bytes(int64_t nt);
 int uj_num_splits(int64_t nt, int64_t ns, int num_sms);
 size_t uj_partial_bytes(int64_t nt, int nsplit);
+// The far pairs' sums of a set on itself on the tensor cores (uj_tc.cu).
+bool uj_takes_tiles(const UJArgs& a);
+size_t uj_tc_bytes(int64_t n);
+int uj_tc_splits(int64_t n, int num_sms);
+cudaError_t launch_uj_tc(const UJArgs& a, const TgtPos* tgt, const SrcMixed* src, void* work, int nsplit,
+                         double* partial, int64_t nt_pad, cudaStream_t st, int64_t* launches);
 
-// Morton-order the nt targets xt; *out receives nt TgtPos records in scratch.
+// Curve-order the nt targets xt; *out receives nt TgtPos records in scratch.
 cudaError_t order_targets(int64_t nt, const double* xt, void* scratch, size_t scratch_bytes, cudaStream_t st,
                           int64_t* launches, const TgtPos** out);
 

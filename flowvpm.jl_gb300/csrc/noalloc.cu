@@ -5,7 +5,7 @@
 // framework's caching pool, an arena reserved at start-up) or must not
 // allocate once they are running, so they cannot let the library call
 // cudaMalloc.  This entry point needs no context and allocates nothing: the
-// kernels' scratch (packed sources, the Morton ordering of the targets and
+// kernels' scratch (packed sources, the curve ordering of the targets and
 // the split-source partial sums) lives in one file-scope __device__ array of
 // VPM_NOALLOC_SCRATCH_BYTES, which every GPU that loads this library's code
 // for this entry point holds until the process exits.
@@ -129,6 +129,14 @@ int vpm_uj_dev_noalloc(int64_t nt, const double* xt, int64_t ns, const double* x
     a.nt = nt; a.ns = ns; a.xt = xt; a.xs = xs; a.gs = gs; a.sgs = sgs;
     a.U = U; a.ldU = 3; a.J = J; a.ldJ = 9; a.kernel = kernel; a.precision = precision;
     a.self = (xt == xs) && (nt == ns);
+    // the tensor pass of vpm_uj_dev where its tiles fit the scratch too
+    const size_t tc_part = align256(vpm::uj_partial_bytes(nt, vpm::uj_tc_splits(nt, sms)));
+    const size_t tiles = align256(vpm::uj_tc_bytes(ns));
+    if (vpm::uj_takes_tiles(a) && pack + order + tc_part + tiles <= (size_t)VPM_NOALLOC_SCRATCH_BYTES) {
+        w.partial = tc_part ? (double*)p : nullptr;
+        w.partial_bytes = tc_part;
+        w.tiles = p + tc_part;
+    }
     cudaStream_t st = (cudaStream_t)stream;
     int64_t launches = 0;
     cudaError_t e = vpm::launch_uj(a, w, sms, st, &launches);

@@ -3,8 +3,8 @@
 // src/FLOWVPM_UJ.jl:35).
 //
 // Layout: one target per thread, UJ_THREADS targets per block, targets in
-// Morton order (order.cu) so each warp holds 32 neighbouring targets.  Sources
-// are packed once per call (in the same Morton order when they are the
+// curve order (order.cu) so each warp holds 32 neighbouring targets.  Sources
+// are packed once per call (in the same curve order when they are the
 // targets).  The FP64 kernel streams them through shared memory in block-wide
 // tiles of UJ_TILE; in the mixed kernel every warp streams them on its own in
 // tiles of 32, double-buffered with cp.async, so warps never wait for one
@@ -59,6 +59,12 @@ int uj_num_splits(int64_t nt, int64_t ns, int num_sms)
     return (int)nsplit;
 }
 
+// The tile kernels (uj_tc.cu) take a set on itself from 12,288 particles.  Below, most tiles of
+// 64 are near ones (4,099 random particles: 73 % of the pairs) and the tile pack is pure cost:
+// 4,000 to 10,000 particles ran within 3 % of uj_mixed_kernel (Winckelmans 4,099 20 % slower),
+// 16,384 10 % faster (741 against 820 us), 65,536 1.6 times.
+bool uj_takes_tiles(const UJArgs& a) { return a.self && a.precision == 1 && a.ns >= 12288; }
+
 size_t uj_partial_bytes(int64_t nt, int nsplit)
 {
     return nsplit > 1 ? (size_t)nsplit * 12 * (size_t)round_up(nt, UJ_THREADS) * sizeof(double) : 0;
@@ -67,7 +73,7 @@ size_t uj_partial_bytes(int64_t nt, int nsplit)
 
 // ------------------------------------------------------------------ packing
 // When `order` is given (sources = targets), source i of the pack is particle
-// order[i].idx, i.e. the sources follow the targets' Morton order: a warp's
+// order[i].idx, i.e. the sources follow the targets' curve order: a warp's
 // near sources then sit in few 4-source groups, so fewer groups take the near
 // path.  The order of a sum's terms does not otherwise matter.
 template <int K>
@@ -167,22 +173,6 @@ __device__ __forceinline__ void pair_f64(double tx, double ty, double tz, const 
 #endif
 
 // --------------------------------------------------------------- epilogue
-__device__ __forceinline__ void write_uj(int64_t t, int32_t idx, const double (&acc)[12], double* U,
-                                         int64_t ldU, double* J, int64_t ldJ, double* partial, int64_t nt_pad)
-{
-    if (partial) {
-        double* p = partial + (int64_t)blockIdx.y * 12 * nt_pad + t;
-#pragma unroll
-        for (int k = 0; k < 12; k++) p[k * nt_pad] = acc[k];
-    } else {
-        const int64_t i = idx;
-#pragma unroll
-        for (int k = 0; k < 3; k++) U[i * ldU + k] += acc[k];
-#pragma unroll
-        for (int k = 0; k < 9; k++) J[i * ldJ + k] += acc[3 + k];
-    }
-}
-
 __global__ void uj_reduce(int64_t nt, int nsplit, const double* __restrict__ partial, int64_t nt_pad,
                           const TgtPos* __restrict__ tgt, double* U, int64_t ldU, double* J, int64_t ldJ)
 {
@@ -571,7 +561,7 @@ uj_mixed_kernel(int64_t nt, const TgtPos* __restrict__ tgt, int64_t ns_pad,
     write_uj(t, idx, acc, U, ldU, J, ldJ, partial, nt_pad);
 }
 // --------------------------------------------- mixed kernel, two targets a lane
-// uj_mixed_kernel with two targets per lane: a warp takes 64 Morton-consecutive
+// uj_mixed_kernel with two targets per lane: a warp takes 64 curve-consecutive
 // targets (lane l: base + l and base + 32 + l), so that each source's shared-memory
 // reads, its tile's far flag and the tile's loads and conversions serve two pairs.
 // Blocks of 128 threads take 256 targets; the register budget is 3 resident blocks
@@ -1076,7 +1066,8 @@ static cudaError_t launch_uj_k(const UJArgs& a, const Workspace& w, int num_sms,
 {
     const int64_t ns_pad = round_up(a.ns, UJ_TILE);
     const int64_t nt_pad = round_up(a.nt, UJ_THREADS);
-    const int nsplit = uj_num_splits(a.nt, a.ns, num_sms);
+    const bool tc = uj_takes_tiles(a) && w.tiles;
+    const int nsplit = tc ? uj_tc_splits(a.nt, num_sms) : uj_num_splits(a.nt, a.ns, num_sms);
     const int64_t tiles = ns_pad / UJ_TILE;
     const int64_t per_split = ((tiles + nsplit - 1) / nsplit) * UJ_TILE;
     double* partial = nsplit > 1 ? w.partial : nullptr;
@@ -1094,6 +1085,10 @@ static cudaError_t launch_uj_k(const UJArgs& a, const Workspace& w, int num_sms,
         SrcMixed* src = (SrcMixed*)w.src_pack;
         pack_src_mixed<K><<<(unsigned)((ns_pad + pb - 1) / pb), pb, 0, st>>>(a.ns, ns_pad, a.xs, a.gs, a.sgs,
                                                                              a.self ? tgt : nullptr, src);
+        if (tc) {
+            e = launch_uj_tc(a, tgt, src, w.tiles, nsplit, partial, nt_pad, st, launches);
+            if (e != cudaSuccess) return e;
+        } else
 #if VPM_UJ_F32X2
         uj_mixed_x2_kernel<K><<<grid, UJ_THREADS, 0, st>>>(a.nt, tgt, ns_pad, src, per_split, a.U, a.ldU,
                                                             a.J, a.ldJ, partial, nt_pad);

@@ -315,4 +315,38 @@ __device__ __forceinline__ void uj_f64_finish(const double (&u)[3], const double
     acc[10] += wx;
 }
 
+// U and J of one target from the mixed kernels' sums f = (U, W, J'): J = -3 J' (J'_33 =
+// -J'_11 - J'_22) plus the Kronecker term of src/FLOWVPM_fmm.jl:148-159 (W = sum aux2 Gamma).
+__device__ __forceinline__ void uj_mixed_finish(const double (&f)[14], double (&acc)[12])
+{
+#pragma unroll
+    for (int k = 0; k < 3; k++) acc[k] = f[k];
+#pragma unroll
+    for (int k = 0; k < 8; k++) acc[3 + k] = -3.0 * f[6 + k];
+    acc[11] = 3.0 * (f[6] + f[10]);
+    acc[4] -= f[5];
+    acc[5] += f[4];
+    acc[6] += f[5];
+    acc[8] -= f[3];
+    acc[9] -= f[4];
+    acc[10] += f[3];
+}
+
+// One target's sums: added to its rows, or written to its split's partial sums.
+__device__ __forceinline__ void write_uj(int64_t t, int32_t idx, const double (&acc)[12], double* U,
+                                         int64_t ldU, double* J, int64_t ldJ, double* partial, int64_t nt_pad)
+{
+    if (partial) {
+        double* p = partial + (int64_t)blockIdx.y * 12 * nt_pad + t;
+#pragma unroll
+        for (int k = 0; k < 12; k++) p[k * nt_pad] = acc[k];
+    } else {
+        const int64_t i = idx;
+#pragma unroll
+        for (int k = 0; k < 3; k++) U[i * ldU + k] += acc[k];
+#pragma unroll
+        for (int k = 0; k < 9; k++) J[i * ldJ + k] += acc[3 + k];
+    }
+}
+
 }  // namespace vpm

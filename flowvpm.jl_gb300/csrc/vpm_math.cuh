@@ -304,7 +304,13 @@ __device__ __forceinline__ void near_GQ(float s, float isig2, float& G, float& Q
         G = (s + 2.5f) * t2u;
         Q = (s + 3.5f) * t * t2u * isig2;
     } else if constexpr (K == K_SING) {
-        far_GQ(s, isig2, G, Q);
+        // J of a singular cloud is a handful of its nearest pairs, and Q = r^-5 carries five
+        // times the error of rsqrt.approx: one Newton step
+        float rs = frsqrt(s);
+        rs = fmaf(0.5f * rs, fmaf(-s * rs, rs, 1.0f), rs);
+        const float rs2 = rs * rs;
+        G = rs * rs2;
+        Q = G * (rs2 * isig2);
     } else if constexpr (K == K_GAUSERF) {
         gerf_GQ<FAR>(s, isig2, G, Q);
     } else {  // Gaussian
