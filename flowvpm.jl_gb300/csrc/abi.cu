@@ -311,8 +311,9 @@ int ensure_work(vpm_ctx* c, int64_t nt, int64_t ns, int precision, bool estr, Wo
     size_t sp = uj_src_pack_bytes(ns, precision);
     if (estr) { size_t e = estr_src_pack_bytes(ns, precision); if (e > sp) sp = e; }
     const size_t ob = order_bytes(nt);
-    const int nsplit = uj_num_splits(nt, ns, c->num_sms);
-    const size_t pb = uj_partial_bytes(nt, nsplit);
+    const int nsplit = uj_num_splits(nt, ns, c->num_sms, precision);
+    size_t pb = uj_partial_bytes(nt, nsplit);
+    if (precision && nt == ns) pb = std::max(pb, uj_partial_bytes(nt, uj_tc_splits(nt, c->num_sms)));
     if (c->src_pack.grow(sp) != cudaSuccess || c->order.grow(ob) != cudaSuccess ||
         (pb && c->partial.grow(pb) != cudaSuccess)) {
         cudaGetLastError();
@@ -329,14 +330,8 @@ int ensure_work(vpm_ctx* c, int64_t nt, int64_t ns, int precision, bool estr, Wo
 void ensure_tiles(vpm_ctx* c, const UJArgs& a, Workspace* w)
 {
     if (!uj_takes_tiles(a)) return;
-    if (c->tiles.grow(uj_tc_bytes(a.ns)) != cudaSuccess ||
-        c->partial.grow(uj_partial_bytes(a.nt, uj_tc_splits(a.nt, c->num_sms))) != cudaSuccess) {
-        cudaGetLastError();
-        return;
-    }
-    w->tiles = c->tiles.p;
-    w->partial = (double*)c->partial.p;
-    w->partial_bytes = c->partial.cap;
+    if (c->tiles.grow(uj_tc_bytes(a.ns)) == cudaSuccess) w->tiles = c->tiles.p;
+    else cudaGetLastError();
 }
 
 int grow(vpm_ctx* c, DevBuf& b, size_t bytes, const char* what)

@@ -153,8 +153,7 @@ template <int K>
 __global__ void __launch_bounds__(UJ_THREADS)
 uj_adjoint_f64_kernel(int64_t nt, const TgtPos* __restrict__ tgt, const double* __restrict__ Ubar,
                       const double* __restrict__ Jbar, int64_t ns, int64_t ns_pad,
-                      const SrcF64* __restrict__ src, int64_t per_split, double* xbar, double* gbar,
-                      double* sbar)
+                      const SrcF64* __restrict__ src, double* xbar, double* gbar, double* sbar)
 {
     __shared__ SrcF64 tile[UJ_TILE];
     __shared__ double red[UJ_WARPS][UJ_TILE][7];
@@ -177,13 +176,14 @@ uj_adjoint_f64_kernel(int64_t nt, const TgtPos* __restrict__ tgt, const double* 
     // wbar_l = eps_abl Jbar_ab with Jbar_ab at Jb[a + 3b]
     const double wb[3] = {Jb[1 + 3 * 2] - Jb[2 + 3 * 1], Jb[2 + 3 * 0] - Jb[0 + 3 * 2], Jb[0 + 3 * 1] - Jb[1 + 3 * 0]};
     double acc[3] = {0.0, 0.0, 0.0};
-    const int64_t s0 = (int64_t)blockIdx.y * per_split;
-    const int64_t s1 = min(s0 + per_split, ns_pad);
-    for (int64_t base = s0; base < s1; base += UJ_TILE) {
+    const int64_t nq = split_count(ns_pad, blockIdx.y, gridDim.y);
+    for (int64_t base = 0; base < nq; base += UJ_TILE) {
         __syncthreads();
-        tile[threadIdx.x] = src[base + threadIdx.x];
+        const int m = (int)min((int64_t)UJ_TILE, nq - base);      // a multiple of F64_UNIT
+        const int64_t si = split_source(base + threadIdx.x, blockIdx.y, gridDim.y);
+        if (threadIdx.x < m) tile[threadIdx.x] = src[si];
         __syncthreads();
-        for (int j = 0; j < UJ_TILE; j += 4) {
+        for (int j = 0; j < m; j += 4) {
             double o0[7], o1[7], o2[7], o3[7];
             {
                 const SrcF64& s = tile[j];
@@ -211,8 +211,7 @@ uj_adjoint_f64_kernel(int64_t nt, const TgtPos* __restrict__ tgt, const double* 
             }
         }
         __syncthreads();
-        const int64_t si = base + threadIdx.x;
-        if (si < ns) {
+        if (threadIdx.x < m && si < ns) {
             double v[7];
 #pragma unroll
             for (int k = 0; k < 7; k++) v[k] = red[0][threadIdx.x][k] + red[1][threadIdx.x][k] +
@@ -674,7 +673,7 @@ static cudaError_t launch_adj_k(const AdjArgs& a, const Workspace& w, int num_sm
     const int64_t nt_pad = (a.n + UJ_THREADS - 1) / UJ_THREADS * UJ_THREADS;
     const int64_t tiles = ns_pad / UJ_TILE;
     const int nsplit = a.precision ? adj_splits(uj_adjoint_mixed_kernel<K>, nt_pad / UJ_THREADS, tiles, num_sms)
-                                   : uj_num_splits(a.n, a.n, num_sms);
+                                   : uj_num_splits(a.n, a.n, num_sms, 0);
     const int64_t per_split = ((tiles + nsplit - 1) / nsplit) * UJ_TILE;
     const TgtPos* tgt = nullptr;
     cudaError_t e = order_targets(a.n, a.x, w.order, w.order_bytes, st, launches, &tgt);
@@ -689,7 +688,7 @@ static cudaError_t launch_adj_k(const AdjArgs& a, const Workspace& w, int num_sm
     } else {
         SrcF64* src = (SrcF64*)w.src_pack;
         pack_src_adj<K><<<(unsigned)((ns_pad + 255) / 256), 256, 0, st>>>(a.n, ns_pad, a.x, a.gam, a.sig, src);
-        uj_adjoint_f64_kernel<K><<<grid, UJ_THREADS, 0, st>>>(a.n, tgt, a.Ubar, a.Jbar, a.n, ns_pad, src, per_split,
+        uj_adjoint_f64_kernel<K><<<grid, UJ_THREADS, 0, st>>>(a.n, tgt, a.Ubar, a.Jbar, a.n, ns_pad, src,
                                                               a.xbar, a.gbar, a.sbar);
     }
     *launches += 2;

@@ -153,11 +153,11 @@ __global__ void estr_reduce(int64_t nt, int nsplit, const double* __restrict__ p
     if (t >= nt) return;
     const int64_t i = tgt[t].idx;
     if (static_t && static_t[i]) return;
-    for (int k = 0; k < 3; k++) {
-        double s = 0.0;
-        for (int sp = 0; sp < nsplit; sp++) s += partial[((int64_t)sp * 3 + k) * nt_pad + t];
-        SFS[i * ldS + k] += s;
-    }
+    const double* p = partial + blockIdx.y * nt_pad + t;
+    double s = 0.0;
+#pragma unroll 8
+    for (int sp = 0; sp < nsplit; sp++) s += p[(int64_t)sp * 3 * nt_pad];
+    SFS[i * ldS + blockIdx.y] += s;
 }
 
 // With ZETA the kernels evaluate zeta_direct instead (src/FLOWVPM_viscous.jl:467-488):
@@ -167,8 +167,7 @@ template <int K, bool ZETA>
 __global__ void __launch_bounds__(UJ_THREADS)
 estr_f64_kernel(int64_t nt, const TgtPos* __restrict__ tgt, const double* __restrict__ Jt, int64_t ldJt,
                 const uint8_t* __restrict__ static_t, int64_t ns_pad, const SrcEstrF64* __restrict__ src,
-                int64_t per_split, bool self, bool transposed, double* SFS, int64_t ldS,
-                double* partial, int64_t nt_pad)
+                bool self, bool transposed, double* SFS, int64_t ldS, double* partial, int64_t nt_pad)
 {
     __shared__ SrcEstrF64 tile[UJ_TILE];
     const int64_t t = (int64_t)blockIdx.x * UJ_THREADS + threadIdx.x;
@@ -179,18 +178,18 @@ estr_f64_kernel(int64_t nt, const TgtPos* __restrict__ tgt, const double* __rest
         tx = p.x; ty = p.y; tz = p.z; idx = p.idx;
     }
     const bool valid = t < nt && (ZETA || !(static_t && static_t[idx]));
-    const int64_t self_idx = (self && !ZETA) ? idx : -1;
+    const int64_t self_q = (self && !ZETA) ? split_position(idx, blockIdx.y, gridDim.y) : -1;
     double zg[3] = {0.0, 0.0, 0.0}, zv[3] = {0.0, 0.0, 0.0};
-    const int64_t s0 = (int64_t)blockIdx.y * per_split;
-    const int64_t s1 = min(s0 + per_split, ns_pad);
-    for (int64_t base = s0; base < s1; base += UJ_TILE) {
+    const int64_t nq = split_count(ns_pad, blockIdx.y, gridDim.y);
+    for (int64_t base = 0; base < nq; base += UJ_TILE) {
         __syncthreads();
-        tile[threadIdx.x] = src[base + threadIdx.x];
+        if (base + threadIdx.x < nq) tile[threadIdx.x] = src[split_source(base + threadIdx.x, blockIdx.y, gridDim.y)];
         __syncthreads();
+        const int m = (int)min((int64_t)UJ_TILE, nq - base);
 #pragma unroll 2
-        for (int j = 0; j < UJ_TILE; j++) {
+        for (int j = 0; j < m; j++) {
             const SrcEstrF64& p = tile[j];
-            if (base + j == self_idx) continue;
+            if (base + j == self_q) continue;
             const double dx = p.xy.x - tx, dy = p.xy.y - ty, dz = p.z_isig.x - tz;
             const double r = sqrt(dx * dx + dy * dy + dz * dz);
             const double isig = p.z_isig.y;
@@ -409,9 +408,7 @@ static cudaError_t launch_estr_k(const EstrArgs& a, const Workspace& w, int num_
 {
     const int64_t ns_pad = round_up(a.ns, UJ_TILE);
     const int64_t nt_pad = round_up(a.nt, UJ_THREADS);
-    const int nsplit = uj_num_splits(a.nt, a.ns, num_sms);
-    const int64_t tiles = ns_pad / UJ_TILE;
-    const int64_t per_split = ((tiles + nsplit - 1) / nsplit) * UJ_TILE;
+    const int nsplit = uj_num_splits(a.nt, a.ns, num_sms, a.precision);
     double* partial = nsplit > 1 ? w.partial : nullptr;
     const dim3 grid((unsigned)(nt_pad / UJ_THREADS), (unsigned)nsplit);
     const int pb = 256;
@@ -428,12 +425,12 @@ static cudaError_t launch_estr_k(const EstrArgs& a, const Workspace& w, int num_
                                                 static_s, a.transposed, src);
         if (a.zeta)
             estr_f64_kernel<K, true><<<grid, UJ_THREADS, 0, st>>>(a.nt, tgt, a.Jt, a.ldJt, static_t, ns_pad, src,
-                                                                  per_split, a.self, a.transposed, a.SFS, a.ldS,
-                                                                  partial, nt_pad);
+                                                                  a.self, a.transposed, a.SFS, a.ldS, partial,
+                                                                  nt_pad);
         else
             estr_f64_kernel<K, false><<<grid, UJ_THREADS, 0, st>>>(a.nt, tgt, a.Jt, a.ldJt, static_t, ns_pad, src,
-                                                                   per_split, a.self, a.transposed, a.SFS, a.ldS,
-                                                                   partial, nt_pad);
+                                                                   a.self, a.transposed, a.SFS, a.ldS, partial,
+                                                                   nt_pad);
     } else {
         SrcEstrDF* src = (SrcEstrDF*)w.src_pack;
         float4* box = (float4*)(src + ns_pad);   // the tile boxes follow the records
@@ -457,7 +454,7 @@ static cudaError_t launch_estr_k(const EstrArgs& a, const Workspace& w, int num_
     }
     *launches += 2;
     if (partial) {
-        estr_reduce<<<(unsigned)((a.nt + pb - 1) / pb), pb, 0, st>>>(a.nt, nsplit, partial, nt_pad, tgt,
+        estr_reduce<<<dim3((unsigned)((a.nt + 127) / 128), 3), 128, 0, st>>>(a.nt, nsplit, partial, nt_pad, tgt,
                                                                    static_t, a.SFS, a.ldS);
         *launches += 1;
     }

@@ -148,21 +148,22 @@ __device__ __forceinline__ void write_partial(double* partial, int nacc, int64_t
 template <int K>
 __global__ void __launch_bounds__(UJ_THREADS)
 ea1_f64(int64_t n, const TgtPos* __restrict__ tgt, const EA2F64* __restrict__ self, int64_t n_pad,
-        const EA1F64* __restrict__ src, int64_t per_split, double* __restrict__ partial)
+        const EA1F64* __restrict__ src, double* __restrict__ partial)
 {
     __shared__ EA1F64 tile[UJ_TILE];
     const int64_t t = (int64_t)blockIdx.x * UJ_THREADS + threadIdx.x;
     const EA2F64 me = self[t < n ? t : n_pad - 1];     // a_t, Sbar_t (zero for static targets)
     double acc[NACC1] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-    const int64_t s0 = (int64_t)blockIdx.y * per_split, s1 = min(s0 + per_split, n_pad);
-    for (int64_t base = s0; base < s1; base += UJ_TILE) {
+    const int64_t nq = split_count(n_pad, blockIdx.y, gridDim.y), self_q = split_position(t, blockIdx.y, gridDim.y);
+    for (int64_t base = 0; base < nq; base += UJ_TILE) {
         __syncthreads();
-        tile[threadIdx.x] = src[base + threadIdx.x];
+        if (base + threadIdx.x < nq) tile[threadIdx.x] = src[split_source(base + threadIdx.x, blockIdx.y, gridDim.y)];
         __syncthreads();
+        const int m = (int)min((int64_t)UJ_TILE, nq - base);
 #pragma unroll 2
-        for (int j = 0; j < UJ_TILE; j++) {
+        for (int j = 0; j < m; j++) {
             const EA1F64& p = tile[j];
-            if (base + j == t) continue;
+            if (base + j == self_q) continue;
             const double dx = me.x - p.x, dy = me.y - p.y, dz = me.z - p.z;
             const double r2 = dx * dx + dy * dy + dz * dz;
             const double r = sqrt(r2);
@@ -180,7 +181,7 @@ ea1_f64(int64_t n, const TgtPos* __restrict__ tgt, const EA2F64* __restrict__ se
 template <int K>
 __global__ void __launch_bounds__(UJ_THREADS)
 ea2_f64(int64_t n, const EA1F64* __restrict__ self, int64_t n_pad, const EA2F64* __restrict__ src,
-        int64_t per_split, double* __restrict__ partial)
+        double* __restrict__ partial)
 {
     __shared__ EA2F64 tile[UJ_TILE];
     const int64_t s = (int64_t)blockIdx.x * UJ_THREADS + threadIdx.x;
@@ -189,15 +190,16 @@ ea2_f64(int64_t n, const EA1F64* __restrict__ self, int64_t n_pad, const EA2F64*
 #pragma unroll
     for (int k = 0; k < NACC2; k++) acc[k] = 0.0;
     const double isig2 = me.isig * me.isig;
-    const int64_t s0 = (int64_t)blockIdx.y * per_split, s1 = min(s0 + per_split, n_pad);
-    for (int64_t base = s0; base < s1; base += UJ_TILE) {
+    const int64_t nq = split_count(n_pad, blockIdx.y, gridDim.y), self_q = split_position(s, blockIdx.y, gridDim.y);
+    for (int64_t base = 0; base < nq; base += UJ_TILE) {
         __syncthreads();
-        tile[threadIdx.x] = src[base + threadIdx.x];
+        if (base + threadIdx.x < nq) tile[threadIdx.x] = src[split_source(base + threadIdx.x, blockIdx.y, gridDim.y)];
         __syncthreads();
+        const int m = (int)min((int64_t)UJ_TILE, nq - base);
 #pragma unroll 2
-        for (int j = 0; j < UJ_TILE; j++) {
+        for (int j = 0; j < m; j++) {
             const EA2F64& p = tile[j];
-            if (base + j == s) continue;
+            if (base + j == self_q) continue;
             const double dx = me.x - p.x, dy = me.y - p.y, dz = me.z - p.z;   // x_s - x_t
             const double r2 = dx * dx + dy * dy + dz * dz;
             const double ss = r2 * isig2;
@@ -561,9 +563,7 @@ cudaError_t launch_k(const EstrAdjArgs& a, const EstrAdjWork& w, int num_sms, cu
 {
     const int64_t n = a.n;
     const int64_t n_pad = round_up(n, UJ_TILE);
-    const int nsplit = uj_num_splits(n, n, num_sms);
-    const int64_t tiles = n_pad / UJ_TILE;
-    const int64_t per_split = ((tiles + nsplit - 1) / nsplit) * UJ_TILE;
+    const int nsplit = uj_num_splits(n, n, num_sms, a.precision);
     const dim3 grid((unsigned)(n_pad / UJ_THREADS), (unsigned)nsplit);
     const int pb = 256;
     const unsigned pg = (unsigned)((n_pad + pb - 1) / pb), eg = (unsigned)((n + pb - 1) / pb);
@@ -577,20 +577,23 @@ cudaError_t launch_k(const EstrAdjArgs& a, const EstrAdjWork& w, int num_sms, cu
                                   w.pack1, w.pack2, box);
     if (!mixed) {
         ea1_f64<K><<<grid, UJ_THREADS, 0, st>>>(n, tgt, (const EA2F64*)w.pack2, n_pad, (const EA1F64*)w.pack1,
-                                                per_split, w.partial);
-        ea1_epilogue<<<eg, pb, 0, st>>>(n, nsplit, w.partial, n_pad, tgt, a.static_flags, a.Sbar, a.transposed,
+                                                w.partial);
+        sum_splits(w.partial, nsplit, NACC1, n, n_pad, st, launches);
+        ea1_epilogue<<<eg, pb, 0, st>>>(n, 1, w.partial, n_pad, tgt, a.static_flags, a.Sbar, a.transposed,
                                         a.xbar, a.Jbar);
-        ea2_f64<K><<<grid, UJ_THREADS, 0, st>>>(n, (const EA1F64*)w.pack1, n_pad, (const EA2F64*)w.pack2, per_split,
+        ea2_f64<K><<<grid, UJ_THREADS, 0, st>>>(n, (const EA1F64*)w.pack1, n_pad, (const EA2F64*)w.pack2,
                                                 w.partial);
     } else {
         ea1_mx<K><<<grid, UJ_THREADS, 0, st>>>(n, tgt, (const EA2Mx*)w.pack2, n_pad, (const EA1Mx*)w.pack1, box,
                                                w.partial);
-        ea1_epilogue<<<eg, pb, 0, st>>>(n, nsplit, w.partial, n_pad, tgt, a.static_flags, a.Sbar, a.transposed,
+        sum_splits(w.partial, nsplit, NACC1, n, n_pad, st, launches);
+        ea1_epilogue<<<eg, pb, 0, st>>>(n, 1, w.partial, n_pad, tgt, a.static_flags, a.Sbar, a.transposed,
                                         a.xbar, a.Jbar);
         ea2_mx<K><<<grid, UJ_THREADS, 0, st>>>(n, (const EA1Mx*)w.pack1, a.gam, tgt, a.J, a.static_flags,
                                                a.transposed, n_pad, (const EA2Mx*)w.pack2, box, w.partial);
     }
-    ea2_epilogue<K><<<eg, pb, 0, st>>>(n, nsplit, w.partial, n_pad, tgt, a.static_flags, a.gam, a.sig, a.J,
+    sum_splits(w.partial, nsplit, NACC2, n, n_pad, st, launches);
+    ea2_epilogue<K><<<eg, pb, 0, st>>>(n, 1, w.partial, n_pad, tgt, a.static_flags, a.gam, a.sig, a.J,
                                        a.transposed, mixed, a.xbar, a.gbar, a.sbar, a.Jbar);
     *launches += 5;
     return cudaGetLastError();
@@ -605,7 +608,7 @@ EstrAdjSizes estr_adjoint_sizes(int64_t n, int num_sms)
     // the larger of the FP64 (80 B) and mixed (64 B) records; pack 1's mixed tile boxes
     // (1 B a particle) fit in the difference
     z.pack = (size_t)n_pad * 80;
-    z.partial = (size_t)uj_num_splits(n, n, num_sms) * NACC2 * (size_t)n_pad * sizeof(double);
+    z.partial = (size_t)uj_num_splits(n, n, num_sms, 0) * NACC2 * (size_t)n_pad * sizeof(double);
     return z;
 }
 

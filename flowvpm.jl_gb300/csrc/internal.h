@@ -124,7 +124,25 @@ struct Workspace {
 size_t uj_src_pack_bytes(int64_t ns, int precision);
 size_t estr_src_pack_bytes(int64_t ns, int precision);
 size_t order_bytes(int64_t nt);
-int uj_num_splits(int64_t nt, int64_t ns, int num_sms);
+int uj_num_splits(int64_t nt, int64_t ns, int num_sms, int precision);
+// Sources of the FP64 kernels' splits: units of F64_UNIT consecutive ones, dealt out in turn
+// (split y of ny has units y, y + ny, ...), so that a target's near sources, which cost most,
+// spread over the splits when the caller's order is a spatial one.
+constexpr int F64_UNIT = 16;
+__host__ __device__ inline int64_t split_count(int64_t ns_pad, int y, int ny)    // ns_pad: a multiple of F64_UNIT
+{
+    return (ns_pad / F64_UNIT - y + ny - 1) / ny * F64_UNIT;
+}
+__host__ __device__ inline int64_t split_source(int64_t q, int y, int ny)        // the split's q-th source
+{
+    return (q / F64_UNIT * ny + y) * F64_UNIT + q % F64_UNIT;
+}
+// the position of source i in split y, or -1 when it is in another one
+__host__ __device__ inline int64_t split_position(int64_t i, int y, int ny)
+{
+    const int64_t u = i / F64_UNIT;
+    return i >= 0 && u % ny == y ? u / ny * F64_UNIT + i % F64_UNIT : -1;
+}
 size_t uj_partial_bytes(int64_t nt, int nsplit);
 // The far pairs' sums of a set on itself on the tensor cores (uj_tc.cu).
 bool uj_takes_tiles(const UJArgs& a);
@@ -139,6 +157,9 @@ cudaError_t order_targets(int64_t nt, const double* xt, void* scratch, size_t sc
 
 // Sets the calling thread's context-free error text (vpm_last_error(NULL)).
 void set_thread_error(const char* msg);
+
+// p[0][k][t] += p[1][k][t] + ... + p[nsplit-1][k][t], k < nk (split partial sums, in split order)
+void sum_splits(double* p, int nsplit, int nk, int64_t nt, int64_t nt_pad, cudaStream_t st, int64_t* launches);
 
 // Launchers; return cudaError_t of the launches and count kernel launches.
 cudaError_t launch_uj(const UJArgs& a, const Workspace& w, int num_sms, cudaStream_t st,
