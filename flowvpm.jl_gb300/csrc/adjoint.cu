@@ -115,12 +115,15 @@ __device__ __forceinline__ void adj_pair_f64(double dx, double dy, double dz, co
     const double P = Ub[0] * cx + Ub[1] * cy + Ub[2] * cz + wb[0] * Gx + wb[1] * Gy + wb[2] * Gz;
     const double Q = cx * JDx + cy * JDy + cz * JDz;
     const double sc = B * P + Bpr * Q;
-    o[0] = sc * dx + A * (Gy * Ub[2] - Gz * Ub[1]) + B * (Gy * JDz - Gz * JDy + JTcx);
-    o[1] = sc * dy + A * (Gz * Ub[0] - Gx * Ub[2]) + B * (Gz * JDx - Gx * JDz + JTcy);
-    o[2] = sc * dz + A * (Gx * Ub[1] - Gy * Ub[0]) + B * (Gx * JDy - Gy * JDx + JTcz);
-    o[3] = A * (Ub[1] * dz - Ub[2] * dy + wb[0]) + B * (JDy * dz - JDz * dy);
-    o[4] = A * (Ub[2] * dx - Ub[0] * dz + wb[1]) + B * (JDz * dx - JDx * dz);
-    o[5] = A * (Ub[0] * dy - Ub[1] * dx + wb[2]) + B * (JDx * dy - JDy * dx);
+    // v = A Ubar + B Jbar dx is in both strength-side and position-side terms:
+    //   dphi/d(dx) = sc dx + Gamma x v + B Jbar^T c,   dphi/dGamma = A wbar + v x dx
+    const double vx = A * Ub[0] + B * JDx, vy = A * Ub[1] + B * JDy, vz = A * Ub[2] + B * JDz;
+    o[0] = sc * dx + B * JTcx + Gy * vz - Gz * vy;
+    o[1] = sc * dy + B * JTcy + Gz * vx - Gx * vz;
+    o[2] = sc * dz + B * JTcz + Gx * vy - Gy * vx;
+    o[3] = A * wb[0] + vy * dz - vz * dy;
+    o[4] = A * wb[1] + vz * dx - vx * dz;
+    o[5] = A * wb[2] + vx * dy - vy * dx;
     o[6] = (K == K_SING) ? 0.0 : dA * P + dB * Q;
 }
 
@@ -423,12 +426,14 @@ __device__ __forceinline__ void adj_pair_f32(float dx, float dy, float dz, float
     const float P = fmaf(Ub[0], cx, fmaf(Ub[1], cy, fmaf(Ub[2], cz, fmaf(wb[0], Gx, fmaf(wb[1], Gy, wb[2] * Gz)))));
     const float Q = fmaf(cx, JDx, fmaf(cy, JDy, cz * JDz));
     const float sc = fmaf(B, P, Bpr * Q);
-    o[0] = fmaf(sc, dx, fmaf(A, fmaf(Gy, Ub[2], -Gz * Ub[1]), B * (fmaf(Gy, JDz, -Gz * JDy) + JTcx)));
-    o[1] = fmaf(sc, dy, fmaf(A, fmaf(Gz, Ub[0], -Gx * Ub[2]), B * (fmaf(Gz, JDx, -Gx * JDz) + JTcy)));
-    o[2] = fmaf(sc, dz, fmaf(A, fmaf(Gx, Ub[1], -Gy * Ub[0]), B * (fmaf(Gx, JDy, -Gy * JDx) + JTcz)));
-    o[3] = fmaf(A, fmaf(Ub[1], dz, fmaf(-Ub[2], dy, wb[0])), B * fmaf(JDy, dz, -JDz * dy));
-    o[4] = fmaf(A, fmaf(Ub[2], dx, fmaf(-Ub[0], dz, wb[1])), B * fmaf(JDz, dx, -JDx * dz));
-    o[5] = fmaf(A, fmaf(Ub[0], dy, fmaf(-Ub[1], dx, wb[2])), B * fmaf(JDx, dy, -JDy * dx));
+    // v = A Ubar + B Jbar dx, as in adj_pair_f64
+    const float vx = fmaf(A, Ub[0], B * JDx), vy = fmaf(A, Ub[1], B * JDy), vz = fmaf(A, Ub[2], B * JDz);
+    o[0] = fmaf(sc, dx, fmaf(B, JTcx, fmaf(Gy, vz, -Gz * vy)));
+    o[1] = fmaf(sc, dy, fmaf(B, JTcy, fmaf(Gz, vx, -Gx * vz)));
+    o[2] = fmaf(sc, dz, fmaf(B, JTcz, fmaf(Gx, vy, -Gy * vx)));
+    o[3] = fmaf(A, wb[0], fmaf(vy, dz, -vz * dy));
+    o[4] = fmaf(A, wb[1], fmaf(vz, dx, -vx * dz));
+    o[5] = fmaf(A, wb[2], fmaf(vx, dy, -vy * dx));
     o[6] = fmaf(dA, P, dB * Q);
 }
 
@@ -592,17 +597,21 @@ uj_adjoint_mixed_kernel(int64_t nt, const TgtPos* __restrict__ tgt, const double
                 // lanes 16-31 / 0-15 keep sources {2,3} / {0,1}, then lanes with bit 3 set / clear
                 // keep the odd / even one, then a butterfly over the remaining 8 lanes; lane 8 g
                 // ends with source g's seven sums (21 + 21 shuffles per four sources, not 4 x 35)
+                // (the singular form of a far group has no sigma term)
                 const bool b4 = (lane & 16) != 0, b3 = (lane & 8) != 0;
                 float r[7];
-#pragma unroll
-                for (int k = 0; k < 7; k++) {
+                auto scatter = [&](int k) {
                     const float p0 = (b4 ? o[2][k] : o[0][k]) + __shfl_xor_sync(0xffffffffu, b4 ? o[0][k] : o[2][k], 16);
                     const float p1 = (b4 ? o[3][k] : o[1][k]) + __shfl_xor_sync(0xffffffffu, b4 ? o[1][k] : o[3][k], 16);
                     float v = (b3 ? p1 : p0) + __shfl_xor_sync(0xffffffffu, b3 ? p0 : p1, 8);
 #pragma unroll
                     for (int m = 4; m > 0; m >>= 1) v += __shfl_xor_sync(0xffffffffu, v, m);
                     r[k] = v;
-                }
+                };
+#pragma unroll
+                for (int k = 0; k < 6; k++) scatter(k);
+                r[6] = 0.f;
+                if (!allfar) scatter(6);
                 if ((lane & 7) == 0) {
                     const int q = (b4 ? 2 : 0) + (b3 ? 1 : 0);
 #pragma unroll
