@@ -314,6 +314,8 @@ int ensure_work(vpm_ctx* c, int64_t nt, int64_t ns, int precision, bool estr, Wo
     const int nsplit = uj_num_splits(nt, ns, c->num_sms, precision);
     size_t pb = uj_partial_bytes(nt, nsplit);
     if (precision && nt == ns) pb = std::max(pb, uj_partial_bytes(nt, uj_tc_splits(nt, c->num_sms)));
+    if (estr)   // 3 sums an Estr target, 9 a filter difference's
+        pb = std::max(pb, uj_partial_bytes(nt, uj_num_splits(nt, ns, c->num_sms, precision, REACH_SPLITS), 9));
     if (c->src_pack.grow(sp) != cudaSuccess || c->order.grow(ob) != cudaSuccess ||
         (pb && c->partial.grow(pb) != cudaSuccess)) {
         cudaGetLastError();
@@ -924,7 +926,7 @@ int vpm_dynamic_diff_dev(vpm_ctx* c, int64_t n, const double* x, const double* g
     if (precision == VPM_FP32COMP) {
         CK(cudaMemsetAsync(dJ, 0, 9 * n * sizeof(double), st), "memset dJ");
         CK(cudaMemsetAsync(dSFS, 0, 3 * n * sizeof(double), st), "memset dSFS");
-        CK(launch_uj_filter_diff(n, x, gam, sig, alpha, dJ, kernel, w, st, &c->launches), "filter-difference UJ");
+        CK(launch_uj_filter_diff(n, x, gam, sig, alpha, dJ, kernel, c->num_sms, w, st, &c->launches), "filter-difference UJ");
         // the weight difference at J, then an ordinary Estr of dJ at alpha sigma
         e.Jt = J; e.Js = J; e.sgs = sig; e.SFS = dSFS; e.dz_alpha = alpha;
         CK(launch_estr(e, w, c->num_sms, st, &c->launches), "weight-difference Estr");

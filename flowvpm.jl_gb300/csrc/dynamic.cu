@@ -64,7 +64,8 @@ __device__ __forceinline__ void dyn_wait() { asm volatile("cp.async.wait_group %
 template <int K, int M>
 __global__ void __launch_bounds__(DYN_THREADS)
 uj_filter_diff_kernel(int64_t nt, const TgtPos* __restrict__ tgt, int64_t ns_pad, const SrcMixed* __restrict__ src,
-                      const float4* __restrict__ box, float hm, int panels, double* __restrict__ dJ)
+                      const float4* __restrict__ box, float hm, int panels, double* __restrict__ dJ,
+                      double* __restrict__ partial, int64_t nt_pad)
 {
     __shared__ SrcMixed stage[DYN_WARPS][2][DYN_WT];
     __shared__ float4 offs[DYN_WARPS][2][DYN_WT];
@@ -114,7 +115,7 @@ uj_filter_diff_kernel(int64_t nt, const TgtPos* __restrict__ tgt, int64_t ns_pad
     const int ntiles = (int)(ns_pad / DYN_WT);
     const SrcMixed* wsrc = src + lane;
     TileWalk walk;
-    walk.init(ntiles);
+    walk.init(ntiles, blockIdx.y, gridDim.y);
     int cur = walk.next_s(box, wbox[warp][2], wbox[warp][3], lane, skip);
     if (cur >= 0) dyn_stage(&stage[warp][0][lane], wsrc + (int64_t)cur * DYN_WT);
     int in_flush = 0, buf = 0;
@@ -181,7 +182,23 @@ uj_filter_diff_kernel(int64_t nt, const TgtPos* __restrict__ tgt, int64_t ns_pad
     }
     if (!valid) return;
 #pragma unroll
-    for (int k = 0; k < 9; k++) dJ[9 * (int64_t)idx + k] += acc[k] + (double)f[k];
+    for (int k = 0; k < 9; k++) {
+        const double v = acc[k] + (double)f[k];
+        if (partial) partial[((int64_t)blockIdx.y * 9 + k) * nt_pad + t] = v;
+        else dJ[9 * (int64_t)idx + k] += v;
+    }
+}
+
+__global__ void filter_diff_reduce(int64_t nt, int nsplit, const double* __restrict__ partial, int64_t nt_pad,
+                                   const TgtPos* __restrict__ tgt, double* __restrict__ dJ)
+{
+    const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (t >= nt) return;
+    const double* p = partial + blockIdx.y * nt_pad + t;
+    double s = 0.0;
+#pragma unroll 8
+    for (int sp = 0; sp < nsplit; sp++) s += p[(int64_t)sp * 9 * nt_pad];
+    dJ[9 * (int64_t)tgt[t].idx + blockIdx.y] += s;
 }
 
 // Sources in the targets' curve order, so that the 32-source tiles are compact whatever the
@@ -221,8 +238,8 @@ size_t dyn_src_pack_bytes(int64_t ns)
 
 template <int K>
 static cudaError_t launch_uj_filter_diff_k(int64_t n, const double* x, const double* gam, const double* sig,
-                                           double alpha, double* dJ, const Workspace& w, cudaStream_t st,
-                                           int64_t* launches)
+                                           double alpha, double* dJ, int num_sms, const Workspace& w,
+                                           cudaStream_t st, int64_t* launches)
 {
     const int64_t ns_pad = (n + DYN_TILE - 1) / DYN_TILE * DYN_TILE;
     const TgtPos* tgt = nullptr;
@@ -232,26 +249,37 @@ static cudaError_t launch_uj_filter_diff_k(int64_t n, const double* x, const dou
     SrcMixed* src = (SrcMixed*)w.src_pack;
     float4* box = (float4*)(src + ns_pad);
     pack_src_dyn<K><<<(unsigned)((ns_pad + 255) / 256), 256, 0, st>>>(n, ns_pad, x, gam, sig, tgt, src, box);
-    const unsigned grid = (unsigned)((n + DYN_THREADS - 1) / DYN_THREADS);
+    const int64_t nt_pad = (n + DYN_THREADS - 1) / DYN_THREADS * DYN_THREADS;
+    // The blocks differ by how many tiles are in their reach: as one launch of 782 (100,000 particles
+    // of the rings), a wave of 912, the SMs were busy for 54 % of it.
+    const int nsplit = uj_num_splits(n, n, num_sms, 1, REACH_SPLITS);
+    double* partial = nsplit > 1 ? w.partial : nullptr;
+    const dim3 grid((unsigned)(nt_pad / DYN_THREADS), (unsigned)nsplit);
     const double ha = 1.0 / alpha - 1.0;
     const int m = filter_panels(ha);
     if (m == 1)
-        uj_filter_diff_kernel<K, 1><<<grid, DYN_THREADS, 0, st>>>(n, tgt, ns_pad, src, box, (float)ha, 1, dJ);
+        uj_filter_diff_kernel<K, 1><<<grid, DYN_THREADS, 0, st>>>(n, tgt, ns_pad, src, box, (float)ha, 1, dJ, partial,
+                                                              nt_pad);
     else
-        uj_filter_diff_kernel<K, 0><<<grid, DYN_THREADS, 0, st>>>(n, tgt, ns_pad, src, box, (float)(ha / m), m, dJ);
+        uj_filter_diff_kernel<K, 0><<<grid, DYN_THREADS, 0, st>>>(n, tgt, ns_pad, src, box, (float)(ha / m), m, dJ,
+                                                              partial, nt_pad);
     *launches += 2;
+    if (partial) {
+        filter_diff_reduce<<<dim3((unsigned)((n + 127) / 128), 9), 128, 0, st>>>(n, nsplit, partial, nt_pad, tgt, dJ);
+        *launches += 1;
+    }
     return cudaGetLastError();
 }
 
 cudaError_t launch_uj_filter_diff(int64_t n, const double* x, const double* gam, const double* sig, double alpha,
-                                  double* dJ, int kernel, const Workspace& w, cudaStream_t st, int64_t* launches)
+                                  double* dJ, int kernel, int num_sms, const Workspace& w, cudaStream_t st, int64_t* launches)
 {
     if (n <= 0) return cudaSuccess;
     switch (kernel) {
     case K_SING: return cudaSuccess;   // g = 1: no sigma dependence
-    case K_GAUS: return launch_uj_filter_diff_k<K_GAUS>(n, x, gam, sig, alpha, dJ, w, st, launches);
-    case K_GAUSERF: return launch_uj_filter_diff_k<K_GAUSERF>(n, x, gam, sig, alpha, dJ, w, st, launches);
-    case K_WNKLMNS: return launch_uj_filter_diff_k<K_WNKLMNS>(n, x, gam, sig, alpha, dJ, w, st, launches);
+    case K_GAUS: return launch_uj_filter_diff_k<K_GAUS>(n, x, gam, sig, alpha, dJ, num_sms, w, st, launches);
+    case K_GAUSERF: return launch_uj_filter_diff_k<K_GAUSERF>(n, x, gam, sig, alpha, dJ, num_sms, w, st, launches);
+    case K_WNKLMNS: return launch_uj_filter_diff_k<K_WNKLMNS>(n, x, gam, sig, alpha, dJ, num_sms, w, st, launches);
     default: return cudaErrorInvalidValue;
     }
 }

@@ -408,7 +408,7 @@ static cudaError_t launch_estr_k(const EstrArgs& a, const Workspace& w, int num_
 {
     const int64_t ns_pad = round_up(a.ns, UJ_TILE);
     const int64_t nt_pad = round_up(a.nt, UJ_THREADS);
-    const int nsplit = uj_num_splits(a.nt, a.ns, num_sms, a.precision);
+    const int nsplit = uj_num_splits(a.nt, a.ns, num_sms, a.precision, REACH_SPLITS);
     double* partial = nsplit > 1 ? w.partial : nullptr;
     const dim3 grid((unsigned)(nt_pad / UJ_THREADS), (unsigned)nsplit);
     const int pb = 256;

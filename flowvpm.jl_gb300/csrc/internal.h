@@ -124,7 +124,8 @@ struct Workspace {
 size_t uj_src_pack_bytes(int64_t ns, int precision);
 size_t estr_src_pack_bytes(int64_t ns, int precision);
 size_t order_bytes(int64_t nt);
-int uj_num_splits(int64_t nt, int64_t ns, int num_sms, int precision);
+int uj_num_splits(int64_t nt, int64_t ns, int num_sms, int precision, int per_sm = 24);
+constexpr int REACH_SPLITS = 32;   // per_sm of the kernels that walk the tiles in reach (Estr, filter differences)
 // Sources of the FP64 kernels' splits: units of F64_UNIT consecutive ones, dealt out in turn
 // (split y of ny has units y, y + ny, ...), so that a target's near sources, which cost most,
 // spread over the splits when the caller's order is a spatial one.
@@ -143,7 +144,7 @@ __host__ __device__ inline int64_t split_position(int64_t i, int y, int ny)
     const int64_t u = i / F64_UNIT;
     return i >= 0 && u % ny == y ? u / ny * F64_UNIT + i % F64_UNIT : -1;
 }
-size_t uj_partial_bytes(int64_t nt, int nsplit);
+size_t uj_partial_bytes(int64_t nt, int nsplit, int components = 12);
 // The far pairs' sums of a set on itself on the tensor cores (uj_tc.cu).
 bool uj_takes_tiles(const UJArgs& a);
 size_t uj_tc_bytes(int64_t n);
@@ -171,7 +172,8 @@ cudaError_t launch_uj_adjoint(const AdjArgs& a, const Workspace& w, int num_sms,
 // dJ[n,9] += J(alpha sigma) - J(sigma) of one particle set, all pairs, FP32-comp (dynamic.cu)
 size_t dyn_src_pack_bytes(int64_t ns);
 cudaError_t launch_uj_filter_diff(int64_t n, const double* x, const double* gam, const double* sig, double alpha,
-                                  double* dJ, int kernel, const Workspace& w, cudaStream_t st, int64_t* launches);
+                                  double* dJ, int kernel, int num_sms, const Workspace& w, cudaStream_t st,
+                                  int64_t* launches);
 
 // ------------------------------------------------------------------ near field
 // A device allocation that grows on demand and never shrinks.

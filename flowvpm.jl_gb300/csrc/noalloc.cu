@@ -107,9 +107,13 @@ int vpm_uj_dev_noalloc(int64_t nt, const double* xt, int64_t ns, const double* x
         !is_device_ptr(U, dev) || !is_device_ptr(J, dev))
         return nerr(VPM_ERR_ARG, "vpm_uj_dev_noalloc: every array must be device memory of the current device %d",
                     dev);
-    const int nsplit = vpm::uj_num_splits(nt, ns, sms, precision);
     const size_t pack = align256(vpm::uj_src_pack_bytes(ns, precision));
     const size_t order = align256(vpm::order_bytes(nt));
+    // vpm_uj_dev's splits, or as many as their partial sums leave room for
+    const int want = vpm::uj_num_splits(nt, ns, sms, precision);
+    int nsplit = want;
+    while (nsplit > 1 && pack + order + align256(vpm::uj_partial_bytes(nt, nsplit)) > (size_t)VPM_NOALLOC_SCRATCH_BYTES)
+        nsplit--;
     const size_t part = align256(vpm::uj_partial_bytes(nt, nsplit));
     if (pack + order + part > (size_t)VPM_NOALLOC_SCRATCH_BYTES)
         return nerr(VPM_ERR_CAPACITY,

@@ -43,14 +43,17 @@ size_t uj_src_pack_bytes(int64_t ns, int precision)
     return (size_t)n * (precision ? sizeof(SrcMixed) : sizeof(SrcF64));
 }
 
-int uj_num_splits(int64_t nt, int64_t ns, int num_sms, int precision)
+int uj_num_splits(int64_t nt, int64_t ns, int num_sms, int precision, int per_sm)
 {
-    // About two waves of ~6 resident blocks per SM, from shares of at least one unit (FP64) or
-    // two warp tiles.  With shares of at least 512 sources, as this rule had them, 1,400
-    // particles made 22 blocks for 152 SMs: UJ 2.39 ms and Estr 1.27 ms in FP64.
+    // per_sm blocks per SM (about four waves at the default), from shares of at least one unit
+    // (FP64) or two warp tiles.  With shares of at least 512 sources 1,400 particles made 22
+    // blocks for 152 SMs (UJ 2.39 ms, Estr 1.27 ms in FP64); with 12 blocks a SM the uneven
+    // blocks left SMs idle at the end: FP64 gradient of 5,600 particles 21.1 ms, 20.4 at 24 and
+    // 20.3 at 36; Estr of the 200,000-particle rings 4.20, 3.78 and 3.77 ms; filter differences
+    // of 100,000 8.9 ms unsplit, 6.8, 6.1 and 5.7 (whole calls).
     const int64_t tblocks = (nt + UJ_THREADS - 1) / UJ_THREADS;
     const int64_t units = precision ? (ns + 63) / 64 : (ns + F64_UNIT - 1) / F64_UNIT;
-    const int64_t want = 12LL * num_sms;
+    const int64_t want = (int64_t)per_sm * num_sms;
     int64_t nsplit = (want + tblocks - 1) / tblocks;
     if (nsplit > units) nsplit = units;
     if (nsplit < 1) nsplit = 1;
@@ -63,9 +66,9 @@ int uj_num_splits(int64_t nt, int64_t ns, int num_sms, int precision)
 // 16,384 10 % faster (741 against 820 us), 65,536 1.6 times.
 bool uj_takes_tiles(const UJArgs& a) { return a.self && a.precision == 1 && a.ns >= 12288; }
 
-size_t uj_partial_bytes(int64_t nt, int nsplit)
+size_t uj_partial_bytes(int64_t nt, int nsplit, int components)
 {
-    return nsplit > 1 ? (size_t)nsplit * 12 * (size_t)round_up(nt, UJ_THREADS) * sizeof(double) : 0;
+    return nsplit > 1 ? (size_t)nsplit * components * (size_t)round_up(nt, UJ_THREADS) * sizeof(double) : 0;
 }
 
 
@@ -386,7 +389,8 @@ static cudaError_t launch_uj_k(const UJArgs& a, const Workspace& w, int num_sms,
     const int64_t ns_pad = round_up(a.ns, UJ_TILE);
     const int64_t nt_pad = round_up(a.nt, UJ_THREADS);
     const bool tc = uj_takes_tiles(a) && w.tiles;
-    const int nsplit = tc ? uj_tc_splits(a.nt, num_sms) : uj_num_splits(a.nt, a.ns, num_sms, a.precision);
+    int nsplit = tc ? uj_tc_splits(a.nt, num_sms) : uj_num_splits(a.nt, a.ns, num_sms, a.precision);
+    while (!tc && nsplit > 1 && uj_partial_bytes(a.nt, nsplit) > w.partial_bytes) nsplit--;   // a caller's fixed scratch
     double* partial = nsplit > 1 ? w.partial : nullptr;
     const dim3 grid((unsigned)(nt_pad / UJ_THREADS), (unsigned)nsplit);
     const int pb = 256;
