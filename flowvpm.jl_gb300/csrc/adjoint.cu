@@ -30,7 +30,7 @@ namespace vpm {
 // (g, g', g'') of kernel K at rho, FP64 (derivatives of src/FLOWVPM_kernel.jl:45-84).
 // Beyond rho = 9 (Gaussian-erf) / 3.5 (Gaussian) g = 1 and g' = g'' = 0 to FP64.
 template <int K>
-__device__ __forceinline__ void g_d1_d2_f64(double rho, double& g, double& d1, double& d2)
+__device__ __forceinline__ void g_d1_d2_f64(double rho, double& g, double& d1, double& d2, const double* T)
 {
     if constexpr (K == K_SING) {
         g = 1.0; d1 = 0.0; d2 = 0.0;
@@ -38,21 +38,23 @@ __device__ __forceinline__ void g_d1_d2_f64(double rho, double& g, double& d1, d
         if (rho > 3.5) { g = 1.0; d1 = 0.0; d2 = 0.0; }
         else {
             const double r3 = rho * rho * rho;
-            const double e = exp(-r3);
+            const double e = exp_neg(-r3, T);
             g = 1.0 - e; d1 = 3.0 * rho * rho * e; d2 = (6.0 * rho - 9.0 * r3 * rho) * e;
         }
     } else if constexpr (K == K_GAUSERF) {
         if (rho > 9.0) { g = 1.0; d1 = 0.0; d2 = 0.0; }
         else {
-            const double e = C2 * exp(-0.5 * rho * rho);
-            g = erf(rho * INV_SQRT2) - rho * e;
-            d1 = rho * rho * e;
-            d2 = (2.0 * rho - rho * rho * rho) * e;
+            const double s = rho * rho;
+            const double e0 = exp_neg(-0.5 * s, T), e = C2 * e0;
+            if (s < 2.0) g = e * rho * s * fma(s, gerf_S2_f64(s), 1.0 / 3.0);
+            else g = fma(-e0, gerf_h_f64(rho), 1.0);
+            d1 = s * e;
+            d2 = (2.0 - s) * rho * e;
         }
     } else {
         const double q = rho * rho + 1.0;
-        const double iq = 1.0 / q;
-        const double iq25 = iq * iq * sqrt(iq);           // q^-2.5
+        const double t = rsqrt(q), iq = t * t;
+        const double iq25 = iq * iq * t;                  // q^-2.5
         g = rho * rho * rho * (rho * rho + 2.5) * iq25;
         d1 = 7.5 * rho * rho * iq25 * iq;
         d2 = 7.5 * rho * (2.0 - 5.0 * rho * rho) * iq25 * iq * iq;
@@ -75,10 +77,10 @@ __host__ __device__ constexpr double adj_far_s()
 template <int K>
 __device__ __forceinline__ void adj_pair_f64(double dx, double dy, double dz, const SrcF64& s,
                                              const double (&Ub)[3], const double (&Jb)[9], const double (&wb)[3],
-                                             double (&o)[7])
+                                             double (&o)[7], const double* T)
 {
     const double r2 = dx * dx + dy * dy + dz * dz;
-    if (r2 == 0.0) {
+    if ((__double2hiint(r2) | __double2loint(r2)) == 0) {   // on the words: a compare costs an FP64-pipe slot
 #pragma unroll
         for (int k = 0; k < 7; k++) o[k] = 0.0;
         return;
@@ -86,7 +88,7 @@ __device__ __forceinline__ void adj_pair_f64(double dx, double dy, double dz, co
     const double rinv = rsqrt(r2);
     const double ri2 = rinv * rinv, ri3 = ri2 * rinv;
     double A, B, Bpr, dA = 0.0, dB = 0.0;
-    if (K == K_SING || (adj_far_s<K>() > 0.0 && r2 > s.gz_sig.y)) {
+    if (K == K_SING || (adj_far_s<K>() > 0.0 && __double2hiint(r2) > __double2hiint(s.gz_sig.y))) {
         const double ri5 = ri3 * ri2;
         A = -C4 * ri3;
         B = (3.0 * C4) * ri5;
@@ -95,7 +97,7 @@ __device__ __forceinline__ void adj_pair_f64(double dx, double dy, double dz, co
         const double isig = s.z_isig.y;
         const double rho = r2 * rinv * isig;
         double g, g1, g2;
-        g_d1_d2_f64<K>(rho, g, g1, g2);
+        g_d1_d2_f64<K>(rho, g, g1, g2, T);
         const double ri4 = ri2 * ri2, ri5 = ri4 * rinv;
         A = -C4 * g * ri3;
         B = -C4 * (g1 * isig * ri4 - 3.0 * g * ri5);
@@ -160,6 +162,8 @@ uj_adjoint_f64_kernel(int64_t nt, const TgtPos* __restrict__ tgt, const double* 
 {
     __shared__ SrcF64 tile[UJ_TILE];
     __shared__ double red[UJ_WARPS][UJ_TILE][7];
+    __shared__ double T[64];
+    exp_table(T);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t t = (int64_t)blockIdx.x * UJ_THREADS + threadIdx.x;
     const bool valid = t < nt;
@@ -190,19 +194,19 @@ uj_adjoint_f64_kernel(int64_t nt, const TgtPos* __restrict__ tgt, const double* 
             double o0[7], o1[7], o2[7], o3[7];
             {
                 const SrcF64& s = tile[j];
-                adj_pair_f64<K>(tx - s.xy.x, ty - s.xy.y, tz - s.z_isig.x, s, Ub, Jb, wb, o0);
+                adj_pair_f64<K>(tx - s.xy.x, ty - s.xy.y, tz - s.z_isig.x, s, Ub, Jb, wb, o0, T);
             }
             {
                 const SrcF64& s = tile[j + 1];
-                adj_pair_f64<K>(tx - s.xy.x, ty - s.xy.y, tz - s.z_isig.x, s, Ub, Jb, wb, o1);
+                adj_pair_f64<K>(tx - s.xy.x, ty - s.xy.y, tz - s.z_isig.x, s, Ub, Jb, wb, o1, T);
             }
             {
                 const SrcF64& s = tile[j + 2];
-                adj_pair_f64<K>(tx - s.xy.x, ty - s.xy.y, tz - s.z_isig.x, s, Ub, Jb, wb, o2);
+                adj_pair_f64<K>(tx - s.xy.x, ty - s.xy.y, tz - s.z_isig.x, s, Ub, Jb, wb, o2, T);
             }
             {
                 const SrcF64& s = tile[j + 3];
-                adj_pair_f64<K>(tx - s.xy.x, ty - s.xy.y, tz - s.z_isig.x, s, Ub, Jb, wb, o3);
+                adj_pair_f64<K>(tx - s.xy.x, ty - s.xy.y, tz - s.z_isig.x, s, Ub, Jb, wb, o3, T);
             }
 #pragma unroll
             for (int k = 0; k < 3; k++) acc[k] += (o0[k] + o1[k]) + (o2[k] + o3[k]);

@@ -107,11 +107,13 @@ __global__ void pack_estr_f64(int64_t ns, int64_t ns_pad, const double* __restri
     SrcEstrF64 p;
     if (i < ns) {
         const bool off = static_s && static_s[i];
-        const double gx = off ? 0.0 : gs[3 * i], gy = off ? 0.0 : gs[3 * i + 1], gz = off ? 0.0 : gs[3 * i + 2];
+        const double isig = 1.0 / sgs[i], k = off ? 0.0 : zeta_norm(K) * isig * isig * isig;
+        const double gx = off ? 0.0 : k * gs[3 * i], gy = off ? 0.0 : k * gs[3 * i + 1],
+                     gz = off ? 0.0 : k * gs[3 * i + 2];
         double vx = 0.0, vy = 0.0, vz = 0.0;
         if (Js) stretch_vec(Js + i * ldJs, gx, gy, gz, transposed, vx, vy, vz);
         p.xy = make_double2(xs[3 * i], xs[3 * i + 1]);
-        p.z_isig = make_double2(xs[3 * i + 2], 1.0 / sgs[i]);
+        p.z_isig = make_double2(xs[3 * i + 2], isig * isig);
         p.gxy = make_double2(gx, gy);
         p.gz_vx = make_double2(gz, vx);
         p.vyz = make_double2(vy, vz);
@@ -170,6 +172,8 @@ estr_f64_kernel(int64_t nt, const TgtPos* __restrict__ tgt, const double* __rest
                 bool self, bool transposed, double* SFS, int64_t ldS, double* partial, int64_t nt_pad)
 {
     __shared__ SrcEstrF64 tile[UJ_TILE];
+    __shared__ double T[64];
+    exp_table(T);
     const int64_t t = (int64_t)blockIdx.x * UJ_THREADS + threadIdx.x;
     double tx = 1.0e3, ty = 1.0e3, tz = 1.0e3;
     int64_t idx = -1;
@@ -191,9 +195,7 @@ estr_f64_kernel(int64_t nt, const TgtPos* __restrict__ tgt, const double* __rest
             const SrcEstrF64& p = tile[j];
             if (base + j == self_q) continue;
             const double dx = p.xy.x - tx, dy = p.xy.y - ty, dz = p.z_isig.x - tz;
-            const double r = sqrt(dx * dx + dy * dy + dz * dz);
-            const double isig = p.z_isig.y;
-            const double z = zeta_f64<K>(r * isig) * isig * isig * isig;
+            const double z = zhat_f64<K>((dx * dx + dy * dy + dz * dz) * p.z_isig.y, T);
             zg[0] += z * p.gxy.x; zg[1] += z * p.gxy.y; zg[2] += z * p.gz_vx.x;
             if constexpr (!ZETA) { zv[0] += z * p.gz_vx.y; zv[1] += z * p.vyz.x; zv[2] += z * p.vyz.y; }
         }

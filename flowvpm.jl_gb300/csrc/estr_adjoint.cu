@@ -151,6 +151,8 @@ ea1_f64(int64_t n, const TgtPos* __restrict__ tgt, const EA2F64* __restrict__ se
         const EA1F64* __restrict__ src, double* __restrict__ partial)
 {
     __shared__ EA1F64 tile[UJ_TILE];
+    __shared__ double T[64];
+    exp_table(T);
     const int64_t t = (int64_t)blockIdx.x * UJ_THREADS + threadIdx.x;
     const EA2F64 me = self[t < n ? t : n_pad - 1];     // a_t, Sbar_t (zero for static targets)
     double acc[NACC1] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
@@ -166,11 +168,11 @@ ea1_f64(int64_t n, const TgtPos* __restrict__ tgt, const EA2F64* __restrict__ se
             if (base + j == self_q) continue;
             const double dx = me.x - p.x, dy = me.y - p.y, dz = me.z - p.z;
             const double r2 = dx * dx + dy * dy + dz * dz;
-            const double r = sqrt(r2);
-            const double z = zeta_f64<K>(r * p.isig) * p.isig * p.isig * p.isig;
+            const double isig2 = p.isig * p.isig, s = r2 * isig2;
+            const double z = zhat_f64<K>(s, T) * (zeta_norm(K) * p.isig * isig2);
             const double w = p.gx * me.ax + p.gy * me.ay + p.gz * me.az - (p.vx * me.sx + p.vy * me.sy + p.vz * me.sz);
             acc[0] += z * p.gx; acc[1] += z * p.gy; acc[2] += z * p.gz;
-            const double c = w * z * kappa_f64<K>(r2 * p.isig * p.isig) * p.isig * p.isig;
+            const double c = w * z * (kappa_f64<K>(s) * isig2);
             acc[3] += c * dx; acc[4] += c * dy; acc[5] += c * dz;
         }
     }
@@ -184,6 +186,8 @@ ea2_f64(int64_t n, const EA1F64* __restrict__ self, int64_t n_pad, const EA2F64*
         double* __restrict__ partial)
 {
     __shared__ EA2F64 tile[UJ_TILE];
+    __shared__ double T[64];
+    exp_table(T);
     const int64_t s = (int64_t)blockIdx.x * UJ_THREADS + threadIdx.x;
     const EA1F64 me = self[s < n ? s : n_pad - 1];     // Gamma_s, v_s (zero for static sources)
     double acc[NACC2];
@@ -203,7 +207,7 @@ ea2_f64(int64_t n, const EA1F64* __restrict__ self, int64_t n_pad, const EA2F64*
             const double dx = me.x - p.x, dy = me.y - p.y, dz = me.z - p.z;   // x_s - x_t
             const double r2 = dx * dx + dy * dy + dz * dz;
             const double ss = r2 * isig2;
-            const double zh = zeta_f64<K>(sqrt(r2) * me.isig);            // the 1/sigma_s^3 comes at the end
+            const double zh = zhat_f64<K>(ss, T);            // ZNORM/sigma_s^3 comes at the end
             const double w = me.gx * p.ax + me.gy * p.ay + me.gz * p.az - (me.vx * p.sx + me.vy * p.sy + me.vz * p.sz);
             const double kp = kappa_f64<K>(ss);
             acc[0] += zh * p.ax; acc[1] += zh * p.ay; acc[2] += zh * p.az;
@@ -543,7 +547,7 @@ __global__ void ea2_epilogue(int64_t n, int nsplit, const double* __restrict__ p
         a[k] = v;
     }
     const double is = 1.0 / sig[i];
-    const double zn = mixed ? zeta_norm(K) : 1.0;
+    const double zn = zeta_norm(K);
     const double c3 = zn * is * is * is, c5 = c3 * is * is, c4 = -c3 * is;
     double A[3], B[3];
     for (int k = 0; k < 3; k++) { A[k] = c3 * a[k]; B[k] = c3 * a[3 + k]; }

@@ -38,8 +38,9 @@ struct __align__(16) SrcF64 { double2 xy, z_isig, gxy, gz_sig; };
 struct __align__(16) SrcEstrDF { float4 a, b, g, v; };
 
 // Packed source of the FP64 Estr kernel, 80 B:
-//   (x, y), (z, 1/sigma), (Gamma_x, Gamma_y), (Gamma_z, v_x), (v_y, v_z)
-// with Gamma and v = J^T Gamma zero for static sources.
+//   (x, y), (z, 1/sigma^2), (g_x, g_y), (g_z, v_x), (v_y, v_z)
+// with g = ZNORM Gamma / sigma^3 and v = J^T g, zero for static sources.  (The near-field
+// pack holds 1/sigma, Gamma and J^T Gamma in their places.)
 struct __align__(16) SrcEstrF64 { double2 xy, z_isig, gxy, gz_vx, vyz; };
 
 constexpr int UJ_THREADS = 128;   // targets per block, one per thread

@@ -955,6 +955,9 @@ nf_uj_f64(int64_t n, int64_t ngroups, const TgtPos* __restrict__ tgt, const int3
 {
     __shared__ SrcF64 tile[NF_WARPS][32];
     __shared__ unsigned tmask[NF_WARPS][32];
+    __shared__ double T[64];
+    exp_table(T);
+    __syncthreads();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t grp = (int64_t)blockIdx.x * NF_WARPS + warp;
     if (grp >= ngroups) return;
@@ -974,7 +977,7 @@ nf_uj_f64(int64_t n, int64_t ngroups, const TgtPos* __restrict__ tgt, const int3
         tmask[warp][lane] = smask;
         __syncwarp();
         for (int j = 0; j < cnt; j++)
-            if (tmask[warp][j] & me.bit) pair_f64_acc<K>(me.tx, me.ty, me.tz, tile[warp][j], u, w, jq);
+            if (tmask[warp][j] & me.bit) pair_f64_acc<K>(me.tx, me.ty, me.tz, tile[warp][j], u, w, jq, T);
     }
     if (!me.valid) return;
     double acc[12];
@@ -1008,6 +1011,11 @@ nf_estr(int64_t n, int64_t ngroups, const TgtPos* __restrict__ tgt, const int32_
     __shared__ SrcEstrF64 dtile[MIXED ? 1 : NF_WARPS][32];
     __shared__ int spos[NF_WARPS][32];                          // source position, -1 for padding
     __shared__ unsigned tmask[NF_WARPS][32];
+    __shared__ double T[64];
+    if constexpr (!MIXED) {
+        exp_table(T);
+        __syncthreads();
+    }
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t grp = (int64_t)blockIdx.x * NF_WARPS + warp;
     if (grp >= ngroups) return;
@@ -1091,7 +1099,8 @@ nf_estr(int64_t n, int64_t ngroups, const TgtPos* __restrict__ tgt, const int32_
                 const SrcEstrF64& p = dtile[warp][j];
                 const double dx = p.xy.x - me.tx, dy = p.xy.y - me.ty, dz = p.z_isig.x - me.tz;
                 const double isig = p.z_isig.y;
-                const double z = zeta_f64<K>(sqrt(dx * dx + dy * dy + dz * dz) * isig) * isig * isig * isig;
+                const double isig2 = isig * isig;
+                const double z = zhat_f64<K>((dx * dx + dy * dy + dz * dz) * isig2, T) * (zeta_norm(K) * isig * isig2);
                 zg[0] += z * p.gxy.x; zg[1] += z * p.gxy.y; zg[2] += z * p.gz_vx.x;
                 zv[0] += z * p.gz_vx.y; zv[1] += z * p.vyz.x; zv[2] += z * p.vyz.y;
             }

@@ -170,6 +170,8 @@ uj_f64_kernel(int64_t nt, const TgtPos* __restrict__ tgt, int64_t ns_pad, const 
               double* U, int64_t ldU, double* J, int64_t ldJ, double* partial, int64_t nt_pad)
 {
     __shared__ SrcF64 tile[UJ_TILE];
+    __shared__ double T[64];
+    exp_table(T);
     const int64_t t = (int64_t)blockIdx.x * UJ_THREADS + threadIdx.x;
     const bool valid = t < nt;
     double tx = 1.0e3, ty = 1.0e3, tz = 1.0e3;
@@ -189,7 +191,7 @@ uj_f64_kernel(int64_t nt, const TgtPos* __restrict__ tgt, int64_t ns_pad, const 
         __syncthreads();
         const int m = (int)min((int64_t)UJ_TILE, nq - base);
 #pragma unroll 2
-        for (int j = 0; j < m; j++) pair_f64_acc<K>(tx, ty, tz, tile[j], u, w, jq);
+        for (int j = 0; j < m; j++) pair_f64_acc<K>(tx, ty, tz, tile[j], u, w, jq, T);
     }
     uj_f64_finish(u, w, jq, acc);
     if (valid) write_uj(t, idx, acc, U, ldU, J, ldJ, partial, nt_pad);

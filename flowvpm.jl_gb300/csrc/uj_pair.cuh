@@ -224,26 +224,52 @@ __device__ __forceinline__ void pair4_mixed(const float3& to, const float3& th, 
 // (uj_f64_finish).  Algebraically the reference's terms, regrouped so that the strength
 // factor -1/(4 pi) and the products shared by the nine J entries are taken once.
 // Gaussian-erf pairs past rho = 9 take g = 1, g' = 0 (the reference's cut) from the
-// pack's threshold 81 sigma^2 without forming rho.  Pairs with r^2 == 0 are skipped.
+// pack's threshold 81 sigma^2 without forming rho.  Pairs with r^2 == 0 are skipped.  Both
+// tests are made on the words of r^2 (a compare costs an FP64-pipe slot); r^2 between the
+// threshold and the next higher top word takes the near form, which holds there too.
+// T: exp_table.
 template <int K>
 __device__ __forceinline__ void pair_f64_acc(double tx, double ty, double tz, const SrcF64& s, double (&u)[3],
-                                             double (&w)[3], double (&jq)[9])
+                                             double (&w)[3], double (&jq)[9], const double* T)
 {
     const double dx = tx - s.xy.x, dy = ty - s.xy.y, dz = tz - s.z_isig.x;
     const double r2 = dx * dx + dy * dy + dz * dz;
-    if (r2 == 0.0) return;
-    const double rinv = rsqrt(r2);
-    const double rinv2 = rinv * rinv;
+    if ((__double2hiint(r2) | __double2loint(r2)) == 0) return;
     double G, Q;
-    if (K == K_SING || (K == K_GAUSERF && r2 > s.gz_sig.y)) {
+    if constexpr (K == K_WNKLMNS) {
+        // (s + 2.5) q^-2.5 / sigma^3 and (s + 3.5) q^-3.5 / sigma^5, q = s + 1
+        const double isig = s.z_isig.y, isig2 = isig * isig;
+        const double sq = r2 * isig2;
+        const double t = rsqrt(sq + 1.0), t2 = t * t;
+        const double f = t2 * t2 * t * (isig2 * isig);
+        G = (sq + 2.5) * f;
+        Q = (sq + 3.5) * f * (t2 * isig2);
+    } else if (K == K_SING || (K == K_GAUSERF && __double2hiint(r2) > __double2hiint(s.gz_sig.y))) {
+        const double rinv = rsqrt(r2), rinv2 = rinv * rinv;
         G = rinv * rinv2;
         Q = G * rinv2;
-    } else {
+    } else if constexpr (K == K_GAUSERF) {
+        const double isig = s.z_isig.y, isig2 = isig * isig;
+        const double sq = r2 * isig2;
+        const double e = C2 * exp_neg(-0.5 * sq, T);
+        if (sq < 2.0) {
+            const double p = gerf_S2_f64(sq), f = e * (isig2 * isig);
+            G = f * fma(sq, p, 1.0 / 3.0);
+            Q = f * p * isig2;
+        } else {
+            const double rinv = rsqrt(r2), rinv2 = rinv * rinv, rinv3 = rinv * rinv2;
+            const double rho = r2 * rinv * isig;
+            const double g = fma(-e, gerf_h_f64(rho) * (1.0 / C2), 1.0);
+            G = g * rinv3;
+            Q = fma(-e * (1.0 / 3.0), rho * sq, g) * (rinv3 * rinv2);
+        }
+    } else {   // Gaussian: g = 1 - e^{-rho^3}, rho g' = 3 rho^3 e^{-rho^3}
+        const double rinv = rsqrt(r2), rinv2 = rinv * rinv, rinv3 = rinv * rinv2;
         const double isig = s.z_isig.y;
-        double g, dg;
-        g_dgdr_f64<K>(r2 * rinv * isig, g, dg);
-        G = g * rinv * rinv2;
-        Q = (G - dg * isig * rinv2 * (1.0 / 3.0)) * rinv2;
+        const double rho = r2 * rinv * isig, t = rho * rho * rho;
+        const double e = exp_neg(-t, T);
+        G = (1.0 - e) * rinv3;
+        Q = fma(-t, e, 1.0 - e) * (rinv3 * rinv2);
     }
     const double gx = s.gxy.x, gy = s.gxy.y, gz = s.gz_sig.x;
     const double cx = dy * gz - dz * gy, cy = dz * gx - dx * gz, cz = dx * gy - dy * gx;

@@ -3,11 +3,10 @@
 //
 // Two forms are provided:
 //
-//  * FP64, the reference formula: (g, dg/dr) of src/FLOWVPM_kernel.jl:45-84 and
-//    zeta of the same file, used by the plain FP64 kernels.  The only change is
-//    an exact far-field shortcut for the Gaussian-erf kernel: for rho > 9 the
-//    terms erf(rho/sqrt2)-1 and sqrt(2/pi)*rho*exp(-rho^2/2) are below 2^-56, so
-//    g = 1 and dg = 0 to FP64 rounding.
+//  * FP64: the functions of src/FLOWVPM_kernel.jl:45-84 to FP64 rounding, used by the plain
+//    FP64 kernels.  Gaussian-erf is evaluated without the reference's cancellation at small rho,
+//    and for rho > 9, where erf(rho/sqrt2)-1 and sqrt(2/pi)*rho*exp(-rho^2/2) are below 2^-56,
+//    as g = 1, dg = 0.
 //
 //  * FP32, a regular reformulation used by the mixed kernels.  With
 //    s = rho^2 = r^2/sigma^2 the pair terms of src/FLOWVPM_fmm.jl:130-160 are
@@ -43,39 +42,99 @@ __host__ __device__ constexpr double zeta_norm(int K)
 }
 
 // ------------------------------------------------------------------ FP64
-template <int K>
-__device__ __forceinline__ void g_dgdr_f64(double rho, double& g, double& dg)
+// The FP64 pipe runs at 1/64 of the FP32 rate and bounds every FP64 kernel, so the forms below
+// count its instructions: an exponential from a table (11 of them), Gaussian-erf from that one
+// exponential and a polynomial (no erf call, no square root), Winckelmans from one rsqrt (no
+// division).
+
+// e^x for x <= 0 by Tang's table method (P. T. P. Tang, "Table-driven implementation of the
+// exponential function in IEEE floating-point arithmetic", ACM TOMS 15, 1989): x = (k/64) ln 2 + r,
+// e^x = 2^(k div 64) T[k mod 64] (1 + p(r)), |r| <= ln 2/128, p the Taylor polynomial of degree 5
+// (3.5e-17 relative).  T: 2^(j/64), j < 64, in shared memory (exp_table).  Results below
+// 2^-1021 and non-finite x take the library's exp.
+__device__ __forceinline__ void exp_table(double* T)
 {
-    if constexpr (K == K_SING) {
-        g = 1.0; dg = 0.0;
-    } else if constexpr (K == K_GAUS) {
-        const double aux = exp(-rho * rho * rho);
-        g = 1.0 - aux; dg = 3.0 * rho * rho * aux;
-    } else if constexpr (K == K_GAUSERF) {
-        if (rho > 9.0) { g = 1.0; dg = 0.0; }
-        else {
-            const double aux = C2 * rho * exp(-0.5 * rho * rho);
-            g = erf(rho * INV_SQRT2) - aux; dg = rho * aux;
-        }
-    } else {  // Winckelmans
-        const double q = rho * rho + 1.0;
-        const double q2 = q * q;
-        const double q25 = sqrt(q2 * q2 * q);
-        g = rho * rho * rho * (rho * rho + 2.5) / q25;
-        dg = 7.5 * rho * rho / (q25 * q);
-    }
+    for (int j = threadIdx.x; j < 64; j += blockDim.x) T[j] = exp2(j * (1.0 / 64.0));
+}
+__device__ __forceinline__ double exp_neg(double x, const double* T)
+{
+    if ((unsigned)__double2hiint(x) >= 0xC0862000u) return exp(x);     // x <= -708, -inf
+    constexpr double magic = 6755399441055744.0;                       // 1.5 2^52
+    double kd = fma(x, 92.33248261689366, magic);                      // 64/ln 2
+    const int k = __double2loint(kd);
+    kd -= magic;
+    double r = fma(kd, -0.010830424695086549, x);                      // ln 2/64: 33 bits, and the rest
+    r = fma(kd, -1.162596423439437e-12, r);
+    double p = fma(r, 1.0 / 120.0, 1.0 / 24.0);
+    p = fma(p, r, 1.0 / 6.0);
+    p = fma(p, r, 0.5);
+    p = fma(p * r, r, r);
+    const double t = T[k & 63];
+    const double ts = __hiloint2double(__double2hiint(t) + ((k >> 6) << 20), __double2loint(t));
+    return fma(ts, p, ts);
 }
 
-template <int K>
-__device__ __forceinline__ double zeta_f64(double rho)
+// Gaussian-erf below s = 2: g = c2 e rho^3 K(s) and -H/3 = c2 e S2(s) with K = 1/3 + s S2 the
+// Kummer series sum s^m/(2m+3)!! (positive terms: none of the cancellation of erf against
+// sqrt(2/pi) rho e); S2 by its degree-11 Chebyshev fit on [0, 2] (2e-17).
+__device__ __forceinline__ double gerf_S2_f64(double s)
 {
-    if constexpr (K == K_SING) return rho == 0.0 ? 1.0 : 0.0;
-    else if constexpr (K == K_GAUS) return C3 * exp(-rho * rho * rho);
-    else if constexpr (K == K_GAUSERF) return C1 * exp(-0.5 * rho * rho);
+    double p = 7.117914962008134e-15;
+    p = fma(p, s, 1.12787989755004e-13);
+    p = fma(p, s, 3.2049748194948006e-12);
+    p = fma(p, s, 7.26474696490197e-11);
+    p = fma(p, s, 1.5274561118204643e-09);
+    p = fma(p, s, 2.9019546056094325e-08);
+    p = fma(p, s, 4.933338773525617e-07);
+    p = fma(p, s, 7.400007382107342e-06);
+    p = fma(p, s, 9.620009620382055e-05);
+    p = fma(p, s, 0.0010582010582006584);
+    p = fma(p, s, 0.00952380952380954);
+    p = fma(p, s, 0.06666666666666667);
+    return p;
+}
+// ... and from s = 2 to rho = 9: g = 1 - e h, h = erfcx(rho/sqrt2) + c2 rho, with
+// erfcx(rho/sqrt2) = t P(w), t = 1/(1 + rho/2), w = A t + B, P a degree-16 Chebyshev fit (3e-17).
+__device__ __forceinline__ double gerf_h_f64(double rho)
+{
+    const double d = fma(0.5, rho, 1.0);
+    double t;                                   // 1/d: the approximate reciprocal and two Newton steps
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(t) : "d"(d));
+    double e = fma(-d, t, 1.0);
+    t = fma(t, e, t);
+    e = fma(-d, t, 1.0);
+    t = fma(t, e, t);
+    const double w = fma(t, 4.950884063887905, -1.9001607388887100);
+    double p = -1.5660591337542868e-11;
+    p = fma(p, w, 5.63460752287977e-11);
+    p = fma(p, w, 5.1974104520460814e-11);
+    p = fma(p, w, -9.507498606778384e-10);
+    p = fma(p, w, 2.8308353212461513e-09);
+    p = fma(p, w, 3.3164182614796496e-09);
+    p = fma(p, w, -5.620367325865092e-08);
+    p = fma(p, w, 1.4651970275804292e-07);
+    p = fma(p, w, 4.7370926853939187e-07);
+    p = fma(p, w, -4.228927081890189e-06);
+    p = fma(p, w, 2.9494713884413277e-06);
+    p = fma(p, w, 8.528834233914718e-05);
+    p = fma(p, w, -0.0002486943660856597);
+    p = fma(p, w, -0.002127601067365253);
+    p = fma(p, w, 0.008702997368809272);
+    p = fma(p, w, 0.12611846511040975);
+    p = fma(p, w, 0.5974010771326975);
+    return fma(C2, rho, p * t);
+}
+
+// zeta(rho)/ZNORM as a function of s = rho^2 (src/FLOWVPM_kernel.jl)
+template <int K>
+__device__ __forceinline__ double zhat_f64(double s, const double* T)
+{
+    if constexpr (K == K_SING) return s == 0.0 ? 1.0 : 0.0;
+    else if constexpr (K == K_GAUS) return exp_neg(-s * sqrt(s), T);
+    else if constexpr (K == K_GAUSERF) return exp_neg(-0.5 * s, T);
     else {
-        const double t = rho * rho + 1.0;
-        const double t3 = t * t * t;
-        return C4 * 7.5 / sqrt(t3 * t3 * t);
+        const double t = rsqrt(s + 1.0), t2 = t * t, t4 = t2 * t2;
+        return t4 * t2 * t;
     }
 }
 
