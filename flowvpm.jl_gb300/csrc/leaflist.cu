@@ -1006,7 +1006,9 @@ nf_estr(int64_t n, int64_t ngroups, const TgtPos* __restrict__ tgt, const int32_
 {
     static_assert(MIXED || !DZ, "weight differences are FP32-comp only");
     static_assert(!(DZ && ZETA), "one mode at a time");
-    // mixed: per source (x_hi, 1/sigma^2), (x_lo), g, v;  FP64: the packed source
+    // mixed: per source (x_hi, 1/sigma^2), (x_lo, target mask), g, v;  FP64: the packed source.  The
+    // kernel is bound by these loads, broadcast reads of every source by every lane (73 % of the
+    // shared-memory rate with the masks in an array of their own).
     __shared__ __align__(16) float4 mtile[MIXED ? NF_WARPS : 1][4][32];
     __shared__ SrcEstrF64 dtile[MIXED ? 1 : NF_WARPS][32];
     __shared__ int spos[NF_WARPS][32];                          // source position, -1 for padding
@@ -1044,20 +1046,22 @@ nf_estr(int64_t n, int64_t ngroups, const TgtPos* __restrict__ tgt, const int32_
             if (sp >= 0) {
                 const SrcEstrDF p = ((const SrcEstrDF*)srcv)[sp];
                 mtile[warp][0][lane] = p.a;
-                mtile[warp][1][lane] = p.b;
+                mtile[warp][1][lane] = make_float4(p.b.x, p.b.y, p.b.z, __uint_as_float(smask));
                 mtile[warp][2][lane] = p.g;
                 mtile[warp][3][lane] = p.v;
             } else {   // padding: far away, no payload (read by the unrolled sub-blocks with mask 0)
                 mtile[warp][0][lane] = make_float4(1.0e6f, 1.0e6f, 1.0e6f, 1.f);
-                mtile[warp][1][lane] = make_float4(0.f, 0.f, 0.f, 0.f);
+                mtile[warp][1][lane] = make_float4(0.f, 0.f, 0.f, __uint_as_float(smask));
                 mtile[warp][2][lane] = make_float4(0.f, 0.f, 0.f, 0.f);
                 mtile[warp][3][lane] = make_float4(0.f, 0.f, 0.f, 0.f);
             }
         } else {
             if (sp >= 0) dtile[warp][lane] = ((const SrcEstrF64*)srcv)[sp];
         }
-        spos[warp][lane] = sp;
-        tmask[warp][lane] = smask;
+        if constexpr (!MIXED) {
+            spos[warp][lane] = sp;
+            tmask[warp][lane] = smask;
+        }
         __syncwarp();
         if constexpr (MIXED) {
             for (int j0 = 0; j0 < cnt; j0 += 8) {   // cnt <= 32: j0 + 7 stays in the tile (padding has mask 0)
@@ -1072,7 +1076,7 @@ nf_estr(int64_t n, int64_t ngroups, const TgtPos* __restrict__ tgt, const int32_
                     float z = zhat_f32<K>(r2 * h.w);
                     if constexpr (DZ) z *= zeta_ratio_m1<K>(r2 * h.w, fd);
                     // pairs at r = 0 are skipped (ZETA: kept, the self pair included)
-                    const bool on = (tmask[warp][j] & bit) != 0u && (ZETA || r2 != 0.0f);
+                    const bool on = (__float_as_uint(l.w) & bit) != 0u && (ZETA || r2 != 0.0f);
                     z = on ? z : 0.0f;
                     const float4 g = mtile[warp][2][j];
                     fg[0] = fmaf(z, g.x, fg[0]); fg[1] = fmaf(z, g.y, fg[1]); fg[2] = fmaf(z, g.z, fg[2]);

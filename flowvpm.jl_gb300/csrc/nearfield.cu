@@ -344,7 +344,8 @@ __global__ void nt_cr(const ull* __restrict__ ctr, const double* __restrict__ bo
 // (GB300's FP64 pipe runs at 1/64 of the FP32 rate: the FP64 test was most of
 // this kernel's time).
 __global__ void nt_trav(int step, double theta, const TravNode* __restrict__ cr, const int2* __restrict__ fin,
-                        int2* __restrict__ fout, uint64_t* __restrict__ near, ull* __restrict__ ctr, ull capF, ull capN)
+                        int2* __restrict__ fout, uint64_t* __restrict__ near, ull* __restrict__ ctr, ull capF, ull capN,
+                        int shift)
 {
     __shared__ unsigned sw[GS_THREADS / 32];
     __shared__ ull sb;
@@ -398,7 +399,7 @@ __global__ void nt_trav(int step, double theta, const TravNode* __restrict__ cr,
         }
         const ull sn = block_append(&ctr[C_NEAR], knear, sw, &sb);
         if (knear) {
-            if (sn < capN) near[sn] = ((uint64_t)(uint32_t)la_leaf << 32) | (uint32_t)lb_leaf;
+            if (sn < capN) near[sn] = ((uint64_t)(uint32_t)la_leaf << shift) | (uint32_t)lb_leaf;
             else ctr[C_OVFN] = 1;
         }
         const ull sf = block_append(&ctr[C_F + step + 1], ksplit, sw, &sb);
@@ -428,15 +429,15 @@ __global__ void nt_trav_init(int2* __restrict__ fr0, ull* __restrict__ ctr)
 }
 
 // ------------------------------------------------------------------- CSR
-__global__ void nt_csr_col(int64_t m, const uint64_t* __restrict__ keys, int32_t* __restrict__ col)
+__global__ void nt_csr_col(int64_t m, const uint64_t* __restrict__ keys, int shift, int32_t* __restrict__ col)
 {
-    for (int64_t i = gtid(); i < m; i += gstride()) col[i] = (int32_t)(uint32_t)(keys[i] & 0xffffffffULL);
+    for (int64_t i = gtid(); i < m; i += gstride()) col[i] = (int32_t)(keys[i] & ((1ull << shift) - 1));
 }
 
-__global__ void nt_csr_row(int64_t m, int64_t nl, const uint64_t* __restrict__ keys, int32_t* __restrict__ row)
+__global__ void nt_csr_row(int64_t m, int64_t nl, const uint64_t* __restrict__ keys, int shift, int32_t* __restrict__ row)
 {
     for (int64_t l = gtid(); l <= nl; l += gstride()) {
-        const uint64_t want = (uint64_t)l << 32;
+        const uint64_t want = (uint64_t)l << shift;
         int64_t lo = 0, hi = m;
         while (lo < hi) {
             const int64_t mid = lo + ((hi - lo) >> 1);
@@ -640,6 +641,10 @@ cudaError_t near_build(NearScratch& s, int64_t n, const double* x, int leaf_size
     // a uniform cloud at leaf size 64 and theta 0.4 needs ~32 n frontier pairs and ~16 n near pairs
     if (s.capF == 0) s.capF = (size_t)(n < 4096 ? 4096 : n) * 40;
     if (s.capN == 0) s.capN = (size_t)(n < 4096 ? 4096 : n) * 24;
+    // near pairs are the keys (target leaf << shift) | source leaf, with only as many bits for the
+    // source as n leaves need: the sort's passes go by key bits (37 instead of 49 at 2^20)
+    int shift = 1;
+    while (((int64_t)1 << shift) < n) shift++;
     for (int attempt = 0;; attempt++) {
         NT_TRY(s.fr0.grow(s.capF * sizeof(int2)));
         NT_TRY(s.fr1.grow(s.capF * sizeof(int2)));
@@ -650,7 +655,7 @@ cudaError_t near_build(NearScratch& s, int64_t n, const double* x, int leaf_size
             const int2* fin = (k & 1) ? s.fr1.as<int2>() : s.fr0.as<int2>();
             int2* fout = (k & 1) ? s.fr0.as<int2>() : s.fr1.as<int2>();
             nt_trav<<<GS_BLOCKS, GS_THREADS, 0, st>>>(k, theta, s.node_cr.as<TravNode>(), fin, fout,
-                                                       s.near0.as<uint64_t>(), ctr, (ull)s.capF, (ull)s.capN);
+                                                       s.near0.as<uint64_t>(), ctr, (ull)s.capF, (ull)s.capN, shift);
         }
         *launches += TRAV_STEPS + 1;
         NT_TRY(cudaGetLastError());
@@ -678,14 +683,15 @@ cudaError_t near_build(NearScratch& s, int64_t n, const double* x, int leaf_size
     int hb = 1;
     while (((int64_t)1 << hb) <= nl) hb++;
     NT_TRY(cub::DeviceRadixSort::SortKeys(nullptr, tb, s.near0.as<uint64_t>(), s.near1.as<uint64_t>(), (int)m, 0,
-                                          32 + hb, st));
+                                          shift + hb, st));
     NT_TRY(grow_cub(s, tb));
     NT_TRY(cub::DeviceRadixSort::SortKeys(s.cub.p, tb, s.near0.as<uint64_t>(), s.near1.as<uint64_t>(), (int)m, 0,
-                                          32 + hb, st));
+                                          shift + hb, st));
     NT_TRY(s.row.grow((nl + 1) * sizeof(int32_t)));
     NT_TRY(s.col.grow((m > 0 ? m : 1) * sizeof(int32_t)));
-    nt_csr_col<<<gs_blocks(m), GS_THREADS, 0, st>>>(m, s.near1.as<uint64_t>(), s.col.as<int32_t>());
-    nt_csr_row<<<gs_blocks(nl + 1), GS_THREADS, 0, st>>>(m, nl, s.near1.as<uint64_t>(), s.row.as<int32_t>());
+    nt_csr_col<<<gs_blocks(m), GS_THREADS, 0, st>>>(m, s.near1.as<uint64_t>(), shift, s.col.as<int32_t>());
+    nt_csr_row<<<gs_blocks(nl + 1), GS_THREADS, 0, st>>>(m, nl, s.near1.as<uint64_t>(), shift,
+                                                      s.row.as<int32_t>());
     *launches += 4;
     NT_TRY(cudaGetLastError());
     L->perm = s.perm.as<int32_t>();
