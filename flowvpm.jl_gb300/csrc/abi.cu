@@ -998,8 +998,9 @@ static int near_run(vpm_ctx* c, NearLists& L, int64_t n, const double* x, const 
                     const uint8_t* static_flags, double* U, double* J, double* SFS, int kernel, int precision,
                     int flags, int64_t* stats)
 {
-    RC(grow(c, c->leaf, leaf_work_bytes(n), "near-field packs"));
+    RC(grow(c, c->leaf, leaf_work_bytes(n, c->num_sms), "near-field packs"));
     LeafArgs a;
+    a.num_sms = c->num_sms;
     a.n = n; a.x = x; a.gam = gam; a.sig = sig; a.U = U; a.J = J; a.SFS = SFS; a.static_flags = static_flags;
     a.kernel = kernel; a.precision = precision; a.sfs = (flags & VPM_SFS) != 0;
     a.transposed = (flags & VPM_TRANSPOSED) != 0;
@@ -1139,8 +1140,9 @@ int vpm_zeta_leaflist_dev(vpm_ctx* c, int64_t n, const double* x, const double* 
         return fail(c, VPM_ERR_ARG, "%s: every array must be a device pointer", fn);
     NearLists L;
     RC(near_lists(c, n, x, leaf_size, theta, (flags & VPM_REUSE_LISTS) != 0, &L));
-    RC(grow(c, c->leaf, leaf_work_bytes(n), "near-field packs"));
+    RC(grow(c, c->leaf, leaf_work_bytes(n, c->num_sms), "near-field packs"));
     LeafArgs a;
+    a.num_sms = c->num_sms;
     a.n = n; a.x = x; a.gam = gam; a.sig = sig; a.U = nullptr; a.J = nullptr; a.SFS = nullptr;
     a.static_flags = nullptr; a.kernel = kernel; a.precision = precision; a.sfs = false; a.transposed = true;
     CK(launch_leaf_zeta(a, L, W, c->leaf.p, c->stream, &c->launches), "near-field zeta");
@@ -1180,7 +1182,7 @@ int vpm_dynamic_diff_leaflist_dev(vpm_ctx* c, int64_t n, const double* x, const 
     cudaStream_t st = c->stream;
     NearLists L;
     RC(near_lists(c, n, x, leaf_size, theta, (flags & VPM_REUSE_LISTS) != 0, &L));
-    RC(grow(c, c->leaf, leaf_work_bytes(n), "near-field packs"));
+    RC(grow(c, c->leaf, leaf_work_bytes(n, c->num_sms), "near-field packs"));
     RC(grow(c, c->s, n * sizeof(double), "test-filter core sizes"));
     double* sig_a = (double*)c->s.p;
     scale_copy<<<nblk(n), EB, 0, st>>>(n, sig, alpha, sig_a);
@@ -1188,6 +1190,7 @@ int vpm_dynamic_diff_leaflist_dev(vpm_ctx* c, int64_t n, const double* x, const 
     CK(cudaMemsetAsync(dJ, 0, 9 * n * sizeof(double), st), "memset dJ");
     CK(cudaMemsetAsync(dSFS, 0, 3 * n * sizeof(double), st), "memset dSFS");
     LeafArgs a;
+    a.num_sms = c->num_sms;
     a.n = n; a.x = x; a.gam = gam; a.sig = sig; a.U = nullptr; a.J = const_cast<double*>(J); a.SFS = dSFS;
     a.static_flags = static_flags; a.kernel = kernel; a.precision = precision; a.sfs = true;
     a.transposed = (flags & VPM_TRANSPOSED) != 0;

@@ -111,6 +111,7 @@ struct LeafArgs {
     const uint8_t* static_flags;                              // [n] or null
     int kernel, precision;
     bool sfs, transposed;
+    int num_sms;
     bool uj = true;                                           // false: the Estr pass alone (J is input)
 };
 
@@ -247,7 +248,7 @@ cudaError_t near_groups(NearScratch& s, NearLists* L, cudaStream_t st, SyncFn sy
                         int64_t* launches);
 
 constexpr int LEAF_SIZE_MAX = 4096;
-size_t leaf_work_bytes(int64_t n);
+size_t leaf_work_bytes(int64_t n, int num_sms);
 cudaError_t launch_leaflist(const LeafArgs& a, const NearLists& L, void* work, cudaStream_t st, int64_t* launches);
 // The per-particle work of an RK3 step (step.cu).
 struct StageArgs {
