@@ -578,6 +578,7 @@ static int uj_full_matrix(vpm_ctx* c, double* particles, int64_t np, int kernel,
         e.SFS = mat + R_SFS; e.ldS = VPM_NFIELDS;
         e.kernel = kernel; e.precision = precision;
         e.transposed = (flags & VPM_TRANSPOSED) != 0; e.self = true;
+        e.ordered = true;   // by the UJ launch
         CK(launch_estr(e, w, c->num_sms, st, &c->launches), "Estr kernels");
     }
     int* dflag = (int*)c->flag.p;
@@ -665,6 +666,7 @@ static int uj_staged(vpm_ctx* c, double* particles, int64_t np, int kernel, int 
         e.SFS = dS; e.ldS = 3;
         e.kernel = kernel; e.precision = precision;
         e.transposed = (flags & VPM_TRANSPOSED) != 0; e.self = true;
+        e.ordered = true;   // by the UJ launch
         CK(launch_estr(e, w, c->num_sms, st, &c->launches), "Estr kernels");
     }
     CK(cudaMemcpyAsync(hout, dU, (size_t)nout * np * sizeof(double), cudaMemcpyDeviceToHost, st), "D2H staged outputs");
@@ -928,8 +930,10 @@ int vpm_dynamic_diff_dev(vpm_ctx* c, int64_t n, const double* x, const double* g
         CK(launch_uj_filter_diff(n, x, gam, sig, alpha, dJ, kernel, c->num_sms, w, st, &c->launches), "filter-difference UJ");
         // the weight difference at J, then an ordinary Estr of dJ at alpha sigma
         e.Jt = J; e.Js = J; e.sgs = sig; e.SFS = dSFS; e.dz_alpha = alpha;
+        e.ordered = kernel != K_SING;   // by the filter difference (nothing to do for the singular kernel)
         CK(launch_estr(e, w, c->num_sms, st, &c->launches), "weight-difference Estr");
         e.Jt = dJ; e.Js = dJ; e.sgs = sig_a; e.dz_alpha = 0.0;
+        e.ordered = true;
         CK(launch_estr(e, w, c->num_sms, st, &c->launches), "test-filter Estr");
     } else {
         // FP64: the reference's two evaluations, then their differences
@@ -944,6 +948,7 @@ int vpm_dynamic_diff_dev(vpm_ctx* c, int64_t n, const double* x, const double* g
         a.U = Ua; a.ldU = 3; a.J = Ja; a.ldJ = 9; a.kernel = kernel; a.precision = precision; a.self = true;
         CK(launch_uj(a, w, c->num_sms, st, &c->launches), "test-filter UJ");
         e.Jt = Ja; e.Js = Ja; e.sgs = sig_a; e.SFS = Sa;
+        e.ordered = true;   // by the UJ launch
         CK(launch_estr(e, w, c->num_sms, st, &c->launches), "test-filter Estr");
         e.Jt = J; e.Js = J; e.sgs = sig; e.SFS = S0;
         CK(launch_estr(e, w, c->num_sms, st, &c->launches), "Estr");

@@ -416,8 +416,12 @@ static cudaError_t launch_estr_k(const EstrArgs& a, const Workspace& w, int num_
     const int pb = 256;
     const unsigned pgrid = (unsigned)((ns_pad + pb - 1) / pb);
     const TgtPos* tgt = nullptr;
-    cudaError_t e = order_targets(a.nt, a.xt, w.order, w.order_bytes, st, launches, &tgt);
-    if (e != cudaSuccess) return e;
+    if (a.ordered) {
+        tgt = ordered_targets(a.nt, w.order);
+    } else {
+        cudaError_t e = order_targets(a.nt, a.xt, w.order, w.order_bytes, st, launches, &tgt);
+        if (e != cudaSuccess) return e;
+    }
     const uint8_t* static_s = a.zeta ? nullptr : a.static_s;
     const uint8_t* static_t = a.zeta ? nullptr : a.static_t;
     if (a.dz_alpha > 0.0 && a.precision == 0) return cudaErrorInvalidValue;   // FP32-comp only

@@ -71,6 +71,7 @@ struct EstrArgs {
     int kernel, precision;
     bool transposed, self;
     bool zeta = false;    // zeta_direct instead: SFS receives W = sum zeta Gamma (J unused, statics included)
+    bool ordered = false;    // Workspace.order holds the order of these targets already (same library call)
     double dz_alpha = 0.0;   // > 0: the weight difference zeta~(r, alpha sigma) - zeta~(r, sigma) (mixed only)
 };
 
@@ -157,6 +158,9 @@ cudaError_t launch_uj_tc(const UJArgs& a, const TgtPos* tgt, const SrcMixed* src
 // Curve-order the nt targets xt; *out receives nt TgtPos records in scratch.
 cudaError_t order_targets(int64_t nt, const double* xt, void* scratch, size_t scratch_bytes, cudaStream_t st,
                           int64_t* launches, const TgtPos** out);
+
+// Where order_targets left the order of nt targets in this scratch (the records come last).
+const TgtPos* ordered_targets(int64_t nt, void* scratch);
 
 // Sets the calling thread's context-free error text (vpm_last_error(NULL)).
 void set_thread_error(const char* msg);

@@ -16,9 +16,11 @@
 // Steps: per-block bounding boxes (bbox_partial), curve keys (hilbert_keys), CUB radix sort of
 // (key, index), and a gather of the sorted positions into TgtPos records.  Keys have 10 bits an
 // axis up to 2^16 particles (a cell of the cube then holds at most a few of a uniform set; four
-// 8-bit sort passes, each about 9 us at these sizes) and 20 beyond (eight passes).
+// 8-bit sort passes, each about 9 us at these sizes) and 20 beyond (eight passes).  Up to 6,144
+// particles one block does all of it (order_block): a launch instead of eight.
 #include "internal.h"
 
+#include <cub/block/block_radix_sort.cuh>
 #include <cub/device/device_radix_sort.cuh>
 
 namespace vpm {
@@ -144,6 +146,78 @@ __global__ void gather_targets(int64_t n, const double* __restrict__ x, const in
 
 static inline size_t align256(size_t b) { return (b + 255) / 256 * 256; }
 
+// Everything in one block: thread t holds particles t ITEMS .. t ITEMS + ITEMS - 1.
+constexpr int OB_THREADS = 1024;
+constexpr int64_t OB_MAX = OB_THREADS * 6;
+constexpr int OB_BITS = 8;                // key bits an axis: seven 4-bit passes with the flag of absent ones
+template <int ITEMS>
+__global__ void __launch_bounds__(OB_THREADS)
+order_block(int n, const double* __restrict__ x, TgtPos* __restrict__ out)
+{
+    typedef cub::BlockRadixSort<uint32_t, OB_THREADS, ITEMS, int32_t> Sort;
+    __shared__ union { typename Sort::TempStorage sort; float red[6][OB_THREADS / 32]; } sm;
+    // Offsets from the first particle, rounded to FP32 (two FP64 operations a coordinate; box, scale
+    // and cells in FP64 took a single SM longer than the eight launches).
+    float p[ITEMS][3], v[6] = {INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+    for (int j = 0; j < ITEMS; j++) {
+        const int i = min((int)threadIdx.x * ITEMS + j, n - 1);
+#pragma unroll
+        for (int k = 0; k < 3; k++) {
+            p[j][k] = (float)(x[3 * i + k] - x[k]);
+            v[k] = fminf(v[k], p[j][k]);
+            v[3 + k] = fmaxf(v[3 + k], p[j][k]);
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < 6; k++) {
+#pragma unroll
+        for (int m = 16; m > 0; m >>= 1) {
+            const float o = __shfl_xor_sync(0xffffffffu, v[k], m);
+            v[k] = k < 3 ? fminf(v[k], o) : fmaxf(v[k], o);
+        }
+        if ((threadIdx.x & 31) == 0) sm.red[k][threadIdx.x >> 5] = v[k];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < 6; k++) {
+        v[k] = sm.red[k][threadIdx.x & 31];
+#pragma unroll
+        for (int m = 16; m > 0; m >>= 1) {
+            const float o = __shfl_xor_sync(0xffffffffu, v[k], m);
+            v[k] = k < 3 ? fminf(v[k], o) : fmaxf(v[k], o);
+        }
+    }
+    __syncthreads();
+    const float ext = fmaxf(v[3] - v[0], fmaxf(v[4] - v[1], v[5] - v[2]));
+    constexpr float top = (float)((1 << OB_BITS) - 1);
+    const float sc = ext > 0.f ? top / ext : 0.f;
+    uint32_t key[ITEMS];
+    int32_t idx[ITEMS];
+#pragma unroll
+    for (int j = 0; j < ITEMS; j++) {
+        const int i = threadIdx.x * ITEMS + j;
+        idx[j] = i;
+        uint32_t q[3];
+#pragma unroll
+        for (int k = 0; k < 3; k++) q[k] = (uint32_t)fminf(fmaxf((p[j][k] - v[k]) * sc, 0.f), top);
+        key[j] = i < n ? hilbert_index<uint32_t>(q, OB_BITS) : 1u << (3 * OB_BITS);     // past n: behind every particle
+    }
+    Sort(sm.sort).Sort(key, idx, 0, 3 * OB_BITS + 1);
+#pragma unroll
+    for (int j = 0; j < ITEMS; j++) {
+        const int o = threadIdx.x * ITEMS + j;
+        if (o >= n) continue;
+        TgtPos t;
+        t.x = x[3 * (int64_t)idx[j]];
+        t.y = x[3 * (int64_t)idx[j] + 1];
+        t.z = x[3 * (int64_t)idx[j] + 2];
+        t.idx = idx[j];
+        t.pad = 0;
+        out[o] = t;
+    }
+}
+
 constexpr int64_t SMALL_KEYS = 1 << 16;   // up to here 10-bit axes and 32-bit keys
 
 template <typename Key>
@@ -169,6 +243,11 @@ size_t order_bytes(int64_t nt)
            2 * align256(nt * sizeof(int32_t)) + align256(sort_tmp(nt)) + align256(nt * sizeof(TgtPos));
 }
 
+const TgtPos* ordered_targets(int64_t nt, void* scratch)
+{
+    return (const TgtPos*)((char*)scratch + order_bytes(nt) - align256(nt * sizeof(TgtPos)));
+}
+
 cudaError_t order_targets(int64_t nt, const double* xt, void* scratch, size_t scratch_bytes, cudaStream_t st,
                           int64_t* launches, const TgtPos** out)
 {
@@ -184,6 +263,16 @@ cudaError_t order_targets(int64_t nt, const double* xt, void* scratch, size_t sc
     if ((size_t)(p - (char*)scratch) > scratch_bytes) return cudaErrorInvalidValue;
     const unsigned nb = (unsigned)((nt + BB_THREADS - 1) / BB_THREADS);
     const int32_t* perm = nullptr;
+    if (nt > 1 && nt <= OB_MAX) {
+        const int items = (int)((nt + OB_THREADS - 1) / OB_THREADS), m = (int)nt;
+        if (items <= 1) order_block<1><<<1, OB_THREADS, 0, st>>>(m, xt, tp);
+        else if (items <= 2) order_block<2><<<1, OB_THREADS, 0, st>>>(m, xt, tp);
+        else if (items <= 4) order_block<4><<<1, OB_THREADS, 0, st>>>(m, xt, tp);
+        else order_block<6><<<1, OB_THREADS, 0, st>>>(m, xt, tp);
+        *launches += 1;
+        *out = tp;
+        return cudaGetLastError();
+    }
     if (nt > 1) {
         bbox_partial<<<BB_BLOCKS, BB_THREADS, 0, st>>>(nt, xt, part);
         cudaError_t e;
