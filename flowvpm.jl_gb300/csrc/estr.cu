@@ -39,8 +39,8 @@ constexpr int EWT = EST_TILE;   // sources per tile of the mixed kernel's stream
 size_t estr_src_pack_bytes(int64_t ns, int precision)
 {
     const int64_t n = round_up(ns, UJ_TILE);
-    // FP32-comp: the records, then two float4 per 32-source tile (estr_tile_boxes)
-    return precision ? (size_t)n * sizeof(SrcEstrDF) + (size_t)(n / EWT) * 2 * sizeof(float4)
+    // FP32-comp: the tiles, then two float4 a tile (estr_tile_box)
+    return precision ? (size_t)(n / EWT) * (sizeof(EstrTile) + 2 * sizeof(float4))
                      : (size_t)n * sizeof(SrcEstrF64);
 }
 
@@ -64,35 +64,40 @@ __global__ void pack_estr_mixed(int64_t ns, int64_t ns_pad, const double* __rest
                                 const double* __restrict__ gs, const double* __restrict__ sgs,
                                 const double* __restrict__ Js, int64_t ldJs,
                                 const uint8_t* __restrict__ static_s, bool transposed,
-                                const TgtPos* __restrict__ order, SrcEstrDF* __restrict__ out,
+                                const TgtPos* __restrict__ order, EstrTile* __restrict__ out,
                                 float4* __restrict__ box)
 {
     // with `order` (sources = targets) the pack follows the targets' curve order
     const int64_t o = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (o >= ns_pad) return;   // whole warps: ns_pad is a multiple of 32
-    SrcEstrDF p;
-    if (o < ns) {
+    float x[3] = {1.0e6f, 1.0e6f, 1.0e6f}, xl[3] = {0.f, 0.f, 0.f}, w = 1.f, g[3] = {0.f, 0.f, 0.f}, v[3] = {0.f, 0.f, 0.f};
+    if (o < ns) {   // past ns: far away, no strength
         const int64_t i = order ? (int64_t)order[o].idx : o;
         const double isig = 1.0 / sgs[i];
         const double isig2 = isig * isig;
-        const double x = xs[3 * i], y = xs[3 * i + 1], z = xs[3 * i + 2];
-        const float xh = (float)x, yh = (float)y, zh = (float)z;
-        p.a = make_float4(xh, yh, zh, (float)isig2);
-        p.b = make_float4((float)(x - (double)xh), (float)(y - (double)yh), (float)(z - (double)zh), 0.f);
+        w = (float)isig2;
         const bool off = static_s && static_s[i];
         const double k = off ? 0.0 : zeta_norm(K) * isig2 * isig;
         const double gx = gs[3 * i], gy = gs[3 * i + 1], gz = gs[3 * i + 2];
-        double vx = 0.0, vy = 0.0, vz = 0.0;   // the zeta field (Js null) needs no v
-        if (Js) stretch_vec(Js + i * ldJs, gx, gy, gz, transposed, vx, vy, vz);
-        p.g = make_float4((float)(k * gx), (float)(k * gy), (float)(k * gz), 0.f);
-        p.v = make_float4((float)(k * vx), (float)(k * vy), (float)(k * vz), 0.f);
-    } else {   // padding: far away, no strength
-        p.a = make_float4(1.0e6f, 1.0e6f, 1.0e6f, 1.f);
-        p.b = make_float4(0.f, 0.f, 0.f, 0.f);
-        p.g = p.v = make_float4(0.f, 0.f, 0.f, 0.f);
+        double vv[3] = {0.0, 0.0, 0.0};   // the zeta field (Js null) needs no v
+        if (Js) stretch_vec(Js + i * ldJs, gx, gy, gz, transposed, vv[0], vv[1], vv[2]);
+#pragma unroll
+        for (int m = 0; m < 3; m++) {
+            const double c = xs[3 * i + m];
+            x[m] = (float)c;
+            xl[m] = (float)(c - (double)x[m]);
+            g[m] = (float)(k * gs[3 * i + m]);
+            v[m] = (float)(k * vv[m]);
+        }
     }
-    out[o] = p;
-    estr_tile_box(o, ns, p.a.x, p.a.y, p.a.z, p.a.w, box);
+    EstrTile& T = out[o / EWT];
+    const int l = (int)(o % EWT);
+    T.x[l] = x[0]; T.y[l] = x[1]; T.z[l] = x[2]; T.w[l] = w;
+    T.xl[l] = xl[0]; T.yl[l] = xl[1]; T.zl[l] = xl[2];
+    T.gv[3 * l] = make_float2(g[0], g[1]);
+    T.gv[3 * l + 1] = make_float2(g[2], v[0]);
+    T.gv[3 * l + 2] = make_float2(v[1], v[2]);
+    estr_tile_box(o, ns, x[0], x[1], x[2], w, box);
 }
 
 template <int K>
@@ -217,7 +222,7 @@ __device__ __forceinline__ void ecp_commit() { asm volatile("cp.async.commit_gro
 template <int N>
 __device__ __forceinline__ void ecp_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
 
-constexpr int ESTR_FLUSH_TILES = 8;      // evaluated warp tiles between FP64 adds (256 sources)
+constexpr int ESTR_FLUSH_TILES = 24;     // evaluated warp tiles between FP64 adds (768 sources)
 
 // The mixed Estr.  Each warp streams the sources on its own, 32 per tile,
 // double-buffered with cp.async (no block-wide barrier); the loading lane
@@ -229,10 +234,15 @@ constexpr int ESTR_FLUSH_TILES = 8;      // evaluated warp tiles between FP64 ad
 // rounding, at the largest weight).  For the Gaussian kernels the terms past
 // zeta_skip_s (zeta/zeta(0) < 1e-13: below the FP32 resolution of the sums) are
 // skipped at three levels: a tile whose pack box is out of reach of the warp's
-// targets is not loaded (TileWalk); a loaded tile is skipped when every one of its
-// sources is out of reach of the warp's target box; an 8-source sub-block when
-// every pair of the warp is.  Sums: 8-source FP32 partials added with
-// compensation (comp_add), FP64 every ESTR_FLUSH_TILES evaluated tiles.
+// targets is not loaded (TileWalk); of a loaded tile, the 8-source sub-blocks whose
+// sources are all out of reach of the warp's target box, before their distances are
+// formed, or of every target, after.  Sums: 8-source FP32 partials added with
+// compensation (comp_add2), FP64 every ESTR_FLUSH_TILES evaluated tiles.
+// Bound: the FMA pipe (61 % busy) and shared-memory reads (67 %).  With two sources to an f32x2
+// instruction and 16-byte reads of four sources' coordinates a pair takes 18 issue slots; one
+// source at a time from 64-byte records took 24 and 80 % of the shared-memory rate (every lane
+// reads every source, and the records' copies and conversions met bank conflicts).  Rings of
+// 200,000: 3.77 -> 3.01 ms; jet of 100,000, Winckelmans (no reach): 9.70 -> 8.55 ms.
 // With DZ (the weight difference of the dynamic procedure's test filter,
 // dynamic.cu) each weight zeta~(r, sigma_s) is replaced by
 // zeta~(r, alpha sigma_s) - zeta~(r, sigma_s) = zeta~(r, sigma_s) (ratio - 1),
@@ -240,12 +250,11 @@ constexpr int ESTR_FLUSH_TILES = 8;      // evaluated warp tiles between FP64 ad
 template <int K, bool ZETA, bool DZ = false>
 __global__ void __launch_bounds__(UJ_THREADS)
 estr_mixed_kernel(int64_t nt, const TgtPos* __restrict__ tgt, const double* __restrict__ Jt, int64_t ldJt,
-                  const uint8_t* __restrict__ static_t, int64_t ns_pad, const SrcEstrDF* __restrict__ src,
+                  const uint8_t* __restrict__ static_t, int64_t ns_pad, const EstrTile* __restrict__ src,
                   const float4* __restrict__ box, bool self, bool transposed, double* SFS,
                   int64_t ldS, double* partial, int64_t nt_pad, float3 fd = make_float3(0.f, 0.f, 0.f))
 {
-    __shared__ SrcEstrDF stage[UJ_WARPS][2][EWT];
-    __shared__ float4 offs[UJ_WARPS][2][EWT];
+    __shared__ EstrTile stage[UJ_WARPS][2];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t t = (int64_t)blockIdx.x * UJ_THREADS + threadIdx.x;
     double tx = 0.0, ty = 0.0, tz = 0.0;
@@ -296,107 +305,84 @@ estr_mixed_kernel(int64_t nt, const TgtPos* __restrict__ tgt, const double* __re
         __syncwarp();
     }
     double zg[3] = {0.0, 0.0, 0.0}, zv[3] = {0.0, 0.0, 0.0};
-    float sg[3] = {0.f, 0.f, 0.f}, cg[3] = {0.f, 0.f, 0.f}, sv[3] = {0.f, 0.f, 0.f}, cv[3] = {0.f, 0.f, 0.f};
-    const SrcEstrDF* wsrc = src + lane;
+    f32x2 sm[3] = {0ull, 0ull, 0ull}, cm[3] = {0ull, 0ull, 0ull};   // compensated sums (gx gy)(gz vx)(vy vz)
+    const f32x2 TX = pk(-to.x, -to.x), TY = pk(-to.y, -to.y), TZ = pk(-to.z, -to.z);
+    auto load = [&](int tile, int b) {   // 104 chunks of 16 bytes
+        const float4* g = (const float4*)&src[tile];
+        float4* d = (float4*)&stage[warp][b];
+#pragma unroll
+        for (int q = 0; q < 3; q++) ecp_async16(d + 32 * q + lane, g + 32 * q + lane);
+        if (lane < 8) ecp_async16(d + 96 + lane, g + 96 + lane);
+        ecp_commit();
+    };
     // the split's tiles within reach of the warp's targets, 32 tiles per ballot
     TileWalk walk;
     walk.init((int)(ns_pad / EWT), blockIdx.y, gridDim.y);
     int cur = walk.next<K>(box, wbox[warp][2], wbox[warp][3], lane);
-    if (cur >= 0) {
-        SrcEstrDF* d = &stage[warp][0][lane];
-        const SrcEstrDF* gp = wsrc + (int64_t)cur * EWT;
-        ecp_async16(&d->a, &gp->a); ecp_async16(&d->b, &gp->b);
-        ecp_async16(&d->g, &gp->g); ecp_async16(&d->v, &gp->v);
-        ecp_commit();
-    }
+    if (cur >= 0) load(cur, 0);
     int in_flush = 0, buf = 0;
     while (cur >= 0) {
         const int nxt = walk.next<K>(box, wbox[warp][2], wbox[warp][3], lane);
         if (nxt >= 0) {
-            const SrcEstrDF* gp = wsrc + (int64_t)nxt * EWT;
-            SrcEstrDF* d = &stage[warp][buf ^ 1][lane];
-            ecp_async16(&d->a, &gp->a); ecp_async16(&d->b, &gp->b);
-            ecp_async16(&d->g, &gp->g); ecp_async16(&d->v, &gp->v);
-            ecp_commit();
+            load(nxt, buf ^ 1);
             ecp_wait<1>();
         } else {
             ecp_wait<0>();
         }
         __syncwarp();
-        bool beyond;
-        {   // this lane's source: FP32 offset, and whether it is out of reach of the whole target box
-            const float4 a = stage[warp][buf][lane].a, b = stage[warp][buf][lane].b;
-            const float px = df_offset(a.x, b.x, oh.x, ol.x), py = df_offset(a.y, b.y, oh.y, ol.y),
-                        pz = df_offset(a.z, b.z, oh.z, ol.z);
-            offs[warp][buf][lane] = make_float4(px, py, pz, a.w);
+        EstrTile& T = stage[warp][buf];
+        // the tile's sources out of reach of the whole target box, and those inside it, the only
+        // ones that can be at r = 0 from a target
+        unsigned beyond, inside;
+        {   // this lane's source: FP32 offset
+            const float px = df_offset(T.x[lane], T.xl[lane], oh.x, ol.x), py = df_offset(T.y[lane], T.yl[lane], oh.y, ol.y),
+                        pz = df_offset(T.z[lane], T.zl[lane], oh.z, ol.z);
+            T.x[lane] = px; T.y[lane] = py; T.z[lane] = pz;
             const float4 lo = wbox[warp][0], hi = wbox[warp][1];
             const float ex = fmaxf(fmaxf(lo.x - px, px - hi.x), 0.0f);
             const float ey = fmaxf(fmaxf(lo.y - py, py - hi.y), 0.0f);
             const float ez = fmaxf(fmaxf(lo.z - pz, pz - hi.z), 0.0f);
-            beyond = fmaf(ex, ex, fmaf(ey, ey, ez * ez)) * a.w > zeta_skip_s<K>();
+            const float d2 = fmaf(ex, ex, fmaf(ey, ey, ez * ez));
+            beyond = __ballot_sync(0xffffffffu, zeta_skip_s<K>() > 0.0f && d2 * T.w[lane] > zeta_skip_s<K>());
+            inside = __ballot_sync(0xffffffffu, !(d2 > 0.0f));
         }
         __syncwarp();
-        if (!(zeta_skip_s<K>() > 0.0f && __all_sync(0xffffffffu, beyond))) {
+        if (beyond != 0xffffffffu) {
 #pragma unroll 1
             for (int sub = 0; sub < EWT; sub += ESTR_SUB) {
-                float sv8[ESTR_SUB], r28[ESTR_SUB];
-                bool far = true;
+                if (((beyond >> sub) & 0xffu) == 0xffu) continue;
+                f32x2 r2[4], s[4];
 #pragma unroll
-                for (int jj = 0; jj < ESTR_SUB; jj++) {
-                    const float4 h = offs[warp][buf][sub + jj];
-                    const float dx = to.x - h.x, dy = to.y - h.y, dz = to.z - h.z;
-                    r28[jj] = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-                    sv8[jj] = r28[jj] * h.w;
-                    far = far && sv8[jj] > zeta_skip_s<K>();
+                for (int q = 0; q < 2; q++) {
+                    const ulonglong2 X = *(const ulonglong2*)&T.x[sub + 4 * q], Y = *(const ulonglong2*)&T.y[sub + 4 * q],
+                                     Z = *(const ulonglong2*)&T.z[sub + 4 * q], W = *(const ulonglong2*)&T.w[sub + 4 * q];
+                    f32x2 dx = add2(X.x, TX), dy = add2(Y.x, TY), dz = add2(Z.x, TZ);
+                    r2[2 * q] = fma2(dx, dx, fma2(dy, dy, mul2(dz, dz)));
+                    s[2 * q] = mul2(r2[2 * q], W.x);
+                    dx = add2(X.y, TX); dy = add2(Y.y, TY); dz = add2(Z.y, TZ);
+                    r2[2 * q + 1] = fma2(dx, dx, fma2(dy, dy, mul2(dz, dz)));
+                    s[2 * q + 1] = mul2(r2[2 * q + 1], W.y);
                 }
-                if (zeta_skip_s<K>() > 0.0f && __all_sync(0xffffffffu, far)) continue;
-                float fg[3] = {0.f, 0.f, 0.f}, fv[3] = {0.f, 0.f, 0.f};
+                if (zeta_skip_s<K>() > 0.0f && __all_sync(0xffffffffu, min8_nan(s) > zeta_skip_s<K>())) continue;
+                f32x2 f[3] = {0ull, 0ull, 0ull};
+                if (!ZETA && ((inside >> sub) & 0xffu))
+                    estr_add8<K, ZETA, DZ, false, !ZETA>(r2, s, &T.gv[3 * sub], 0u, fd, f);
+                else
+                    estr_add8<K, ZETA, DZ, false, false>(r2, s, &T.gv[3 * sub], 0u, fd, f);
 #pragma unroll
-                for (int jj = 0; jj < ESTR_SUB; jj++) {
-                    const int j = sub + jj;
-                    float z = zhat_f32<K>(sv8[jj]);
-                    if constexpr (DZ) z *= zeta_ratio_m1<K>(sv8[jj], fd);
-                    if constexpr (!ZETA) z = (r28[jj] == 0.0f) ? 0.0f : z;
-                    const float4 g = stage[warp][buf][j].g;
-                    fg[0] = fmaf(z, g.x, fg[0]);
-                    fg[1] = fmaf(z, g.y, fg[1]);
-                    fg[2] = fmaf(z, g.z, fg[2]);
-                    if constexpr (!ZETA) {
-                        const float4 v = stage[warp][buf][j].v;
-                        fv[0] = fmaf(z, v.x, fv[0]);
-                        fv[1] = fmaf(z, v.y, fv[1]);
-                        fv[2] = fmaf(z, v.z, fv[2]);
-                    }
-                }
-#pragma unroll
-                for (int k = 0; k < 3; k++) {
-                    comp_add(sg[k], cg[k], fg[k]);
-                    if constexpr (!ZETA) comp_add(sv[k], cv[k], fv[k]);
-                }
+                for (int k = 0; k < (ZETA ? 2 : 3); k++) comp_add2(sm[k], cm[k], f[k]);
             }
             // skipped tiles add nothing, so only the tiles taken count towards a flush
             if (++in_flush == ESTR_FLUSH_TILES) {
                 in_flush = 0;
-#pragma unroll
-                for (int k = 0; k < 3; k++) {
-                    zg[k] += (double)sg[k] + (double)cg[k];
-                    sg[k] = cg[k] = 0.f;
-                    if constexpr (!ZETA) {
-                        zv[k] += (double)sv[k] + (double)cv[k];
-                        sv[k] = cv[k] = 0.f;
-                    }
-                }
+                estr_flush(sm, cm, zg, zv);
             }
         }
         __syncwarp();   // every lane is done with `buf` before it is refilled
         cur = nxt;
         buf ^= 1;
     }
-#pragma unroll
-    for (int k = 0; k < 3; k++) {
-        zg[k] += (double)sg[k] + (double)cg[k];
-        if constexpr (!ZETA) zv[k] += (double)sv[k] + (double)cv[k];
-    }
+    estr_flush(sm, cm, zg, zv);
     if (!valid) return;
     double o[3];
     if constexpr (ZETA) { o[0] = zg[0]; o[1] = zg[1]; o[2] = zg[2]; }
@@ -438,8 +424,8 @@ static cudaError_t launch_estr_k(const EstrArgs& a, const Workspace& w, int num_
                                                                    a.self, a.transposed, a.SFS, a.ldS, partial,
                                                                    nt_pad);
     } else {
-        SrcEstrDF* src = (SrcEstrDF*)w.src_pack;
-        float4* box = (float4*)(src + ns_pad);   // the tile boxes follow the records
+        EstrTile* src = (EstrTile*)w.src_pack;
+        float4* box = (float4*)(src + ns_pad / EWT);   // the tile boxes follow the tiles
         pack_estr_mixed<K><<<pgrid, pb, 0, st>>>(a.ns, ns_pad, a.xs, a.gs, a.sgs, a.zeta ? nullptr : a.Js, a.ldJs,
                                                   static_s, a.transposed, a.self ? tgt : nullptr, src, box);
         if (a.zeta)

@@ -4,12 +4,80 @@
 // below FP32 resolution past a reach (zeta_skip_s, dyn_skip_s), so whole 32-source tiles
 // out of a warp's reach need not be loaded.
 #pragma once
+#include "dyn_math.cuh"
 #include "internal.h"
 #include "vpm_math.cuh"
 
 namespace vpm {
 
 constexpr int EST_TILE = 32;   // particles per tile (one per lane of a warp)
+
+// A tile of sources for the mixed Estr kernels (estr.cu, leaflist.cu), in the form their inner loop
+// reads: coordinates (x, y, z high parts, turned into offsets in place by estr.cu; xl, yl, zl low
+// parts) and w = 1/sigma^2 as arrays, so that one 16-byte broadcast read serves four sources and
+// f32x2 instructions take two of them; and the payload g, v = ZNORM (Gamma, J^T Gamma)/sigma^3 as
+// (gx gy)(gz vx)(vy vz), three f32x2 a source, 24 bytes instead of two float4.
+struct __align__(128) EstrTile {
+    float x[EST_TILE], y[EST_TILE], z[EST_TILE], w[EST_TILE], xl[EST_TILE], yl[EST_TILE], zl[EST_TILE];
+    float2 gv[3 * EST_TILE];
+};
+static_assert(sizeof(EstrTile) == 1664, "whole 16-byte chunks, no padding");
+
+// Payload sums of 8 sources: f[0..2] += z (gx gy)(gz vx)(vy vz) for the weights of r2/s pairs
+// (s = r2/sigma^2).  MASKED: `on` has a bit per source and those without add nothing.
+// ZERO: sources at r2 = 0 may be among them, which add nothing.
+template <int K, bool ZETA, bool DZ, bool MASKED, bool ZERO>
+__device__ __forceinline__ void estr_add8(const f32x2 (&r2)[4], const f32x2 (&s)[4], const float2* gv, unsigned on,
+                                          float3 fd, f32x2 (&f)[3])
+{
+    const ulonglong2* p = (const ulonglong2*)gv;
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        float s0, s1;
+        upk(s[q], s0, s1);
+        float z0 = zhat_f32<K>(s0), z1 = zhat_f32<K>(s1);
+        if constexpr (DZ) { z0 *= zeta_ratio_m1<K>(s0, fd); z1 *= zeta_ratio_m1<K>(s1, fd); }
+        if constexpr (MASKED) {
+            z0 = (on >> (2 * q)) & 1u ? z0 : 0.0f;
+            z1 = (on >> (2 * q + 1)) & 1u ? z1 : 0.0f;
+        }
+        if constexpr (ZERO) {
+            float a, b;
+            upk(r2[q], a, b);
+            z0 = a == 0.0f ? 0.0f : z0;
+            z1 = b == 0.0f ? 0.0f : z1;
+        }
+        const ulonglong2 a = p[3 * q], b = p[3 * q + 1], c = p[3 * q + 2];
+        const f32x2 Z0 = pk(z0, z0), Z1 = pk(z1, z1);
+        f[0] = fma2(Z0, a.x, f[0]);
+        f[1] = fma2(Z0, a.y, f[1]);
+        if constexpr (!ZETA) f[2] = fma2(Z0, b.x, f[2]);
+        f[0] = fma2(Z1, b.y, f[0]);
+        f[1] = fma2(Z1, c.x, f[1]);
+        if constexpr (!ZETA) f[2] = fma2(Z1, c.y, f[2]);
+    }
+}
+
+// The compensated sums sm + cm, added to FP64.  A branch of its own (the warp barriers): as a
+// predicated block in the tile loop its FP64 instructions took their turn in the FP64 pipe for every
+// tile (24 % busy).
+__device__ __forceinline__ void estr_flush(f32x2 (&sm)[3], f32x2 (&cm)[3], double (&zg)[3], double (&zv)[3])
+{
+    __syncwarp();
+    float a[6], c[6];
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        upk(sm[k], a[2 * k], a[2 * k + 1]);
+        upk(cm[k], c[2 * k], c[2 * k + 1]);
+        sm[k] = cm[k] = 0ull;
+    }
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+        zg[k] += (double)a[k] + (double)c[k];
+        zv[k] += (double)a[3 + k] + (double)c[3 + k];
+    }
+    __syncwarp();
+}
 
 // The box of every 32-source tile of a pack of ns_pad sources (ns real ones): for tile i,
 // box[2 i] = (min x, min y, min z, min 1/sigma^2) and box[2 i + 1] = (max x, max y, max z, 0)

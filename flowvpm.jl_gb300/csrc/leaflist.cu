@@ -16,6 +16,7 @@
 // formula for FP64); Estr uses the factored form of estr.cu with the self
 // pair excluded by position.
 #include "dyn_math.cuh"
+#include "estr_tiles.cuh"
 #include "internal.h"
 #include "uj_pair.cuh"
 #include "vpm_math.cuh"
@@ -25,7 +26,7 @@ namespace vpm {
 constexpr int NF_WARPS = 4;                  // warp groups per block
 constexpr int NF_THREADS = 32 * NF_WARPS;
 constexpr int NF_BLK_TILES = 2;              // 32-source tiles summed in FP32 per block
-constexpr int NF_ESTR_FLUSH = 8;             // nf_estr: tiles of compensated FP32 sums between FP64 adds
+constexpr int NF_ESTR_FLUSH = 24;            // nf_estr: tiles of compensated FP32 sums between FP64 adds
 constexpr int NF_MIN_BLOCKS = 4;             // resident blocks per SM the UJ kernel is compiled for
 constexpr int NF_MID_BLKS = 4;               // blocks summed in FP32 before the FP64 add
 
@@ -472,10 +473,10 @@ nf_estr(int64_t n, int64_t ngroups, const TgtPos* __restrict__ tgt, const int32_
 {
     static_assert(MIXED || !DZ, "weight differences are FP32-comp only");
     static_assert(!(DZ && ZETA), "one mode at a time");
-    // mixed: per source (x_hi, 1/sigma^2), (x_lo, target mask), g, v;  FP64: the packed source.  The
-    // kernel is bound by these loads, broadcast reads of every source by every lane (73 % of the
-    // shared-memory rate with the masks in an array of their own).
-    __shared__ __align__(16) float4 mtile[MIXED ? NF_WARPS : 1][4][32];
+    // mixed: the sources as in the all-pairs kernel (estr.cu), two to an f32x2 instruction, without a
+    // look at the masks where the group's targets all take all eight sources (jet of 2^20 with the
+    // list build and UJ: 22.05 -> 21.34 ms);  FP64: the packed source
+    __shared__ EstrTile mtile[MIXED ? NF_WARPS : 1];
     __shared__ SrcEstrF64 dtile[MIXED ? 1 : NF_WARPS][32];
     __shared__ int spos[NF_WARPS][32];                          // source position, -1 for padding
     __shared__ unsigned tmask[NF_WARPS][32];
@@ -498,7 +499,27 @@ nf_estr(int64_t n, int64_t ngroups, const TgtPos* __restrict__ tgt, const int32_
     double zg[3] = {0.0, 0.0, 0.0}, zv[3] = {0.0, 0.0, 0.0};
     // mixed: compensated FP32 sums of 8-source partial sums (comp_add), FP64 every NF_ESTR_FLUSH tiles
     // (as the all-pairs mixed Estr; the FP64 pipe runs at 1/64 of the FP32 rate)
-    float sg[3] = {0.f, 0.f, 0.f}, cg[3] = {0.f, 0.f, 0.f}, sv[3] = {0.f, 0.f, 0.f}, cv[3] = {0.f, 0.f, 0.f};
+    f32x2 sm[3] = {0ull, 0ull, 0ull}, cm[3] = {0ull, 0ull, 0ull};
+    const f32x2 HX = pk(-th.x, -th.x), HY = pk(-th.y, -th.y), HZ = pk(-th.z, -th.z);
+    const f32x2 LX = pk(-tl.x, -tl.x), LY = pk(-tl.y, -tl.y), LZ = pk(-tl.z, -tl.z);
+    const unsigned all = __reduce_or_sync(0xffffffffu, bit);   // the group's live leaves
+    // box of the group's targets (high parts): sources out of its reach are skipped as in the
+    // all-pairs kernel, and only those inside it can be at r = 0 from a target
+    __shared__ float4 gbox[MIXED ? NF_WARPS : 1][2];
+    if constexpr (MIXED) {
+        float3 lo = th, hi = th;
+#pragma unroll
+        for (int m = 16; m > 0; m >>= 1) {
+            lo.x = fminf(lo.x, __shfl_xor_sync(0xffffffffu, lo.x, m)); hi.x = fmaxf(hi.x, __shfl_xor_sync(0xffffffffu, hi.x, m));
+            lo.y = fminf(lo.y, __shfl_xor_sync(0xffffffffu, lo.y, m)); hi.y = fmaxf(hi.y, __shfl_xor_sync(0xffffffffu, hi.y, m));
+            lo.z = fminf(lo.z, __shfl_xor_sync(0xffffffffu, lo.z, m)); hi.z = fmaxf(hi.z, __shfl_xor_sync(0xffffffffu, hi.z, m));
+        }
+        if (lane == 0) {
+            gbox[warp][0] = make_float4(lo.x, lo.y, lo.z, 0.f);
+            gbox[warp][1] = make_float4(hi.x, hi.y, hi.z, 0.f);
+        }
+        __syncwarp();
+    }
     int tiles = 0;
     PartTurn part;
     IntervalWalk walk;
@@ -510,19 +531,29 @@ nf_estr(int64_t n, int64_t ngroups, const TgtPos* __restrict__ tgt, const int32_
         if (cnt == 0) break;
         if (!part.mine()) continue;
         __syncwarp();
+        unsigned beyond = 0u, inside = 0u;
         if constexpr (MIXED) {
+            EstrTile& q = mtile[warp];
+            SrcEstrDF p;
             if (sp >= 0) {
-                const SrcEstrDF p = ((const SrcEstrDF*)srcv)[sp];
-                mtile[warp][0][lane] = p.a;
-                mtile[warp][1][lane] = make_float4(p.b.x, p.b.y, p.b.z, __uint_as_float(smask));
-                mtile[warp][2][lane] = p.g;
-                mtile[warp][3][lane] = p.v;
-            } else {   // padding: far away, no payload (read by the unrolled sub-blocks with mask 0)
-                mtile[warp][0][lane] = make_float4(1.0e6f, 1.0e6f, 1.0e6f, 1.f);
-                mtile[warp][1][lane] = make_float4(0.f, 0.f, 0.f, __uint_as_float(smask));
-                mtile[warp][2][lane] = make_float4(0.f, 0.f, 0.f, 0.f);
-                mtile[warp][3][lane] = make_float4(0.f, 0.f, 0.f, 0.f);
+                p = ((const SrcEstrDF*)srcv)[sp];
+            } else {   // padding: far away, no payload, mask 0
+                p.a = make_float4(1.0e6f, 1.0e6f, 1.0e6f, 1.f);
+                p.b = p.g = p.v = make_float4(0.f, 0.f, 0.f, 0.f);
             }
+            q.x[lane] = p.a.x; q.y[lane] = p.a.y; q.z[lane] = p.a.z; q.w[lane] = p.a.w;
+            q.xl[lane] = p.b.x; q.yl[lane] = p.b.y; q.zl[lane] = p.b.z;
+            q.gv[3 * lane] = make_float2(p.g.x, p.g.y);
+            q.gv[3 * lane + 1] = make_float2(p.g.z, p.v.x);
+            q.gv[3 * lane + 2] = make_float2(p.v.y, p.v.z);
+            tmask[warp][lane] = smask;
+            const float4 lo = gbox[warp][0], hi = gbox[warp][1];
+            const float ex = fmaxf(fmaxf(lo.x - p.a.x, p.a.x - hi.x), 0.0f);
+            const float ey = fmaxf(fmaxf(lo.y - p.a.y, p.a.y - hi.y), 0.0f);
+            const float ez = fmaxf(fmaxf(lo.z - p.a.z, p.a.z - hi.z), 0.0f);
+            const float d2 = fmaf(ex, ex, fmaf(ey, ey, ez * ez));
+            beyond = __ballot_sync(0xffffffffu, zeta_skip_s<K>() > 0.0f && d2 * p.a.w > zeta_skip_s<K>());
+            inside = __ballot_sync(0xffffffffu, !(d2 > 0.0f));
         } else {
             if (sp >= 0) dtile[warp][lane] = ((const SrcEstrF64*)srcv)[sp];
         }
@@ -532,38 +563,42 @@ nf_estr(int64_t n, int64_t ngroups, const TgtPos* __restrict__ tgt, const int32_
         }
         __syncwarp();
         if constexpr (MIXED) {
+            const EstrTile& q = mtile[warp];
+            const unsigned whole = __ballot_sync(0xffffffffu, (smask & all) == all);   // sources of every target
             for (int j0 = 0; j0 < cnt; j0 += 8) {   // cnt <= 32: j0 + 7 stays in the tile (padding has mask 0)
-                float fg[3] = {0.f, 0.f, 0.f}, fv[3] = {0.f, 0.f, 0.f};
+                if (((beyond >> j0) & 0xffu) == 0xffu) continue;
+                f32x2 r2[4], s[4], f[3] = {0ull, 0ull, 0ull};
 #pragma unroll
-                for (int j = j0; j < j0 + 8; j++) {
-                    const float4 h = mtile[warp][0][j], l = mtile[warp][1][j];
-                    const float dx = (th.x - h.x) + (tl.x - l.x);
-                    const float dy = (th.y - h.y) + (tl.y - l.y);
-                    const float dz = (th.z - h.z) + (tl.z - l.z);
-                    const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-                    float z = zhat_f32<K>(r2 * h.w);
-                    if constexpr (DZ) z *= zeta_ratio_m1<K>(r2 * h.w, fd);
-                    // pairs at r = 0 are skipped (ZETA: kept, the self pair included)
-                    const bool on = (__float_as_uint(l.w) & bit) != 0u && (ZETA || r2 != 0.0f);
-                    z = on ? z : 0.0f;
-                    const float4 g = mtile[warp][2][j];
-                    fg[0] = fmaf(z, g.x, fg[0]); fg[1] = fmaf(z, g.y, fg[1]); fg[2] = fmaf(z, g.z, fg[2]);
-                    if constexpr (!ZETA) {
-                        const float4 v = mtile[warp][3][j];
-                        fv[0] = fmaf(z, v.x, fv[0]); fv[1] = fmaf(z, v.y, fv[1]); fv[2] = fmaf(z, v.z, fv[2]);
-                    }
+                for (int c = 0; c < 2; c++) {
+                    const int j = j0 + 4 * c;
+                    const ulonglong2 X = *(const ulonglong2*)&q.x[j], Y = *(const ulonglong2*)&q.y[j],
+                                     Z = *(const ulonglong2*)&q.z[j], W = *(const ulonglong2*)&q.w[j],
+                                     XL = *(const ulonglong2*)&q.xl[j], YL = *(const ulonglong2*)&q.yl[j],
+                                     ZL = *(const ulonglong2*)&q.zl[j];
+                    f32x2 dx = add2(add2(X.x, HX), add2(XL.x, LX)), dy = add2(add2(Y.x, HY), add2(YL.x, LY)),
+                          dz = add2(add2(Z.x, HZ), add2(ZL.x, LZ));
+                    r2[2 * c] = fma2(dx, dx, fma2(dy, dy, mul2(dz, dz)));
+                    s[2 * c] = mul2(r2[2 * c], W.x);
+                    dx = add2(add2(X.y, HX), add2(XL.y, LX)); dy = add2(add2(Y.y, HY), add2(YL.y, LY));
+                    dz = add2(add2(Z.y, HZ), add2(ZL.y, LZ));
+                    r2[2 * c + 1] = fma2(dx, dx, fma2(dy, dy, mul2(dz, dz)));
+                    s[2 * c + 1] = mul2(r2[2 * c + 1], W.y);
+                }
+                if (zeta_skip_s<K>() > 0.0f && __all_sync(0xffffffffu, min8_nan(s) > zeta_skip_s<K>())) continue;
+                if (((whole >> j0) & 0xffu) == 0xffu && (ZETA || !((inside >> j0) & 0xffu))) {
+                    estr_add8<K, ZETA, DZ, false, false>(r2, s, &q.gv[3 * j0], 0u, fd, f);
+                } else {
+                    unsigned on = 0u;
+#pragma unroll
+                    for (int j = 0; j < 8; j++) on |= (tmask[warp][j0 + j] & bit) ? 1u << j : 0u;
+                    estr_add8<K, ZETA, DZ, true, !ZETA>(r2, s, &q.gv[3 * j0], on, fd, f);
                 }
 #pragma unroll
-                for (int k = 0; k < 3; k++) { comp_add(sg[k], cg[k], fg[k]); comp_add(sv[k], cv[k], fv[k]); }
+                for (int k = 0; k < (ZETA ? 2 : 3); k++) comp_add2(sm[k], cm[k], f[k]);
             }
             if (++tiles == NF_ESTR_FLUSH) {
                 tiles = 0;
-#pragma unroll
-                for (int k = 0; k < 3; k++) {
-                    zg[k] += (double)sg[k] + (double)cg[k];
-                    zv[k] += (double)sv[k] + (double)cv[k];
-                    sg[k] = cg[k] = sv[k] = cv[k] = 0.f;
-                }
+                estr_flush(sm, cm, zg, zv);
             }
         } else {
             for (int j = 0; j < cnt; j++) {
@@ -578,10 +613,7 @@ nf_estr(int64_t n, int64_t ngroups, const TgtPos* __restrict__ tgt, const int32_
             }
         }
     }
-    if constexpr (MIXED) {
-#pragma unroll
-        for (int k = 0; k < 3; k++) { zg[k] += (double)sg[k] + (double)cg[k]; zv[k] += (double)sv[k] + (double)cv[k]; }
-    }
+    if constexpr (MIXED) estr_flush(sm, cm, zg, zv);
     if (!live && !(partial && me.valid)) return;
     double o[3] = {0.0, 0.0, 0.0};
     if constexpr (ZETA) {

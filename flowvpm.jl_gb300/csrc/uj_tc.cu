@@ -197,26 +197,6 @@ pack_tiles(int64_t n, const double* __restrict__ gs, const double* __restrict__ 
 }
 
 // ---------------------------------------------------------- packed FP32 pairs
-typedef unsigned long long f32x2;
-__device__ __forceinline__ f32x2 pk(float a, float b)
-{
-    f32x2 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-    return r;
-}
-__device__ __forceinline__ void upk(f32x2 v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
-__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c)
-{
-    f32x2 r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b)
-{
-    f32x2 r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
 // hi = the two values as f16x2; nlo = minus their remainders as f16x2
 __device__ __forceinline__ void split2(f32x2 v, uint32_t& hi, uint32_t& nlo)
 {

@@ -417,6 +417,46 @@ __device__ __forceinline__ float df_offset(float a, float b, float oh, float ol)
     return s + (e + (b - ol));
 }
 
+// ---------------------------------------------------------- packed FP32 pairs
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pk(float a, float b)
+{
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void upk(f32x2 v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c)
+{
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b)
+{
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b)
+{
+    f32x2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 sub2(f32x2 a, f32x2 b) { return fma2(b, pk(-1.f, -1.f), a); }
+// the least of the eight (a NaN if one is)
+__device__ __forceinline__ float min8_nan(const f32x2 (&v)[4])
+{
+    float a[8], r;
+#pragma unroll
+    for (int k = 0; k < 4; k++) upk(v[k], a[2 * k], a[2 * k + 1]);
+    asm("{\n\t.reg .f32 t;\n\tmin.NaN.f32 t, %1, %2, %3;\n\tmin.NaN.f32 t, t, %4, %5;\n\t"
+        "min.NaN.f32 t, t, %6, %7;\n\tmin.NaN.f32 %0, t, %8;\n\t}"
+        : "=f"(r) : "f"(a[0]), "f"(a[1]), "f"(a[2]), "f"(a[3]), "f"(a[4]), "f"(a[5]), "f"(a[6]), "f"(a[7]));
+    return r;
+}
+
 // s += y, with the rounding error of the addition accumulated in c (Fast2Sum;
 // exact when |s| >= |y|, which a running sum of like terms keeps after its
 // first additions).  s + c is the compensated sum.
@@ -424,6 +464,12 @@ __device__ __forceinline__ void comp_add(float& s, float& c, float y)
 {
     const float t = s + y;
     c += (s - t) + y;
+    s = t;
+}
+__device__ __forceinline__ void comp_add2(f32x2& s, f32x2& c, f32x2 y)
+{
+    const f32x2 t = add2(s, y);
+    c = add2(c, add2(sub2(s, t), y));
     s = t;
 }
 
