@@ -366,9 +366,9 @@ estr_mixed_kernel(int64_t nt, const TgtPos* __restrict__ tgt, const double* __re
                 if (zeta_skip_s<K>() > 0.0f && __all_sync(0xffffffffu, min8_nan(s) > zeta_skip_s<K>())) continue;
                 f32x2 f[3] = {0ull, 0ull, 0ull};
                 if (!ZETA && ((inside >> sub) & 0xffu))
-                    estr_add8<K, ZETA, DZ, false, !ZETA>(r2, s, &T.gv[3 * sub], 0u, fd, f);
+                    estr_add8<K, ZETA, DZ, false, !ZETA>(r2, s, &T.gv[3 * sub], 0u, nullptr, fd, f);
                 else
-                    estr_add8<K, ZETA, DZ, false, false>(r2, s, &T.gv[3 * sub], 0u, fd, f);
+                    estr_add8<K, ZETA, DZ, false, false>(r2, s, &T.gv[3 * sub], 0u, nullptr, fd, f);
 #pragma unroll
                 for (int k = 0; k < (ZETA ? 2 : 3); k++) comp_add2(sm[k], cm[k], f[k]);
             }

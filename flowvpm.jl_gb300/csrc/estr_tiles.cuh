@@ -24,11 +24,11 @@ struct __align__(128) EstrTile {
 static_assert(sizeof(EstrTile) == 1664, "whole 16-byte chunks, no padding");
 
 // Payload sums of 8 sources: f[0..2] += z (gx gy)(gz vx)(vy vz) for the weights of r2/s pairs
-// (s = r2/sigma^2).  MASKED: `on` has a bit per source and those without add nothing.
+// (s = r2/sigma^2).  MASKED: sources whose target mask (`mask`) lacks `bit` add nothing.
 // ZERO: sources at r2 = 0 may be among them, which add nothing.
 template <int K, bool ZETA, bool DZ, bool MASKED, bool ZERO>
-__device__ __forceinline__ void estr_add8(const f32x2 (&r2)[4], const f32x2 (&s)[4], const float2* gv, unsigned on,
-                                          float3 fd, f32x2 (&f)[3])
+__device__ __forceinline__ void estr_add8(const f32x2 (&r2)[4], const f32x2 (&s)[4], const float2* gv, unsigned bit,
+                                          const uint4* mask, float3 fd, f32x2 (&f)[3])
 {
     const ulonglong2* p = (const ulonglong2*)gv;
 #pragma unroll
@@ -38,8 +38,9 @@ __device__ __forceinline__ void estr_add8(const f32x2 (&r2)[4], const f32x2 (&s)
         float z0 = zhat_f32<K>(s0), z1 = zhat_f32<K>(s1);
         if constexpr (DZ) { z0 *= zeta_ratio_m1<K>(s0, fd); z1 *= zeta_ratio_m1<K>(s1, fd); }
         if constexpr (MASKED) {
-            z0 = (on >> (2 * q)) & 1u ? z0 : 0.0f;
-            z1 = (on >> (2 * q + 1)) & 1u ? z1 : 0.0f;
+            const uint4 m = mask[q >> 1];
+            z0 = (q & 1 ? m.z : m.x) & bit ? z0 : 0.0f;
+            z1 = (q & 1 ? m.w : m.y) & bit ? z1 : 0.0f;
         }
         if constexpr (ZERO) {
             float a, b;

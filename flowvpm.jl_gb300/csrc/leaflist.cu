@@ -27,7 +27,9 @@ constexpr int NF_WARPS = 4;                  // warp groups per block
 constexpr int NF_THREADS = 32 * NF_WARPS;
 constexpr int NF_BLK_TILES = 2;              // 32-source tiles summed in FP32 per block
 constexpr int NF_ESTR_FLUSH = 24;            // nf_estr: tiles of compensated FP32 sums between FP64 adds
-constexpr int NF_MIN_BLOCKS = 4;             // resident blocks per SM the UJ kernel is compiled for
+// Resident blocks per SM the UJ kernel is compiled for; a fifth hides the Gaussian kernel's divergent
+// branches (jet of 200,000: 4.05 -> 3.85 ms) and gains nothing elsewhere.
+constexpr int nf_min_blocks(int kernel) { return kernel == K_GAUS ? 5 : 4; }
 constexpr int NF_MID_BLKS = 4;               // blocks summed in FP32 before the FP64 add
 
 __global__ void tgt_from_perm(int64_t n, const double* __restrict__ x, const int32_t* __restrict__ perm,
@@ -238,46 +240,93 @@ __global__ void leaf_pack_lane(int64_t n, const double* __restrict__ x, const do
     out[o] = p;
 }
 
-// Sources from leaf_pack_lane: 1/sigma^2 in a.w and the near form's 1/sigma^3 in gam, so
-// that a pair takes neither (pair4_mixed with SCALED).
+// A tile of nf_uj_mixed: minus the positions (nx, ny, nz + their low parts), w = 1/sigma^2, the
+// strength and its negative (f32x2 instructions have no subtraction), as arrays, so that a 16-byte
+// broadcast read serves four sources and an f32x2 instruction takes two.
+struct __align__(16) UjTile {
+    float nx[32], ny[32], nz[32], w[32], nxl[32], nyl[32], nzl[32];
+    float g[3][32], ng[3][32];
+    unsigned mask[32];
+};
+
+// Box of a warp's targets (FP32 high parts), by its lane 0 to box[0..1].
+__device__ __forceinline__ void target_box(const float3& th, int lane, float4* box)
+{
+    float3 lo = th, hi = th;
+#pragma unroll
+    for (int m = 16; m > 0; m >>= 1) {
+        lo.x = fminf(lo.x, __shfl_xor_sync(0xffffffffu, lo.x, m)); hi.x = fmaxf(hi.x, __shfl_xor_sync(0xffffffffu, hi.x, m));
+        lo.y = fminf(lo.y, __shfl_xor_sync(0xffffffffu, lo.y, m)); hi.y = fmaxf(hi.y, __shfl_xor_sync(0xffffffffu, hi.y, m));
+        lo.z = fminf(lo.z, __shfl_xor_sync(0xffffffffu, lo.z, m)); hi.z = fmaxf(hi.z, __shfl_xor_sync(0xffffffffu, hi.z, m));
+    }
+    if (lane == 0) {
+        box[0] = make_float4(lo.x, lo.y, lo.z, 0.f);
+        box[1] = make_float4(hi.x, hi.y, hi.z, 0.f);
+    }
+    __syncwarp();
+}
+
+// Squared distance of a source (high parts) from that box; 0 (or NaN) inside.
+__device__ __forceinline__ float box_d2(const float4* box, float x, float y, float z)
+{
+    const float4 lo = box[0], hi = box[1];
+    const float ex = fmaxf(fmaxf(lo.x - x, x - hi.x), 0.0f);
+    const float ey = fmaxf(fmaxf(lo.y - y, y - hi.y), 0.0f);
+    const float ez = fmaxf(fmaxf(lo.z - z, z - hi.z), 0.0f);
+    return fmaf(ex, ex, fmaf(ey, ey, ez * ez));
+}
+
+// The two halves of an f32x2 sum.
+__device__ __forceinline__ float halves(f32x2 v)
+{
+    float a, b;
+    upk(v, a, b);
+    return a + b;
+}
+
+// Sums of four sources at a time, two to an instruction.  Masks and r = 0 are looked at only in
+// groups of four where a source does not act on all of the group's targets or lies inside their
+// box, the series form of Gaussian-erf (s < 2) only where one is that near to the box.
+// Bound: the FMA pipe; f32x2 instructions with three distinct operands take about 2.4 of its cycles
+// (62 % busy at 2), and the issue slots fell from 82 % to 56 %.  Kernel at jet 2^20 10.0 -> 9.3 ms
+// against one source at a time with masks, r = 0 and form looked at in every pair; errors 0.65
+// times as large, each half being a sum of its own.  Tried: offsets from the group's first target
+// for sources far enough away (3 operations instead of 9 for a displacement): 4 % slower, few are.
 template <int K>
-__global__ void __launch_bounds__(NF_THREADS, NF_MIN_BLOCKS)
+__global__ void __launch_bounds__(NF_THREADS, nf_min_blocks(K))
 nf_uj_mixed(int64_t n, int64_t ngroups, const TgtPos* __restrict__ tgt, const int32_t* __restrict__ leaf_of,
             const int32_t* __restrict__ grp_row, const int4* __restrict__ ivs, const SrcMixed* __restrict__ src,
             double* U, double* J, double* __restrict__ partial, int64_t n_pad)
 {
-    __shared__ SrcMixed tile[NF_WARPS][32];
-    __shared__ float4 off[NF_WARPS][32];
+    __shared__ UjTile tiles_s[NF_WARPS];
+    __shared__ float4 box[NF_WARPS][2];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t grp = (int64_t)blockIdx.x * NF_WARPS + warp;
     if (grp >= ngroups) return;
     const int64_t p0 = 32 * grp;
     const GroupTarget me = group_target(n, p0, lane, tgt, leaf_of);
-    const TgtPos o = tgt[p0];
     const float3 th = make_float3((float)me.tx, (float)me.ty, (float)me.tz);
     const float3 tl = make_float3((float)(me.tx - (double)th.x), (float)(me.ty - (double)th.y),
                                   (float)(me.tz - (double)th.z));
-    const float3 oh = make_float3((float)o.x, (float)o.y, (float)o.z);
-    const float3 ol = make_float3((float)(o.x - (double)oh.x), (float)(o.y - (double)oh.y), (float)(o.z - (double)oh.z));
-    const float3 to = make_float3((float)(me.tx - o.x), (float)(me.ty - o.y), (float)(me.tz - o.z));
-    float b2 = fmaf(to.x, to.x, fmaf(to.y, to.y, to.z * to.z));
-#pragma unroll
-    for (int m = 16; m > 0; m >>= 1) b2 = fmaxf(b2, __shfl_xor_sync(0xffffffffu, b2, m));
-    const float r2n = fmaxf(4.0f * b2, 1.0e-30f);
+    target_box(th, lane, box[warp]);
+    const unsigned all = __reduce_or_sync(0xffffffffu, me.bit);
+    const f32x2 HX = pk(th.x, th.x), HY = pk(th.y, th.y), HZ = pk(th.z, th.z);
+    const f32x2 LX = pk(tl.x, tl.x), LY = pk(tl.y, tl.y), LZ = pk(tl.z, tl.z);
 
-    // FP64 sums of this lane in shared memory ([0..2] U, [3..5] W, [6..13] J'), touched once per
-    // NF_MID_BLKS blocks: the registers go to occupancy instead
+    // sums of this lane ([0..2] U, [3..5] W, [6..13] J'): FP32 over NF_BLK_TILES tiles in registers,
+    // FP32 over NF_MID_BLKS of those and FP64 in shared memory
     __shared__ double acc64[14][NF_THREADS];
+    __shared__ float mid[14][NF_THREADS];
 #pragma unroll
-    for (int k = 0; k < 14; k++) acc64[k][threadIdx.x] = 0.0;
-    float mu[3] = {0.f, 0.f, 0.f}, mw[3] = {0.f, 0.f, 0.f}, mj[8];
-    float u[3] = {0.f, 0.f, 0.f}, w[3] = {0.f, 0.f, 0.f}, jq[8];
+    for (int k = 0; k < 14; k++) { acc64[k][threadIdx.x] = 0.0; mid[k][threadIdx.x] = 0.f; }
+    f32x2 a[14];
 #pragma unroll
-    for (int k = 0; k < 8; k++) { mj[k] = 0.f; jq[k] = 0.f; }
+    for (int k = 0; k < 14; k++) a[k] = 0ull;
     int tiles = 0, blks = 0;
     PartTurn part;
     IntervalWalk walk;
     walk.init(ivs, grp_row[grp], grp_row[grp + 1], lane);
+    UjTile& T = tiles_s[warp];
     for (;;) {
         int sp;
         unsigned smask;
@@ -289,45 +338,100 @@ nf_uj_mixed(int64_t n, int64_t ngroups, const TgtPos* __restrict__ tgt, const in
             sj = src[sp];
         } else {   // padding: far away, no strength, no target
             sj.a = make_float4(1.0e6f, 1.0e6f, 1.0e6f, 1.f);
-            sj.b = make_float4(0.f, 0.f, 0.f, 1.f);
-            sj.gam = make_float4(0.f, 0.f, 0.f, 0.f);
+            sj.b = sj.gam = make_float4(0.f, 0.f, 0.f, 0.f);
         }
-        sj.gam.w = __uint_as_float(smask);
         __syncwarp();
-        tile[warp][lane] = sj;
-        off[warp][lane] = make_float4((sj.a.x - oh.x) + (sj.b.x - ol.x), (sj.a.y - oh.y) + (sj.b.y - ol.y),
-                                      (sj.a.z - oh.z) + (sj.b.z - ol.z), sj.a.w);
+        T.nx[lane] = -sj.a.x; T.ny[lane] = -sj.a.y; T.nz[lane] = -sj.a.z; T.w[lane] = sj.a.w;
+        T.nxl[lane] = -sj.b.x; T.nyl[lane] = -sj.b.y; T.nzl[lane] = -sj.b.z;
+        T.g[0][lane] = sj.gam.x; T.g[1][lane] = sj.gam.y; T.g[2][lane] = sj.gam.z;
+        T.ng[0][lane] = -sj.gam.x; T.ng[1][lane] = -sj.gam.y; T.ng[2][lane] = -sj.gam.z;
+        T.mask[lane] = smask;
+        const float d2 = box_d2(box[warp], sj.a.x, sj.a.y, sj.a.z);
+        const unsigned care = __ballot_sync(0xffffffffu, !(d2 > 0.0f) || (smask & all) != all);
+        const unsigned close = __ballot_sync(0xffffffffu, !(d2 * sj.a.w > 2.5f));   // 2, and room for the low parts
         __syncwarp();
-        const int ng = (cnt + 3) >> 2;
-        for (int q = 0; q < ng; q++)
-            pair4_mixed<K, true, false, true>(to, th, tl, r2n, off[warp], tile[warp], 4 * q, u, jq, w, me.bit);
+#pragma unroll 1
+        for (int j = 0; j < cnt; j += 4) {   // cnt <= 32: j + 3 stays in the tile
+            const bool series = ((close >> j) & 0xfu) != 0u;
+            f32x2 dx[2], dy[2], dz[2], r2[2], G[2], Q[2];
+            {
+                const ulonglong2 X = *(const ulonglong2*)&T.nx[j], Y = *(const ulonglong2*)&T.ny[j],
+                                 Z = *(const ulonglong2*)&T.nz[j], XL = *(const ulonglong2*)&T.nxl[j],
+                                 YL = *(const ulonglong2*)&T.nyl[j], ZL = *(const ulonglong2*)&T.nzl[j],
+                                 W = *(const ulonglong2*)&T.w[j];
+#pragma unroll
+                for (int q = 0; q < 2; q++) {
+                    dx[q] = add2(add2(HX, q ? X.y : X.x), add2(LX, q ? XL.y : XL.x));
+                    dy[q] = add2(add2(HY, q ? Y.y : Y.x), add2(LY, q ? YL.y : YL.x));
+                    dz[q] = add2(add2(HZ, q ? Z.y : Z.x), add2(LZ, q ? ZL.y : ZL.x));
+                    r2[q] = fma2(dx[q], dx[q], fma2(dy[q], dy[q], mul2(dz[q], dz[q])));
+                }
+                const f32x2 w[2] = {W.x, W.y}, s[2] = {mul2(r2[0], W.x), mul2(r2[1], W.y)};
+                near_GQ2<K, 2>(s, w, series, G, Q);
+            }
+            if ((care >> j) & 0xfu) {
+                const uint4 m = *(const uint4*)&T.mask[j];
+#pragma unroll
+                for (int q = 0; q < 2; q++) {
+                    float r0, r1, g0, g1, q0, q1;
+                    upk(r2[q], r0, r1);
+                    upk(G[q], g0, g1);
+                    upk(Q[q], q0, q1);
+                    const bool on0 = r0 > 0.0f && ((q ? m.z : m.x) & me.bit), on1 = r1 > 0.0f && ((q ? m.w : m.y) & me.bit);
+                    G[q] = pk(on0 ? g0 : 0.f, on1 ? g1 : 0.f);
+                    Q[q] = pk(on0 ? q0 : 0.f, on1 ? q1 : 0.f);
+                }
+            }
+            const ulonglong2 GX = *(const ulonglong2*)&T.g[0][j], GY = *(const ulonglong2*)&T.g[1][j],
+                             GZ = *(const ulonglong2*)&T.g[2][j], NX = *(const ulonglong2*)&T.ng[0][j],
+                             NY = *(const ulonglong2*)&T.ng[1][j], NZ = *(const ulonglong2*)&T.ng[2][j];
+#pragma unroll
+            for (int q = 0; q < 2; q++) {   // accum_pair
+                const f32x2 gx = q ? GX.y : GX.x, gy = q ? GY.y : GY.x, gz = q ? GZ.y : GZ.x;
+                const f32x2 cx = fma2(dy[q], gz, mul2(dz[q], q ? NY.y : NY.x));
+                const f32x2 cy = fma2(dz[q], gx, mul2(dx[q], q ? NZ.y : NZ.x));
+                const f32x2 cz = fma2(dx[q], gy, mul2(dy[q], q ? NX.y : NX.x));
+                a[0] = fma2(G[q], cx, a[0]);
+                a[1] = fma2(G[q], cy, a[1]);
+                a[2] = fma2(G[q], cz, a[2]);
+                a[3] = fma2(G[q], gx, a[3]);
+                a[4] = fma2(G[q], gy, a[4]);
+                a[5] = fma2(G[q], gz, a[5]);
+                const f32x2 bx = mul2(Q[q], cx), by = mul2(Q[q], cy), bz = mul2(Q[q], cz);
+                a[6] = fma2(bx, dx[q], a[6]);
+                a[7] = fma2(by, dx[q], a[7]);
+                a[8] = fma2(bz, dx[q], a[8]);
+                a[9] = fma2(bx, dy[q], a[9]);
+                a[10] = fma2(by, dy[q], a[10]);
+                a[11] = fma2(bz, dy[q], a[11]);
+                a[12] = fma2(bx, dz[q], a[12]);
+                a[13] = fma2(by, dz[q], a[13]);
+            }
+        }
         if (++tiles == NF_BLK_TILES) {
             tiles = 0;
+            __syncwarp();   // these flushes are branches of their own, not predicated
+            const bool up = ++blks == NF_MID_BLKS;
 #pragma unroll
-            for (int k = 0; k < 3; k++) { mu[k] += u[k]; mw[k] += w[k]; u[k] = 0.f; w[k] = 0.f; }
-#pragma unroll
-            for (int k = 0; k < 8; k++) { mj[k] += jq[k]; jq[k] = 0.f; }
-            if (++blks == NF_MID_BLKS) {
+            for (int k = 0; k < 14; k++) {
+                mid[k][threadIdx.x] += halves(a[k]);
+                a[k] = 0ull;
+            }
+            if (up) {
                 blks = 0;
+                __syncwarp();
 #pragma unroll
-                for (int k = 0; k < 3; k++) {
-                    acc64[k][threadIdx.x] += (double)mu[k];
-                    acc64[3 + k][threadIdx.x] += (double)mw[k];
-                    mu[k] = 0.f; mw[k] = 0.f;
+                for (int k = 0; k < 14; k++) {
+                    acc64[k][threadIdx.x] += (double)mid[k][threadIdx.x];
+                    mid[k][threadIdx.x] = 0.f;
                 }
-#pragma unroll
-                for (int k = 0; k < 8; k++) { acc64[6 + k][threadIdx.x] += (double)mj[k]; mj[k] = 0.f; }
+                __syncwarp();
             }
         }
     }
     double f[14], acc[12];
 #pragma unroll
-    for (int k = 0; k < 3; k++) {
-        f[k] = acc64[k][threadIdx.x] + ((double)mu[k] + (double)u[k]);
-        f[3 + k] = acc64[3 + k][threadIdx.x] + ((double)mw[k] + (double)w[k]);
-    }
-#pragma unroll
-    for (int k = 0; k < 8; k++) f[6 + k] = acc64[6 + k][threadIdx.x] + ((double)mj[k] + (double)jq[k]);
+    for (int k = 0; k < 14; k++) f[k] = acc64[k][threadIdx.x] + ((double)mid[k][threadIdx.x] + (double)halves(a[k]));
     if (!me.valid) return;
     uj_mixed_finish(f, acc);
     write_uj(p0 + lane, me.idx, acc, U, 3, J, 9, partial, n_pad);
@@ -479,7 +583,7 @@ nf_estr(int64_t n, int64_t ngroups, const TgtPos* __restrict__ tgt, const int32_
     __shared__ EstrTile mtile[MIXED ? NF_WARPS : 1];
     __shared__ SrcEstrF64 dtile[MIXED ? 1 : NF_WARPS][32];
     __shared__ int spos[NF_WARPS][32];                          // source position, -1 for padding
-    __shared__ unsigned tmask[NF_WARPS][32];
+    __shared__ __align__(16) unsigned tmask[NF_WARPS][32];
     __shared__ double T[64];
     if constexpr (!MIXED) {
         exp_table(T);
@@ -506,20 +610,7 @@ nf_estr(int64_t n, int64_t ngroups, const TgtPos* __restrict__ tgt, const int32_
     // box of the group's targets (high parts): sources out of its reach are skipped as in the
     // all-pairs kernel, and only those inside it can be at r = 0 from a target
     __shared__ float4 gbox[MIXED ? NF_WARPS : 1][2];
-    if constexpr (MIXED) {
-        float3 lo = th, hi = th;
-#pragma unroll
-        for (int m = 16; m > 0; m >>= 1) {
-            lo.x = fminf(lo.x, __shfl_xor_sync(0xffffffffu, lo.x, m)); hi.x = fmaxf(hi.x, __shfl_xor_sync(0xffffffffu, hi.x, m));
-            lo.y = fminf(lo.y, __shfl_xor_sync(0xffffffffu, lo.y, m)); hi.y = fmaxf(hi.y, __shfl_xor_sync(0xffffffffu, hi.y, m));
-            lo.z = fminf(lo.z, __shfl_xor_sync(0xffffffffu, lo.z, m)); hi.z = fmaxf(hi.z, __shfl_xor_sync(0xffffffffu, hi.z, m));
-        }
-        if (lane == 0) {
-            gbox[warp][0] = make_float4(lo.x, lo.y, lo.z, 0.f);
-            gbox[warp][1] = make_float4(hi.x, hi.y, hi.z, 0.f);
-        }
-        __syncwarp();
-    }
+    if constexpr (MIXED) target_box(th, lane, gbox[warp]);
     int tiles = 0;
     PartTurn part;
     IntervalWalk walk;
@@ -547,11 +638,7 @@ nf_estr(int64_t n, int64_t ngroups, const TgtPos* __restrict__ tgt, const int32_
             q.gv[3 * lane + 1] = make_float2(p.g.z, p.v.x);
             q.gv[3 * lane + 2] = make_float2(p.v.y, p.v.z);
             tmask[warp][lane] = smask;
-            const float4 lo = gbox[warp][0], hi = gbox[warp][1];
-            const float ex = fmaxf(fmaxf(lo.x - p.a.x, p.a.x - hi.x), 0.0f);
-            const float ey = fmaxf(fmaxf(lo.y - p.a.y, p.a.y - hi.y), 0.0f);
-            const float ez = fmaxf(fmaxf(lo.z - p.a.z, p.a.z - hi.z), 0.0f);
-            const float d2 = fmaf(ex, ex, fmaf(ey, ey, ez * ez));
+            const float d2 = box_d2(gbox[warp], p.a.x, p.a.y, p.a.z);
             beyond = __ballot_sync(0xffffffffu, zeta_skip_s<K>() > 0.0f && d2 * p.a.w > zeta_skip_s<K>());
             inside = __ballot_sync(0xffffffffu, !(d2 > 0.0f));
         } else {
@@ -586,12 +673,11 @@ nf_estr(int64_t n, int64_t ngroups, const TgtPos* __restrict__ tgt, const int32_
                 }
                 if (zeta_skip_s<K>() > 0.0f && __all_sync(0xffffffffu, min8_nan(s) > zeta_skip_s<K>())) continue;
                 if (((whole >> j0) & 0xffu) == 0xffu && (ZETA || !((inside >> j0) & 0xffu))) {
-                    estr_add8<K, ZETA, DZ, false, false>(r2, s, &q.gv[3 * j0], 0u, fd, f);
+                    estr_add8<K, ZETA, DZ, false, false>(r2, s, &q.gv[3 * j0], 0u, nullptr, fd, f);
                 } else {
-                    unsigned on = 0u;
-#pragma unroll
-                    for (int j = 0; j < 8; j++) on |= (tmask[warp][j0 + j] & bit) ? 1u << j : 0u;
-                    estr_add8<K, ZETA, DZ, true, !ZETA>(r2, s, &q.gv[3 * j0], on, fd, f);
+                    const uint4* m = (const uint4*)&tmask[warp][j0];
+                    const uint4 on[2] = {m[0], m[1]};
+                    estr_add8<K, ZETA, DZ, true, !ZETA>(r2, s, &q.gv[3 * j0], bit, on, fd, f);
                 }
 #pragma unroll
                 for (int k = 0; k < (ZETA ? 2 : 3); k++) comp_add2(sm[k], cm[k], f[k]);

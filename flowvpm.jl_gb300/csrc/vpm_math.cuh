@@ -243,6 +243,34 @@ __device__ __forceinline__ void far_GQ(float s, float isig2, float& G, float& Q)
     Q = G * (rs2 * isig2);
 }
 
+// ---------------------------------------------------------- packed FP32 pairs
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pk(float a, float b)
+{
+    f32x2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void upk(f32x2 v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c)
+{
+    f32x2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b)
+{
+    f32x2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b)
+{
+    f32x2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f32x2 sub2(f32x2 a, f32x2 b) { return fma2(b, pk(-1.f, -1.f), a); }
 // G = g/rho^3 of Gaussian-erf for s >= 2 from the erfcx fit, given e = e^{-s/2}, rs = s^-1/2
 __device__ __forceinline__ float gerf_G_erfcx(float s, float e, float rs)
 {
@@ -303,54 +331,6 @@ __device__ __forceinline__ void gerf_GQ(float s, float isig2, float& G, float& Q
     }
 }
 
-// gerf_GQ for four pairs of one lane, with the choice of forms made for the
-// whole warp so that the four pairs' chains interleave: every lane past s = 50
-// (FAR only): the singular form; otherwise the s >= 2 form for all four (valid
-// at any s > 0), replaced by the series, per pair, where s < 2 when any lane
-// of the warp has such a pair.  All 32 lanes must call it.
-template <bool FAR>
-__device__ __forceinline__ void gerf_GQ4(const float (&s)[4], const float (&isig2)[4], float (&G)[4], float (&Q)[4])
-{
-    bool allfar = FAR, anyser = false;
-#pragma unroll
-    for (int q = 0; q < 4; q++) {
-        allfar = allfar && s[q] > S_FAR_GERF;
-        anyser = anyser || s[q] < S_SERIES;
-    }
-    if (FAR && __all_sync(0xffffffffu, allfar)) {
-#pragma unroll
-        for (int q = 0; q < 4; q++) far_GQ(s[q], isig2[q], G[q], Q[q]);
-        return;
-    }
-    float e[4];
-#pragma unroll
-    for (int q = 0; q < 4; q++) {
-        e[q] = fexp2(s[q] * -0.72134752044448170f);
-        const float rs = frsqrt(s[q]);
-        G[q] = gerf_G_erfcx(s[q], e[q], rs);
-        Q[q] = fmaf(F_C2 * -0.33333333333333333f, e[q], G[q]) * (rs * rs) * isig2[q];
-    }
-    if (__any_sync(0xffffffffu, anyser)) {
-#pragma unroll
-        for (int q = 0; q < 4; q++) {
-            float p = 3.1622138893727926e-12f;
-            p = fmaf(p, s[q], 7.273091945557423e-11f);
-            p = fmaf(p, s[q], 1.5273493085670588e-09f);
-            p = fmaf(p, s[q], 2.901963686277412e-08f);
-            p = fmaf(p, s[q], 4.9333382666716e-07f);
-            p = fmaf(p, s[q], 7.4000074000074e-06f);
-            p = fmaf(p, s[q], 9.62000962000962e-05f);
-            p = fmaf(p, s[q], 0.0010582010582010583f);
-            p = fmaf(p, s[q], 0.009523809523809525f);
-            p = fmaf(p, s[q], 0.06666666666666667f);
-            const float ce = F_C2 * e[q];
-            const bool ser = s[q] < S_SERIES;
-            G[q] = ser ? ce * fmaf(s[q], p, 0.33333333333333333f) : G[q];
-            Q[q] = ser ? ce * p * isig2[q] : Q[q];
-        }
-    }
-}
-
 // Full form of kernel K for one lane (any s > 0); FAR as in gerf_GQ.
 template <int K, bool FAR = true>
 __device__ __forceinline__ void near_GQ(float s, float isig2, float& G, float& Q)
@@ -392,15 +372,80 @@ __device__ __forceinline__ void near_GQ(float s, float isig2, float& G, float& Q
     }
 }
 
-// near_GQ for four pairs of one lane; all 32 lanes must call it.
-template <int K, bool FAR = true>
-__device__ __forceinline__ void near_GQ4(const float (&s)[4], const float (&isig2)[4], float (&G)[4], float (&Q)[4])
+// near_GQ of N pairs of f32x2, without the singular branches.  Gaussian-erf: the s >= 2 form (valid at
+// any s > 0), replaced by the series where s < 2 when `series` says that one may be.
+template <int K, int N>
+__device__ __forceinline__ void near_GQ2(const f32x2 (&s)[N], const f32x2 (&isig2)[N], bool series, f32x2 (&G)[N],
+                                         f32x2 (&Q)[N])
 {
+    auto both = [](float v) { return pk(v, v); };
     if constexpr (K == K_GAUSERF) {
-        gerf_GQ4<FAR>(s, isig2, G, Q);
+        constexpr float P[8] = {5.1560079373370265e-06f, -5.998428003101994e-06f, -0.00010125038777505872f,
+                                0.00030713426402493693f, 0.0023330098304451836f, -0.009623567049071946f,
+                                -0.13016216050000662f, -0.5926831417002281f};   // minus gerf_G_erfcx's
+        constexpr float S2[10] = {3.1622138893727926e-12f, 7.273091945557423e-11f, 1.5273493085670588e-09f,
+                                  2.901963686277412e-08f, 4.9333382666716e-07f, 7.4000074000074e-06f,
+                                  9.62000962000962e-05f, 0.0010582010582010583f, 0.009523809523809525f,
+                                  0.06666666666666667f};
+        f32x2 e[N];
+#pragma unroll
+        for (int q = 0; q < N; q++) {
+            float v0, v1;
+            upk(s[q], v0, v1);
+            const f32x2 rs = pk(frsqrt(v0), frsqrt(v1));
+            upk(mul2(s[q], both(-0.72134752044448170f)), v0, v1);
+            e[q] = pk(fexp2(v0), fexp2(v1));
+            const f32x2 rho = mul2(s[q], rs);
+            upk(fma2(rho, both(0.5f), both(1.f)), v0, v1);
+            const f32x2 t = pk(frcp(v0), frcp(v1));
+            const f32x2 w = fma2(t, both(4.77190564267067f), both(-1.795317607111778f));
+            f32x2 p = both(P[0]);
+#pragma unroll
+            for (int k = 1; k < 8; k++) p = fma2(p, w, both(P[k]));
+            const f32x2 nh = fma2(rho, both(-F_C2), mul2(p, t));
+            const f32x2 g = fma2(e[q], nh, both(1.f)), rs2 = mul2(rs, rs);
+            G[q] = mul2(mul2(g, rs), rs2);
+            Q[q] = mul2(mul2(fma2(e[q], both(F_C2 * -0.33333333333333333f), G[q]), rs2), isig2[q]);
+        }
+        if (series) {
+#pragma unroll
+            for (int q = 0; q < N; q++) {
+                f32x2 p = both(S2[0]);
+#pragma unroll
+                for (int k = 1; k < 10; k++) p = fma2(p, s[q], both(S2[k]));
+                const f32x2 ce = mul2(e[q], both(F_C2));
+                float s0, s1, a0, a1, b0, b1, g0, g1, q0, q1;
+                upk(s[q], s0, s1);
+                upk(mul2(ce, fma2(s[q], p, both(0.33333333333333333f))), a0, a1);
+                upk(mul2(mul2(ce, p), isig2[q]), b0, b1);
+                upk(G[q], g0, g1);
+                upk(Q[q], q0, q1);
+                const bool l0 = s0 < S_SERIES, l1 = s1 < S_SERIES;
+                G[q] = pk(l0 ? a0 : g0, l1 ? a1 : g1);
+                Q[q] = pk(l0 ? b0 : q0, l1 ? b1 : q1);
+            }
+        }
     } else {
 #pragma unroll
-        for (int q = 0; q < 4; q++) near_GQ<K, FAR>(s[q], isig2[q], G[q], Q[q]);
+        for (int q = 0; q < N; q++) {
+            float s0, s1;
+            upk(s[q], s0, s1);
+            if constexpr (K == K_WNKLMNS) {
+                float q0, q1;
+                upk(add2(s[q], both(1.f)), q0, q1);
+                const f32x2 t = pk(frcp(q0), frcp(q1));
+                const f32x2 t2u = mul2(mul2(t, t), pk(frsqrt(q0), frsqrt(q1)));
+                G[q] = mul2(add2(s[q], both(2.5f)), t2u);
+                Q[q] = mul2(mul2(mul2(add2(s[q], both(3.5f)), t), t2u), isig2[q]);
+            } else {
+                float i0, i1, g0, g1, q0, q1;
+                upk(isig2[q], i0, i1);
+                near_GQ<K, false>(s0, i0, g0, q0);
+                near_GQ<K, false>(s1, i1, g1, q1);
+                G[q] = pk(g0, g1);
+                Q[q] = pk(q0, q1);
+            }
+        }
     }
 }
 
@@ -417,34 +462,6 @@ __device__ __forceinline__ float df_offset(float a, float b, float oh, float ol)
     return s + (e + (b - ol));
 }
 
-// ---------------------------------------------------------- packed FP32 pairs
-typedef unsigned long long f32x2;
-__device__ __forceinline__ f32x2 pk(float a, float b)
-{
-    f32x2 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-    return r;
-}
-__device__ __forceinline__ void upk(f32x2 v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
-__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c)
-{
-    f32x2 r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b)
-{
-    f32x2 r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b)
-{
-    f32x2 r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ f32x2 sub2(f32x2 a, f32x2 b) { return fma2(b, pk(-1.f, -1.f), a); }
 // the least of the eight (a NaN if one is)
 __device__ __forceinline__ float min8_nan(const f32x2 (&v)[4])
 {

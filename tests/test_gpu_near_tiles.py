@@ -1,0 +1,32 @@
+"""The near-field UJ sums, FP32-comp against FP64 on the same lists, where the groups of four sources
+take each of their branches: targets of several leaves in a group (masks), coincident particles,
+pairs on both sides of the series' limit, list lengths that are no multiple of four or 32."""
+import numpy as np
+import pytest
+import torch
+
+import vpm_gb300 as vpm
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("kernel", [0, 1, 2, 3])
+@pytest.mark.parametrize("n,leaf", [(1, 1), (33, 5), (130, 7), (1501, 50), (4099, 20)])
+def test_near_uj_blocks(n, leaf, kernel):
+    rng = np.random.default_rng(n + kernel)
+    x = rng.random((n, 3))
+    if n > 40:
+        x[5:9], x[n // 2] = x[4], x[20]                     # coincident
+    T = lambda a: torch.tensor(a, device="cuda", dtype=torch.float64)       # noqa: E731
+    h = n ** (-1 / 3)
+    x, gam, sig = T(x), T(rng.standard_normal((n, 3))), T(h * (0.4 + 1.2 * rng.random(n)))
+    ctx = vpm.default_context()
+    out = []
+    for precision in (0, 1):
+        U, J = (torch.zeros(n, k, device="cuda", dtype=torch.float64) for k in (3, 9))
+        ctx.p2p_leaflist_dev(x, gam, sig, U, J, leaf_size=leaf, theta=0.5, kernel=kernel, precision=precision)
+        out.append((U, J))
+    # a pair's terms are rounded to ~16 ulp (displacement, weight, products; J's r^-5 and the singular
+    # kernel's nearest pairs included), its distance to one ulp of the unit cube's coordinates' low parts
+    for a, b in zip(out[1], out[0]):
+        assert (a - b).norm() <= 16 * 2.0 ** -24 * b.norm() + 1e-14
