@@ -19,9 +19,9 @@
 //   3. geometry: bounding box of each node's particles (leaves directly,
 //      inner nodes as the union of their children), centre = box centre,
 //      R = half the box diagonal;
-//   4. dual-tree traversal from (root, root), one frontier of node pairs per
-//      step: far when A != B and theta*r >= R_A + R_B, a near leaf pair when
-//      both are leaves, otherwise the larger non-leaf node (the target on a
+//   4. dual-tree traversal from (root, root), one frontier of node pairs to be
+//      split per step: far when A != B and theta*r >= R_A + R_B, a near leaf pair
+//      when both are leaves, otherwise the larger non-leaf node (the target on a
 //      tie) is split;
 //   5. the near pairs sorted into CSR rows per target leaf, and the warp-group
 //      source intervals used by the kernels of leaflist.cu.
@@ -62,6 +62,7 @@ typedef unsigned long long ull;
 
 // what the traversal reads of a node, in one 64-B record: centre, radius,
 // first child, number of children (0: a leaf) and the leaf's index
+// (pos, below, holds what most tests need of it)
 struct __align__(64) TravNode { double x, y, z, w; int first, nkid, leaf; float w32; int pad[4]; };
 
 __device__ __forceinline__ uint64_t spread3(uint64_t v)
@@ -77,37 +78,6 @@ __device__ __forceinline__ uint64_t spread3(uint64_t v)
 
 __device__ __forceinline__ int64_t gtid() { return blockIdx.x * (int64_t)blockDim.x + threadIdx.x; }
 __device__ __forceinline__ int64_t gstride() { return (int64_t)gridDim.x * blockDim.x; }
-
-// Every thread of the block calls this (no early exit: it holds barriers);
-// returns the thread's slot in a shared append counter, with one atomic per
-// block.  sw: GS_THREADS/32 words of shared memory, sb: one.
-__device__ __forceinline__ ull block_append(ull* ctr, unsigned k, unsigned* sw, ull* sb)
-{
-    const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-    unsigned incl = k;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const unsigned v = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= (unsigned)o) incl += v;
-    }
-    if (lane == 31) sw[warp] = incl;
-    __syncthreads();
-    if (warp == 0) {
-        const unsigned t = lane < nw ? sw[lane] : 0u;
-        unsigned w = t;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const unsigned v = __shfl_up_sync(0xffffffffu, w, o);
-            if (lane >= (unsigned)o) w += v;
-        }
-        if (lane < nw) sw[lane] = w - t;                  // exclusive offset of each warp
-        if (lane == nw - 1) *sb = w ? atomicAdd(ctr, (ull)w) : 0ull;
-    }
-    __syncthreads();
-    const ull slot = *sb + sw[warp] + incl - k;
-    __syncthreads();                                      // sw, sb are reused by the next call
-    return slot;
-}
 
 // ------------------------------------------------------------------ keys
 __global__ void nt_bbox_partial(int64_t n, const double* __restrict__ x, double* __restrict__ part)
@@ -315,9 +285,11 @@ __global__ void nt_box_inner(int d, const int4* __restrict__ nodes, const ull* _
 
 // centre and radius, in tree.cpp's operation order: c = 0.5 (lo + hi), R = 0.5 sqrt(sum (hi - lo)^2)
 __global__ void nt_cr(const ull* __restrict__ ctr, const double* __restrict__ box, const int4* __restrict__ nodes,
-                      const int32_t* __restrict__ node_leaf, TravNode* __restrict__ cr)
+                      const int32_t* __restrict__ node_leaf, TravNode* __restrict__ cr, float4* __restrict__ pos)
 {
     const int64_t nn = (int64_t)ctr[C_NODES];
+    double rc[3];   // the root's centre
+    for (int k = 0; k < 3; k++) rc[k] = 0.5 * (box[k] + box[3 + k]);
     for (int64_t id = gtid(); id < nn; id += gstride()) {
         const double* b = box + 6 * id;
         double c[3], d2 = 0.0;
@@ -333,99 +305,151 @@ __global__ void nt_cr(const ull* __restrict__ ctr, const double* __restrict__ bo
         t.w32 = (float)t.w;
         for (int k = 0; k < 4; k++) t.pad[k] = 0;
         cr[id] = t;
+        // the centre relative to the root's, and the radius, negative for a leaf, in FP32
+        pos[id] = make_float4((float)(c[0] - rc[0]), (float)(c[1] - rc[1]), (float)(c[2] - rc[2]),
+                              t.nkid ? t.w32 : __uint_as_float(__float_as_uint(t.w32) | 0x80000000u));
     }
 }
 
 // -------------------------------------------------------------- traversal
-// The acceptance test theta r >= R_A + R_B is decided in FP32 on the squares,
-// from the FP64 centre differences (each rounded once to FP32): the FP32 sides
-// carry < 2^-20 relative error, so a difference above 2^-17 of their sum gives
-// tree.cpp's FP64 decision; closer calls, and A = B, take the FP64 test itself
-// (GB300's FP64 pipe runs at 1/64 of the FP32 rate: the FP64 test was most of
-// this kernel's time).
-__global__ void nt_trav(int step, double theta, const TravNode* __restrict__ cr, const int2* __restrict__ fin,
-                        int2* __restrict__ fout, uint64_t* __restrict__ near, ull* __restrict__ ctr, ull capF, ull capN,
-                        int shift)
+// A frontier entry is a node pair that is to be split: the node that stays, and the children of the
+// other one (first, count; side 1: they are the targets).  A step tests every child pair of its
+// entries, 8 lanes an entry, TRAV_E entries a lane in flight: leaf pairs go to the near list, far
+// pairs nowhere, pairs to be split to the next frontier, and one append a block serves both lists.
+// Entries hold what the next step needs, so a step reads two node records a test, one of them
+// shared by the 8 lanes and the others next to each other.  With a frontier of pairs to be tested
+// (every child pair written, read back, and its two 64-byte nodes gathered) the traversal of a jet
+// of 2^20 took 2.4 ms; in this form 1.66, with 16 bytes a node for the test 1.17.
+//
+// The acceptance test theta r >= R_A + R_B is decided on 16 bytes a node (`pos`), in FP32 on the
+// squares.  Against tree.cpp's FP64 test the two sides carry < 2^-20 relative error from their own
+// roundings, and r is off by at most d = sqrt(3) 2^-23 root radii from the rounded centres (half an
+// ulp of at most one root radius in each coordinate of each), the left side by
+// 2 theta^2 r d + theta^2 d^2.  A difference above 2^-17 of the sides' sum plus that (with
+// slack = 4 theta 2^-23 root radii > 2 theta d) gives tree.cpp's decision; closer calls, and A = B,
+// take the FP64 test itself (GB300's FP64 pipe runs at 1/64 of the FP32 rate).
+struct __align__(16) TravEntry { int other, first, nkid, side; };
+
+__device__ __forceinline__ TravEntry trav_entry(int A, int B, const TravNode& a, const TravNode& c)
+{
+    // the larger non-leaf node is split, the target on a tie
+    const bool split_a = a.nkid != 0 && (c.nkid == 0 || a.w >= c.w);
+    TravEntry t;
+    t.other = split_a ? B : A;
+    t.first = split_a ? a.first : c.first;
+    t.nkid = split_a ? a.nkid : c.nkid;
+    t.side = split_a;
+    return t;
+}
+
+constexpr int TRAV_E = 4;
+
+__global__ void __launch_bounds__(GS_THREADS)
+nt_trav(int step, double theta, const TravNode* __restrict__ cr, const float4* __restrict__ pos,
+        const int32_t* __restrict__ leaf, const TravEntry* __restrict__ fin, TravEntry* __restrict__ fout,
+        uint64_t* __restrict__ near, ull* __restrict__ ctr, ull capF, ull capN, int shift)
 {
     __shared__ unsigned sw[GS_THREADS / 32];
-    __shared__ ull sb;
+    __shared__ ull sb[2];
     __shared__ int stop;
     // After an overflow in an earlier step, the slots of this step's frontier past the last
     // write were counted but never written: read nothing, the host grows the buffers and
-    // repeats the traversal.  One read per block keeps the exit block-uniform (block_append
+    // repeats the traversal.  One read per block keeps the exit block-uniform (the append
     // holds barriers); the flag is read once, before this launch writes anything.
     if (threadIdx.x == 0) stop = ctr[C_OVF] != 0ull;
     __syncthreads();
     if (stop) return;
-    const float th2 = (float)(theta * theta);
+    const float th2 = (float)(theta * theta), slack = 4.0f * (float)theta * 1.1920928955078125e-07f * cr[0].w32;
     const ull raw = ctr[C_F + step];
     const int64_t cnt = (int64_t)(raw < capF ? raw : capF);
-    // block-strided so that every thread of a block runs the same iterations (block_append)
-    for (int64_t base = (int64_t)blockIdx.x * blockDim.x; base < cnt; base += gstride()) {
-        const int64_t i = base + threadIdx.x;
-        unsigned knear = 0, ksplit = 0;
-        int A = 0, B = 0, first = 0, la_leaf = 0, lb_leaf = 0;
-        bool split_a = false;
-        if (i < cnt) {
-            const int2 ab = fin[i];
-            A = ab.x;
-            B = ab.y;
-            const TravNode a = cr[A], c = cr[B];
-            const double dx = __dsub_rn(a.x, c.x), dy = __dsub_rn(a.y, c.y), dz = __dsub_rn(a.z, c.z);
-            const float fx = (float)dx, fy = (float)dy, fz = (float)dz;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, kid = threadIdx.x & 7;
+    constexpr int PER = TRAV_E * GS_THREADS / 8;   // entries a block and iteration
+    for (int64_t base = (int64_t)blockIdx.x * PER; base < cnt; base += (int64_t)gridDim.x * PER) {
+        uint64_t key[TRAV_E];
+        TravEntry ent[TRAV_E];
+        unsigned kinds = 0;                        // bit e: near; bit 8 + e: to be split
+#pragma unroll
+        for (int e = 0; e < TRAV_E; e++) {
+            const int64_t i = base + e * (GS_THREADS / 8) + (threadIdx.x >> 3);
+            if (i >= cnt) continue;
+            const TravEntry p = fin[i];
+            if (kid >= p.nkid) continue;
+            const int A = p.side ? p.first + kid : p.other, B = p.side ? p.other : p.first + kid;
+            const float4 pa = pos[A], pc = pos[B];
+            const float fx = pa.x - pc.x, fy = pa.y - pc.y, fz = pa.z - pc.z;
             const float lhs = th2 * fmaf(fx, fx, fmaf(fy, fy, fz * fz));
-            const float rs = a.w32 + c.w32;
+            const float rs = fabsf(pa.w) + fabsf(pc.w);
             const float rhs = rs * rs;
             bool far;
-            if (A != B && fabsf(lhs - rhs) > 7.62939453125e-06f * (lhs + rhs)) {
+            if (A != B && fabsf(lhs - rhs) > fmaf(7.62939453125e-06f, lhs + rhs, slack * (sqrtf(lhs) + slack))) {
                 far = lhs > rhs;
             } else {   // tree.cpp's FP64 test, in its operation order
+                const TravNode a = cr[A], c = cr[B];
+                const double dx = __dsub_rn(a.x, c.x), dy = __dsub_rn(a.y, c.y), dz = __dsub_rn(a.z, c.z);
                 const double r = __dsqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)),
                                                       __dmul_rn(dz, dz)));
                 far = (A != B) && (__dmul_rn(theta, r) >= __dadd_rn(a.w, c.w));
             }
-            if (!far) {
-                const bool la = a.nkid == 0, lb = c.nkid == 0;
-                if (la && lb) {
-                    knear = 1;
-                    la_leaf = a.leaf;
-                    lb_leaf = c.leaf;
-                } else {
-                    split_a = !la && (lb || a.w >= c.w);
-                    first = split_a ? a.first : c.first;
-                    ksplit = (unsigned)(split_a ? a.nkid : c.nkid);
-                }
+            if (far) continue;
+            if (__float_as_uint(pa.w) & __float_as_uint(pc.w) & 0x80000000u) {
+                kinds |= 1u << e;
+                key[e] = ((uint64_t)(uint32_t)leaf[A] << shift) | (uint32_t)leaf[B];
+            } else {
+                kinds |= 256u << e;
+                ent[e] = trav_entry(A, B, cr[A], cr[B]);
             }
         }
-        const ull sn = block_append(&ctr[C_NEAR], knear, sw, &sb);
-        if (knear) {
-            if (sn < capN) near[sn] = ((uint64_t)(uint32_t)la_leaf << shift) | (uint32_t)lb_leaf;
-            else ctr[C_OVFN] = 1;
+        // one append for both lists: counts packed 16 + 16 bits (a block appends at most 1,024 each)
+        const unsigned k = (unsigned)__popc(kinds & 255u) | (unsigned)__popc(kinds >> 8) << 16;
+        unsigned incl = k;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned v = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += v;
         }
-        const ull sf = block_append(&ctr[C_F + step + 1], ksplit, sw, &sb);
-        if (ksplit) {
-            if (sf + ksplit <= capF) {
-                for (unsigned k = 0; k < ksplit; k++) {
-                    const int ch = first + (int)k;
-                    fout[sf + k] = split_a ? make_int2(ch, B) : make_int2(A, ch);
-                }
-            } else {
-                ctr[C_OVF] = 1;
+        if (lane == 31) sw[warp] = incl;
+        __syncthreads();
+        unsigned before = 0, all = 0;
+#pragma unroll
+        for (int w = 0; w < GS_THREADS / 32; w++) {
+            if (w < warp) before += sw[w];
+            all += sw[w];
+        }
+        if (threadIdx.x == 0) sb[0] = all & 0xffffu ? atomicAdd(&ctr[C_NEAR], (ull)(all & 0xffffu)) : 0ull;
+        if (threadIdx.x == 32) sb[1] = all >> 16 ? atomicAdd(&ctr[C_F + step + 1], (ull)(all >> 16)) : 0ull;
+        __syncthreads();
+        before += incl - k;
+        ull sn = sb[0] + (before & 0xffffu), sf = sb[1] + (before >> 16);
+#pragma unroll
+        for (int e = 0; e < TRAV_E; e++) {
+            if (kinds >> e & 1u) {
+                if (sn < capN) near[sn] = key[e];
+                else ctr[C_OVFN] = 1;
+                sn++;
+            }
+            if (kinds >> (8 + e) & 1u) {
+                if (sf < capF) fout[sf] = ent[e];
+                else ctr[C_OVF] = 1;
+                sf++;
             }
         }
     }
 }
 
-// the root pair starts the traversal; every frontier count and the near count are reset
-__global__ void nt_trav_init(int2* __restrict__ fr0, ull* __restrict__ ctr)
+// The root pair starts the traversal; every frontier count and the near count are reset.
+__global__ void nt_trav_init(const TravNode* __restrict__ cr, TravEntry* __restrict__ fr0, uint64_t* __restrict__ near,
+                             ull* __restrict__ ctr)
 {
     if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    fr0[0] = make_int2(0, 0);
-    ctr[C_NEAR] = 0;
+    const TravNode root = cr[0];
+    const bool leaf = root.nkid == 0;
+    if (leaf) near[0] = 0;                        // leaf 0 with itself
+    else fr0[0] = trav_entry(0, 0, root, root);
+    ctr[C_NEAR] = leaf;
     ctr[C_OVF] = 0;
     ctr[C_OVFN] = 0;
     for (int k = 0; k < TRAV_STEPS + 2; k++) ctr[C_F + k] = 0;
-    ctr[C_F] = 1;
+    ctr[C_F] = !leaf;
 }
 
 // ------------------------------------------------------------------- CSR
@@ -588,7 +612,7 @@ cudaError_t near_build(NearScratch& s, int64_t n, const double* x, int leaf_size
     NT_TRY(s.nodes.grow(ncap * sizeof(int4)));
     NT_TRY(s.node_lvl.grow(ncap * sizeof(int32_t)));
     NT_TRY(s.node_box.grow(6 * ncap * sizeof(double)));
-    NT_TRY(s.node_cr.grow(ncap * sizeof(TravNode)));
+    NT_TRY(s.node_cr.grow(ncap * (sizeof(TravNode) + sizeof(float4))));
     NT_TRY(s.node_leaf.grow(ncap * sizeof(int32_t)));
     NT_TRY(s.flag.grow(n * sizeof(int32_t)));
     NT_TRY(s.lb.grow(n * sizeof(int32_t)));
@@ -632,29 +656,30 @@ cudaError_t near_build(NearScratch& s, int64_t n, const double* x, int leaf_size
     double* nbox = s.node_box.as<double>();
     nt_box_leaf<<<gs_blocks(2 * n), GS_THREADS, 0, st>>>(nodes, ctr, s.xs.as<double>(), nbox);
     for (int d = MAX_DEPTH; d >= 0; d--) nt_box_inner<<<gs_blocks(n / 2 + 1), GS_THREADS, 0, st>>>(d, nodes, ctr, nbox);
-    nt_cr<<<gs_blocks(2 * n), GS_THREADS, 0, st>>>(ctr, nbox, nodes, s.node_leaf.as<int32_t>(),
-                                                   s.node_cr.as<TravNode>());
+    TravNode* cr = s.node_cr.as<TravNode>();
+    float4* pos = (float4*)(cr + ncap);
+    nt_cr<<<gs_blocks(2 * n), GS_THREADS, 0, st>>>(ctr, nbox, nodes, s.node_leaf.as<int32_t>(), cr, pos);
     *launches += 2 * MAX_DEPTH + 1 + 4 + (MAX_DEPTH + 1) + 2;
     NT_TRY(cudaGetLastError());
 
     // 4. traversal; on overflow of a frontier or of the near list, grow and repeat
-    // a uniform cloud at leaf size 64 and theta 0.4 needs ~32 n frontier pairs and ~16 n near pairs
-    if (s.capF == 0) s.capF = (size_t)(n < 4096 ? 4096 : n) * 40;
+    // a uniform cloud at leaf size 64 and theta 0.4 needs ~6 n frontier entries and ~20 n near pairs
+    if (s.capF == 0) s.capF = (size_t)(n < 4096 ? 4096 : n) * 10;
     if (s.capN == 0) s.capN = (size_t)(n < 4096 ? 4096 : n) * 24;
     // near pairs are the keys (target leaf << shift) | source leaf, with only as many bits for the
     // source as n leaves need: the sort's passes go by key bits (37 instead of 49 at 2^20)
     int shift = 1;
     while (((int64_t)1 << shift) < n) shift++;
     for (int attempt = 0;; attempt++) {
-        NT_TRY(s.fr0.grow(s.capF * sizeof(int2)));
-        NT_TRY(s.fr1.grow(s.capF * sizeof(int2)));
+        NT_TRY(s.fr0.grow(s.capF * sizeof(TravEntry)));
+        NT_TRY(s.fr1.grow(s.capF * sizeof(TravEntry)));
         NT_TRY(s.near0.grow(s.capN * sizeof(uint64_t)));
         NT_TRY(s.near1.grow(s.capN * sizeof(uint64_t)));
-        nt_trav_init<<<1, 32, 0, st>>>(s.fr0.as<int2>(), ctr);
+        nt_trav_init<<<1, 32, 0, st>>>(cr, s.fr0.as<TravEntry>(), s.near0.as<uint64_t>(), ctr);
         for (int k = 0; k < TRAV_STEPS; k++) {
-            const int2* fin = (k & 1) ? s.fr1.as<int2>() : s.fr0.as<int2>();
-            int2* fout = (k & 1) ? s.fr0.as<int2>() : s.fr1.as<int2>();
-            nt_trav<<<GS_BLOCKS, GS_THREADS, 0, st>>>(k, theta, s.node_cr.as<TravNode>(), fin, fout,
+            const TravEntry* fin = (k & 1) ? s.fr1.as<TravEntry>() : s.fr0.as<TravEntry>();
+            TravEntry* fout = (k & 1) ? s.fr0.as<TravEntry>() : s.fr1.as<TravEntry>();
+            nt_trav<<<GS_BLOCKS, GS_THREADS, 0, st>>>(k, theta, cr, pos, s.node_leaf.as<int32_t>(), fin, fout,
                                                        s.near0.as<uint64_t>(), ctr, (ull)s.capF, (ull)s.capN, shift);
         }
         *launches += TRAV_STEPS + 1;

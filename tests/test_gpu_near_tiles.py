@@ -30,3 +30,17 @@ def test_near_uj_blocks(n, leaf, kernel):
     # kernel's nearest pairs included), its distance to one ulp of the unit cube's coordinates' low parts
     for a, b in zip(out[1], out[0]):
         assert (a - b).norm() <= 16 * 2.0 ** -24 * b.norm() + 1e-14
+
+
+@pytest.mark.parametrize("leaf,theta", [(1, 0.4), (3, 0.9), (64, 0.0)])
+@pytest.mark.parametrize("spread", [1e-9, 3e-8, 1e-7, 1e-6])
+def test_lists_of_points_closer_than_fp32_centres(spread, leaf, theta):
+    """Points far closer than FP32 resolves across the field: the device's FP32 acceptance test has to
+    leave these to FP64, and the lists stay the host builder's."""
+    rng = np.random.default_rng(3)
+    n = 1200
+    x = rng.random((40, 3)).repeat(n // 40, 0) + spread * rng.standard_normal((n, 3)) + 5.0
+    host = vpm._lib.leaflist_host(x, leaf, theta)
+    dev = vpm.default_context().leaflist_dev(torch.tensor(x, device="cuda"), leaf, theta)
+    for h, d in zip(host, dev):
+        assert np.array_equal(np.asarray(h), np.asarray(d.cpu() if isinstance(d, torch.Tensor) else d))
