@@ -14,13 +14,12 @@
 // times as wide as high (tile radius 0.161 against 0.074).
 //
 // Steps: per-block bounding boxes (bbox_partial), curve keys (hilbert_keys), CUB radix sort of
-// (key, index), and a gather of the sorted positions into TgtPos records.  Keys have 10 bits an
-// axis up to 2^16 particles (a cell of the cube then holds at most a few of a uniform set; four
-// 8-bit sort passes, each about 9 us at these sizes) and 20 beyond (eight passes).  Up to 6,144
-// particles one block does all of it (order_block): a launch instead of eight.
+// (key, index), and a gather of the sorted positions into TgtPos records; up to RANK_MAX
+// particles order_rank counts places instead.  Keys have 10 bits an axis up to 2^16 particles (a
+// cell of the cube then holds at most a few of a uniform set; four 8-bit sort passes, each about
+// 9 us at these sizes) and 20 beyond (eight passes).
 #include "internal.h"
 
-#include <cub/block/block_radix_sort.cuh>
 #include <cub/device/device_radix_sort.cuh>
 
 namespace vpm {
@@ -146,76 +145,48 @@ __global__ void gather_targets(int64_t n, const double* __restrict__ x, const in
 
 static inline size_t align256(size_t b) { return (b + 255) / 256 * 256; }
 
-// Everything in one block: thread t holds particles t ITEMS .. t ITEMS + ITEMS - 1.
-constexpr int OB_THREADS = 1024;
-constexpr int64_t OB_MAX = OB_THREADS * 6;
-constexpr int OB_BITS = 8;                // key bits an axis: seven 4-bit passes with the flag of absent ones
-template <int ITEMS>
-__global__ void __launch_bounds__(OB_THREADS)
-order_block(int n, const double* __restrict__ x, TgtPos* __restrict__ out)
+// Up to RANK_MAX particles: each one's place is the number of keys before it, counted (lane =
+// particle, the block's warps share the keys), and its record goes there: one launch for the sort's
+// six and the gather.  n^2 compares are 4 us at 8,192 particles, but 60 us at 32,000, where the
+// sort takes 45.  UJ calls with the sort -> with ranks: 8,192 356 -> 300 us, 16,000 594 -> 579,
+// 24,000 976 -> 1004; a sort of everything in one block takes 20 us more at 6,100 than the ranks
+// and as long at 1,400.
+constexpr int64_t RANK_MAX = 16384;
+constexpr int RANK_THREADS = 1024;
+__global__ void __launch_bounds__(RANK_THREADS)
+order_rank(int n, const double* __restrict__ x, const uint32_t* __restrict__ keys, TgtPos* __restrict__ out)
 {
-    typedef cub::BlockRadixSort<uint32_t, OB_THREADS, ITEMS, int32_t> Sort;
-    __shared__ union { typename Sort::TempStorage sort; float red[6][OB_THREADS / 32]; } sm;
-    // Offsets from the first particle, rounded to FP32 (two FP64 operations a coordinate; box, scale
-    // and cells in FP64 took a single SM longer than the eight launches).
-    float p[ITEMS][3], v[6] = {INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY};
-#pragma unroll
-    for (int j = 0; j < ITEMS; j++) {
-        const int i = min((int)threadIdx.x * ITEMS + j, n - 1);
-#pragma unroll
-        for (int k = 0; k < 3; k++) {
-            p[j][k] = (float)(x[3 * i + k] - x[k]);
-            v[k] = fminf(v[k], p[j][k]);
-            v[3 + k] = fmaxf(v[3 + k], p[j][k]);
+    __shared__ int part[RANK_THREADS / 32][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int i0 = blockIdx.x * 32, i = i0 + lane;
+    const uint32_t key = keys[min(i, n - 1)];
+    TgtPos t;
+    if (warp == 0) {
+        const int j = min(i, n - 1);
+        t.x = x[3 * j]; t.y = x[3 * j + 1]; t.z = x[3 * j + 2];
+        t.idx = j; t.pad = 0;
+    }
+    int c = 0;
+    for (int q = warp; q < n / 4; q += RANK_THREADS / 32) {   // equal keys keep the caller's order
+        const uint4 k = ((const uint4*)keys)[q];
+        if (4 * q < i0) {
+            c += (k.x <= key) + (k.y <= key) + (k.z <= key) + (k.w <= key);
+        } else if (4 * q >= i0 + 32) {
+            c += (k.x < key) + (k.y < key) + (k.z < key) + (k.w < key);
+        } else {
+            c += (k.x < key || (k.x == key && 4 * q < i)) + (k.y < key || (k.y == key && 4 * q + 1 < i)) +
+                 (k.z < key || (k.z == key && 4 * q + 2 < i)) + (k.w < key || (k.w == key && 4 * q + 3 < i));
         }
     }
-#pragma unroll
-    for (int k = 0; k < 6; k++) {
-#pragma unroll
-        for (int m = 16; m > 0; m >>= 1) {
-            const float o = __shfl_xor_sync(0xffffffffu, v[k], m);
-            v[k] = k < 3 ? fminf(v[k], o) : fmaxf(v[k], o);
-        }
-        if ((threadIdx.x & 31) == 0) sm.red[k][threadIdx.x >> 5] = v[k];
-    }
+    if (warp == 0)
+        for (int j = n / 4 * 4; j < n; j++) c += keys[j] < key || (keys[j] == key && j < i);
+    part[warp][lane] = c;
     __syncthreads();
+    if (warp != 0 || i >= n) return;
+    c = 0;
 #pragma unroll
-    for (int k = 0; k < 6; k++) {
-        v[k] = sm.red[k][threadIdx.x & 31];
-#pragma unroll
-        for (int m = 16; m > 0; m >>= 1) {
-            const float o = __shfl_xor_sync(0xffffffffu, v[k], m);
-            v[k] = k < 3 ? fminf(v[k], o) : fmaxf(v[k], o);
-        }
-    }
-    __syncthreads();
-    const float ext = fmaxf(v[3] - v[0], fmaxf(v[4] - v[1], v[5] - v[2]));
-    constexpr float top = (float)((1 << OB_BITS) - 1);
-    const float sc = ext > 0.f ? top / ext : 0.f;
-    uint32_t key[ITEMS];
-    int32_t idx[ITEMS];
-#pragma unroll
-    for (int j = 0; j < ITEMS; j++) {
-        const int i = threadIdx.x * ITEMS + j;
-        idx[j] = i;
-        uint32_t q[3];
-#pragma unroll
-        for (int k = 0; k < 3; k++) q[k] = (uint32_t)fminf(fmaxf((p[j][k] - v[k]) * sc, 0.f), top);
-        key[j] = i < n ? hilbert_index<uint32_t>(q, OB_BITS) : 1u << (3 * OB_BITS);     // past n: behind every particle
-    }
-    Sort(sm.sort).Sort(key, idx, 0, 3 * OB_BITS + 1);
-#pragma unroll
-    for (int j = 0; j < ITEMS; j++) {
-        const int o = threadIdx.x * ITEMS + j;
-        if (o >= n) continue;
-        TgtPos t;
-        t.x = x[3 * (int64_t)idx[j]];
-        t.y = x[3 * (int64_t)idx[j] + 1];
-        t.z = x[3 * (int64_t)idx[j] + 2];
-        t.idx = idx[j];
-        t.pad = 0;
-        out[o] = t;
-    }
+    for (int w = 0; w < RANK_THREADS / 32; w++) c += part[w][lane];
+    out[c] = t;
 }
 
 constexpr int64_t SMALL_KEYS = 1 << 16;   // up to here 10-bit axes and 32-bit keys
@@ -263,19 +234,16 @@ cudaError_t order_targets(int64_t nt, const double* xt, void* scratch, size_t sc
     if ((size_t)(p - (char*)scratch) > scratch_bytes) return cudaErrorInvalidValue;
     const unsigned nb = (unsigned)((nt + BB_THREADS - 1) / BB_THREADS);
     const int32_t* perm = nullptr;
-    if (nt > 1 && nt <= OB_MAX) {
-        const int items = (int)((nt + OB_THREADS - 1) / OB_THREADS), m = (int)nt;
-        if (items <= 1) order_block<1><<<1, OB_THREADS, 0, st>>>(m, xt, tp);
-        else if (items <= 2) order_block<2><<<1, OB_THREADS, 0, st>>>(m, xt, tp);
-        else if (items <= 4) order_block<4><<<1, OB_THREADS, 0, st>>>(m, xt, tp);
-        else order_block<6><<<1, OB_THREADS, 0, st>>>(m, xt, tp);
-        *launches += 1;
-        *out = tp;
-        return cudaGetLastError();
-    }
     if (nt > 1) {
         bbox_partial<<<BB_BLOCKS, BB_THREADS, 0, st>>>(nt, xt, part);
         cudaError_t e;
+        if (nt <= RANK_MAX) {
+            hilbert_keys<<<nb, BB_THREADS, 0, st>>>(nt, xt, part, 10, (uint32_t*)k0, i0);
+            order_rank<<<(unsigned)((nt + 31) / 32), RANK_THREADS, 0, st>>>((int)nt, xt, (uint32_t*)k0, tp);
+            *launches += 3;
+            *out = tp;
+            return cudaGetLastError();
+        }
         if (nt <= SMALL_KEYS) {
             hilbert_keys<<<nb, BB_THREADS, 0, st>>>(nt, xt, part, 10, (uint32_t*)k0, i0);
             e = sort_keys(tmpp, tmp, (uint32_t*)k0, (uint32_t*)k1, i0, i1, nt, 10, st);

@@ -1,6 +1,6 @@
-"""The curve ordering of the targets and sources at its edges: one and two particles, the last
-sizes of the one-block kernel and of the 32-bit keys and the next ones, and sets without extent along some or all
-axes.  The FP32-comp U, J of the ordered set against the FP64 form's (whose sums do not depend
+"""The curve ordering of the targets and sources at its edges: one and two particles, remainders of
+the counted ranks (33, 35, ...), their last size and that of the 32-bit keys and the next ones, and
+sets without extent along some or all axes.  The FP32-comp U, J of the ordered set against the FP64 form's (whose sums do not depend
 on the order); tolerance: the FP32-comp bound of test_gpu_uj.py.  The Winckelmans kernel: 65,536
 random points of a line have neighbours at 1e-7 core sizes, where the literal FP64 form of the
 Gaussian-erf kernel, a difference of nearly equal terms, has no digits left to compare with."""
@@ -14,7 +14,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("shape", ["cloud", "line", "plane", "point"])
-@pytest.mark.parametrize("n", [1, 2, 700, 1024, 1025, 2049, 4097, 6144, 6145, 65536, 65537])
+@pytest.mark.parametrize("n", [1, 2, 700, 1024, 1025, 2049, 4097, 6144, 6145, 65536, 65537, 31, 33, 35, 16383, 16384, 16385])
 def test_ordered_sums(ctx, n, shape):
     X, G, s = random_cloud(n, seed=n)
     if shape == "line":
