@@ -46,6 +46,7 @@ namespace {
 constexpr int KEY_LEVELS = 21;                 // 3 x 21 = 63 key bits
 constexpr int MAX_DEPTH = KEY_LEVELS + 1;      // breadth-first node depths
 constexpr int TRAV_STEPS = 2 * MAX_DEPTH + 2;  // each step descends one side
+constexpr int TRAV_FIRST = 20;                 // steps before the host looks whether any are left
 constexpr int GS_THREADS = 256;
 constexpr int GS_BLOCKS = 8 * 152;
 
@@ -53,8 +54,8 @@ constexpr int GS_BLOCKS = 8 * 152;
 enum : int {
     C_NODES = 0, C_NEAR = 1, C_OVF = 2, C_PAIRS = 3, C_NL = 4,
     C_OVFN = 5,                                 // the near list overflowed (the traversal itself stays valid)
-    C_LVL = 8,                                  // [C_LVL + 2d, C_LVL + 2d + 1) = node ids of depth d
-    C_F = C_LVL + 2 * (MAX_DEPTH + 2),          // C_F + s = frontier size of traversal step s
+    C_LVL = 8,                                  // C_LVL + d = nodes of depth d
+    C_F = C_LVL + MAX_DEPTH + 2,                // C_F + s = frontier size of traversal step s
     C_COUNT = C_F + TRAV_STEPS + 2
 };
 
@@ -164,9 +165,18 @@ __global__ void nt_init(int64_t n, int4* __restrict__ nodes, int32_t* __restrict
     nodes[0] = make_int4(0, (int)n, -1, 0);
     lvl[0] = 0;
     ctr[C_NODES] = 1;
-    ctr[C_LVL] = 0;
-    ctr[C_LVL + 1] = 1;
-    ctr[C_F] = 1;
+    ctr[C_LVL] = 1;
+}
+
+// The node ids [s, e) of depth d, from the counts of the depths up to it; whole warps call this.
+static_assert(MAX_DEPTH + 1 <= 32, "one depth a lane");
+__device__ __forceinline__ void level_range(const ull* ctr, int d, int64_t& s, int64_t& e)
+{
+    const int lane = threadIdx.x & 31;
+    const unsigned c = lane <= d ? (unsigned)ctr[C_LVL + lane] : 0u;
+    const unsigned all = __reduce_add_sync(0xffffffffu, c);
+    e = (int64_t)all;
+    s = (int64_t)(all - __shfl_sync(0xffffffffu, c, d));
 }
 
 // first position in [lo, hi) whose octant digit at `shift` is >= oct (digits are sorted there)
@@ -183,7 +193,8 @@ __device__ __forceinline__ int digit_lower_bound(const uint64_t* __restrict__ ke
 __global__ void nt_split(int d, const uint64_t* __restrict__ key, int leaf_size, int4* __restrict__ nodes,
                          int32_t* __restrict__ lvl, ull* __restrict__ ctr)
 {
-    const int64_t s = (int64_t)ctr[C_LVL + 2 * d], e = (int64_t)ctr[C_LVL + 2 * d + 1];
+    int64_t s, e;
+    level_range(ctr, d, s, e);
     for (int64_t id = s + gtid(); id < e; id += gstride()) {
         const int4 nd = nodes[id];
         int L = lvl[id];
@@ -201,7 +212,8 @@ __global__ void nt_split(int d, const uint64_t* __restrict__ key, int leaf_size,
             if (++L >= KEY_LEVELS) { nk = 0; break; }   // one octant down to the last key bit: a leaf
         }
         if (nk == 0) continue;
-        const int64_t slot = (int64_t)atomicAdd(&ctr[C_NODES], (ull)nk);
+        const int64_t slot = e + (int64_t)atomicAdd(&ctr[C_LVL + d + 1], (ull)nk);   // depth d + 1 follows depth d
+        atomicAdd(&ctr[C_NODES], (ull)nk);
         int j = 0;
         for (int o = 0; o < 8; o++)
             if (st[o + 1] > st[o]) {
@@ -211,13 +223,6 @@ __global__ void nt_split(int d, const uint64_t* __restrict__ key, int leaf_size,
             }
         nodes[id] = make_int4(nd.x, nd.y, (int)slot, nk);
     }
-}
-
-__global__ void nt_mark(int d, ull* __restrict__ ctr)
-{
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    ctr[C_LVL + 2 * (d + 1)] = ctr[C_LVL + 2 * d + 1];
-    ctr[C_LVL + 2 * (d + 1) + 1] = ctr[C_NODES];
 }
 
 __global__ void nt_leaf_flag(const int4* __restrict__ nodes, const ull* __restrict__ ctr, int32_t* __restrict__ flag)
@@ -269,7 +274,8 @@ __global__ void nt_box_leaf(const int4* __restrict__ nodes, const ull* __restric
 
 __global__ void nt_box_inner(int d, const int4* __restrict__ nodes, const ull* __restrict__ ctr, double* __restrict__ box)
 {
-    const int64_t s = (int64_t)ctr[C_LVL + 2 * d], e = (int64_t)ctr[C_LVL + 2 * d + 1];
+    int64_t s, e;
+    level_range(ctr, d, s, e);
     for (int64_t id = s + gtid(); id < e; id += gstride()) {
         const int4 nd = nodes[id];
         if (nd.w == 0) continue;
@@ -639,10 +645,8 @@ cudaError_t near_build(NearScratch& s, int64_t n, const double* x, int leaf_size
     // 2. nodes, breadth first
     int4* nodes = s.nodes.as<int4>();
     nt_init<<<1, 32, 0, st>>>(n, nodes, s.node_lvl.as<int32_t>(), ctr);
-    for (int d = 0; d < MAX_DEPTH; d++) {
+    for (int d = 0; d < MAX_DEPTH; d++)
         nt_split<<<gs_blocks(n / 2 + 1), GS_THREADS, 0, st>>>(d, skey, leaf_size, nodes, s.node_lvl.as<int32_t>(), ctr);
-        nt_mark<<<1, 32, 0, st>>>(d, ctr);
-    }
     // leaves in Morton order
     NT_TRY(cudaMemsetAsync(s.flag.p, 0, n * sizeof(int32_t), st));
     nt_leaf_flag<<<gs_blocks(n), GS_THREADS, 0, st>>>(nodes, ctr, s.flag.as<int32_t>());
@@ -659,7 +663,7 @@ cudaError_t near_build(NearScratch& s, int64_t n, const double* x, int leaf_size
     TravNode* cr = s.node_cr.as<TravNode>();
     float4* pos = (float4*)(cr + ncap);
     nt_cr<<<gs_blocks(2 * n), GS_THREADS, 0, st>>>(ctr, nbox, nodes, s.node_leaf.as<int32_t>(), cr, pos);
-    *launches += 2 * MAX_DEPTH + 1 + 4 + (MAX_DEPTH + 1) + 2;
+    *launches += MAX_DEPTH + 1 + 4 + (MAX_DEPTH + 1) + 2;
     NT_TRY(cudaGetLastError());
 
     // 4. traversal; on overflow of a frontier or of the near list, grow and repeat
@@ -676,17 +680,26 @@ cudaError_t near_build(NearScratch& s, int64_t n, const double* x, int leaf_size
         NT_TRY(s.near0.grow(s.capN * sizeof(uint64_t)));
         NT_TRY(s.near1.grow(s.capN * sizeof(uint64_t)));
         nt_trav_init<<<1, 32, 0, st>>>(cr, s.fr0.as<TravEntry>(), s.near0.as<uint64_t>(), ctr);
-        for (int k = 0; k < TRAV_STEPS; k++) {
-            const TravEntry* fin = (k & 1) ? s.fr1.as<TravEntry>() : s.fr0.as<TravEntry>();
-            TravEntry* fout = (k & 1) ? s.fr0.as<TravEntry>() : s.fr1.as<TravEntry>();
-            nt_trav<<<GS_BLOCKS, GS_THREADS, 0, st>>>(k, theta, cr, pos, s.node_leaf.as<int32_t>(), fin, fout,
-                                                       s.near0.as<uint64_t>(), ctr, (ull)s.capF, (ull)s.capN, shift);
+        // the first TRAV_FIRST steps finish trees up to half as deep (an empty step costs a launch,
+        // the look at the counters in between the deeper ones a wait)
+        int k = 0;
+        for (int last : {TRAV_FIRST, TRAV_STEPS}) {
+            *launches += last - k;
+            for (; k < last; k++) {
+                const TravEntry* fin = (k & 1) ? s.fr1.as<TravEntry>() : s.fr0.as<TravEntry>();
+                TravEntry* fout = (k & 1) ? s.fr0.as<TravEntry>() : s.fr1.as<TravEntry>();
+                nt_trav<<<GS_BLOCKS, GS_THREADS, 0, st>>>(k, theta, cr, pos, s.node_leaf.as<int32_t>(), fin, fout,
+                                                           s.near0.as<uint64_t>(), ctr, (ull)s.capF, (ull)s.capN,
+                                                           shift);
+            }
+            NT_TRY(cudaGetLastError());
+            NT_TRY(read_counters(s, st, sync, sync_ctx));
+            const ull* h = (const ull*)s.hctr;
+            if (h[C_OVF] || h[C_F + k] == 0) break;
         }
-        *launches += TRAV_STEPS + 1;
-        NT_TRY(cudaGetLastError());
-        NT_TRY(read_counters(s, st, sync, sync_ctx));
+        *launches += 1;   // nt_trav_init
         const ull* h = (const ull*)s.hctr;
-        if (!h[C_OVF] && !h[C_OVFN] && h[C_F + TRAV_STEPS] == 0) break;
+        if (!h[C_OVF] && !h[C_OVFN] && h[C_F + k] == 0) break;
         // The counters hold the full sizes of every frontier up to the one that overflowed
         // (appends are counted even when they do not fit) and the near pairs found so far:
         // grow past them, so that each retry gets at least one step further.
