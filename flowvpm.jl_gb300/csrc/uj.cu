@@ -63,11 +63,11 @@ int uj_num_splits(int64_t nt, int64_t ns, int num_sms, int precision, int per_sm
     return (int)nsplit;
 }
 
-// The tile kernels (uj_tc.cu) take a set on itself from 12,288 particles.  Below, most tiles of
-// 64 are near ones (4,099 random particles: 73 % of the pairs) and the tile pack is pure cost:
-// 4,000 to 10,000 particles ran within 3 % of uj_mixed_kernel (Winckelmans 4,099 20 % slower),
-// 16,384 10 % faster (741 against 820 us), 65,536 1.6 times.
-bool uj_takes_tiles(const UJArgs& a) { return a.self && a.precision == 1 && a.ns >= 12288; }
+// The tile kernels (uj_tc.cu) take a set on itself from 10,240 particles.  Below, most tiles of
+// 64 are near ones (4,099 random particles: 73 % of the pairs) and the tile pack is pure cost.
+// With uj_mixed_kernel / with tiles, us: random 6,500 269 / 275, 8,192 307 / 293, 10,000 378 / 360,
+// 12,000 450 / 424; ring of 8,000 291 / 305, of 12,000 445 / 431; Winckelmans 8,192 287 / 290.
+bool uj_takes_tiles(const UJArgs& a) { return a.self && a.precision == 1 && a.ns >= 10240; }
 
 size_t uj_partial_bytes(int64_t nt, int nsplit, int components)
 {

@@ -19,16 +19,16 @@
 // warp's targets from the tile (so that G <= 2^9, Q <= 2^15 and, within a factor of 8 in
 // distance, both keep a normal lo part), y in units of the tile's radius, gam in units of the
 // tile's largest strength / 64.  Errors against 64 bits stay at or below the mixed kernel's
-// (U / J, 2-norm): rings of 29,600 3.7e-8 / 4.8e-8 (5.4e-8 / 9.9e-8 there), random cloud of
-// 60,000 1.9e-7 / 2.9e-7 (2.2e-7 / 3.2e-7).
+// (U / J, 2-norm): rings of 60,000 4.1e-8 / 5.0e-8 (4.5e-8 / 8.1e-8 there), random cloud of
+// 65,536 1.9e-7 / 2.8e-7 (2.2e-7 / 3.2e-7).
 //
 // Classes, box to box, for a warp's 32 targets and a tile (tile_class):
-//   far   every pair past the kernel's singular reach and past 1.5 tile radii (little
+//   far   every pair past the kernel's singular reach and past TC_RAD tile radii (little
 //         cancellation in the polynomials), distances within a factor of 8 (the f16 range):
 //         the singular weights (Winckelmans has no reach: its own weights);
 //   mid   within the reach, past s = 2 (Gaussian-erf): the kernel's full form as the weight;
 //   near  the rest, pair by pair after the tensor pass as in uj_mixed_kernel.
-// At 65,536 random particles 87 / 8 / 5 % of the pairs, at 2^20 93 / 6 / 1 %.
+// At 65,536 random particles 87.6 / 9.2 / 3.2 % of the pairs, at 2^20 94.1 / 5.5 / 0.4 %.
 //
 // Layout: blocks of 128 targets in curve order, one a thread (4 warps), and a fifth warp that
 // loads the tiles (bulk copies, two stages) and issues the MMAs from uniform registers (12 to
@@ -42,8 +42,8 @@
 // MUFU, the f16 splits) plus 4 for its share of a tile's set-up, waits and recombination,
 // against 40.4 in uj_mixed_kernel; 66 % of the issue slots are used (4 warps a scheduler, the
 // TMEM's limit), the tensor pipe 17 %.  Measured, whole calls, Gaussian-erf: N = 2^20 1360 ->
-// 737 ms, 262,144 102.8 -> 54.1, 65,536 7.83 -> 4.3, rings of 200,000 57.8 -> 39.2, ring of
-// 32,000 2.40 -> 1.57; Winckelmans 50,001 4.61 -> 2.93.  Tried: packed pairs split back to
+// 735 ms, 262,144 102.8 -> 52.0, 65,536 7.83 -> 4.00, rings of 200,000 57.8 -> 39.5, ring of
+// 32,000 2.40 -> 1.52; Winckelmans 50,001 4.61 -> 2.66.  Tried: packed pairs split back to
 // scalar FP32 13 % slower, f16 remainders by conversion instead of the mixed-precision
 // subtraction 11 %, three blocks a SM 6 %, two A buffers of 16 sources (twice the barriers)
 // 16 %.
@@ -80,7 +80,7 @@ struct __align__(16) TileHdr {
     float chx, chy, chz, rad;
     float clx, cly, clz, sig2;     // sig2: the tile's largest sigma^2
     float hx, hy, hz, gscale;      // gscale: gam = gscale * (the pack's strength)
-    float yscale, ok, p0, p1;      // yscale: y = yscale * (the pack's y)
+    float yscale, ok, sig2lo, p1;  // yscale: y = yscale * (the pack's y); sig2lo: the smallest sigma^2
 };
 static_assert(sizeof(TileHdr) == 64, "header layout");
 
@@ -105,7 +105,7 @@ pack_tiles(int64_t n, const double* __restrict__ gs, const double* __restrict__ 
            const TgtPos* __restrict__ order, TileHdr* __restrict__ hdr, char* __restrict__ rec)
 {
     __shared__ double red[2][7];
-    __shared__ float redf[2][2];
+    __shared__ float redf[2][3];
     __shared__ __align__(16) char img[TC_B];
     const int k = threadIdx.x, warp = k >> 5, lane = k & 31;
     const int64_t o = (int64_t)blockIdx.x * TCS + k;
@@ -138,7 +138,7 @@ pack_tiles(int64_t n, const double* __restrict__ gs, const double* __restrict__ 
         y[m] = x[m] - c[m];
     }
     const float gmax = (float)fmax(red[0][6], red[1][6]);
-    float r2 = (float)(y[0] * y[0] + y[1] * y[1] + y[2] * y[2]), s2 = on ? (float)(sig * sig) : 0.f;
+    float r2 = (float)(y[0] * y[0] + y[1] * y[1] + y[2] * y[2]), s2 = on ? (float)(sig * sig) : 0.f, s2lo = on ? s2 : 3.0e38f;
     // the tile's fourth array: sigma^2 for Winckelmans, 1/sigma for the kernels with a singular tail
     const float mys2 = !on ? 1.f : singular_tail<K>() ? (float)(1.0 / sig) : s2;
     // a NaN position or core size must not hide in a maximum: it clears `ok`
@@ -146,8 +146,9 @@ pack_tiles(int64_t n, const double* __restrict__ gs, const double* __restrict__ 
     for (int s = 16; s > 0; s >>= 1) {
         r2 = fmaxf(r2, __shfl_xor_sync(0xffffffffu, r2, s));
         s2 = fmaxf(s2, __shfl_xor_sync(0xffffffffu, s2, s));
+        s2lo = fminf(s2lo, __shfl_xor_sync(0xffffffffu, s2lo, s));
     }
-    if (lane == 0) { redf[warp][0] = r2; redf[warp][1] = s2; }
+    if (lane == 0) { redf[warp][0] = r2; redf[warp][1] = s2; redf[warp][2] = s2lo; }
     const bool ok = __syncthreads_and(fine) && gmax < 1e30f && (gmax > 1e-30f || gmax == 0.f);
     const float rad = sqrtf(fmaxf(redf[0][0], redf[1][0])) * 1.000001f;
     const float ys = rad > 1e-30f ? pow2_at_least(rad) : 1.f;
@@ -190,7 +191,7 @@ pack_tiles(int64_t n, const double* __restrict__ gs, const double* __restrict__ 
         h.sig2 = fmaxf(redf[0][1], redf[1][1]);
         h.hx = half[0]; h.hy = half[1]; h.hz = half[2];
         h.gscale = gsc;
-        h.yscale = ys; h.ok = ok ? 1.f : 0.f; h.p0 = 0.f; h.p1 = 0.f;
+        h.yscale = ys; h.ok = ok ? 1.f : 0.f; h.sig2lo = fminf(redf[0][2], redf[1][2]); h.p1 = 0.f;
         hdr[blockIdx.x] = h;
         *(TileHdr*)(out + TC_B + 4 * TC_POS) = h;
     }
@@ -313,9 +314,15 @@ __device__ __forceinline__ void store_a(uint32_t a, const uint32_t (&gh)[8], con
 // extents wh): TILE_FAR, every pair past the kernel's singular reach; TILE_MID, within it but
 // past s = 2 (Gaussian-erf); both past the geometry's limits; else TILE_NEAR.  iR receives 1/R.
 enum : int { TILE_NEAR = 0, TILE_MID = 1, TILE_FAR = 2 };
-constexpr float TC_RAD = 1.5f;     // least distance of a far or mid tile, in tile radii
+// Least distance of a far or mid tile, in tile radii.  Nearer ones are evaluated pair by pair, at four
+// times the cost: 1.5 / 1.0 / 0.75 / 0.5 radii measured 4.30 / 4.06 / 4.00 / 3.92 ms at 65,536 random
+// particles, with the same errors but at 0.5 (rings of 30,000, Winckelmans: largest error of J
+// 3.7e-7 -> 6.6e-7 of the rms).
+constexpr float TC_RAD = 0.75f;
+// (A call of its own: it runs once for 32 tiles, and inlined its square roots cost the tile loop up to
+// 10 % through the registers and the order of the code around it: Winckelmans 100,000 10.0 -> 9.04 ms.)
 template <int K>
-__device__ __forceinline__ int tile_class(const TileHdr& h, const float3& wch, const float3& wcl, const float3& wh,
+__device__ __noinline__ int tile_class(const TileHdr& h, const float3& wch, const float3& wcl, const float3& wh,
                                           float wdiag, float& iR)
 {
     const float ax = fmaxf(fabsf((h.chx - wch.x) + (h.clx - wcl.x)) - h.hx - wh.x, 0.f);
@@ -324,9 +331,17 @@ __device__ __forceinline__ int tile_class(const TileHdr& h, const float3& wch, c
     const float d2 = fmaf(ax, ax, fmaf(ay, ay, az * az));
     const float dmin = sqrtf(d2);
     const float span = 2.f * (sqrtf(fmaf(h.hx, h.hx, fmaf(h.hy, h.hy, h.hz * h.hz))) + wdiag);
-    // R: the power of two in (4, 8] dmin
-    iR = __uint_as_float((251u << 23) - (__float_as_uint(dmin) & 0x7f800000u));
-    if (!(h.ok != 0.f && dmin > TC_RAD * h.rad && span < 7.f * dmin && dmin > 1e-9f && dmin < 1e9f)) return TILE_NEAR;
+    // R: the power of two in (4, 8] dmin.  Winckelmans' weights go by p = r^2 + sigma^2, up to 3.5 p^-2.5:
+    // there dmin^2 is the least p times 3.5^-0.4, and the p of the tile stay within 8^2
+    float unit = dmin;
+    bool range = span < 7.f * dmin;
+    if constexpr (!singular_tail<K>()) {
+        const float p = d2 + h.sig2lo, far = dmin + span;
+        unit = 0.778f * sqrtf(p);
+        range = fmaf(far, far, h.sig2) < 64.f * p;
+    }
+    iR = __uint_as_float((251u << 23) - (__float_as_uint(unit) & 0x7f800000u));
+    if (!(h.ok != 0.f && dmin > TC_RAD * h.rad && range && dmin > 1e-9f && unit < 1e9f)) return TILE_NEAR;
     const float sw = h.gscale * iR * iR * iR;      // the sums' unit stays well inside FP32
     if (!(sw > 1e-30f && sw < 1e30f)) return TILE_NEAR;
     if (!singular_tail<K>() || d2 > s_far<K>() * h.sig2) return TILE_FAR;
