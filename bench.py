@@ -39,19 +39,19 @@ N_PARTICLES = 1 << 20
 KERNEL = 2            # gaussianerf
 FLOP_PER_PAIR = 74    # VPM_FLOP_PER_UJ_PAIR
 FLOP_PER_ADJ_PAIR = 186   # VPM_FLOP_PER_UJ_ADJ_PAIR
-# DRAM bytes of one uj_mixed_kernel<gaussianerf> launch at N = 2^20, measured by ncu
+# DRAM bytes of one uj_tc_kernel<gaussianerf> launch at N = 2^20, measured by ncu
 # (`ncu --metrics gpu__time_duration.sum,dram__bytes_read.sum,dram__bytes_write.sum
-#  --clock-control none -k regex:uj_mixed_kernel -c 1 python bench.py --kernel-only --n 1048576
-#  --warmup 0 --steps 1`): 405,746,944 read + 181,722,112 written.  The compulsory traffic is
-# ~0.16 GB (56 B in, 96 B out a particle); the rest is re-reads of the 50 MB source pack that
-# miss L2.  Either way it is ~0.42 GB/s over the 1.41 s launch: the kernel is FP32-bound.
-UJ_DRAM_BYTES_2P20 = 405_746_944 + 181_722_112
+#  --clock-control none -k regex:uj_tc_kernel -c 1 python bench.py --kernel-only --n 1048576
+#  --warmup 0 --steps 1`): 145,001,999,360 read + 13,305,452,032 written.  The compulsory traffic is
+# ~0.16 GB (56 B in, 96 B out a particle); the rest is re-reads of the 154 MB of tiles that miss
+# the 129 MB L2 (30 MB at 2^18 fit: 0.15 GB in all).  It is 216 GB/s over the 0.734 s launch, 3 % of
+# the measured copy rate.
+UJ_DRAM_BYTES_2P20 = 145_001_999_360 + 13_305_452_032
 # (warp, 32-source tile) pairs within reach that one estr_mixed_kernel<gaussianerf> launch
-# loads on the 200,000-particle leapfrog rings: one cp.async commit (LDGDEPBAR) per loaded tile
-# in ncu's per-opcode counts of `python bench.py --kernel-only --estr --cloud rings --n 200000
-# --warmup 0 --steps 1` (2,967,977 commits, 4 LDGSTS each), of the 6,250 x 6,250 tile pairs.
+# loads on the 200,000-particle leapfrog rings, of the 6,250 x 6,250 tile pairs: the pairs whose
+# FP32 boxes lie within the kernel's reach, counted on the host over the curve order.
 # The reach depends on the positions and core sizes only, which the workload fixes.
-ESTR_TILES_IN_REACH_RINGS200K = 2_967_977
+ESTR_TILES_IN_REACH_RINGS200K = 2_941_019
 # the headline metric as the reference's benchmark definition names it; `value` is the
 # FP32-comp rate, `fp64_gpu` / `mixed_over_fp64` and `adjoint` carry the other two parts
 METRIC = "UJ pair-interactions/s, FP32-comp vs FP64 GPU @≤1e-6 rel err; adjoint/fwd ratio"
@@ -320,14 +320,16 @@ def run_gpu(args, rank, world):
             "e2e": {"value": e2e_value, "unit": "pairs/s", "h2d_bytes_per_step": 8 * 8 * n,
                     "d2h_bytes_per_step": 12 * 8 * n, "ms_per_step": 1e3 * statistics.mean(e2e_times),
                     "call": "vpm_uj(ctx, host 46xN matrix, RESET) = UJ_gb300_mixed(pfield)"},
-            "roofline": {"bound": "fp32", "achieved": achieved_tflops, "peak": peak_tflops,
+            "roofline": {"bound": "issue", "achieved": achieved_tflops, "peak": peak_tflops,
                          "unit": "TFLOP/s", "frac": achieved_tflops / peak_tflops,
                          "traffic": UJ_DRAM_BYTES_2P20 if n == 1 << 20 else None,
                          "traffic_unit": "bytes per launch",
                          "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of one N=2^20 launch "
-                                           "(405.7 + 181.7 MB; 1 pass, --clock-control none)",
-                         "kernel": "uj_mixed_kernel<gaussianerf>",
+                                           "(145.0 + 13.3 GB; 1 pass, --clock-control none)",
+                         "kernel": "uj_tc_kernel<gaussianerf>",
                          "flop_per_pair": FLOP_PER_PAIR,
+                         "note": "algorithmic flop over the FFMA peak; the far pairs' contraction runs on the "
+                                 "tensor cores, so frac reads above 1",
                          "peak_source": "FFMA-loop kernel measured in this run (no FP32 figure in "
                                         "MEASURED_PEAKS.json)",
                          "peak_nominal_2070MHz": 152 * 128 * 2 * 2.07e9 / 1e12,
@@ -437,7 +439,7 @@ def rings_blocks(ctx, vpm, torch, peak_tflops):
                     "them; tiles and 8-source sub-blocks whose every pair is past zeta/zeta(0) < 1e-13 are "
                     "skipped (their terms are below FP32 resolution), so that figure reads above 1. "
                     "tile_pairs_in_reach = the 32 x 32 pair slots of the (warp, source tile) pairs the kernel "
-                    "loads (ncu count of one launch on this workload); in_reach_frac counts those at 25 flop"}
+                    "loads (counted on the host on this workload); in_reach_frac counts those at 25 flop"}
     fld = ds.DeviceField(x.clone(), g.clone(), sg.clone(), kernel=KERNEL, precision=vpm.FP32COMP)
     sfs = ds.DynamicSFSParams()
     visc = ds.CoreSpreadingParams(nu=1e-4, sgm0=0.05)
@@ -502,7 +504,7 @@ def winckelmans_rate(ctx, vpm, torch, X, G, s):
     Ur, Jr = oracle.uj_pairs(X[sub], X, G, s, vpm._lib.KERNEL_WINCKELMANS)
     Uh, Jh = U.cpu().numpy()[sub], J.cpu().numpy()[sub]
     return {"value": float(n) * n / (ms / 1e3), "unit": "pairs/s", "n_particles": n, "ms": ms,
-            "kernel": "uj_mixed_kernel<winckelmans>",
+            "kernel": "uj_tc_kernel<winckelmans>",
             "error_vs_oracle": {"U_max_rel": float(np.abs(Uh - Ur).max() / np.abs(Ur).max()),
                                 "J_max_rel": float(np.abs(Jh - Jr).max() / np.abs(Jr).max()),
                                 "targets_checked": 256}}

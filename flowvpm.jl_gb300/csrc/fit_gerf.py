@@ -1,5 +1,6 @@
 """Generates the coefficients of the Gaussian-erf pair functions in vpm_math.cuh
-(gerf_GQ).  Run by hand (numpy + scipy); its output is pasted into the header.
+(gerf_GQ; gerf_S2_f64 and gerf_h_f64 in FP64).  Run by hand (numpy + scipy, mpmath for the FP64
+forms); its output is pasted into the header.
 
 The Gaussian-erf kernel's g(rho) = erf(rho/sqrt2) - sqrt(2/pi) rho e^{-rho^2/2}
 (src/FLOWVPM_kernel.jl:45-84) enters the pair term through, with s = rho^2,
@@ -41,6 +42,39 @@ def fit():
     return c, 1 / th, -tc / th
 
 
+def fit_f64():
+    """FP64 forms: Chebyshev interpolation in 50 digits.  erfcx(rho/sqrt2) = t P(w), P of degree 16
+    over rho in [sqrt2, 9]; S2 on [0, 2], degree 11.  Lowest powers first."""
+    import mpmath as mp
+    mp.mp.dps = 50
+
+    def interp(f, deg):   # power coefficients in w on [-1, 1]
+        nodes = [mp.cos(mp.pi * (k + mp.mpf(1) / 2) / (deg + 1)) for k in range(deg + 1)]
+        V = mp.matrix(deg + 1, deg + 1)
+        for i, x in enumerate(nodes):
+            for j in range(deg + 1):
+                V[i, j] = x ** j
+        return mp.lu_solve(V, mp.matrix([f(x) for x in nodes]))
+
+    tlo, thi = 1 / (1 + mp.mpf(9) / 2), 1 / (1 + mp.sqrt(2) / 2)
+    tc, th = (thi + tlo) / 2, (thi - tlo) / 2
+
+    def ex(w):
+        t = tc + th * w
+        rho = 2 * (1 / t - 1)
+        return mp.exp(rho * rho / 2) * mp.erfc(rho / mp.sqrt(2)) / t
+
+    def s2(s):
+        return mp.nsum(lambda m: s ** m / mp.fac2(2 * m + 5), [0, mp.inf])
+
+    c = interp(lambda w: s2(1 + w), 11)
+    poly = [mp.mpf(0)] * 12                       # back to powers of s = 1 + w
+    for j in range(12):
+        for i in range(j + 1):
+            poly[i] += c[j] * mp.binomial(j, i) * mp.mpf(-1) ** (j - i)
+    return interp(ex, 16), 1 / th, -tc / th, poly
+
+
 def main():
     c, A, B = fit()
     rho = np.linspace(RHO_LO, RHO_HI, 100001)
@@ -54,6 +88,13 @@ def main():
     for m in range(10):
         print(f"    {1.0 / d!r}f,")
         d *= 2 * m + 7
+    c, A, B, p = fit_f64()
+    print(f"// FP64: w = {float(A)!r} t + {float(B)!r}")
+    for a in list(c)[::-1]:
+        print(f"    {float(a)!r},")
+    print("// FP64 S2")
+    for a in p[::-1]:
+        print(f"    {float(a)!r},")
 
 
 if __name__ == "__main__":

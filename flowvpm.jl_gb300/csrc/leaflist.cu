@@ -12,8 +12,8 @@
 // running on across interval boundaries so that they are full, each source
 // carrying its interval's mask; a lane whose leaf is not in a source's mask
 // computes that pair with zero weight.  Pair math is
-// that of the all-pairs kernels (uj_pair.cuh for FP32-comp, the reference
-// formula for FP64); Estr uses the factored form of estr.cu with the self
+// that of the all-pairs kernels (two sources to an f32x2 instruction for FP32-comp, uj_pair.cuh for
+// FP64); Estr uses the factored form of estr.cu with the self
 // pair excluded by position.
 #include "dyn_math.cuh"
 #include "estr_tiles.cuh"

@@ -5,8 +5,8 @@
 // framework's caching pool, an arena reserved at start-up) or must not
 // allocate once they are running, so they cannot let the library call
 // cudaMalloc.  This entry point needs no context and allocates nothing: the
-// kernels' scratch (packed sources, the curve ordering of the targets and
-// the split-source partial sums) lives in one file-scope __device__ array of
+// kernels' scratch (packed sources, the curve ordering of the targets, the
+// split-source partial sums and, where they fit, the tensor pass's tiles) lives in one file-scope __device__ array of
 // VPM_NOALLOC_SCRATCH_BYTES, which every GPU that loads this library's code
 // for this entry point holds until the process exits.
 //

@@ -119,8 +119,8 @@ int vpm_ctx_set_stream(vpm_ctx* ctx, void* stream);
  * context unusable. */
 int vpm_ctx_set_timeout(vpm_ctx* ctx, double seconds);
 /* Capacities, in pairs, of the near-field list builder's traversal buffers for
- * the next build of this context: node pairs of one frontier and near leaf
- * pairs (by default 40 n and 24 n, n >= 4096).  A build that overflows them
+ * the next build of this context: node pairs to be split of one frontier and near leaf
+ * pairs (by default 10 n and 24 n, n >= 4096).  A build that overflows them
  * doubles them and traverses again, so they only trade device memory for
  * repeated traversals; the lists do not depend on them.  Library plumbing (the
  * reference's FastMultipole sizes its own lists). */
