@@ -92,38 +92,38 @@ __global__ void __launch_bounds__(BB_THREADS)
 hilbert_keys(int64_t n, const double* __restrict__ x, const double* __restrict__ part, int bits,
              Key* __restrict__ keys, int32_t* __restrict__ idx)
 {
-    // the box from the 256 partial ones, one a thread
-    __shared__ double red[6][BB_THREADS / 32];
-    static_assert(BB_BLOCKS == BB_THREADS, "one partial box a thread");
+    // The box from the 256 partial ones, a warp a side, and the scale, once a block: the FP64 pipe
+    // (16 cycles a warp instruction) is what this kernel waits for, and with every thread at all of
+    // it 5,600 particles took 11.2 us and 100,000 took 28.
+    __shared__ double box[6], scale;
+    static_assert(BB_BLOCKS == 256 && BB_THREADS >= 192, "six warps, eight boxes a lane");
+    const double top = (double)((1u << bits) - 1u);
+    if (threadIdx.x < 192) {
+        const int k = threadIdx.x >> 5, lane = threadIdx.x & 31;
+        double v[8];
 #pragma unroll
-    for (int k = 0; k < 6; k++) {
-        double v = part[threadIdx.x * 6 + k];
+        for (int j = 0; j < 8; j++) v[j] = part[(lane + 32 * j) * 6 + k];
+#pragma unroll
+        for (int j = 1; j < 8; j++) v[0] = k < 3 ? fmin(v[0], v[j]) : fmax(v[0], v[j]);
 #pragma unroll
         for (int m = 16; m > 0; m >>= 1) {
-            const double o = __shfl_xor_sync(0xffffffffu, v, m);
-            v = k < 3 ? fmin(v, o) : fmax(v, o);
+            const double o = __shfl_xor_sync(0xffffffffu, v[0], m);
+            v[0] = k < 3 ? fmin(v[0], o) : fmax(v[0], o);
         }
-        if ((threadIdx.x & 31) == 0) red[k][threadIdx.x >> 5] = v;
+        if (lane == 0) box[k] = v[0];
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        const double ext = fmax(fmax(fmax(box[3] - box[0], box[4] - box[1]), box[5] - box[2]), 0.0);
+        scale = ext > 0.0 ? top / ext : 0.0;
     }
     __syncthreads();
     const int64_t i = blockIdx.x * (int64_t)BB_THREADS + threadIdx.x;
     if (i >= n) return;
-    double lo[3], ext = 0.0;
-#pragma unroll
-    for (int k = 0; k < 3; k++) {
-        double a = red[k][0], b = red[3 + k][0];
-#pragma unroll
-        for (int w = 1; w < BB_THREADS / 32; w++) {
-            a = fmin(a, red[k][w]);
-            b = fmax(b, red[3 + k][w]);
-        }
-        lo[k] = a;
-        ext = fmax(ext, b - a);
-    }
     uint32_t q[3];
-    const double top = (double)((1u << bits) - 1u), sc = ext > 0.0 ? top / ext : 0.0;
 #pragma unroll
-    for (int k = 0; k < 3; k++) q[k] = (uint32_t)fmin(fmax((x[3 * i + k] - lo[k]) * sc, 0.0), top);
+    for (int k = 0; k < 3; k++)   // the conversion takes values below 0 to 0, the minimum the rest (NaN too) to the top
+        q[k] = min(__double2uint_rz((x[3 * i + k] - box[k]) * scale), (1u << bits) - 1u);
     keys[i] = hilbert_index<Key>(q, bits);
     idx[i] = (int32_t)i;
 }
@@ -148,8 +148,8 @@ static inline size_t align256(size_t b) { return (b + 255) / 256 * 256; }
 // Up to RANK_MAX particles: each one's place is the number of keys before it, counted (lane =
 // particle, the block's warps share the keys), and its record goes there: one launch for the sort's
 // six and the gather.  n^2 compares are 4 us at 8,192 particles, but 60 us at 32,000, where the
-// sort takes 45.  UJ calls with the sort -> with ranks: 8,192 356 -> 300 us, 16,000 594 -> 579,
-// 24,000 976 -> 1004; a sort of everything in one block takes 20 us more at 6,100 than the ranks
+// sort takes 45.  UJ calls with the sort -> with ranks (before the key reads were unrolled):
+// 8,192 356 -> 300 us, 16,000 594 -> 579, 24,000 976 -> 1004; a sort of everything in one block takes 20 us more at 6,100 than the ranks
 // and as long at 1,400.
 constexpr int64_t RANK_MAX = 16384;
 constexpr int RANK_THREADS = 1024;
@@ -167,16 +167,24 @@ order_rank(int n, const double* __restrict__ x, const uint32_t* __restrict__ key
         t.idx = j; t.pad = 0;
     }
     int c = 0;
-    for (int q = warp; q < n / 4; q += RANK_THREADS / 32) {   // equal keys keep the caller's order
-        const uint4 k = ((const uint4*)keys)[q];
-        if (4 * q < i0) {
-            c += (k.x <= key) + (k.y <= key) + (k.z <= key) + (k.w <= key);
-        } else if (4 * q >= i0 + 32) {
-            c += (k.x < key) + (k.y < key) + (k.z < key) + (k.w < key);
-        } else {
-            c += (k.x < key || (k.x == key && 4 * q < i)) + (k.y < key || (k.y == key && 4 * q + 1 < i)) +
-                 (k.z < key || (k.z == key && 4 * q + 2 < i)) + (k.w < key || (k.w == key && 4 * q + 3 < i));
-        }
+    // equal keys keep the caller's order; the block's own 32 keys are quads i0/4 .. i0/4 + 7
+    const uint4* k4 = (const uint4*)keys;
+    const int own = i0 / 4, quads = n / 4;
+#pragma unroll 4
+    for (int q = warp; q < own; q += RANK_THREADS / 32) {
+        const uint4 k = k4[q];
+        c += (k.x <= key) + (k.y <= key) + (k.z <= key) + (k.w <= key);
+    }
+    if (warp < 8 && own + warp < quads) {
+        const int j = 4 * (own + warp);
+        const uint4 k = k4[own + warp];
+        c += (k.x < key || (k.x == key && j < i)) + (k.y < key || (k.y == key && j + 1 < i)) +
+             (k.z < key || (k.z == key && j + 2 < i)) + (k.w < key || (k.w == key && j + 3 < i));
+    }
+#pragma unroll 4
+    for (int q = own + 8 + warp; q < quads; q += RANK_THREADS / 32) {
+        const uint4 k = k4[q];
+        c += (k.x < key) + (k.y < key) + (k.z < key) + (k.w < key);
     }
     if (warp == 0)
         for (int j = n / 4 * 4; j < n; j++) c += keys[j] < key || (keys[j] == key && j < i);
