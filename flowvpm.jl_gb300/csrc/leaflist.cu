@@ -249,7 +249,8 @@ struct __align__(16) UjTile {
     unsigned mask[32];
 };
 
-// Box of a warp's targets (FP32 high parts), by its lane 0 to box[0..1].
+// Box of a warp's targets, by its lane 0 to box[0..1]: their FP32 high parts, widened by 2^-21 of
+// the coordinates, more than what the low parts of targets and sources can add to a distance.
 __device__ __forceinline__ void target_box(const float3& th, int lane, float4* box)
 {
     float3 lo = th, hi = th;
@@ -260,8 +261,10 @@ __device__ __forceinline__ void target_box(const float3& th, int lane, float4* b
         lo.z = fminf(lo.z, __shfl_xor_sync(0xffffffffu, lo.z, m)); hi.z = fmaxf(hi.z, __shfl_xor_sync(0xffffffffu, hi.z, m));
     }
     if (lane == 0) {
-        box[0] = make_float4(lo.x, lo.y, lo.z, 0.f);
-        box[1] = make_float4(hi.x, hi.y, hi.z, 0.f);
+        const float d = 4.76837158203125e-07f * fmaxf(fmaxf(fmaxf(fabsf(lo.x), fabsf(hi.x)), fmaxf(fabsf(lo.y), fabsf(hi.y))),
+                                                      fmaxf(fabsf(lo.z), fabsf(hi.z)));
+        box[0] = make_float4(lo.x - d, lo.y - d, lo.z - d, 0.f);
+        box[1] = make_float4(hi.x + d, hi.y + d, hi.z + d, 0.f);
     }
     __syncwarp();
 }
@@ -348,7 +351,7 @@ nf_uj_mixed(int64_t n, int64_t ngroups, const TgtPos* __restrict__ tgt, const in
         T.mask[lane] = smask;
         const float d2 = box_d2(box[warp], sj.a.x, sj.a.y, sj.a.z);
         const unsigned care = __ballot_sync(0xffffffffu, !(d2 > 0.0f) || (smask & all) != all);
-        const unsigned close = __ballot_sync(0xffffffffu, !(d2 * sj.a.w > 2.5f));   // 2, and room for the low parts
+        const unsigned close = __ballot_sync(0xffffffffu, !(d2 * sj.a.w > 2.01f));   // 2, and room for roundings
         __syncwarp();
 #pragma unroll 1
         for (int j = 0; j < cnt; j += 4) {   // cnt <= 32: j + 3 stays in the tile

@@ -32,6 +32,24 @@ def test_near_uj_blocks(n, leaf, kernel):
         assert (a - b).norm() <= 16 * 2.0 ** -24 * b.norm() + 1e-14
 
 
+@pytest.mark.parametrize("shift", [0.0, 1e5, 1e7])
+def test_near_sums_far_from_the_origin(shift):
+    """Coordinates of up to 10^8 core sizes, where FP32 does not resolve a core: the box tests that choose
+    the pair form and skip sources have to see the low parts too."""
+    rng = np.random.default_rng(8)
+    n = 2000
+    T = lambda a: torch.tensor(a, device="cuda", dtype=torch.float64)       # noqa: E731
+    x, gam, sig = T(rng.random((n, 3)) + shift), T(rng.standard_normal((n, 3))), T(0.1 * (0.7 + 0.6 * rng.random(n)))
+    out = []
+    for precision in (0, 1):
+        U, J, S = (torch.zeros(n, k, device="cuda", dtype=torch.float64) for k in (3, 9, 3))
+        vpm.default_context().p2p_leaflist_dev(x, gam, sig, U, J, S, leaf_size=20, theta=0.5, precision=precision, sfs=True)
+        out.append((U, J))
+    # as above, and the coordinates' own rounding to 2^-48 of the shift against distances near 0.03
+    for a, b in zip(out[1], out[0]):
+        assert (a - b).norm() <= (16 * 2.0 ** -24 + 5 * shift * 2.0 ** -48 / 0.03) * b.norm()
+
+
 @pytest.mark.parametrize("leaf,theta", [(1, 0.4), (3, 0.9), (64, 0.0)])
 @pytest.mark.parametrize("spread", [1e-9, 3e-8, 1e-7, 1e-6])
 def test_lists_of_points_closer_than_fp32_centres(spread, leaf, theta):
