@@ -238,7 +238,7 @@ constexpr int ESTR_FLUSH_TILES = 24;     // evaluated warp tiles between FP64 ad
 // sources are all out of reach of the warp's target box, before their distances are
 // formed, or of every target, after.  Sums: 8-source FP32 partials added with
 // compensation (comp_add2), FP64 every ESTR_FLUSH_TILES evaluated tiles.
-// Bound: the FMA pipe (61 % busy) and shared-memory reads (67 %).  With two sources to an f32x2
+// Bound: shared-memory reads (74 % of the rate) and the FMA pipe (61 % busy).  With two sources to an f32x2
 // instruction and 16-byte reads of four sources' coordinates a pair takes 18 issue slots; one
 // source at a time from 64-byte records took 24 and 80 % of the shared-memory rate (every lane
 // reads every source, and the records' copies and conversions met bank conflicts).  Rings of

@@ -725,8 +725,9 @@ nf_estr(int64_t n, int64_t ngroups, const TgtPos* __restrict__ tgt, const int32_
 static inline size_t al256(size_t b) { return (b + 255) / 256 * 256; }
 
 // Warps a group: enough for 16 blocks a SM, at most 8 (each walks the whole list to find its
-// tiles).  One block a SM's worth of uneven groups left most of it idle: near-field call of a
-// 100,000-particle jet 6.4 ms, of 1,048,576 21.7 ms.
+// tiles).  With one warp a group a few blocks of uneven groups left most of the chip idle: near-field
+// UJ and Estr calls of a 20,000-particle jet 1.94 -> 1.70 ms, 100,000 6.34 -> 5.52, 2^20 unchanged
+// (one warp a group there).
 static int near_parts(int64_t n, int num_sms)
 {
     const int64_t blocks = (n + NF_THREADS - 1) / NF_THREADS;
