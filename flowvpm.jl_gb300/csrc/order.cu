@@ -147,11 +147,10 @@ static inline size_t align256(size_t b) { return (b + 255) / 256 * 256; }
 
 // Up to RANK_MAX particles: each one's place is the number of keys before it, counted (lane =
 // particle, the block's warps share the keys), and its record goes there: one launch for the sort's
-// six and the gather.  n^2 compares are 4 us at 8,192 particles, but 60 us at 32,000, where the
-// sort takes 45.  UJ calls with the sort -> with ranks (before the key reads were unrolled):
-// 8,192 356 -> 300 us, 16,000 594 -> 579, 24,000 976 -> 1004; a sort of everything in one block takes 20 us more at 6,100 than the ranks
-// and as long at 1,400.
-constexpr int64_t RANK_MAX = 16384;
+// six and the gather, but n^2 compares.  UJ calls with the sort / with ranks, us: 8,192 356 / 290,
+// 18,000 627 / 599, 20,000 706 / 694, 24,000 890 / 889, 28,000 1060 / 1087.  A sort of everything in
+// one block took 20 us more at 6,100 than the ranks, and as long at 1,400.
+constexpr int64_t RANK_MAX = 20480;
 constexpr int RANK_THREADS = 1024;
 __global__ void __launch_bounds__(RANK_THREADS)
 order_rank(int n, const double* __restrict__ x, const uint32_t* __restrict__ keys, TgtPos* __restrict__ out)

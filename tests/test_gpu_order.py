@@ -14,7 +14,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("shape", ["cloud", "line", "plane", "point"])
-@pytest.mark.parametrize("n", [1, 2, 700, 1024, 1025, 2049, 4097, 6144, 6145, 65536, 65537, 31, 33, 35, 16383, 16384, 16385])
+@pytest.mark.parametrize("n", [1, 2, 700, 1024, 1025, 2049, 4097, 6144, 6145, 65536, 65537, 31, 33, 35, 20479, 20480, 20481])
 def test_ordered_sums(ctx, n, shape):
     X, G, s = random_cloud(n, seed=n)
     if shape == "line":
