@@ -21,6 +21,8 @@
 #include "internal.h"
 #include "vpm_math.cuh"
 
+#include <type_traits>
+
 namespace vpm {
 
 static inline int64_t round_up(int64_t a, int64_t b) { return (a + b - 1) / b * b; }
@@ -231,7 +233,9 @@ constexpr int ESTR_FLUSH_TILES = 24;     // evaluated warp tiles between FP64 ad
 // own offset is formed by the same operations, so that the self pair and
 // coincident particles have
 // r^2 == 0 exactly (they are skipped: their terms would only cancel to FP32
-// rounding, at the largest weight).  For the Gaussian kernels the terms past
+// rounding, at the largest weight).  Where the targets' box is wide against a source's
+// core and the source close to it, the displacement takes in what the offsets' rounding left
+// and is rounded to its own size: ESTR_WIDE, ESTR_CLOSE.  For the Gaussian kernels the terms past
 // zeta_skip_s (zeta/zeta(0) < 1e-13: below the FP32 resolution of the sums) are
 // skipped at three levels: a tile whose pack box is out of reach of the warp's
 // targets is not loaded (TileWalk); of a loaded tile, the 8-source sub-blocks whose
@@ -242,7 +246,8 @@ constexpr int ESTR_FLUSH_TILES = 24;     // evaluated warp tiles between FP64 ad
 // instruction and 16-byte reads of four sources' coordinates a pair takes 18 issue slots; one
 // source at a time from 64-byte records took 24 and 80 % of the shared-memory rate (every lane
 // reads every source, and the records' copies and conversions met bank conflicts).  Rings of
-// 200,000: 3.77 -> 3.01 ms; jet of 100,000, Winckelmans (no reach): 9.70 -> 8.55 ms.
+// 200,000: 3.77 -> 3.08 ms; jet of 100,000, Winckelmans (no reach): 9.70 -> 8.69 ms (3.01 and
+// 8.55 before the test for coarse offsets).
 // With DZ (the weight difference of the dynamic procedure's test filter,
 // dynamic.cu) each weight zeta~(r, sigma_s) is replaced by
 // zeta~(r, alpha sigma_s) - zeta~(r, sigma_s) = zeta~(r, sigma_s) (ratio - 1),
@@ -271,18 +276,19 @@ estr_mixed_kernel(int64_t nt, const TgtPos* __restrict__ tgt, const double* __re
     const float3 ol = make_float3((float)(ox - (double)oh.x), (float)(oy - (double)oh.y), (float)(oz - (double)oh.z));
     // the target's offset by the same FP32 double-float operations as the sources' (below);
     // padding lanes sit at the origin
-    float3 to = make_float3(0.f, 0.f, 0.f);
+    float3 to = make_float3(0.f, 0.f, 0.f), tr = to;      // and what its rounding left
     if (t < nt) {
         const float3 th = make_float3((float)tx, (float)ty, (float)tz);
         const float3 tl = make_float3((float)(tx - (double)th.x), (float)(ty - (double)th.y),
                                       (float)(tz - (double)th.z));
-        to = make_float3(df_offset(th.x, tl.x, oh.x, ol.x), df_offset(th.y, tl.y, oh.y, ol.y),
-                         df_offset(th.z, tl.z, oh.z, ol.z));
+        to = make_float3(df_offset(th.x, tl.x, oh.x, ol.x, tr.x), df_offset(th.y, tl.y, oh.y, ol.y, tr.y),
+                         df_offset(th.z, tl.z, oh.z, ol.z, tr.z));
     }
     // the warp's target boxes: offsets (for the per-source test of a tile) and FP32
     // positions of its targets (for the tile boxes of the pack); [0], [1] = offsets low,
     // high; [2], [3] = positions low, high (empty without a target)
     __shared__ float4 wbox[UJ_WARPS][4];
+    float ext;
     {
         float v[12] = {to.x, to.y, to.z, -to.x, -to.y, -to.z};
         const bool real = t < nt;
@@ -296,6 +302,7 @@ estr_mixed_kernel(int64_t nt, const TgtPos* __restrict__ tgt, const double* __re
         for (int m = 16; m > 0; m >>= 1)
 #pragma unroll
             for (int k = 0; k < 12; k++) v[k] = fminf(v[k], __shfl_xor_sync(0xffffffffu, v[k], m));
+        ext = fmaxf(fmaxf(-v[3] - v[0], -v[4] - v[1]), -v[5] - v[2]);
         if (lane == 0) {
             wbox[warp][0] = make_float4(v[0], v[1], v[2], 0.f);
             wbox[warp][1] = make_float4(-v[3], -v[4], -v[5], 0.f);
@@ -306,7 +313,7 @@ estr_mixed_kernel(int64_t nt, const TgtPos* __restrict__ tgt, const double* __re
     }
     double zg[3] = {0.0, 0.0, 0.0}, zv[3] = {0.0, 0.0, 0.0};
     f32x2 sm[3] = {0ull, 0ull, 0ull}, cm[3] = {0ull, 0ull, 0ull};   // compensated sums (gx gy)(gz vx)(vy vz)
-    const f32x2 TX = pk(-to.x, -to.x), TY = pk(-to.y, -to.y), TZ = pk(-to.z, -to.z);
+    const float ext2 = ext * ext;
     auto load = [&](int tile, int b) {   // 104 chunks of 16 bytes
         const float4* g = (const float4*)&src[tile];
         float4* d = (float4*)&stage[warp][b];
@@ -331,47 +338,53 @@ estr_mixed_kernel(int64_t nt, const TgtPos* __restrict__ tgt, const double* __re
         }
         __syncwarp();
         EstrTile& T = stage[warp][buf];
-        // the tile's sources out of reach of the whole target box, and those inside it, the only
-        // ones that can be at r = 0 from a target
-        unsigned beyond, inside;
+        // the tile's sources out of reach of the whole target box, those inside it, the only ones that
+        // can be at r = 0 from a target, and those whose offsets are too coarse
+        unsigned beyond, inside, coarse;
         {   // this lane's source: FP32 offset
-            const float px = df_offset(T.x[lane], T.xl[lane], oh.x, ol.x), py = df_offset(T.y[lane], T.yl[lane], oh.y, ol.y),
-                        pz = df_offset(T.z[lane], T.zl[lane], oh.z, ol.z);
+            const float hx = T.x[lane], hy = T.y[lane], hz = T.z[lane], w = T.w[lane];
+            const float lx = T.xl[lane], ly = T.yl[lane], lz = T.zl[lane];
+            const float px = df_offset(hx, lx, oh.x, ol.x), py = df_offset(hy, ly, oh.y, ol.y),
+                        pz = df_offset(hz, lz, oh.z, ol.z);
             T.x[lane] = px; T.y[lane] = py; T.z[lane] = pz;
             const float4 lo = wbox[warp][0], hi = wbox[warp][1];
             const float ex = fmaxf(fmaxf(lo.x - px, px - hi.x), 0.0f);
             const float ey = fmaxf(fmaxf(lo.y - py, py - hi.y), 0.0f);
             const float ez = fmaxf(fmaxf(lo.z - pz, pz - hi.z), 0.0f);
-            const float d2 = fmaf(ex, ex, fmaf(ey, ey, ez * ez));
-            beyond = __ballot_sync(0xffffffffu, zeta_skip_s<K>() > 0.0f && d2 * T.w[lane] > zeta_skip_s<K>());
+            const float d2 = fmaf(ex, ex, fmaf(ey, ey, ez * ez)), ds = d2 * w;
+            beyond = __ballot_sync(0xffffffffu, zeta_skip_s<K>() > 0.0f && ds > zeta_skip_s<K>());
             inside = __ballot_sync(0xffffffffu, !(d2 > 0.0f));
+            coarse = __ballot_sync(0xffffffffu, ext2 * w > ESTR_WIDE && ds < ESTR_CLOSE);
+            if (__builtin_expect(coarse != 0u, 0)) {
+                float rx, ry, rz;
+                df_offset(hx, lx, oh.x, ol.x, rx);
+                df_offset(hy, ly, oh.y, ol.y, ry);
+                df_offset(hz, lz, oh.z, ol.z, rz);
+                T.xl[lane] = rx; T.yl[lane] = ry; T.zl[lane] = rz;
+            }
         }
         __syncwarp();
         if (beyond != 0xffffffffu) {
+            // (two loops: with the choice inside one loop the dense fields took 15 % longer)
+            auto sources = [&](auto two_parts) {
 #pragma unroll 1
-            for (int sub = 0; sub < EWT; sub += ESTR_SUB) {
-                if (((beyond >> sub) & 0xffu) == 0xffu) continue;
-                f32x2 r2[4], s[4];
+                for (int sub = 0; sub < EWT; sub += ESTR_SUB) {
+                    if (((beyond >> sub) & 0xffu) == 0xffu) continue;
+                    f32x2 r2[4], s[4];
+                    if (decltype(two_parts)::value && ((coarse >> sub) & 0xffu)) estr_r2s8(T, sub, to, tr, r2, s);
+                    else estr_r2s8(T, sub, to, r2, s);
+                    if (zeta_skip_s<K>() > 0.0f && __all_sync(0xffffffffu, min8_nan(s) > zeta_skip_s<K>())) continue;
+                    f32x2 f[3] = {0ull, 0ull, 0ull};
+                    if (!ZETA && ((inside >> sub) & 0xffu))
+                        estr_add8<K, ZETA, DZ, false, !ZETA>(r2, s, &T.gv[3 * sub], 0u, nullptr, fd, f);
+                    else
+                        estr_add8<K, ZETA, DZ, false, false>(r2, s, &T.gv[3 * sub], 0u, nullptr, fd, f);
 #pragma unroll
-                for (int q = 0; q < 2; q++) {
-                    const ulonglong2 X = *(const ulonglong2*)&T.x[sub + 4 * q], Y = *(const ulonglong2*)&T.y[sub + 4 * q],
-                                     Z = *(const ulonglong2*)&T.z[sub + 4 * q], W = *(const ulonglong2*)&T.w[sub + 4 * q];
-                    f32x2 dx = add2(X.x, TX), dy = add2(Y.x, TY), dz = add2(Z.x, TZ);
-                    r2[2 * q] = fma2(dx, dx, fma2(dy, dy, mul2(dz, dz)));
-                    s[2 * q] = mul2(r2[2 * q], W.x);
-                    dx = add2(X.y, TX); dy = add2(Y.y, TY); dz = add2(Z.y, TZ);
-                    r2[2 * q + 1] = fma2(dx, dx, fma2(dy, dy, mul2(dz, dz)));
-                    s[2 * q + 1] = mul2(r2[2 * q + 1], W.y);
+                    for (int k = 0; k < (ZETA ? 2 : 3); k++) comp_add2(sm[k], cm[k], f[k]);
                 }
-                if (zeta_skip_s<K>() > 0.0f && __all_sync(0xffffffffu, min8_nan(s) > zeta_skip_s<K>())) continue;
-                f32x2 f[3] = {0ull, 0ull, 0ull};
-                if (!ZETA && ((inside >> sub) & 0xffu))
-                    estr_add8<K, ZETA, DZ, false, !ZETA>(r2, s, &T.gv[3 * sub], 0u, nullptr, fd, f);
-                else
-                    estr_add8<K, ZETA, DZ, false, false>(r2, s, &T.gv[3 * sub], 0u, nullptr, fd, f);
-#pragma unroll
-                for (int k = 0; k < (ZETA ? 2 : 3); k++) comp_add2(sm[k], cm[k], f[k]);
-            }
+            };
+            if (__builtin_expect(coarse != 0u, 0)) sources(std::true_type());
+            else sources(std::false_type());
             // skipped tiles add nothing, so only the tiles taken count towards a flush
             if (++in_flush == ESTR_FLUSH_TILES) {
                 in_flush = 0;

@@ -12,9 +12,19 @@ namespace vpm {
 
 constexpr int EST_TILE = 32;   // particles per tile (one per lane of a warp)
 
+// The rounding of two FP32 offsets of size |o| changes a weight by dlog(zeta)/ds 2 sqrt(s) |o|/sigma
+// 2^-24 or so, with |o| up to the box's extent E plus the distance.  Within E = 4 sigma that is at most
+// 4 ulp of zeta(0) at any distance; in wider boxes sources nearer than 3 sigma to the box take
+// both parts of the offsets (farther ones are below 3 ulp of zeta(0) up to E = 100 sigma, since zeta
+// itself falls off).  A random cloud of 1,600 has E = 40 sigma, and its sums are a few close pairs: their
+// SFS was 2e-6 of its norm off.  Rings of 60,000 and more stay on the offsets (E = 0.9 to 2.7 sigma for
+// nine warps in ten).
+constexpr float ESTR_WIDE = 16.0f;       // (E/sigma)^2
+constexpr float ESTR_CLOSE = 9.0f;       // (distance from the box/sigma)^2
+
 // A tile of sources for the mixed Estr kernels (estr.cu, leaflist.cu), in the form their inner loop
-// reads: coordinates (x, y, z high parts, turned into offsets in place by estr.cu; xl, yl, zl low
-// parts) and w = 1/sigma^2 as arrays, so that one 16-byte broadcast read serves four sources and
+// reads: coordinates (x, y, z high parts, xl, yl, zl low
+// parts; both turned into offsets in place by estr.cu) and w = 1/sigma^2 as arrays, so that one 16-byte broadcast read serves four sources and
 // f32x2 instructions take two of them; and the payload g, v = ZNORM (Gamma, J^T Gamma)/sigma^3 as
 // (gx gy)(gz vx)(vy vz), three f32x2 a source, 24 bytes instead of two float4.
 struct __align__(128) EstrTile {
@@ -22,6 +32,49 @@ struct __align__(128) EstrTile {
     float2 gv[3 * EST_TILE];
 };
 static_assert(sizeof(EstrTile) == 1664, "whole 16-byte chunks, no padding");
+
+// r^2 and s = r^2/sigma^2 of the tile's sources j .. j + 7 for a target at th + tl, from both
+// parts of the positions: the rounding is of the displacement's own size.
+__device__ __forceinline__ void estr_r2s8(const EstrTile& T, int j, const float3& th, const float3& tl, f32x2 (&r2)[4],
+                                          f32x2 (&s)[4])
+{
+    const f32x2 HX = pk(-th.x, -th.x), HY = pk(-th.y, -th.y), HZ = pk(-th.z, -th.z);
+    const f32x2 LX = pk(-tl.x, -tl.x), LY = pk(-tl.y, -tl.y), LZ = pk(-tl.z, -tl.z);
+#pragma unroll
+    for (int c = 0; c < 2; c++) {
+        const int i = j + 4 * c;
+        const ulonglong2 X = *(const ulonglong2*)&T.x[i], Y = *(const ulonglong2*)&T.y[i],
+                         Z = *(const ulonglong2*)&T.z[i], W = *(const ulonglong2*)&T.w[i],
+                         XL = *(const ulonglong2*)&T.xl[i], YL = *(const ulonglong2*)&T.yl[i],
+                         ZL = *(const ulonglong2*)&T.zl[i];
+        f32x2 dx = add2(add2(X.x, HX), add2(XL.x, LX)), dy = add2(add2(Y.x, HY), add2(YL.x, LY)),
+              dz = add2(add2(Z.x, HZ), add2(ZL.x, LZ));
+        r2[2 * c] = fma2(dx, dx, fma2(dy, dy, mul2(dz, dz)));
+        s[2 * c] = mul2(r2[2 * c], W.x);
+        dx = add2(add2(X.y, HX), add2(XL.y, LX)); dy = add2(add2(Y.y, HY), add2(YL.y, LY));
+        dz = add2(add2(Z.y, HZ), add2(ZL.y, LZ));
+        r2[2 * c + 1] = fma2(dx, dx, fma2(dy, dy, mul2(dz, dz)));
+        s[2 * c + 1] = mul2(r2[2 * c + 1], W.y);
+    }
+}
+
+// ... from the high parts (offsets) alone
+__device__ __forceinline__ void estr_r2s8(const EstrTile& T, int j, const float3& to, f32x2 (&r2)[4], f32x2 (&s)[4])
+{
+    const f32x2 TX = pk(-to.x, -to.x), TY = pk(-to.y, -to.y), TZ = pk(-to.z, -to.z);
+#pragma unroll
+    for (int c = 0; c < 2; c++) {
+        const int i = j + 4 * c;
+        const ulonglong2 X = *(const ulonglong2*)&T.x[i], Y = *(const ulonglong2*)&T.y[i],
+                         Z = *(const ulonglong2*)&T.z[i], W = *(const ulonglong2*)&T.w[i];
+        f32x2 dx = add2(X.x, TX), dy = add2(Y.x, TY), dz = add2(Z.x, TZ);
+        r2[2 * c] = fma2(dx, dx, fma2(dy, dy, mul2(dz, dz)));
+        s[2 * c] = mul2(r2[2 * c], W.x);
+        dx = add2(X.y, TX); dy = add2(Y.y, TY); dz = add2(Z.y, TZ);
+        r2[2 * c + 1] = fma2(dx, dx, fma2(dy, dy, mul2(dz, dz)));
+        s[2 * c + 1] = mul2(r2[2 * c + 1], W.y);
+    }
+}
 
 // Payload sums of 8 sources: f[0..2] += z (gx gy)(gz vx)(vy vz) for the weights of r2/s pairs
 // (s = r2/sigma^2).  MASKED: sources whose target mask (`mask`) lacks `bit` add nothing.

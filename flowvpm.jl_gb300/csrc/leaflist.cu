@@ -607,8 +607,6 @@ nf_estr(int64_t n, int64_t ngroups, const TgtPos* __restrict__ tgt, const int32_
     // mixed: compensated FP32 sums of 8-source partial sums (comp_add), FP64 every NF_ESTR_FLUSH tiles
     // (as the all-pairs mixed Estr; the FP64 pipe runs at 1/64 of the FP32 rate)
     f32x2 sm[3] = {0ull, 0ull, 0ull}, cm[3] = {0ull, 0ull, 0ull};
-    const f32x2 HX = pk(-th.x, -th.x), HY = pk(-th.y, -th.y), HZ = pk(-th.z, -th.z);
-    const f32x2 LX = pk(-tl.x, -tl.x), LY = pk(-tl.y, -tl.y), LZ = pk(-tl.z, -tl.z);
     const unsigned all = __reduce_or_sync(0xffffffffu, bit);   // the group's live leaves
     // box of the group's targets (high parts): sources out of its reach are skipped as in the
     // all-pairs kernel, and only those inside it can be at r = 0 from a target
@@ -658,22 +656,7 @@ nf_estr(int64_t n, int64_t ngroups, const TgtPos* __restrict__ tgt, const int32_
             for (int j0 = 0; j0 < cnt; j0 += 8) {   // cnt <= 32: j0 + 7 stays in the tile (padding has mask 0)
                 if (((beyond >> j0) & 0xffu) == 0xffu) continue;
                 f32x2 r2[4], s[4], f[3] = {0ull, 0ull, 0ull};
-#pragma unroll
-                for (int c = 0; c < 2; c++) {
-                    const int j = j0 + 4 * c;
-                    const ulonglong2 X = *(const ulonglong2*)&q.x[j], Y = *(const ulonglong2*)&q.y[j],
-                                     Z = *(const ulonglong2*)&q.z[j], W = *(const ulonglong2*)&q.w[j],
-                                     XL = *(const ulonglong2*)&q.xl[j], YL = *(const ulonglong2*)&q.yl[j],
-                                     ZL = *(const ulonglong2*)&q.zl[j];
-                    f32x2 dx = add2(add2(X.x, HX), add2(XL.x, LX)), dy = add2(add2(Y.x, HY), add2(YL.x, LY)),
-                          dz = add2(add2(Z.x, HZ), add2(ZL.x, LZ));
-                    r2[2 * c] = fma2(dx, dx, fma2(dy, dy, mul2(dz, dz)));
-                    s[2 * c] = mul2(r2[2 * c], W.x);
-                    dx = add2(add2(X.y, HX), add2(XL.y, LX)); dy = add2(add2(Y.y, HY), add2(YL.y, LY));
-                    dz = add2(add2(Z.y, HZ), add2(ZL.y, LZ));
-                    r2[2 * c + 1] = fma2(dx, dx, fma2(dy, dy, mul2(dz, dz)));
-                    s[2 * c + 1] = mul2(r2[2 * c + 1], W.y);
-                }
+                estr_r2s8(q, j0, th, tl, r2, s);
                 if (zeta_skip_s<K>() > 0.0f && __all_sync(0xffffffffu, min8_nan(s) > zeta_skip_s<K>())) continue;
                 if (((whole >> j0) & 0xffu) == 0xffu && (ZETA || !((inside >> j0) & 0xffu))) {
                     estr_add8<K, ZETA, DZ, false, false>(r2, s, &q.gv[3 * j0], 0u, nullptr, fd, f);

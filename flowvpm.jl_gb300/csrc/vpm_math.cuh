@@ -462,6 +462,16 @@ __device__ __forceinline__ float df_offset(float a, float b, float oh, float ol)
     return s + (e + (b - ol));
 }
 
+// ... and `rest`, what its rounding left (two-sum: exact)
+__device__ __forceinline__ float df_offset(float a, float b, float oh, float ol, float& rest)
+{
+    const float s = a - oh, v = s - a;
+    const float t = ((a - (s - v)) + (-oh - v)) + (b - ol);
+    const float h = s + t, w = h - s;
+    rest = (s - (h - w)) + (t - w);
+    return h;
+}
+
 // the least of the eight (a NaN if one is)
 __device__ __forceinline__ float min8_nan(const f32x2 (&v)[4])
 {
