@@ -37,6 +37,8 @@
 #include "internal.h"
 #include "vpm_math.cuh"
 
+#include <type_traits>
+
 namespace vpm {
 
 static inline int64_t round_up(int64_t a, int64_t b) { return (a + b - 1) / b * b; }
@@ -224,7 +226,8 @@ ea2_f64(int64_t n, const EA1F64* __restrict__ self, int64_t n_pad, const EA2F64*
 // Both passes stream the other role's records per warp, 32 per tile,
 // double-buffered with cp.async (no block-wide barrier), as the forward mixed
 // Estr does; offsets from the warp's first particle are formed by df_offset
-// for both roles (the self pair has r^2 == 0 exactly and is skipped).  A tile
+// for both roles (the self pair has r^2 == 0 exactly and is skipped), with what their rounding
+// left where the warp's box is wide against the cores (ESTR_WIDE, ESTR_CLOSE).  A tile
 // is skipped when every pair of it is past zeta_skip_s from the warp's box
 // (pass 1 with each source's own sigma; pass 2 with the warp's smallest lane
 // sigma), then an 8-pair sub-block when every pair of the warp is.  Sums:
@@ -254,17 +257,18 @@ __device__ __forceinline__ void ea_stage(R* d, const R* g)
 // The warp's origin (lane 0's particle, double-float), this lane's offset and the
 // bounding box of the warp's offsets.
 struct EaFrame {
-    float3 oh, ol, me;
-    float bmin[3], bmax[3];
+    float3 oh, ol, me, rest;     // rest: what the rounding of `me` left
+    float bmin[3], bmax[3], ext2;
     __device__ __forceinline__ void init(const float4& h, const float4& l, bool valid)
     {
         oh = make_float3(__shfl_sync(0xffffffffu, h.x, 0), __shfl_sync(0xffffffffu, h.y, 0),
                          __shfl_sync(0xffffffffu, h.z, 0));
         ol = make_float3(__shfl_sync(0xffffffffu, l.x, 0), __shfl_sync(0xffffffffu, l.y, 0),
                          __shfl_sync(0xffffffffu, l.z, 0));
-        me = valid ? make_float3(df_offset(h.x, l.x, oh.x, ol.x), df_offset(h.y, l.y, oh.y, ol.y),
-                                 df_offset(h.z, l.z, oh.z, ol.z))
-                   : make_float3(0.f, 0.f, 0.f);
+        me = rest = make_float3(0.f, 0.f, 0.f);
+        if (valid)
+            me = make_float3(df_offset(h.x, l.x, oh.x, ol.x, rest.x), df_offset(h.y, l.y, oh.y, ol.y, rest.y),
+                             df_offset(h.z, l.z, oh.z, ol.z, rest.z));
         bmin[0] = bmax[0] = me.x; bmin[1] = bmax[1] = me.y; bmin[2] = bmax[2] = me.z;
 #pragma unroll
         for (int m = 16; m > 0; m >>= 1)
@@ -273,6 +277,8 @@ struct EaFrame {
                 bmin[k] = fminf(bmin[k], __shfl_xor_sync(0xffffffffu, bmin[k], m));
                 bmax[k] = fmaxf(bmax[k], __shfl_xor_sync(0xffffffffu, bmax[k], m));
             }
+        const float ext = fmaxf(fmaxf(bmax[0] - bmin[0], bmax[1] - bmin[1]), bmax[2] - bmin[2]);
+        ext2 = ext * ext;
     }
     // the FP32 box of the warp's valid particles (high parts) to wb[0] (low), wb[1] (high)
     __device__ __forceinline__ static void abs_box(const float4& h, bool valid, float4* wb)
@@ -293,6 +299,22 @@ struct EaFrame {
     {
         return make_float3(df_offset(h.x, l.x, oh.x, ol.x), df_offset(h.y, l.y, oh.y, ol.y),
                            df_offset(h.z, l.z, oh.z, ol.z));
+    }
+    __device__ __forceinline__ float3 left(const float4& h, const float4& l) const
+    {
+        float3 r;
+        df_offset(h.x, l.x, oh.x, ol.x, r.x);
+        df_offset(h.y, l.y, oh.y, ol.y, r.y);
+        df_offset(h.z, l.z, oh.z, ol.z, r.z);
+        return r;
+    }
+    // displacement from a record at offset h; TWO: with what both roundings left (l)
+    template <bool TWO>
+    __device__ __forceinline__ float3 disp(const float4& h, const float4& l) const
+    {
+        float3 d = make_float3(me.x - h.x, me.y - h.y, me.z - h.z);
+        if constexpr (TWO) { d.x += rest.x - l.x; d.y += rest.y - l.y; d.z += rest.z - l.z; }
+        return d;
     }
     __device__ __forceinline__ float box_dist2(const float3& p) const
     {
@@ -337,46 +359,57 @@ ea1_mx(int64_t n, const TgtPos* __restrict__ tgt, const EA2Mx* __restrict__ self
             ea_wait<0>();
         }
         __syncwarp();
-        bool beyond;
+        bool beyond, coarse;
         {
-            const EA1Mx& r = stage[warp][buf][lane];
+            EA1Mx& r = stage[warp][buf][lane];
             const float3 p = fr.offset(r.a, r.b);
             offs[warp][buf][lane] = make_float4(p.x, p.y, p.z, r.a.w);
-            beyond = fr.box_dist2(p) * r.a.w > zeta_skip_s<K>();
+            const float d2 = fr.box_dist2(p);
+            beyond = d2 * r.a.w > zeta_skip_s<K>();
+            coarse = __any_sync(0xffffffffu, fr.ext2 * r.a.w > ESTR_WIDE && d2 * r.a.w < ESTR_CLOSE);
+            if (coarse) {
+                const float3 q = fr.left(r.a, r.b);
+                r.b = make_float4(q.x, q.y, q.z, 0.f);
+            }
         }
         __syncwarp();
         if (!(zeta_skip_s<K>() > 0.0f && __all_sync(0xffffffffu, beyond))) {
+            auto pairs = [&](auto two_parts) {
+                constexpr bool TWO = decltype(two_parts)::value;
 #pragma unroll 1
-            for (int sub = 0; sub < EA_WT; sub += EA_SUB) {
-                float sv[EA_SUB], r2v[EA_SUB];
-                bool far = true;
+                for (int sub = 0; sub < EA_WT; sub += EA_SUB) {
+                    float sv[EA_SUB], r2v[EA_SUB];
+                    bool far = true;
 #pragma unroll
-                for (int jj = 0; jj < EA_SUB; jj++) {
-                    const float4 h = offs[warp][buf][sub + jj];
-                    const float dx = fr.me.x - h.x, dy = fr.me.y - h.y, dz = fr.me.z - h.z;
-                    r2v[jj] = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-                    sv[jj] = r2v[jj] * h.w;
-                    far = far && sv[jj] > zeta_skip_s<K>();
+                    for (int jj = 0; jj < EA_SUB; jj++) {
+                        const float4 h = offs[warp][buf][sub + jj];
+                        const float3 d = fr.disp<TWO>(h, stage[warp][buf][sub + jj].b);
+                        r2v[jj] = fmaf(d.x, d.x, fmaf(d.y, d.y, d.z * d.z));
+                        sv[jj] = r2v[jj] * h.w;
+                        far = far && sv[jj] > zeta_skip_s<K>();
+                    }
+                    if (zeta_skip_s<K>() > 0.0f && __all_sync(0xffffffffu, far)) continue;
+                    float f[NACC1] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+                    for (int jj = 0; jj < EA_SUB; jj++) {
+                        const int j = sub + jj;
+                        const float4 h = offs[warp][buf][j];
+                        const float3 d = fr.disp<TWO>(h, stage[warp][buf][j].b);
+                        float zh = zhat_f32<K>(sv[jj]);
+                        zh = r2v[jj] == 0.0f ? 0.0f : zh;     // the self pair and coincident pairs
+                        const float4 g = stage[warp][buf][j].g, v = stage[warp][buf][j].v;
+                        const float wh = fmaf(g.x, me.a.x, fmaf(g.y, me.a.y, g.z * me.a.z)) -
+                                         fmaf(v.x, me.sb.x, fmaf(v.y, me.sb.y, v.z * me.sb.z));
+                        f[0] = fmaf(zh, g.x, f[0]); f[1] = fmaf(zh, g.y, f[1]); f[2] = fmaf(zh, g.z, f[2]);
+                        const float c = zh * wh * kappa_f32<K>(sv[jj]) * h.w;
+                        f[3] = fmaf(c, d.x, f[3]); f[4] = fmaf(c, d.y, f[4]); f[5] = fmaf(c, d.z, f[5]);
+                    }
+#pragma unroll
+                    for (int k = 0; k < NACC1; k++) comp_add(sm[k], cm[k], f[k]);
                 }
-                if (zeta_skip_s<K>() > 0.0f && __all_sync(0xffffffffu, far)) continue;
-                float f[NACC1] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-                for (int jj = 0; jj < EA_SUB; jj++) {
-                    const int j = sub + jj;
-                    const float4 h = offs[warp][buf][j];
-                    const float dx = fr.me.x - h.x, dy = fr.me.y - h.y, dz = fr.me.z - h.z;
-                    float zh = zhat_f32<K>(sv[jj]);
-                    zh = r2v[jj] == 0.0f ? 0.0f : zh;     // the self pair and coincident pairs
-                    const float4 g = stage[warp][buf][j].g, v = stage[warp][buf][j].v;
-                    const float wh = fmaf(g.x, me.a.x, fmaf(g.y, me.a.y, g.z * me.a.z)) -
-                                     fmaf(v.x, me.sb.x, fmaf(v.y, me.sb.y, v.z * me.sb.z));
-                    f[0] = fmaf(zh, g.x, f[0]); f[1] = fmaf(zh, g.y, f[1]); f[2] = fmaf(zh, g.z, f[2]);
-                    const float c = zh * wh * kappa_f32<K>(sv[jj]) * h.w;
-                    f[3] = fmaf(c, dx, f[3]); f[4] = fmaf(c, dy, f[4]); f[5] = fmaf(c, dz, f[5]);
-                }
-#pragma unroll
-                for (int k = 0; k < NACC1; k++) comp_add(sm[k], cm[k], f[k]);
-            }
+            };
+            if (__builtin_expect(coarse, 0)) pairs(std::true_type());
+            else pairs(std::false_type());
             if (++in_flush == EA_FLUSH) {     // evaluated tiles only
                 in_flush = 0;
 #pragma unroll
@@ -421,9 +454,12 @@ ea2_mx(int64_t n, const EA1Mx* __restrict__ self, const double* __restrict__ gam
     fr.init(me.a, me.b, s < n);
     EaFrame::abs_box(me.a, s < n, wbox[warp]);
     const float isig2 = me.a.w;
-    float i2min = s < n ? isig2 : 3.0e38f;
+    float i2min = s < n ? isig2 : 3.0e38f, i2max = s < n ? isig2 : 0.0f;
 #pragma unroll
-    for (int m = 16; m > 0; m >>= 1) i2min = fminf(i2min, __shfl_xor_sync(0xffffffffu, i2min, m));
+    for (int m = 16; m > 0; m >>= 1) {
+        i2min = fminf(i2min, __shfl_xor_sync(0xffffffffu, i2min, m));
+        i2max = fmaxf(i2max, __shfl_xor_sync(0xffffffffu, i2max, m));
+    }
     double acc[NACC2];
     float sm[NACC2], cm[NACC2];
 #pragma unroll
@@ -443,51 +479,62 @@ ea2_mx(int64_t n, const EA1Mx* __restrict__ self, const double* __restrict__ gam
             ea_wait<0>();
         }
         __syncwarp();
-        bool beyond;
+        bool beyond, coarse;
         {
-            const EA2Mx& r = stage[warp][buf][lane];
+            EA2Mx& r = stage[warp][buf][lane];
             const float3 p = fr.offset(r.h, r.l);
             offs[warp][buf][lane] = make_float4(p.x, p.y, p.z, 0.f);
-            beyond = fr.box_dist2(p) * i2min > zeta_skip_s<K>();
+            const float d2 = fr.box_dist2(p);
+            beyond = d2 * i2min > zeta_skip_s<K>();
+            coarse = __any_sync(0xffffffffu, fr.ext2 * i2max > ESTR_WIDE && d2 * i2min < ESTR_CLOSE);
+            if (coarse) {
+                const float3 q = fr.left(r.h, r.l);
+                r.l = make_float4(q.x, q.y, q.z, 0.f);
+            }
         }
         __syncwarp();
         if (!(zeta_skip_s<K>() > 0.0f && __all_sync(0xffffffffu, beyond))) {
+            auto pairs = [&](auto two_parts) {
+                constexpr bool TWO = decltype(two_parts)::value;
 #pragma unroll 1
-            for (int sub = 0; sub < EA_WT; sub += EA_SUB) {
-                float sv[EA_SUB], r2v[EA_SUB];
-                bool far = true;
+                for (int sub = 0; sub < EA_WT; sub += EA_SUB) {
+                    float sv[EA_SUB], r2v[EA_SUB];
+                    bool far = true;
 #pragma unroll
-                for (int jj = 0; jj < EA_SUB; jj++) {
-                    const float4 h = offs[warp][buf][sub + jj];
-                    const float dx = fr.me.x - h.x, dy = fr.me.y - h.y, dz = fr.me.z - h.z;
-                    r2v[jj] = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-                    sv[jj] = r2v[jj] * isig2;
-                    far = far && sv[jj] > zeta_skip_s<K>();
+                    for (int jj = 0; jj < EA_SUB; jj++) {
+                        const float4 h = offs[warp][buf][sub + jj];
+                        const float3 d = fr.disp<TWO>(h, stage[warp][buf][sub + jj].l);
+                        r2v[jj] = fmaf(d.x, d.x, fmaf(d.y, d.y, d.z * d.z));
+                        sv[jj] = r2v[jj] * isig2;
+                        far = far && sv[jj] > zeta_skip_s<K>();
+                    }
+                    if (zeta_skip_s<K>() > 0.0f && __all_sync(0xffffffffu, far)) continue;
+                    float f[NACC2];
+#pragma unroll
+                    for (int k = 0; k < NACC2; k++) f[k] = 0.f;
+#pragma unroll
+                    for (int jj = 0; jj < EA_SUB; jj++) {
+                        const int j = sub + jj;
+                        const float4 h = offs[warp][buf][j];
+                        const float3 d = fr.disp<TWO>(h, stage[warp][buf][j].l);
+                        float zh = zhat_f32<K>(sv[jj]);
+                        zh = r2v[jj] == 0.0f ? 0.0f : zh;
+                        const float4 a = stage[warp][buf][j].a, sb = stage[warp][buf][j].sb;
+                        const float w = fmaf(G.x, a.x, fmaf(G.y, a.y, G.z * a.z)) - fmaf(V.x, sb.x, fmaf(V.y, sb.y, V.z * sb.z));
+                        const float kp = kappa_f32<K>(sv[jj]);
+                        f[0] = fmaf(zh, a.x, f[0]); f[1] = fmaf(zh, a.y, f[1]); f[2] = fmaf(zh, a.z, f[2]);
+                        f[3] = fmaf(zh, sb.x, f[3]); f[4] = fmaf(zh, sb.y, f[4]); f[5] = fmaf(zh, sb.z, f[5]);
+                        const float zw = zh * w;
+                        const float c = zw * kp;
+                        f[6] = fmaf(c, d.x, f[6]); f[7] = fmaf(c, d.y, f[7]); f[8] = fmaf(c, d.z, f[8]);
+                        f[9] = fmaf(zw, fmaf(sv[jj], kp, 3.0f), f[9]);
+                    }
+#pragma unroll
+                    for (int k = 0; k < NACC2; k++) comp_add(sm[k], cm[k], f[k]);
                 }
-                if (zeta_skip_s<K>() > 0.0f && __all_sync(0xffffffffu, far)) continue;
-                float f[NACC2];
-#pragma unroll
-                for (int k = 0; k < NACC2; k++) f[k] = 0.f;
-#pragma unroll
-                for (int jj = 0; jj < EA_SUB; jj++) {
-                    const int j = sub + jj;
-                    const float4 h = offs[warp][buf][j];
-                    const float dx = fr.me.x - h.x, dy = fr.me.y - h.y, dz = fr.me.z - h.z;
-                    float zh = zhat_f32<K>(sv[jj]);
-                    zh = r2v[jj] == 0.0f ? 0.0f : zh;
-                    const float4 a = stage[warp][buf][j].a, sb = stage[warp][buf][j].sb;
-                    const float w = fmaf(G.x, a.x, fmaf(G.y, a.y, G.z * a.z)) - fmaf(V.x, sb.x, fmaf(V.y, sb.y, V.z * sb.z));
-                    const float kp = kappa_f32<K>(sv[jj]);
-                    f[0] = fmaf(zh, a.x, f[0]); f[1] = fmaf(zh, a.y, f[1]); f[2] = fmaf(zh, a.z, f[2]);
-                    f[3] = fmaf(zh, sb.x, f[3]); f[4] = fmaf(zh, sb.y, f[4]); f[5] = fmaf(zh, sb.z, f[5]);
-                    const float zw = zh * w;
-                    const float c = zw * kp;
-                    f[6] = fmaf(c, dx, f[6]); f[7] = fmaf(c, dy, f[7]); f[8] = fmaf(c, dz, f[8]);
-                    f[9] = fmaf(zw, fmaf(sv[jj], kp, 3.0f), f[9]);
-                }
-#pragma unroll
-                for (int k = 0; k < NACC2; k++) comp_add(sm[k], cm[k], f[k]);
-            }
+            };
+            if (__builtin_expect(coarse, 0)) pairs(std::true_type());
+            else pairs(std::false_type());
             if (++in_flush == EA_FLUSH) {     // evaluated tiles only
                 in_flush = 0;
 #pragma unroll

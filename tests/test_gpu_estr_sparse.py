@@ -45,3 +45,41 @@ def test_close_pairs(ctx, n, kernel):
         err = (S[1] - S[0]).norm(dim=1)
         lim = bound(x, g, sig, J, kernel) + 1e-13 * S[0].norm()
         assert (err <= lim).all(), f"seed {seed}: {float((err / lim).max()):.2f}"
+
+
+@pytest.mark.parametrize("kernel", [1, 2, 3])
+@pytest.mark.parametrize("n", [33, 700, 1630, 4099])
+def test_close_pairs_adjoint(ctx, n, kernel):
+    """The same for the Estr adjoint.  Bounds by particle: the terms of the gradients, as the sums of
+    their parts' magnitudes, each rounded to 8 ulp (16 ulp where the displacement, kappa = d log(zeta)/ds
+    and the pair's weight w multiply) and by the rounding of s as above."""
+    k = {1: 3 / (4 * np.pi), 2: (2 * np.pi) ** -1.5, 3: 7.5 / (4 * np.pi)}[kernel]
+    for seed in range(8):
+        x, g, sig, J = sparse(n, seed)
+        Sb = torch.tensor(np.random.default_rng(seed + 99).standard_normal((n, 3)), device="cuda")
+        out = []
+        for precision in (0, 1):
+            o = [torch.zeros(n, *c, device="cuda", dtype=torch.float64) for c in ((3,), (3,), (), (9,))]
+            ctx.estr_adjoint_dev(x, g, sig, J, Sb, *o, kernel, precision)
+            out.append([v.reshape(n, -1) for v in o])
+        Jn, gn, bn = J.norm(dim=1), g.norm(dim=1), Sb.norm(dim=1)
+        lim = [torch.zeros(n, device="cuda", dtype=torch.float64) for _ in range(4)]
+        for a in range(0, n, 2000):
+            t = slice(a, min(n, a + 2000))
+            s = ((x[t, None] - x[None]) ** 2).sum(2) / sig[None] ** 2
+            z, dlog, kap = {1: lambda: (torch.exp(-s ** 1.5), 1.5 * s.sqrt(), 3 * s.sqrt()),
+                            2: lambda: (torch.exp(-s / 2), 0.5 + 0 * s, 1 + 0 * s),
+                            3: lambda: ((1 + s) ** -3.5, 3.5 / (1 + s), 7 / (1 + s))}[kernel]()
+            e = (s > 0) * k / sig[None] ** 3 * (z * 8 * 2.0 ** -24 * (1 + dlog * s) + 1e-13)
+            w = 2 * (Jn[t, None] + Jn[None]) * gn[None] * bn[t, None]
+            ex, es = e * kap * s.sqrt() / sig[None] * w, e * (kap * s + 3) / sig[None] * w
+            lim[0][t] += ex.sum(1)
+            lim[0] += ex.sum(0)
+            lim[1] += (e * (Jn[t, None] + Jn[None]) * bn[t, None]).sum(0)
+            lim[2] += es.sum(0)
+            lim[3][t] += bn[t] * (e * gn[None]).sum(1)
+            lim[3] += gn * (e * bn[t, None]).sum(0)
+        for p, q, m, name in zip(out[1], out[0], lim, ("x", "Gamma", "sigma", "J")):
+            err = (p - q).norm(dim=1)
+            m = m + 1e-13 * q.norm()
+            assert (err <= m).all(), f"{name}, seed {seed}: {float((err / m).max()):.2f}"
