@@ -139,8 +139,7 @@ pack_tiles(int64_t n, const double* __restrict__ gs, const double* __restrict__ 
     }
     const float gmax = (float)fmax(red[0][6], red[1][6]);
     float r2 = (float)(y[0] * y[0] + y[1] * y[1] + y[2] * y[2]), s2 = on ? (float)(sig * sig) : 0.f, s2lo = on ? s2 : 3.0e38f;
-    // the tile's fourth array: sigma^2 for Winckelmans, 1/sigma for the kernels with a singular tail
-    const float mys2 = !on ? 1.f : singular_tail<K>() ? (float)(1.0 / sig) : s2;
+    const float own_s2 = s2;
     // a NaN position or core size must not hide in a maximum: it clears `ok`
     const bool fine = isfinite(r2) && isfinite(s2) && isfinite(g[0]) && isfinite(g[1]) && isfinite(g[2]);
     for (int s = 16; s > 0; s >>= 1) {
@@ -150,6 +149,11 @@ pack_tiles(int64_t n, const double* __restrict__ gs, const double* __restrict__ 
     }
     if (lane == 0) { redf[warp][0] = r2; redf[warp][1] = s2; redf[warp][2] = s2lo; }
     const bool ok = __syncthreads_and(fine) && gmax < 1e30f && (gmax > 1e-30f || gmax == 0.f);
+    // the tile's fourth array: sigma^2 for Winckelmans, 1/sigma for the kernels with a singular tail.  Sources
+    // past n take the tile's largest core: they have no strength, but a weight outside the f16 range that
+    // tile_class works out from the tile's own cores would be infinite, and NaN times their zeros.
+    const float s2max = fmaxf(redf[0][1], redf[1][1]);
+    const float mys2 = singular_tail<K>() ? on ? (float)(1.0 / sig) : 1.f / sqrtf(s2max) : on ? own_s2 : s2max;
     const float rad = sqrtf(fmaxf(redf[0][0], redf[1][0])) * 1.000001f;
     const float ys = rad > 1e-30f ? pow2_at_least(rad) : 1.f;
     const float gsc = gmax > 1e-30f ? pow2_at_least(gmax) * (1.f / 64.f) : 1.f;
@@ -188,7 +192,7 @@ pack_tiles(int64_t n, const double* __restrict__ gs, const double* __restrict__ 
         TileHdr h;
         h.chx = (float)c[0]; h.chy = (float)c[1]; h.chz = (float)c[2]; h.rad = rad;
         h.clx = (float)(c[0] - (double)h.chx); h.cly = (float)(c[1] - (double)h.chy); h.clz = (float)(c[2] - (double)h.chz);
-        h.sig2 = fmaxf(redf[0][1], redf[1][1]);
+        h.sig2 = s2max;
         h.hx = half[0]; h.hy = half[1]; h.hz = half[2];
         h.gscale = gsc;
         h.yscale = ys; h.ok = ok ? 1.f : 0.f; h.sig2lo = fminf(redf[0][2], redf[1][2]); h.p1 = 0.f;

@@ -1,0 +1,35 @@
+"""The tensor pass of the FP32-comp UJ at the limits of its number ranges: length units, core sizes and
+strengths against each other, with ragged last tiles.  The sums are scale-free, so the tolerance is that
+of test_gpu_uj_tiles.py (1e-6 of the largest value) in any unit."""
+import numpy as np
+import pytest
+import torch
+
+from helpers import normwise, random_cloud
+
+pytestmark = pytest.mark.gpu
+
+
+def uj(ctx, X, G, s, k, prec, cross=False):
+    """U, J; cross: with the sources in arrays of their own, which the pairwise kernel takes."""
+    n = X.shape[0]
+    x, g, sg = (torch.tensor(a, device="cuda") for a in (X, G, s))
+    U, J = (torch.zeros(n, c, dtype=torch.float64, device="cuda") for c in (3, 9))
+    ctx.uj_dev(x, x.clone() if cross else x, g, sg, U, J, k, prec)
+    return U.cpu().numpy(), J.cpu().numpy()
+
+
+def check(ctx, X, G, s, k, what):
+    for u, v, name in zip(uj(ctx, X, G, s, k, 1), uj(ctx, X, G, s, k, 0), "UJ"):
+        assert np.isfinite(u).all(), f"{what}: {name} not finite"
+        e = normwise(u, v)[0]
+        assert e <= 1e-6, f"{what}: {name} {e:.3e}"
+
+
+@pytest.mark.parametrize("k", [2, 3])
+@pytest.mark.parametrize("n", [13057, 13060, 13064, 13119])     # last tiles of 1, 4, 8 and 63
+@pytest.mark.parametrize("S", [1e-4, 1.0, 1e2, 1.3e2, 1e5])
+def test_wide_cores_in_any_unit(ctx, k, n, S):
+    X, G, s = random_cloud(n, seed=n)
+    for wide in (3.0, 6.0, 30.0):
+        check(ctx, S * X, S ** 3 * G, wide * S * s, k, f"k={k} n={n} S={S} wide={wide}")
