@@ -151,9 +151,12 @@ pack_tiles(int64_t n, const double* __restrict__ gs, const double* __restrict__ 
     const bool ok = __syncthreads_and(fine) && gmax < 1e30f && (gmax > 1e-30f || gmax == 0.f);
     // the tile's fourth array: sigma^2 for Winckelmans, 1/sigma for the kernels with a singular tail.  Sources
     // past n take the tile's largest core: they have no strength, but a weight outside the f16 range that
-    // tile_class works out from the tile's own cores would be infinite, and NaN times their zeros.
+    // tile_class works out from the tile's own cores would be infinite, and NaN times their zeros.  1/sigma
+    // stays below 1e6 of the largest core's, where the mid form (r > 1.4 of the largest core) is long the
+    // singular one: past rho = 7e12 its rho^3 e^{-rho^2/2} would be infinity times zero.
     const float s2max = fmaxf(redf[0][1], redf[1][1]);
-    const float mys2 = singular_tail<K>() ? on ? (float)(1.0 / sig) : 1.f / sqrtf(s2max) : on ? own_s2 : s2max;
+    const float islo = 1.f / sqrtf(s2max);
+    const float mys2 = singular_tail<K>() ? on ? fminf((float)(1.0 / sig), 1e6f * islo) : islo : on ? own_s2 : s2max;
     const float rad = sqrtf(fmaxf(redf[0][0], redf[1][0])) * 1.000001f;
     const float ys = rad > 1e-30f ? pow2_at_least(rad) : 1.f;
     const float gsc = gmax > 1e-30f ? pow2_at_least(gmax) * (1.f / 64.f) : 1.f;

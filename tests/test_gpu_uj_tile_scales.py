@@ -33,3 +33,14 @@ def test_wide_cores_in_any_unit(ctx, k, n, S):
     X, G, s = random_cloud(n, seed=n)
     for wide in (3.0, 6.0, 30.0):
         check(ctx, S * X, S ** 3 * G, wide * S * s, k, f"k={k} n={n} S={S} wide={wide}")
+
+
+@pytest.mark.parametrize("tiny", [1e-3, 1e-9, 1e-12])
+def test_tiny_cores_among_ordinary_ones(ctx, tiny):
+    """Particles without strength whose cores are 1e-4 to 1e-13 of their neighbours' (particles that have
+    lost theirs): they add nothing to U and J."""
+    X, G, s = random_cloud(13000, seed=11)
+    X, s = 1e3 * X, 3e3 * s
+    G[5::37] = 0.0
+    s[5::37] = tiny
+    check(ctx, X, G, s, 2, f"tiny={tiny}")
