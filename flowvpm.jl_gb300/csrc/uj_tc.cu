@@ -68,6 +68,11 @@ constexpr int TC_THREADS = UJ_THREADS + 32;
 constexpr int TC_COLS = 128;                  // TMEM columns of a block: A 64, G sums 16, Q sums 48
 constexpr int TC_DG = 64, TC_DQ = 80;
 constexpr int WT = 32;
+// Tiles between FP64 adds of the tensor pass (1,024 sources, as in uj_mixed_kernel) and of the near pass,
+// whose terms are the largest (32 and the 32 tiles' near ones: error of J, rings of 100,000, 7.0e-8
+// against 4.1e-8, 6.8e-8 in uj_mixed_kernel in Morton order; UJ of 65,000 random particles 3.92 against 3.98
+// ms, of the rings 9.94 against 10.16).
+constexpr int TC_MID = 16, TC_MID_NEAR = 4;
 // tcgen05.mma truncates its FP32 accumulator: a sum of terms of one sign loses up to 8
 // truncations of half an ulp on average on its way through a tile.  B is scaled up by the mean
 // loss, measured on vortex rings of 30,000 to 100,000 particles, whose far velocities add up
@@ -494,7 +499,7 @@ uj_tc_kernel(int64_t nt, const TgtPos* __restrict__ tgt, int ntiles_all, const T
     };
 
     // ------------------------------------------------- tensor pass over the far tiles
-    // The mid-level sums go to FP64 after 32 tiles (the FP64 adds stand outside the tile loop:
+    // The mid-level sums go to FP64 after TC_MID tiles (the FP64 adds stand outside the tile loop:
     // as a condition inside it they were issued, predicated off, for every tile and kept the
     // FP64 pipe 42 % busy).
     const uint32_t ta = tmem + ((uint32_t)(warp * 32) << 16);
@@ -555,68 +560,70 @@ uj_tc_kernel(int64_t nt, const TgtPos* __restrict__ tgt, int ntiles_all, const T
         }
         const unsigned far = __ballot_sync(0xffffffffu, cls == TILE_FAR);
         const unsigned mid = __ballot_sync(0xffffffffu, cls == TILE_MID);
+        for (int part = base; ok && part < min(base + 32, ntiles); part += TC_MID) {
 #pragma unroll 1
-        for (int it = base; it < min(base + 32, ntiles); it++) {
-            const bool isfar = (far >> (it & 31)) & 1u;
-            if (!isfar && !((mid >> (it & 31)) & 1u)) {
-                // not this warp's: its rows of A keep stale values and its sums are not read
-                ok = mbar_wait(&adone, 1u);      // the previous tile's second half
-                if (!ok) break;
-                tc_fence_after();
-                if (pend) { collect(pdx, pdy, pdz, pR, pg, py); tc_fence_before(); __syncwarp(); }
-                pend = false;
-                if (lane == 0) mbar_arrive(&afull);
-                ok = mbar_wait(&adone, 0u);
-                if (!ok) break;
-                if (lane == 0) mbar_arrive(&afull);
-                continue;
-            }
-            const char* r = stage[it & 1].rec;
-            const float iR = __shfl_sync(0xffffffffu, iRl, it & 31);
-            ok = mbar_wait(&bfull[it & 1], (uint32_t)(it >> 1) & 1u);
-            if (!ok) break;
-            const TileHdr& h = *(const TileHdr*)(r + TC_B + 4 * TC_POS);
-            const float dx = ((th.x - h.chx) + (tl.x - h.clx)) * iR, dy = ((th.y - h.chy) + (tl.y - h.cly)) * iR,
-                        dz = ((th.z - h.chz) + (tl.z - h.clz)) * iR;
-            const float hg = h.gscale, hy = h.yscale;   // the stage is not read after the last arrival
-#pragma unroll 1
-            for (int hh = 0; hh < 2; hh++) {
-                const ulonglong2* p = (const ulonglong2*)(r + TC_B) + hh * 8;
-                if (isfar) {
-                    uint32_t gh[8], gl[8], qh[8], ql[8];
-                    weigh<K, 8>(p, dx, dy, dz, iR, gh, gl, qh, ql);   // while the last step's MMAs run
-                    ok = mbar_wait(&adone, (uint32_t)(hh ^ 1));
+            for (int it = part; it < min(part + TC_MID, ntiles); it++) {
+                const bool isfar = (far >> (it & 31)) & 1u;
+                if (!isfar && !((mid >> (it & 31)) & 1u)) {
+                    // not this warp's: its rows of A keep stale values and its sums are not read
+                    ok = mbar_wait(&adone, 1u);      // the previous tile's second half
                     if (!ok) break;
                     tc_fence_after();
-                    store_a(ta, gh, gl, qh, ql);
-                    if (hh == 0 && pend) collect(pdx, pdy, pdz, pR, pg, py);
-                    weigh<K, 8>(p + 4, dx, dy, dz, iR, gh, gl, qh, ql);
-                    store_a(ta + 8, gh, gl, qh, ql);
-                } else if constexpr (K == K_GAUSERF) {
-                    ok = mbar_wait(&adone, (uint32_t)(hh ^ 1));
+                    if (pend) { collect(pdx, pdy, pdz, pR, pg, py); tc_fence_before(); __syncwarp(); }
+                    pend = false;
+                    if (lane == 0) mbar_arrive(&afull);
+                    ok = mbar_wait(&adone, 0u);
                     if (!ok) break;
-                    tc_fence_after();
-                    if (hh == 0 && pend) collect(pdx, pdy, pdz, pR, pg, py);
-#pragma unroll 1
-                    for (int c = 0; c < 4; c++) {
-                        uint32_t gh[4], gl[4], qh[4], ql[4];
-                        weigh<K, 4, true>(p + 2 * c, dx, dy, dz, iR, gh, gl, qh, ql);
-                        tmem_st4(ta + 4 * c, gh);
-                        tmem_st4(ta + 16 + 4 * c, gl);
-                        tmem_st4(ta + 32 + 4 * c, qh);
-                        tmem_st4(ta + 48 + 4 * c, ql);
-                    }
+                    if (lane == 0) mbar_arrive(&afull);
+                    continue;
                 }
-                tc_wait_st();
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&afull);
+                const char* r = stage[it & 1].rec;
+                const float iR = __shfl_sync(0xffffffffu, iRl, it & 31);
+                ok = mbar_wait(&bfull[it & 1], (uint32_t)(it >> 1) & 1u);
+                if (!ok) break;
+                const TileHdr& h = *(const TileHdr*)(r + TC_B + 4 * TC_POS);
+                const float dx = ((th.x - h.chx) + (tl.x - h.clx)) * iR, dy = ((th.y - h.chy) + (tl.y - h.cly)) * iR,
+                            dz = ((th.z - h.chz) + (tl.z - h.clz)) * iR;
+                const float hg = h.gscale, hy = h.yscale;   // the stage is not read after the last arrival
+#pragma unroll 1
+                for (int hh = 0; hh < 2; hh++) {
+                    const ulonglong2* p = (const ulonglong2*)(r + TC_B) + hh * 8;
+                    if (isfar) {
+                        uint32_t gh[8], gl[8], qh[8], ql[8];
+                        weigh<K, 8>(p, dx, dy, dz, iR, gh, gl, qh, ql);   // while the last step's MMAs run
+                        ok = mbar_wait(&adone, (uint32_t)(hh ^ 1));
+                        if (!ok) break;
+                        tc_fence_after();
+                        store_a(ta, gh, gl, qh, ql);
+                        if (hh == 0 && pend) collect(pdx, pdy, pdz, pR, pg, py);
+                        weigh<K, 8>(p + 4, dx, dy, dz, iR, gh, gl, qh, ql);
+                        store_a(ta + 8, gh, gl, qh, ql);
+                    } else if constexpr (K == K_GAUSERF) {
+                        ok = mbar_wait(&adone, (uint32_t)(hh ^ 1));
+                        if (!ok) break;
+                        tc_fence_after();
+                        if (hh == 0 && pend) collect(pdx, pdy, pdz, pR, pg, py);
+#pragma unroll 1
+                        for (int c = 0; c < 4; c++) {
+                            uint32_t gh[4], gl[4], qh[4], ql[4];
+                            weigh<K, 4, true>(p + 2 * c, dx, dy, dz, iR, gh, gl, qh, ql);
+                            tmem_st4(ta + 4 * c, gh);
+                            tmem_st4(ta + 16 + 4 * c, gl);
+                            tmem_st4(ta + 32 + 4 * c, qh);
+                            tmem_st4(ta + 48 + 4 * c, ql);
+                        }
+                    }
+                    tc_wait_st();
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&afull);
+                }
+                if (!ok) break;
+                pend = true;
+                pdx = dx; pdy = dy; pdz = dz; pR = iR; pg = hg; py = hy;
             }
-            if (!ok) break;
-            pend = true;
-            pdx = dx; pdy = dy; pdz = dz; pR = iR; pg = hg; py = hy;
+            flush();
         }
-        flush();
     }
     if (ok) {
         ok = mbar_wait(&adone, 1u);
@@ -635,6 +642,7 @@ uj_tc_kernel(int64_t nt, const TgtPos* __restrict__ tgt, int ntiles_all, const T
                                       __shfl_sync(0xffffffffu, th.z, 0));
         const float3 ol = make_float3(__shfl_sync(0xffffffffu, tl.x, 0), __shfl_sync(0xffffffffu, tl.y, 0),
                                       __shfl_sync(0xffffffffu, tl.z, 0));
+        int in_mid = 0;
         for (int base = 0; base < ntiles; base += 32) {
             int cls = TILE_FAR;
             if (base + lane < ntiles) {
@@ -677,8 +685,11 @@ uj_tc_kernel(int64_t nt, const TgtPos* __restrict__ tgt, int ntiles_all, const T
                 for (int k = 0; k < 3; k++) { mu[k] += u[k]; mw[k] += w[k]; }
 #pragma unroll
                 for (int k = 0; k < 8; k++) mj[k] += jq[k];
+                if (sub == 0 && ++in_mid == TC_MID_NEAR) {
+                    in_mid = 0;
+                    flush();
+                }
             }
-            flush();
         }
     }
     flush();
