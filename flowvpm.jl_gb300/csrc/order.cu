@@ -13,11 +13,13 @@
 // curve: with each axis scaled to its own extent the cells of a 32,000-particle ring were 11
 // times as wide as high (tile radius 0.161 against 0.074).
 //
-// Steps: per-block bounding boxes (bbox_partial), curve keys (hilbert_keys), CUB radix sort of
-// (key, index), and a gather of the sorted positions into TgtPos records; up to RANK_MAX
-// particles order_rank counts places instead.  Keys have 10 bits an axis up to 2^16 particles (a
-// cell of the cube then holds at most a few of a uniform set; four 8-bit sort passes, each about
-// 9 us at these sizes) and 20 beyond (eight passes).
+// Steps: per-block bounding boxes (bbox_partial), curve keys (hilbert_keys), CUB radix sort and a
+// gather of the sorted positions into TgtPos records; up to RANK_MAX particles order_rank counts
+// places instead.  Keys have 21 bits an axis at every size: the cube is as wide as the farthest
+// particle makes it, and with 10 bits one particle 1,000 extents away left all others in the
+// caller's order, every tile of 64 near every other (FP32-comp UJ of 60,000 3.4 -> 10.8 ms; 4.7
+// with 21, for the few wide tiles and warps that hold the particle).  order_rank compares their
+// top 32 bits at first, four to a 16-byte read, and all 63 where particles share those.
 #include "internal.h"
 
 #include <cub/device/device_radix_sort.cuh>
@@ -27,12 +29,25 @@ namespace vpm {
 constexpr int BB_BLOCKS = 256;
 constexpr int BB_THREADS = 256;
 
-// Index along Hilbert's curve of the cell q of a 2^bits cube (J. Skilling, "Programming the
-// Hilbert curve", AIP Conf. Proc. 707, 2004: axes to transpose, then the bits interleaved).
-template <typename Key>
-__device__ __forceinline__ Key hilbert_index(uint32_t (&q)[3], int bits)
+constexpr int KEY_BITS = 21;   // an axis
+
+// Spread the low 21 bits of v so that bit i moves to bit 3i.
+__device__ __forceinline__ uint64_t spread3(uint64_t v)
 {
-    for (uint32_t m = 1u << (bits - 1); m > 1; m >>= 1) {
+    v &= 0x1fffffULL;
+    v = (v | (v << 32)) & 0x1f00000000ffffULL;
+    v = (v | (v << 16)) & 0x1f0000ff0000ffULL;
+    v = (v | (v << 8)) & 0x100f00f00f00f00fULL;
+    v = (v | (v << 4)) & 0x10c30c30c30c30c3ULL;
+    v = (v | (v << 2)) & 0x1249249249249249ULL;
+    return v;
+}
+
+// Index along Hilbert's curve of the cell q of a 2^KEY_BITS cube (J. Skilling, "Programming the
+// Hilbert curve", AIP Conf. Proc. 707, 2004: axes to transpose, then the bits interleaved).
+__device__ __forceinline__ uint64_t hilbert_index(uint32_t (&q)[3])
+{
+    for (uint32_t m = 1u << (KEY_BITS - 1); m > 1; m >>= 1) {
         const uint32_t p = m - 1;
 #pragma unroll
         for (int i = 0; i < 3; i++) {
@@ -48,14 +63,11 @@ __device__ __forceinline__ Key hilbert_index(uint32_t (&q)[3], int bits)
     q[1] ^= q[0];
     q[2] ^= q[1];
     uint32_t t = 0;
-    for (uint32_t m = 1u << (bits - 1); m > 1; m >>= 1)
+    for (uint32_t m = 1u << (KEY_BITS - 1); m > 1; m >>= 1)
         if (q[2] & m) t ^= m - 1;
 #pragma unroll
     for (int i = 0; i < 3; i++) q[i] ^= t;
-    Key k = 0;
-    for (int b = bits - 1; b >= 0; b--)
-        k = (k << 3) | (Key)((((q[0] >> b) & 1u) << 2) | (((q[1] >> b) & 1u) << 1) | ((q[2] >> b) & 1u));
-    return k;
+    return spread3(q[0]) << 2 | spread3(q[1]) << 1 | spread3(q[2]);
 }
 
 __global__ void __launch_bounds__(BB_THREADS)
@@ -87,17 +99,26 @@ bbox_partial(int64_t n, const double* __restrict__ x, double* __restrict__ part)
     if (threadIdx.x < 6) part[blockIdx.x * 6 + threadIdx.x] = red[threadIdx.x][0];
 }
 
-template <typename Key>
+__device__ __forceinline__ TgtPos target_of(const double* __restrict__ x, int64_t i)
+{
+    TgtPos t;
+    t.x = x[3 * i]; t.y = x[3 * i + 1]; t.z = x[3 * i + 2];
+    t.idx = (int32_t)i; t.pad = 0;
+    return t;
+}
+
+// aux receives the key's top 32 bits (RANK) or the index
+template <bool RANK>
 __global__ void __launch_bounds__(BB_THREADS)
-hilbert_keys(int64_t n, const double* __restrict__ x, const double* __restrict__ part, int bits,
-             Key* __restrict__ keys, int32_t* __restrict__ idx)
+hilbert_keys(int64_t n, const double* __restrict__ x, const double* __restrict__ part, uint64_t* __restrict__ keys,
+             uint32_t* __restrict__ aux)
 {
     // The box from the 256 partial ones, a warp a side, and the scale, once a block: the FP64 pipe
     // (16 cycles a warp instruction) is what this kernel waits for, and with every thread at all of
     // it 5,600 particles took 11.2 us and 100,000 took 28.
     __shared__ double box[6], scale;
     static_assert(BB_BLOCKS == 256 && BB_THREADS >= 192, "six warps, eight boxes a lane");
-    const double top = (double)((1u << bits) - 1u);
+    constexpr uint32_t TOP = (1u << KEY_BITS) - 1u;
     if (threadIdx.x < 192) {
         const int k = threadIdx.x >> 5, lane = threadIdx.x & 31;
         double v[8];
@@ -115,7 +136,7 @@ hilbert_keys(int64_t n, const double* __restrict__ x, const double* __restrict__
     __syncthreads();
     if (threadIdx.x == 0) {
         const double ext = fmax(fmax(fmax(box[3] - box[0], box[4] - box[1]), box[5] - box[2]), 0.0);
-        scale = ext > 0.0 ? top / ext : 0.0;
+        scale = ext > 0.0 ? (double)TOP / ext : 0.0;
     }
     __syncthreads();
     const int64_t i = blockIdx.x * (int64_t)BB_THREADS + threadIdx.x;
@@ -123,70 +144,78 @@ hilbert_keys(int64_t n, const double* __restrict__ x, const double* __restrict__
     uint32_t q[3];
 #pragma unroll
     for (int k = 0; k < 3; k++)   // the conversion takes values below 0 to 0, the minimum the rest (NaN too) to the top
-        q[k] = min(__double2uint_rz((x[3 * i + k] - box[k]) * scale), (1u << bits) - 1u);
-    keys[i] = hilbert_index<Key>(q, bits);
-    idx[i] = (int32_t)i;
+        q[k] = min(__double2uint_rz((x[3 * i + k] - box[k]) * scale), TOP);
+    const uint64_t key = hilbert_index(q);
+    keys[i] = key;
+    aux[i] = RANK ? (uint32_t)(key >> (3 * KEY_BITS - 32)) : (uint32_t)i;
 }
 
-__global__ void gather_targets(int64_t n, const double* __restrict__ x, const int32_t* __restrict__ perm,
+__global__ void gather_targets(int64_t n, const double* __restrict__ x, const uint32_t* __restrict__ perm,
                                TgtPos* __restrict__ out)
 {
-    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const int32_t j = perm ? perm[i] : (int32_t)i;
-    TgtPos t;
-    t.x = x[3 * (int64_t)j];
-    t.y = x[3 * (int64_t)j + 1];
-    t.z = x[3 * (int64_t)j + 2];
-    t.idx = j;
-    t.pad = 0;
-    out[i] = t;
+    const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (t >= n) return;
+    out[t] = target_of(x, perm ? (int64_t)perm[t] : t);
 }
 
 static inline size_t align256(size_t b) { return (b + 255) / 256 * 256; }
 
 // Up to RANK_MAX particles: each one's place is the number of keys before it, counted (lane =
 // particle, the block's warps share the keys), and its record goes there: one launch for the sort's
-// six and the gather, but n^2 compares.  UJ calls with the sort / with ranks, us: 8,192 356 / 290,
-// 18,000 627 / 599, 20,000 706 / 694, 24,000 890 / 889, 28,000 1060 / 1087.  A sort of everything in
-// one block took 20 us more at 6,100 than the ranks, and as long at 1,400.
-constexpr int64_t RANK_MAX = 20480;
+// nine and the gather, but n^2 compares.  UJ calls with the sort / with ranks, us: 4,099 293 / 197,
+// 16,000 618 / 557, 20,000 754 / 710, 24,000 949 / 921, 28,000 1118 / 1125, 32,000 1370 / 1412.  A sort
+// of everything in one block took 20 us more at 6,100 than the ranks, and as long at 1,400.
+constexpr int64_t RANK_MAX = 27648;
 constexpr int RANK_THREADS = 1024;
 __global__ void __launch_bounds__(RANK_THREADS)
-order_rank(int n, const double* __restrict__ x, const uint32_t* __restrict__ keys, TgtPos* __restrict__ out)
+order_rank(int n, const double* __restrict__ x, const uint32_t* __restrict__ hi, const uint64_t* __restrict__ keys,
+           TgtPos* __restrict__ out)
 {
     __shared__ int part[RANK_THREADS / 32][32];
+    constexpr int W = RANK_THREADS / 32;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int i0 = blockIdx.x * 32, i = i0 + lane;
-    const uint32_t key = keys[min(i, n - 1)];
+    const int i0 = blockIdx.x * 32, i = i0 + lane, ic = min(i, n - 1);
+    const uint32_t top = hi[ic];
+    const uint64_t key = keys[ic];
     TgtPos t;
-    if (warp == 0) {
-        const int j = min(i, n - 1);
-        t.x = x[3 * j]; t.y = x[3 * j + 1]; t.z = x[3 * j + 2];
-        t.idx = j; t.pad = 0;
-    }
-    int c = 0;
-    // equal keys keep the caller's order; the block's own 32 keys are quads i0/4 .. i0/4 + 7
-    const uint4* k4 = (const uint4*)keys;
+    if (warp == 0) t = target_of(x, ic);
+    // The keys before the block's own 32 and those after them, by their top bits or, where a lane's own
+    // are among these, in full; then the 32 (quads own .. own + 7).  Equal keys keep the caller's order.
+    const uint4* h4 = (const uint4*)hi;
+    const ulonglong2* k2 = (const ulonglong2*)keys;
     const int own = i0 / 4, quads = n / 4;
+    int c = 0;
+    bool tie = false;
+    auto tops = [&](int q) {
+        const uint4 k = h4[q];
+        c += (k.x < top) + (k.y < top) + (k.z < top) + (k.w < top);
+        tie = tie || k.x == top || k.y == top || k.z == top || k.w == top;
+    };
 #pragma unroll 4
-    for (int q = warp; q < own; q += RANK_THREADS / 32) {
-        const uint4 k = k4[q];
-        c += (k.x <= key) + (k.y <= key) + (k.z <= key) + (k.w <= key);
+    for (int q = warp; q < own; q += W) tops(q);
+#pragma unroll 4
+    for (int q = own + 8 + warp; q < quads; q += W) tops(q);
+    if (__any_sync(0xffffffffu, tie)) {
+        c = 0;
+#pragma unroll 4
+        for (int q = warp; q < own; q += W) {
+            const ulonglong2 a = k2[2 * q], b = k2[2 * q + 1];
+            c += (a.x <= key) + (a.y <= key) + (b.x <= key) + (b.y <= key);
+        }
+#pragma unroll 4
+        for (int q = own + 8 + warp; q < quads; q += W) {
+            const ulonglong2 a = k2[2 * q], b = k2[2 * q + 1];
+            c += (a.x < key) + (a.y < key) + (b.x < key) + (b.y < key);
+        }
     }
+    auto before = [&](uint64_t k, int j) { return k < key || (k == key && j < i); };
     if (warp < 8 && own + warp < quads) {
         const int j = 4 * (own + warp);
-        const uint4 k = k4[own + warp];
-        c += (k.x < key || (k.x == key && j < i)) + (k.y < key || (k.y == key && j + 1 < i)) +
-             (k.z < key || (k.z == key && j + 2 < i)) + (k.w < key || (k.w == key && j + 3 < i));
-    }
-#pragma unroll 4
-    for (int q = own + 8 + warp; q < quads; q += RANK_THREADS / 32) {
-        const uint4 k = k4[q];
-        c += (k.x < key) + (k.y < key) + (k.z < key) + (k.w < key);
+        const ulonglong2 a = k2[j / 2], b = k2[j / 2 + 1];
+        c += before(a.x, j) + before(a.y, j + 1) + before(b.x, j + 2) + before(b.y, j + 3);
     }
     if (warp == 0)
-        for (int j = n / 4 * 4; j < n; j++) c += keys[j] < key || (keys[j] == key && j < i);
+        for (int j = n / 4 * 4; j < n; j++) c += before(keys[j], j);
     part[warp][lane] = c;
     __syncthreads();
     if (warp != 0 || i >= n) return;
@@ -196,22 +225,16 @@ order_rank(int n, const double* __restrict__ x, const uint32_t* __restrict__ key
     out[c] = t;
 }
 
-constexpr int64_t SMALL_KEYS = 1 << 16;   // up to here 10-bit axes and 32-bit keys
-
-template <typename Key>
-static cudaError_t sort_keys(void* tmp, size_t& bytes, Key* k0, Key* k1, int32_t* i0, int32_t* i1, int64_t n,
-                             int bits, cudaStream_t st)
+static cudaError_t sort_keys(void* tmp, size_t& bytes, uint64_t* k0, uint64_t* k1, uint32_t* i0, uint32_t* i1,
+                             int64_t n, cudaStream_t st)
 {
-    return cub::DeviceRadixSort::SortPairs(tmp, bytes, k0, k1, i0, i1, (int)n, 0, 3 * bits, st);
+    return cub::DeviceRadixSort::SortPairs(tmp, bytes, k0, k1, i0, i1, (int)n, 0, 3 * KEY_BITS, st);
 }
 
 static size_t sort_tmp(int64_t nt)
 {
     size_t tmp = 0;
-    if (nt <= SMALL_KEYS)
-        sort_keys<uint32_t>(nullptr, tmp, nullptr, nullptr, nullptr, nullptr, nt, 10, nullptr);
-    else
-        sort_keys<uint64_t>(nullptr, tmp, nullptr, nullptr, nullptr, nullptr, nt, 20, nullptr);
+    sort_keys(nullptr, tmp, nullptr, nullptr, nullptr, nullptr, nt, nullptr);
     return tmp;
 }
 
@@ -233,32 +256,26 @@ cudaError_t order_targets(int64_t nt, const double* xt, void* scratch, size_t sc
     double* part = (double*)p;            p += align256(BB_BLOCKS * 6 * sizeof(double));
     uint64_t* k0 = (uint64_t*)p;          p += align256(nt * sizeof(uint64_t));
     uint64_t* k1 = (uint64_t*)p;          p += align256(nt * sizeof(uint64_t));
-    int32_t* i0 = (int32_t*)p;            p += align256(nt * sizeof(int32_t));
-    int32_t* i1 = (int32_t*)p;            p += align256(nt * sizeof(int32_t));
+    uint32_t* i0 = (uint32_t*)p;          p += align256(nt * sizeof(int32_t));
+    uint32_t* i1 = (uint32_t*)p;          p += align256(nt * sizeof(int32_t));
     size_t tmp = sort_tmp(nt);
     void* tmpp = p;                       p += align256(tmp);
     TgtPos* tp = (TgtPos*)p;              p += align256(nt * sizeof(TgtPos));
     if ((size_t)(p - (char*)scratch) > scratch_bytes) return cudaErrorInvalidValue;
     const unsigned nb = (unsigned)((nt + BB_THREADS - 1) / BB_THREADS);
-    const int32_t* perm = nullptr;
+    const uint32_t* perm = nullptr;
     if (nt > 1) {
         bbox_partial<<<BB_BLOCKS, BB_THREADS, 0, st>>>(nt, xt, part);
-        cudaError_t e;
+        *launches += 2;
         if (nt <= RANK_MAX) {
-            hilbert_keys<<<nb, BB_THREADS, 0, st>>>(nt, xt, part, 10, (uint32_t*)k0, i0);
-            order_rank<<<(unsigned)((nt + 31) / 32), RANK_THREADS, 0, st>>>((int)nt, xt, (uint32_t*)k0, tp);
-            *launches += 3;
+            hilbert_keys<true><<<nb, BB_THREADS, 0, st>>>(nt, xt, part, k0, i0);
+            order_rank<<<(unsigned)((nt + 31) / 32), RANK_THREADS, 0, st>>>((int)nt, xt, i0, k0, tp);
+            *launches += 1;
             *out = tp;
             return cudaGetLastError();
         }
-        if (nt <= SMALL_KEYS) {
-            hilbert_keys<<<nb, BB_THREADS, 0, st>>>(nt, xt, part, 10, (uint32_t*)k0, i0);
-            e = sort_keys(tmpp, tmp, (uint32_t*)k0, (uint32_t*)k1, i0, i1, nt, 10, st);
-        } else {
-            hilbert_keys<<<nb, BB_THREADS, 0, st>>>(nt, xt, part, 20, k0, i0);
-            e = sort_keys(tmpp, tmp, k0, k1, i0, i1, nt, 20, st);
-        }
-        *launches += 2;
+        hilbert_keys<false><<<nb, BB_THREADS, 0, st>>>(nt, xt, part, k0, i0);
+        cudaError_t e = sort_keys(tmpp, tmp, k0, k1, i0, i1, nt, st);
         if (e != cudaSuccess) return e;
         *launches += 1;  // CUB's onesweep passes are counted as one library call
         perm = i1;
