@@ -10,16 +10,19 @@
 //     v = d x sum Q gam - sum Q (y x gam),   T_j = sum Q gam y_j :
 // 26 sums of the two weights G(r), Q(r) times quantities of the source alone.  They are a
 // matrix product, weights[targets x sources] * B[sources x 26], which tcgen05.mma does; the
-// CUDA cores are left with r^2 and the weights (12 of the pair's 37 instructions).
+// CUDA cores are left with r^2 and the weights.
 //
-// Arithmetic.  A weight is split into two f16 numbers, hi + lo (22 to 24 bits), and so is every
-// entry of B; all four products are accumulated in FP32 (TMEM), over one tile of 64 sources at
-// a time, and added to the same FP32 mid-level and FP64 sums as the mixed kernel's.  Scales are
-// powers of two: distances are taken in units of R = 4..8 times the least distance of the
-// warp's targets from the tile (so that G <= 2^9, Q <= 2^15 and, within a factor of 8 in
-// distance, both keep a normal lo part), y in units of the tile's radius, gam in units of the
-// tile's largest strength / 64.  Errors against 64 bits stay at or below the mixed kernel's
-// (U / J, 2-norm): rings of 60,000 4.1e-8 / 5.0e-8 (4.5e-8 / 8.1e-8 there), random cloud of
+// Arithmetic.  A weight is split into two f16 numbers, hi + lo, and so is every entry of B; all
+// four products are accumulated in FP32 (TMEM), over one tile of 64 sources at a time, and added to
+// FP32 mid-level sums (TC_MID tiles) and FP64 ones.  Scales are powers of two: distances are taken
+// in units of R = 4..8 times the least distance of the warp's targets from the tile (so that
+// G <= 2^9, Q <= 2^15), y in units of the tile's radius, and each column of B so that its largest
+// entry is near 2^14: a small component of the strengths or positions keeps its own digits.  hi + lo
+// holds 22 to 24 bits, except for Q past 1.5 R, where lo is subnormal: 20 bits at 2 R, the farthest
+// pairs.  (Pairs alone at 1.5 R, measured: error of J 2.9e-7 to 3.0e-7 rms, 2.4e-7 to 2.9e-7 in
+// uj_mixed_kernel, most of it r^-5 from the approximate square root; R within 6.4..8 of the least
+// distance, 22 bits everywhere, gave 2.9e-7 to 3.1e-7.)  Errors against 64 bits
+// (U / J, 2-norm): rings of 100,000 4.4e-8 / 4.1e-8 (4.0e-8 / 6.8e-8 there, in Morton order), random cloud of
 // 65,536 1.9e-7 / 2.8e-7 (2.2e-7 / 3.2e-7).
 //
 // Classes, box to box, for a warp's 32 targets and a tile (tile_class):
@@ -63,7 +66,9 @@ constexpr int TC_BK = TC_BG + TC_QN * 16 * 2;
 constexpr int TC_B = (TCS / 16) * TC_BK;      // 8192
 constexpr int TC_POS = TCS * 4;               // bytes of one coordinate of the tile's y
 constexpr int TC_REC = TC_B + 4 * TC_POS + 64;      // B, y (x, y, z), sigma^2, header
-constexpr int TC_STRIDE = (TC_REC + 127) / 128 * 128;
+constexpr int TC_SC = 128;                          // then the scales of B's 26 columns
+constexpr int TC_STRIDE = (TC_REC + TC_SC + 127) / 128 * 128;
+constexpr int TC_SIZE = (TC_REC + 127) / 128 * 128; // a stage, without the scales
 constexpr int TC_THREADS = UJ_THREADS + 32;
 constexpr int TC_COLS = 128;                  // TMEM columns of a block: A 64, G sums 16, Q sums 48
 constexpr int TC_DG = 64, TC_DQ = 80;
@@ -111,6 +116,7 @@ pack_tiles(int64_t n, const double* __restrict__ gs, const double* __restrict__ 
 {
     __shared__ double red[2][7];
     __shared__ float redf[2][3];
+    __shared__ uint32_t redc[2][26];
     __shared__ __align__(16) char img[TC_B];
     const int k = threadIdx.x, warp = k >> 5, lane = k & 31;
     const int64_t o = (int64_t)blockIdx.x * TCS + k;
@@ -177,15 +183,24 @@ pack_tiles(int64_t n, const double* __restrict__ gs, const double* __restrict__ 
             col[9 + 3 * j + i] = g[i] * y[j];
             if (3 * j + i < 8) col[18 + 3 * j + i] = mx[i] * y[j];
         }
+    // each column to a largest entry of 2^14 in magnitude
+    for (int m = 0; m < 26; m++) {
+        const uint32_t top = __reduce_max_sync(0xffffffffu, __float_as_uint(fabsf((float)col[m])));
+        if (lane == 0) redc[warp][m] = top;
+    }
     for (int w = k; w < TC_B / 16; w += TCS) ((uint4*)img)[w] = make_uint4(0, 0, 0, 0);
     __syncthreads();
+    auto scale = [&](int m) {
+        const float top = __uint_as_float(max(redc[0][m], redc[1][m]));
+        return top > 1e-30f && top < 1e30f ? pow2_at_least(top) * 0x1p-14f : 1.f;
+    };
     char* kb = img + (k >> 4) * TC_BK;
     const int kc = (k >> 3) & 1, k8 = k & 7;
     for (int m = 0; m < 26; m++) {
         const bool q = m >= 6;
-        const float v = (float)col[m];
-        const __half h = __float2half_rn(v);
-        const __half l = __float2half_rn((float)(col[m] - (double)__half2float(h)));
+        const float sc = scale(m), isc = __uint_as_float((254u << 23) - __float_as_uint(sc));   // a power of two
+        const __half h = __float2half_rn((float)col[m] * isc);
+        const __half l = __float2half_rn((float)(col[m] - (double)(__half2float(h) * sc)) * isc);
         const int base = q ? TC_BG : 0, nh = q ? m - 6 : m, nl = q ? m - 6 + 20 : m + 6;
         *(__half*)(kb + base + ((nh >> 3) * 2 + kc) * 128 + (nh & 7) * 16 + k8 * 2) = h;
         *(__half*)(kb + base + ((nl >> 3) * 2 + kc) * 128 + (nl & 7) * 16 + k8 * 2) = l;
@@ -196,6 +211,7 @@ pack_tiles(int64_t n, const double* __restrict__ gs, const double* __restrict__ 
     // y, in absolute units (the pair's dx needs no scale of its own); sources past n at the centre
     for (int m = 0; m < 3; m++) ((float*)(out + TC_B + m * TC_POS))[k] = on ? (float)(x[m] - c[m]) : 0.f;
     ((float*)(out + TC_B + 3 * TC_POS))[k] = mys2;
+    if (k < 26) ((float*)(out + TC_REC))[k] = scale(k);
     if (k == 0) {
         TileHdr h;
         h.chx = (float)c[0]; h.chy = (float)c[1]; h.chz = (float)c[2]; h.rad = rad;
@@ -360,7 +376,7 @@ __device__ __noinline__ int tile_class(const TileHdr& h, const float3& wch, cons
     return K == K_GAUSERF && d2 > 2.f * h.sig2 ? TILE_MID : TILE_NEAR;
 }
 
-struct TcStage { char rec[TC_STRIDE]; };
+struct TcStage { char rec[TC_SIZE]; };
 
 template <int K>
 __global__ void __launch_bounds__(TC_THREADS, 4)
@@ -369,6 +385,9 @@ uj_tc_kernel(int64_t nt, const TgtPos* __restrict__ tgt, int ntiles_all, const T
              double* U, int64_t ldU, double* J, int64_t ldJ, double* partial, int64_t nt_pad)
 {
     __shared__ __align__(128) TcStage stage[2];
+    // The scales of a tile's columns, read when its sums are, in the next tile's first half: a slot is
+    // filled again three tiles on, after every warp's arrival for that half.
+    __shared__ __align__(16) ulonglong2 scales[3][TC_SC / 16];
     __shared__ SrcMixed near_s[UJ_WARPS][WT];
     __shared__ float4 near_o[UJ_WARPS][WT];
     __shared__ double acc64[14][UJ_THREADS];
@@ -399,11 +418,17 @@ uj_tc_kernel(int64_t nt, const TgtPos* __restrict__ tgt, int ntiles_all, const T
         const bool one = elect_one();
         bool ok = true;
         int loaded = min(ntiles, 2);
-        if (one)
-            for (int q = 0; q < loaded; q++) {
-                mbar_expect_tx(&bfull[q], TC_REC);
-                bulk_load(&stage[q], rec + (int64_t)(t0 + q * tstep) * TC_STRIDE, TC_REC, &bfull[q]);
+        int slot = 0;                       // of the next tile's scales
+        auto load = [&](int q) {
+            if (one) {
+                const char* r = rec + (int64_t)(t0 + q * tstep) * TC_STRIDE;
+                mbar_expect_tx(&bfull[q & 1], TC_REC + TC_SC);
+                bulk_load(&stage[q & 1], r, TC_REC, &bfull[q & 1]);
+                bulk_load(scales[slot], r + TC_REC, TC_SC, &bfull[q & 1]);
             }
+            slot = slot == 2 ? 0 : slot + 1;
+        };
+        for (int q = 0; q < loaded; q++) load(q);
         constexpr uint32_t ig = idesc_f16(128, TC_GN), iq = idesc_f16(128, TC_QN);
         constexpr uint32_t neg = 1u << 13;   // the lo operands are stored negated
         for (int it = 0; ok && it < ntiles; it++) {
@@ -432,11 +457,7 @@ uj_tc_kernel(int64_t nt, const TgtPos* __restrict__ tgt, int ntiles_all, const T
                 // the stage is free: every warp has read its y (afull of the last step), and
                 // the tile's MMAs are done with its B
                 ok = mbar_wait(&adone, 1u);
-                if (ok && one) {
-                    mbar_expect_tx(&bfull[s], TC_REC);
-                    bulk_load(&stage[s], rec + (int64_t)(t0 + loaded * tstep) * TC_STRIDE, TC_REC, &bfull[s]);
-                }
-                loaded += ok;
+                if (ok) load(loaded++);
             }
         }
         if (!ok) {   // a wait that gave up: wait (bounded) for what is in flight
@@ -505,15 +526,18 @@ uj_tc_kernel(int64_t nt, const TgtPos* __restrict__ tgt, int ntiles_all, const T
     const uint32_t ta = tmem + ((uint32_t)(warp * 32) << 16);
     bool ok = true;
     // the tile's sums, back in absolute units
-    auto collect = [&](float pdx, float pdy, float pdz, float iR, float hg, float hy) {
+    auto collect = [&](const ulonglong2* sc, float pdx, float pdy, float pdz, float iR, float hg, float hy) {
         const float kap = hy * iR, su = hg * iR * iR, sw = su * iR;
         {
             float v[16];
             tmem_ld8(ta + TC_DG, v);
             tmem_ld8(ta + TC_DG + 8, v + 8);
             tc_wait_ld(v);
-            const float wx = v[0] + v[6], wy = v[1] + v[7], wz = v[2] + v[8];
-            const float mx = v[3] + v[9], my = v[4] + v[10], mz = v[5] + v[11];
+            const ulonglong2 s0 = sc[0], s1 = sc[1];
+            float wx, wy, wz, mx, my, mz;
+            upk(mul2(add2(pk(v[0], v[1]), pk(v[6], v[7])), s0.x), wx, wy);
+            upk(mul2(add2(pk(v[2], v[3]), pk(v[8], v[9])), s0.y), wz, mx);
+            upk(mul2(add2(pk(v[4], v[5]), pk(v[10], v[11])), s1.x), my, mz);
             mu[0] = fmaf(su, fmaf(pdy, wz, fmaf(-pdz, wy, -kap * mx)), mu[0]);
             mu[1] = fmaf(su, fmaf(pdz, wx, fmaf(-pdx, wz, -kap * my)), mu[1]);
             mu[2] = fmaf(su, fmaf(pdx, wy, fmaf(-pdy, wx, -kap * mz)), mu[2]);
@@ -527,7 +551,10 @@ uj_tc_kernel(int64_t nt, const TgtPos* __restrict__ tgt, int ntiles_all, const T
             for (int k = 0; k < 5; k++) tmem_ld8(ta + TC_DQ + 8 * k, v + 8 * k);
             tc_wait_ld(v);
 #pragma unroll
-            for (int k = 0; k < 20; k++) v[k] += v[20 + k];
+            for (int k = 0; k < 10; k++) {
+                const ulonglong2 s2 = sc[(3 + k) >> 1];
+                upk(mul2(add2(pk(v[2 * k], v[2 * k + 1]), pk(v[20 + 2 * k], v[21 + 2 * k])), k & 1 ? s2.x : s2.y), v[2 * k], v[2 * k + 1]);
+            }
             const float* T = v + 3;          // T[3 j + i] = sum Q gam_i y_j
             const float kx = kap * pdx, ky = kap * pdy, kz = kap * pdz, k2 = kap * kap;
             // v = d x A - kappa sum Q (y x gam), the latter from the antisymmetric part of T
@@ -551,6 +578,7 @@ uj_tc_kernel(int64_t nt, const TgtPos* __restrict__ tgt, int ntiles_all, const T
     };
     bool pend = false;                           // the last tile's sums are still to be read
     float pdx = 0.f, pdy = 0.f, pdz = 0.f, pR = 0.f, pg = 0.f, py = 0.f;   // its d, 1/R and scales
+    int slot = 2;                                // where the scales of the tile before are
     for (int base = 0; ok && base < ntiles; base += 32) {
         float iRl = 0.f;
         int cls = 0;
@@ -569,12 +597,13 @@ uj_tc_kernel(int64_t nt, const TgtPos* __restrict__ tgt, int ntiles_all, const T
                     ok = mbar_wait(&adone, 1u);      // the previous tile's second half
                     if (!ok) break;
                     tc_fence_after();
-                    if (pend) { collect(pdx, pdy, pdz, pR, pg, py); tc_fence_before(); __syncwarp(); }
+                    if (pend) { collect(scales[slot], pdx, pdy, pdz, pR, pg, py); tc_fence_before(); __syncwarp(); }
                     pend = false;
                     if (lane == 0) mbar_arrive(&afull);
                     ok = mbar_wait(&adone, 0u);
                     if (!ok) break;
                     if (lane == 0) mbar_arrive(&afull);
+                    slot = slot == 2 ? 0 : slot + 1;
                     continue;
                 }
                 const char* r = stage[it & 1].rec;
@@ -595,14 +624,14 @@ uj_tc_kernel(int64_t nt, const TgtPos* __restrict__ tgt, int ntiles_all, const T
                         if (!ok) break;
                         tc_fence_after();
                         store_a(ta, gh, gl, qh, ql);
-                        if (hh == 0 && pend) collect(pdx, pdy, pdz, pR, pg, py);
+                        if (hh == 0 && pend) collect(scales[slot], pdx, pdy, pdz, pR, pg, py);
                         weigh<K, 8>(p + 4, dx, dy, dz, iR, gh, gl, qh, ql);
                         store_a(ta + 8, gh, gl, qh, ql);
                     } else if constexpr (K == K_GAUSERF) {
                         ok = mbar_wait(&adone, (uint32_t)(hh ^ 1));
                         if (!ok) break;
                         tc_fence_after();
-                        if (hh == 0 && pend) collect(pdx, pdy, pdz, pR, pg, py);
+                        if (hh == 0 && pend) collect(scales[slot], pdx, pdy, pdz, pR, pg, py);
 #pragma unroll 1
                         for (int c = 0; c < 4; c++) {
                             uint32_t gh[4], gl[4], qh[4], ql[4];
@@ -620,6 +649,7 @@ uj_tc_kernel(int64_t nt, const TgtPos* __restrict__ tgt, int ntiles_all, const T
                 }
                 if (!ok) break;
                 pend = true;
+                slot = slot == 2 ? 0 : slot + 1;
                 pdx = dx; pdy = dy; pdz = dz; pR = iR; pg = hg; py = hy;
             }
             flush();
@@ -628,7 +658,7 @@ uj_tc_kernel(int64_t nt, const TgtPos* __restrict__ tgt, int ntiles_all, const T
     if (ok) {
         ok = mbar_wait(&adone, 1u);
         tc_fence_after();
-        if (ok && pend) collect(pdx, pdy, pdz, pR, pg, py);
+        if (ok && pend) collect(scales[slot], pdx, pdy, pdz, pR, pg, py);
     }
     if (!ok && lane == 0) failed = 1;
 

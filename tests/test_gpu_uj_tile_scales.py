@@ -56,3 +56,16 @@ def test_long_sums_of_one_sign(ctx):
     (_, a), (_, b) = uj(ctx, X, G, s, 2, 1), uj(ctx, X, G, s, 2, 0)
     e = normwise(a, b)[1]
     assert e <= 5e-8, f"{e:.3e}"
+
+
+@pytest.mark.parametrize("k", [2, 3])
+@pytest.mark.parametrize("small", [1e-3, 1e-5, 1e-7])
+def test_small_strength_components(ctx, k, small):
+    """Strengths nearly along z: the small velocity across the plane comes from their small components
+    alone, and is as accurate as the large ones: within 1e-6 of its own largest value."""
+    X, G, s = random_cloud(20_000, seed=31)
+    H = G * [small, small, 1.0]
+    a, b = uj(ctx, X, H, s, k, 1)[0], uj(ctx, X, H, s, k, 0)[0]
+    for c in range(3):
+        e = normwise(a[:, c], b[:, c])[0]
+        assert e <= 1e-6, f"U{c}: {e:.3e}"
