@@ -82,6 +82,9 @@ struct vpm_ctx {
     const double* near_x = nullptr;
     int near_leaf = 0;
     double near_theta = 0.0;
+    // a kernel whose wait gave up sets *gave_up (pinned host memory, read by bounded_wait)
+    int* gave_up = nullptr;
+    int wait_rounds = WAIT_ROUNDS;
     int sync_rc = 0;     // VPM status of the last wait made for the list builder
 };
 
@@ -141,7 +144,12 @@ int bounded_wait(vpm_ctx* c)
     auto t0 = std::chrono::steady_clock::now();
     for (;;) {
         cudaError_t q = cudaEventQuery(c->done);
-        if (q == cudaSuccess) return VPM_OK;
+        if (q == cudaSuccess) {
+            if (!*(volatile int*)c->gave_up) return VPM_OK;
+            *(volatile int*)c->gave_up = 0;
+            return fail(c, VPM_ERR_TIMEOUT, "a wait inside a kernel gave up after %d rounds; the outputs are not valid",
+                        c->wait_rounds);
+        }
         if (q != cudaErrorNotReady) return cuda_fail(c, q, "device work");
         double el = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
         if (el > c->timeout_s) {
@@ -333,6 +341,8 @@ void ensure_tiles(vpm_ctx* c, const UJArgs& a, Workspace* w)
     if (!uj_takes_tiles(a)) return;
     if (c->tiles.grow(uj_tc_bytes(a.ns)) == cudaSuccess) w->tiles = c->tiles.p;
     else cudaGetLastError();
+    w->gave_up = c->gave_up;
+    w->wait_rounds = c->wait_rounds;
 }
 
 int grow(vpm_ctx* c, DevBuf& b, size_t bytes, const char* what)
@@ -411,11 +421,15 @@ int vpm_ctx_create(vpm_ctx** out, int device)
     // a blocking stream: ordered with the legacy default stream's work both ways, so that
     // callers who queue their own work there (frameworks' default streams) need no events
     if (cudaStreamCreateWithFlags(&c->own_stream, cudaStreamDefault) != cudaSuccess ||
-        cudaEventCreateWithFlags(&c->done, cudaEventDisableTiming) != cudaSuccess) {
+        cudaEventCreateWithFlags(&c->done, cudaEventDisableTiming) != cudaSuccess ||
+        cudaHostAlloc((void**)&c->gave_up, sizeof(int), cudaHostAllocMapped) != cudaSuccess) {
         cudaGetLastError();
+        if (c->done) cudaEventDestroy(c->done);
+        if (c->own_stream) cudaStreamDestroy(c->own_stream);
         delete c;
         return fail(nullptr, VPM_ERR_CUDA, "could not create a stream/event on device %d", device);
     }
+    *c->gave_up = 0;
     c->stream = c->own_stream;
     *out = c;
     return VPM_OK;
@@ -436,6 +450,7 @@ int vpm_ctx_destroy(vpm_ctx* c)
         for (DevBuf* b : {&c->din, &c->dout}) b->release();
         c->hin.release();
         c->hout.release();
+        if (c->gave_up) cudaFreeHost(c->gave_up);
         if (c->done) cudaEventDestroy(c->done);
         if (c->own_stream) cudaStreamDestroy(c->own_stream);
         cudaGetLastError();
@@ -460,6 +475,16 @@ int vpm_ctx_set_timeout(vpm_ctx* c, double seconds)
     if (!(seconds > 0)) return fail(c, VPM_ERR_ARG, "timeout must be > 0 s");
     std::lock_guard<std::mutex> lk(c->mu);
     c->timeout_s = seconds;
+    return VPM_OK;
+}
+
+int vpm_ctx_set_wait_rounds(vpm_ctx* c, int rounds)
+{
+    if (!c) return fail(nullptr, VPM_ERR_ARG, "vpm_ctx_set_wait_rounds: ctx is NULL");
+    if (rounds < 0 || rounds > WAIT_ROUNDS)
+        return fail(c, VPM_ERR_ARG, "vpm_ctx_set_wait_rounds: rounds must be in 0..%d", WAIT_ROUNDS);
+    std::lock_guard<std::mutex> lk(c->mu);
+    c->wait_rounds = rounds;
     return VPM_OK;
 }
 

@@ -116,12 +116,17 @@ struct LeafArgs {
     bool uj = true;                                           // false: the Estr pass alone (J is input)
 };
 
+// Rounds after which a wait inside a kernel gives up: seconds, against microseconds in normal running.
+constexpr int WAIT_ROUNDS = 1 << 16;
+
 // Scratch and packing buffers supplied by the caller (the context).
 struct Workspace {
     void* src_pack; size_t src_pack_bytes;
     void* order; size_t order_bytes;          // curve ordering of the targets
     double* partial; size_t partial_bytes;    // split-source partial sums
     void* tiles = nullptr;                    // uj_tc_bytes: the tensor pass's tiles (null: not taken)
+    int wait_rounds = WAIT_ROUNDS;            // its waits' limit, and the word it sets to 1 when one gives up
+    int* gave_up = nullptr;
 };
 
 size_t uj_src_pack_bytes(int64_t ns, int precision);
@@ -152,7 +157,7 @@ size_t uj_partial_bytes(int64_t nt, int nsplit, int components = 12);
 bool uj_takes_tiles(const UJArgs& a);
 size_t uj_tc_bytes(int64_t n);
 int uj_tc_splits(int64_t n, int num_sms);
-cudaError_t launch_uj_tc(const UJArgs& a, const TgtPos* tgt, const SrcMixed* src, void* work, int nsplit,
+cudaError_t launch_uj_tc(const UJArgs& a, const TgtPos* tgt, const SrcMixed* src, const Workspace& w, int nsplit,
                          double* partial, int64_t nt_pad, cudaStream_t st, int64_t* launches);
 
 // Curve-order the nt targets xt; *out receives nt TgtPos records in scratch.

@@ -30,9 +30,12 @@ namespace {
 
 __device__ __align__(256) unsigned char g_noalloc_scratch[VPM_NOALLOC_SCRATCH_BYTES];
 
+__device__ int g_noalloc_gave_up;      // set by a kernel whose wait gave up
+
 constexpr int MAX_DEVICES = 64;
 std::mutex g_setup_mu;
 void* g_scratch_ptr[MAX_DEVICES] = {nullptr};
+int* g_gave_up_ptr[MAX_DEVICES] = {nullptr};
 
 // Errors are reported through vpm_last_error(NULL), like vpm_ctx_create's.
 int nerr(int code, const char* fmt, ...) __attribute__((format(printf, 2, 3)));
@@ -63,22 +66,25 @@ bool is_device_ptr(const void* p, int dev)
     return at.type == cudaMemoryTypeManaged || (at.type == cudaMemoryTypeDevice && at.device == dev);
 }
 
-// Address of the scratch array on the current device (looked up once per device).
-int scratch_address(int dev, void** out)
+// Addresses of the scratch array and of the word beside it on the current device (looked up once per device).
+int scratch_address(int dev, void** out, int** gave_up)
 {
     if (dev < 0 || dev >= MAX_DEVICES) return nerr(VPM_ERR_ARG, "device %d out of range", dev);
     std::lock_guard<std::mutex> lk(g_setup_mu);
     if (!g_scratch_ptr[dev]) {
-        void* ptr = nullptr;
+        void *ptr = nullptr, *word = nullptr;
         cudaError_t e = cudaGetSymbolAddress(&ptr, g_noalloc_scratch);
-        if (e != cudaSuccess || !ptr) {
+        if (e == cudaSuccess) e = cudaGetSymbolAddress(&word, g_noalloc_gave_up);
+        if (e != cudaSuccess || !ptr || !word) {
             cudaGetLastError();
             return nerr(VPM_ERR_CUDA, "cudaGetSymbolAddress of the scratch array failed: %s",
                         cudaGetErrorString(e));
         }
         g_scratch_ptr[dev] = ptr;
+        g_gave_up_ptr[dev] = (int*)word;
     }
     *out = g_scratch_ptr[dev];
+    *gave_up = g_gave_up_ptr[dev];
     return VPM_OK;
 }
 
@@ -122,7 +128,8 @@ int vpm_uj_dev_noalloc(int64_t nt, const double* xt, int64_t ns, const double* x
                     (long long)nt, (long long)ns, pack + order + part,
                     (unsigned long long)VPM_NOALLOC_SCRATCH_BYTES);
     void* base = nullptr;
-    int rc = scratch_address(dev, &base);
+    int* gave_up = nullptr;
+    int rc = scratch_address(dev, &base, &gave_up);
     if (rc != VPM_OK) return rc;
     char* p = (char*)base;
     vpm::Workspace w;
@@ -140,6 +147,7 @@ int vpm_uj_dev_noalloc(int64_t nt, const double* xt, int64_t ns, const double* x
         w.partial = tc_part ? (double*)p : nullptr;
         w.partial_bytes = tc_part;
         w.tiles = p + tc_part;
+        w.gave_up = gave_up;
     }
     cudaStream_t st = (cudaStream_t)stream;
     int64_t launches = 0;
@@ -153,7 +161,14 @@ int vpm_uj_dev_noalloc(int64_t nt, const double* xt, int64_t ns, const double* x
     int sleep_us = 2;
     for (;;) {
         e = cudaStreamQuery(st);
-        if (e == cudaSuccess) return VPM_OK;
+        if (e == cudaSuccess) {
+            int bad = 0;
+            if (!w.tiles || (e = cudaMemcpyAsync(&bad, gave_up, sizeof(int), cudaMemcpyDeviceToHost, st)) == cudaSuccess) {
+                if (!bad) return VPM_OK;
+                cudaMemsetAsync(gave_up, 0, sizeof(int), st);
+                return nerr(VPM_ERR_TIMEOUT, "vpm_uj_dev_noalloc: a wait inside a kernel gave up; U and J are not valid");
+            }
+        }
         if (e != cudaErrorNotReady) {
             cudaGetLastError();
             return nerr(VPM_ERR_CUDA, "vpm_uj_dev_noalloc: device work failed: %s", cudaGetErrorString(e));

@@ -26,19 +26,20 @@ __device__ __forceinline__ void mbar_expect_tx(uint64_t* m, uint32_t bytes)
 {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(m)), "r"(bytes) : "memory");
 }
-// Rounds of try_wait (each suspends the thread for a hardware time slice) before a wait
-// gives up; a wait in normal running ends within the first few.
-constexpr int MBAR_SPIN = 1 << 16;
-// true once the phase of m with this parity has completed, false after MBAR_SPIN rounds
-__device__ __forceinline__ bool mbar_wait(uint64_t* m, uint32_t parity)
+// A wait of a whole warp for the phase of m with this parity: a look, then up to `rounds` rounds of
+// try_wait (each suspends the threads for a hardware time slice; a wait in normal running ends within
+// the first few), after which it gives up.  The same answer in all 32 lanes: true if every lane saw the
+// phase complete.
+__device__ __forceinline__ bool mbar_wait(uint64_t* m, uint32_t parity, uint32_t rounds)
 {
     uint32_t done;
-    asm volatile("{\n\t.reg .pred p, q;\n\t.reg .u32 n;\n\tmov.u32 n, %3;\n"
-                 "WAIT:\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t@p bra DONE;\n\t"
-                 "sub.u32 n, n, 1;\n\tsetp.ne.u32 q, n, 0;\n\t@q bra WAIT;\n"
+    asm volatile("{\n\t.reg .pred p, q;\n\t.reg .u32 n;\n\tmov.u32 n, %3;\n\t"
+                 "mbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+                 "WAIT:\n\t@p bra DONE;\n\tsetp.eq.u32 q, n, 0;\n\t@q bra DONE;\n\tsub.u32 n, n, 1;\n\t"
+                 "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tbra WAIT;\n"
                  "DONE:\n\tselp.u32 %0, 1, 0, p;\n\t}"
-                 : "=r"(done) : "r"(smem_u32(m)), "r"(parity), "n"(MBAR_SPIN) : "memory");
-    return done != 0;
+                 : "=r"(done) : "r"(smem_u32(m)), "r"(parity), "r"(rounds) : "memory");
+    return __all_sync(0xffffffffu, done != 0);
 }
 
 // one lane of a converged warp

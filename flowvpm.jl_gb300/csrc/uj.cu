@@ -399,7 +399,7 @@ static cudaError_t launch_uj_k(const UJArgs& a, const Workspace& w, int num_sms,
 {
     const int64_t ns_pad = round_up(a.ns, UJ_TILE);
     const int64_t nt_pad = round_up(a.nt, UJ_THREADS);
-    const bool tc = uj_takes_tiles(a) && w.tiles;
+    const bool tc = uj_takes_tiles(a) && w.tiles && w.gave_up;
     int nsplit = tc ? uj_tc_splits(a.nt, num_sms) : uj_num_splits(a.nt, a.ns, num_sms, a.precision);
     while (!tc && nsplit > 1 && uj_partial_bytes(a.nt, nsplit) > w.partial_bytes) nsplit--;   // a caller's fixed scratch
     double* partial = nsplit > 1 ? w.partial : nullptr;
@@ -418,7 +418,7 @@ static cudaError_t launch_uj_k(const UJArgs& a, const Workspace& w, int num_sms,
         pack_src_mixed<K><<<(unsigned)((ns_pad + pb - 1) / pb), pb, 0, st>>>(a.ns, ns_pad, a.xs, a.gs, a.sgs,
                                                                              a.self ? tgt : nullptr, src);
         if (tc) {
-            e = launch_uj_tc(a, tgt, src, w.tiles, nsplit, partial, nt_pad, st, launches);
+            e = launch_uj_tc(a, tgt, src, w, nsplit, partial, nt_pad, st, launches);
             if (e != cudaSuccess) return e;
         } else
         uj_mixed_kernel<K><<<grid, UJ_THREADS, 0, st>>>(a.nt, tgt, ns_pad, src, a.U, a.ldU,

@@ -432,7 +432,8 @@ template <int K>
 __global__ void __launch_bounds__(TC_THREADS, 4)
 uj_tc_kernel(int64_t nt, const TgtPos* __restrict__ tgt, int ntiles_all, const TileHdr* __restrict__ hdr,
              const char* __restrict__ rec, const SrcMixed* __restrict__ src,
-             double* U, int64_t ldU, double* J, int64_t ldJ, double* partial, int64_t nt_pad)
+             double* U, int64_t ldU, double* J, int64_t ldJ, double* partial, int64_t nt_pad, uint32_t rounds,
+             int* __restrict__ gave_up)
 {
     __shared__ __align__(128) TcStage stage[2];
     // The scales of a tile's columns, read when its sums are, in the next tile's first half: a slot is
@@ -483,12 +484,12 @@ uj_tc_kernel(int64_t nt, const TgtPos* __restrict__ tgt, int ntiles_all, const T
         constexpr uint32_t neg = 1u << 13;   // the lo operands are stored negated
         for (int it = 0; ok && it < ntiles; it++) {
             const int s = it & 1;
-            ok = mbar_wait(&bfull[s], (uint32_t)(it >> 1) & 1u);
+            ok = mbar_wait(&bfull[s], (uint32_t)(it >> 1) & 1u, rounds);
             const uint32_t b0 = smem_u32(&stage[s]);
             const uint64_t dg0 = smem_desc(b0, 128, 256), dq0 = smem_desc(b0 + TC_BG, 128, 256);
 #pragma unroll 1
             for (int h = 0; ok && h < 2; h++) {   // 32 sources: step 2 it + h
-                ok = mbar_wait(&afull, (uint32_t)h);
+                ok = mbar_wait(&afull, (uint32_t)h, rounds);
                 tc_fence_after();
                 if (ok && one) {
 #pragma unroll
@@ -506,14 +507,14 @@ uj_tc_kernel(int64_t nt, const TgtPos* __restrict__ tgt, int ntiles_all, const T
             if (ok && loaded < ntiles) {
                 // the stage is free: every warp has read its y (afull of the last step), and
                 // the tile's MMAs are done with its B
-                ok = mbar_wait(&adone, 1u);
+                ok = mbar_wait(&adone, 1u, rounds);
                 if (ok) load(loaded++);
             }
         }
         if (!ok) {   // a wait that gave up: wait (bounded) for what is in flight
             if (one) { failed = 1; mma_commit(&drain); }
-            for (int q = max(0, loaded - 2); q < loaded; q++) mbar_wait(&bfull[q & 1], (uint32_t)(q >> 1) & 1u);
-            mbar_wait(&drain, 0);
+            for (int q = max(0, loaded - 2); q < loaded; q++) mbar_wait(&bfull[q & 1], (uint32_t)(q >> 1) & 1u, WAIT_ROUNDS);
+            mbar_wait(&drain, 0, WAIT_ROUNDS);
         }
         __syncwarp();
         tc_fence_before();
@@ -644,13 +645,13 @@ uj_tc_kernel(int64_t nt, const TgtPos* __restrict__ tgt, int ntiles_all, const T
                 const bool isfar = (far >> (it & 31)) & 1u;
                 if (!isfar && !((mid >> (it & 31)) & 1u)) {
                     // not this warp's: its rows of A keep stale values and its sums are not read
-                    ok = mbar_wait(&adone, 1u);      // the previous tile's second half
+                    ok = mbar_wait(&adone, 1u, rounds);      // the previous tile's second half
                     if (!ok) break;
                     tc_fence_after();
                     if (pend) { collect(scales[slot], pdx, pdy, pdz, pR, pg, py); tc_fence_before(); __syncwarp(); }
                     pend = false;
                     if (lane == 0) mbar_arrive(&afull);
-                    ok = mbar_wait(&adone, 0u);
+                    ok = mbar_wait(&adone, 0u, rounds);
                     if (!ok) break;
                     if (lane == 0) mbar_arrive(&afull);
                     slot = slot == 2 ? 0 : slot + 1;
@@ -658,7 +659,7 @@ uj_tc_kernel(int64_t nt, const TgtPos* __restrict__ tgt, int ntiles_all, const T
                 }
                 const char* r = stage[it & 1].rec;
                 const float iR = __shfl_sync(0xffffffffu, iRl, it & 31);
-                ok = mbar_wait(&bfull[it & 1], (uint32_t)(it >> 1) & 1u);
+                ok = mbar_wait(&bfull[it & 1], (uint32_t)(it >> 1) & 1u, rounds);
                 if (!ok) break;
                 const TileHdr& h = *(const TileHdr*)(r + TC_B + 4 * TC_POS);
                 const float dx = ((th.x - h.chx) + (tl.x - h.clx)) * iR, dy = ((th.y - h.chy) + (tl.y - h.cly)) * iR,
@@ -670,7 +671,7 @@ uj_tc_kernel(int64_t nt, const TgtPos* __restrict__ tgt, int ntiles_all, const T
                     if (isfar) {
                         uint32_t gh[8], gl[8], qh[8], ql[8];
                         weigh<K, 8>(p, dx, dy, dz, iR, gh, gl, qh, ql);   // while the last step's MMAs run
-                        ok = mbar_wait(&adone, (uint32_t)(hh ^ 1));
+                        ok = mbar_wait(&adone, (uint32_t)(hh ^ 1), rounds);
                         if (!ok) break;
                         tc_fence_after();
                         store_a(ta, gh, gl, qh, ql);
@@ -678,7 +679,7 @@ uj_tc_kernel(int64_t nt, const TgtPos* __restrict__ tgt, int ntiles_all, const T
                         weigh<K, 8>(p + 4, dx, dy, dz, iR, gh, gl, qh, ql);
                         store_a(ta + 8, gh, gl, qh, ql);
                     } else if constexpr (K == K_GAUSERF) {
-                        ok = mbar_wait(&adone, (uint32_t)(hh ^ 1));
+                        ok = mbar_wait(&adone, (uint32_t)(hh ^ 1), rounds);
                         if (!ok) break;
                         tc_fence_after();
                         if (hh == 0 && pend) collect(scales[slot], pdx, pdy, pdz, pR, pg, py);
@@ -706,7 +707,7 @@ uj_tc_kernel(int64_t nt, const TgtPos* __restrict__ tgt, int ntiles_all, const T
         }
     }
     if (ok) {
-        ok = mbar_wait(&adone, 1u);
+        ok = mbar_wait(&adone, 1u, rounds);
         tc_fence_after();
         if (ok && pend) collect(scales[slot], pdx, pdy, pdz, pR, pg, py);
     }
@@ -775,6 +776,7 @@ uj_tc_kernel(int64_t nt, const TgtPos* __restrict__ tgt, int ntiles_all, const T
     flush();
     tc_fence_before();
     __syncthreads();
+    if (failed && threadIdx.x == 0) *(volatile int*)gave_up = 1;     // and the block's sums are NaN
     if (!valid) return;
     double f[14];
 #pragma unroll
@@ -801,27 +803,29 @@ int uj_tc_splits(int64_t n, int num_sms)
 }
 
 template <int K>
-static cudaError_t launch_k(const UJArgs& a, const TgtPos* tgt, const SrcMixed* src, void* work, int nsplit,
+static cudaError_t launch_k(const UJArgs& a, const TgtPos* tgt, const SrcMixed* src, const Workspace& w, int nsplit,
                             double* partial, int64_t nt_pad, cudaStream_t st)
 {
+    void* work = w.tiles;
     const int tiles = (int)tc_tiles(a.ns);
     TileHdr* hdr = (TileHdr*)work;
     char* rec = (char*)work + align128((size_t)tiles * sizeof(TileHdr));
     pack_tiles<K><<<tiles, TCS, 0, st>>>(a.ns, a.gs, a.sgs, tgt, hdr, rec);
     const dim3 grid((unsigned)(nt_pad / UJ_THREADS), (unsigned)nsplit);
-    uj_tc_kernel<K><<<grid, TC_THREADS, 0, st>>>(a.nt, tgt, tiles, hdr, rec, src, a.U, a.ldU, a.J, a.ldJ, partial, nt_pad);
+    uj_tc_kernel<K><<<grid, TC_THREADS, 0, st>>>(a.nt, tgt, tiles, hdr, rec, src, a.U, a.ldU, a.J, a.ldJ, partial, nt_pad,
+                                              (uint32_t)w.wait_rounds, w.gave_up);
     return cudaGetLastError();
 }
 
-cudaError_t launch_uj_tc(const UJArgs& a, const TgtPos* tgt, const SrcMixed* src, void* work, int nsplit,
-                         double* partial, int64_t nt_pad, cudaStream_t st, int64_t* launches)
+cudaError_t launch_uj_tc(const UJArgs& a, const TgtPos* tgt, const SrcMixed* src, const Workspace& w,
+                         int nsplit, double* partial, int64_t nt_pad, cudaStream_t st, int64_t* launches)
 {
     *launches += 2;
     switch (a.kernel) {
-    case K_SING: return launch_k<K_SING>(a, tgt, src, work, nsplit, partial, nt_pad, st);
-    case K_GAUS: return launch_k<K_GAUS>(a, tgt, src, work, nsplit, partial, nt_pad, st);
-    case K_GAUSERF: return launch_k<K_GAUSERF>(a, tgt, src, work, nsplit, partial, nt_pad, st);
-    default: return launch_k<K_WNKLMNS>(a, tgt, src, work, nsplit, partial, nt_pad, st);
+    case K_SING: return launch_k<K_SING>(a, tgt, src, w, nsplit, partial, nt_pad, st);
+    case K_GAUS: return launch_k<K_GAUS>(a, tgt, src, w, nsplit, partial, nt_pad, st);
+    case K_GAUSERF: return launch_k<K_GAUSERF>(a, tgt, src, w, nsplit, partial, nt_pad, st);
+    default: return launch_k<K_WNKLMNS>(a, tgt, src, w, nsplit, partial, nt_pad, st);
     }
 }
 

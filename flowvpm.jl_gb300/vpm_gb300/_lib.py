@@ -42,6 +42,7 @@ SIGNATURES = {
     "vpm_last_error": (ctypes.c_char_p, [_vp]),
     "vpm_ctx_set_stream": (_int, [_vp, _vp]),
     "vpm_ctx_set_timeout": (_int, [_vp, _dbl]),
+    "vpm_ctx_set_wait_rounds": (_int, [_vp, _int]),
     "vpm_ctx_set_near_capacity": (_int, [_vp, _i64, _i64]),
     "vpm_abi_version": (_int, []),
     "vpm_build_info": (ctypes.c_char_p, []),
@@ -176,6 +177,10 @@ class Context:
 
     def set_timeout(self, seconds: float):
         self._check(self._L.vpm_ctx_set_timeout(self._h, float(seconds)))
+
+    def set_wait_rounds(self, rounds: int):
+        """Limit on the waits inside this context's kernels (a call whose wait gives up raises ERR_TIMEOUT)."""
+        self._check(self._L.vpm_ctx_set_wait_rounds(self._h, int(rounds)))
 
     def set_near_capacity(self, frontier_pairs: int, near_pairs: int):
         """Initial traversal capacities of the next near-field list build (grown on overflow)."""

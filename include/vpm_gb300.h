@@ -118,6 +118,11 @@ int vpm_ctx_set_stream(vpm_ctx* ctx, void* stream);
  * (default 3600).  A wait that runs out returns VPM_ERR_TIMEOUT and marks the
  * context unusable. */
 int vpm_ctx_set_timeout(vpm_ctx* ctx, double seconds);
+/* Limit, in rounds of the hardware's timed wait, on every wait inside this context's kernels
+ * (0..65536, default 65536: seconds, where a wait takes microseconds; 0 looks once).  A kernel
+ * whose wait gives up ends in order; the call returns VPM_ERR_TIMEOUT, its outputs are not
+ * valid (NaN) and the context stays usable.  Library plumbing. */
+int vpm_ctx_set_wait_rounds(vpm_ctx* ctx, int rounds);
 /* Capacities, in pairs, of the near-field list builder's traversal buffers for
  * the next build of this context: node pairs to be split of one frontier and near leaf
  * pairs (by default 10 n and 24 n, n >= 4096).  A build that overflows them
