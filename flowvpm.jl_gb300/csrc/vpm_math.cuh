@@ -344,9 +344,9 @@ __device__ __forceinline__ void near_GQ(float s, float isig2, float& G, float& Q
         Q = (s + 3.5f) * t * t2u * isig2;
     } else if constexpr (K == K_SING) {
         // J of a singular cloud is a handful of its nearest pairs, and Q = r^-5 carries five
-        // times the error of rsqrt.approx: one Newton step
+        // times the error of rsqrt.approx: one Newton step (not where r^2 overflows: infinity times zero)
         float rs = frsqrt(s);
-        rs = fmaf(0.5f * rs, fmaf(-s * rs, rs, 1.0f), rs);
+        if (s < INFINITY) rs = fmaf(0.5f * rs, fmaf(-s * rs, rs, 1.0f), rs);
         const float rs2 = rs * rs;
         G = rs * rs2;
         Q = G * (rs2 * isig2);
