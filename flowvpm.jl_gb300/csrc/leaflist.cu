@@ -163,16 +163,18 @@ struct PartTurn {
 };
 
 __global__ void leaf_reduce(int64_t n, int parts, int na, int nb, const double* __restrict__ partial, int64_t n_pad,
-                            const TgtPos* __restrict__ tgt, double* __restrict__ A, double* __restrict__ B)
+                            const TgtPos* __restrict__ tgt, const uint8_t* __restrict__ skip, double* __restrict__ A,
+                            double* __restrict__ B)
 {
     const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (t >= n) return;
+    const int64_t i = tgt[t].idx;
+    if (skip && skip[i]) return;                 // static targets of Estr
     const int k = blockIdx.y, nk = na + nb;
     const double* p = partial + k * n_pad + t;
     double s = 0.0;
 #pragma unroll 4
     for (int q = 0; q < parts; q++) s += p[(int64_t)q * nk * n_pad];
-    const int64_t i = tgt[t].idx;
     if (k < na) A[na * i + k] += s;
     else B[nb * i + (k - na)] += s;
 }
@@ -686,12 +688,12 @@ nf_estr(int64_t n, int64_t ngroups, const TgtPos* __restrict__ tgt, const int32_
         }
     }
     if constexpr (MIXED) estr_flush(sm, cm, zg, zv);
-    if (!live && !(partial && me.valid)) return;
+    if (!live) return;      // a static target's partial sums are not read
     double o[3] = {0.0, 0.0, 0.0};
     if constexpr (ZETA) {
 #pragma unroll
         for (int k = 0; k < 3; k++) o[k] = zg[k];
-    } else if (live) {
+    } else {
         const double* Jp = Jt + 9 * (int64_t)me.idx;
         const int sr = transposed ? 3 : 1, sc = transposed ? 1 : 3;
 #pragma unroll
@@ -751,11 +753,11 @@ static LeafWork leaf_work(const LeafArgs& a, const NearLists& L, void* work)
 }
 
 static void reduce_parts(const LeafArgs& a, const LeafWork& w, int na, double* A, int nb, double* B, cudaStream_t st,
-                         int64_t* launches)
+                         int64_t* launches, const uint8_t* skip = nullptr)
 {
     if (!w.partial) return;
     leaf_reduce<<<dim3((unsigned)((a.n + 127) / 128), (unsigned)(na + nb)), 128, 0, st>>>(
-        a.n, (int)w.grid.y, na, nb, w.partial, w.n_pad, w.tgt, A, B);
+        a.n, (int)w.grid.y, na, nb, w.partial, w.n_pad, w.tgt, skip, A, B);
     *launches += 1;
 }
 
@@ -792,7 +794,7 @@ static cudaError_t launch_leaf_k(const LeafArgs& a, const NearLists& L, void* wo
                                                              a.J, a.static_flags, a.transposed, a.SFS, w.partial,
                                                              w.n_pad);
         *launches += 2;
-        reduce_parts(a, w, 3, a.SFS, 0, nullptr, st, launches);
+        reduce_parts(a, w, 3, a.SFS, 0, nullptr, st, launches, a.static_flags);
     }
     return cudaGetLastError();
 }
@@ -828,11 +830,11 @@ static cudaError_t launch_leaf_dyn_k(const LeafArgs& a, const NearLists& L, doub
     leaf_pack_estr<K><<<w.gt, 256, 0, st>>>(n, a.x, a.gam, a.sig, a.J, a.static_flags, a.transposed, L.perm, 1, w.src);
     nf_estr<K, true, true><<<w.grid, NF_THREADS, 0, st>>>(n, L.ngroups, w.tgt, L.leaf_of, L.grp_row, L.ivs, w.src, a.J,
                                                           a.static_flags, a.transposed, dSFS, w.partial, w.n_pad, fd);
-    reduce_parts(a, w, 3, dSFS, 0, nullptr, st, launches);
+    reduce_parts(a, w, 3, dSFS, 0, nullptr, st, launches, a.static_flags);
     leaf_pack_estr<K><<<w.gt, 256, 0, st>>>(n, a.x, a.gam, sig_a, dJ, a.static_flags, a.transposed, L.perm, 1, w.src);
     nf_estr<K, true><<<w.grid, NF_THREADS, 0, st>>>(n, L.ngroups, w.tgt, L.leaf_of, L.grp_row, L.ivs, w.src, dJ,
                                                     a.static_flags, a.transposed, dSFS, w.partial, w.n_pad);
-    reduce_parts(a, w, 3, dSFS, 0, nullptr, st, launches);
+    reduce_parts(a, w, 3, dSFS, 0, nullptr, st, launches, a.static_flags);
     *launches += 4;
     return cudaGetLastError();
 }
