@@ -782,7 +782,6 @@ int vpm_uj_cross(vpm_ctx* c, const double* src, int64_t ld_src, int64_t ns, doub
     a.nt = nt; a.ns = ns; a.xt = (double*)c->xt.p; a.xs = (double*)c->x.p; a.gs = (double*)c->g.p;
     a.sgs = (double*)c->s.p; a.U = mt + R_U; a.ldU = VPM_NFIELDS; a.J = mt + R_J; a.ldJ = VPM_NFIELDS;
     a.kernel = kernel; a.precision = precision; a.self = false;
-    ensure_tiles(c, a, &w);
     CK(launch_uj(a, w, c->num_sms, st, &c->launches), "UJ kernels");
     RC(bounded_wait(c));
     const size_t pitch = VPM_NFIELDS * sizeof(double);

@@ -10,8 +10,8 @@
 // contributes exactly zero there, is excluded by index (in the factored form
 // its two terms would only cancel to rounding).  Static sources are packed with
 // zero strength; static targets are left untouched.  Targets run in curve
-// order (order.cu) like the UJ kernels.  The FP64 kernel keeps the reference's
-// zeta formula; the mixed kernel uses FP32 pair math on per-warp FP32 offsets
+// order (order.cu) like the UJ kernels.  The FP64 kernel takes
+// zeta from r^2 with a table exponential or one rsqrt; the mixed kernel uses FP32 pair math on per-warp FP32 offsets
 // (see uj.cu) and FP64 accumulation of FP32 blocks, and skips every pair at
 // r = 0 (the self pair, and coincident particles, whose J are equal so that
 // their reference term is zero; in the factored form their two terms would

@@ -26,7 +26,7 @@
 // source-side sums; z_ts depends on sigma_s only, so every 1/sigma_s factor is a
 // lane constant applied once at the end).  Particles run in curve order
 // (order.cu) in both roles; sums go to FP64 partial arrays per source split,
-// and an epilogue kernel per pass adds the splits in order and forms the
+// added in split order (sum_splits), and an epilogue kernel per pass forms the
 // outputs.  FP64 follows the formulas above pair by pair, coincident pairs
 // (r = 0, s != t) included as in the forward; FP32-comp takes the forward mixed
 // Estr's arithmetic (per-warp streaming, FP32 offsets from a per-warp
@@ -552,7 +552,7 @@ ea2_mx(int64_t n, const EA1Mx* __restrict__ self, const double* __restrict__ gam
 
 // ---------------------------------------------------------------- epilogues
 // Pass 1: x_t and J_t of every non-static target (curve position t).
-__global__ void ea1_epilogue(int64_t n, int nsplit, const double* __restrict__ partial, int64_t n_pad,
+__global__ void ea1_epilogue(int64_t n, const double* __restrict__ sums, int64_t n_pad,
                              const TgtPos* __restrict__ tgt, const uint8_t* __restrict__ st,
                              const double* __restrict__ Sbar, bool transposed, double* xbar, double* Jbar)
 {
@@ -561,11 +561,7 @@ __global__ void ea1_epilogue(int64_t n, int nsplit, const double* __restrict__ p
     const int64_t i = tgt[t].idx;
     if (st && st[i]) return;
     double a[NACC1];
-    for (int k = 0; k < NACC1; k++) {
-        double s = 0.0;
-        for (int sp = 0; sp < nsplit; sp++) s += partial[((int64_t)sp * NACC1 + k) * n_pad + t];
-        a[k] = s;
-    }
+    for (int k = 0; k < NACC1; k++) a[k] = sums[k * n_pad + t];
     for (int k = 0; k < 3; k++) xbar[3 * i + k] += a[3 + k];
     const double* sb = Sbar + 3 * i;
     for (int p = 0; p < 3; p++)
@@ -574,13 +570,13 @@ __global__ void ea1_epilogue(int64_t n, int nsplit, const double* __restrict__ p
 }
 
 // Pass 2: x_s, Gamma_s, sigma_s and J_s of every non-static source (curve position s);
-// `scale` = (ZNORM/sigma^3, ZNORM/sigma^5, -ZNORM/sigma^4) applied to (A, B), X, Sg (FP64:
-// A, B, Sg, X hold zeta itself, with ZNORM; mixed: zeta / ZNORM).
+// ZNORM/sigma^3, ZNORM/sigma^5 and -ZNORM/sigma^4 applied to (A, B), X and Sg, which are sums of
+// zeta / ZNORM.
 template <int K>
-__global__ void ea2_epilogue(int64_t n, int nsplit, const double* __restrict__ partial, int64_t n_pad,
+__global__ void ea2_epilogue(int64_t n, const double* __restrict__ sums, int64_t n_pad,
                              const TgtPos* __restrict__ tgt, const uint8_t* __restrict__ st,
                              const double* __restrict__ gam, const double* __restrict__ sig,
-                             const double* __restrict__ J, bool transposed, bool mixed, double* xbar, double* gbar,
+                             const double* __restrict__ J, bool transposed, double* xbar, double* gbar,
                              double* sbar, double* Jbar)
 {
     const int64_t s = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -588,11 +584,7 @@ __global__ void ea2_epilogue(int64_t n, int nsplit, const double* __restrict__ p
     const int64_t i = tgt[s].idx;
     if (st && st[i]) return;
     double a[NACC2];
-    for (int k = 0; k < NACC2; k++) {
-        double v = 0.0;
-        for (int sp = 0; sp < nsplit; sp++) v += partial[((int64_t)sp * NACC2 + k) * n_pad + s];
-        a[k] = v;
-    }
+    for (int k = 0; k < NACC2; k++) a[k] = sums[k * n_pad + s];
     const double is = 1.0 / sig[i];
     const double zn = zeta_norm(K);
     const double c3 = zn * is * is * is, c5 = c3 * is * is, c4 = -c3 * is;
@@ -630,7 +622,7 @@ cudaError_t launch_k(const EstrAdjArgs& a, const EstrAdjWork& w, int num_sms, cu
         ea1_f64<K><<<grid, UJ_THREADS, 0, st>>>(n, tgt, (const EA2F64*)w.pack2, n_pad, (const EA1F64*)w.pack1,
                                                 w.partial);
         sum_splits(w.partial, nsplit, NACC1, n, n_pad, st, launches);
-        ea1_epilogue<<<eg, pb, 0, st>>>(n, 1, w.partial, n_pad, tgt, a.static_flags, a.Sbar, a.transposed,
+        ea1_epilogue<<<eg, pb, 0, st>>>(n, w.partial, n_pad, tgt, a.static_flags, a.Sbar, a.transposed,
                                         a.xbar, a.Jbar);
         ea2_f64<K><<<grid, UJ_THREADS, 0, st>>>(n, (const EA1F64*)w.pack1, n_pad, (const EA2F64*)w.pack2,
                                                 w.partial);
@@ -638,14 +630,14 @@ cudaError_t launch_k(const EstrAdjArgs& a, const EstrAdjWork& w, int num_sms, cu
         ea1_mx<K><<<grid, UJ_THREADS, 0, st>>>(n, tgt, (const EA2Mx*)w.pack2, n_pad, (const EA1Mx*)w.pack1, box,
                                                w.partial);
         sum_splits(w.partial, nsplit, NACC1, n, n_pad, st, launches);
-        ea1_epilogue<<<eg, pb, 0, st>>>(n, 1, w.partial, n_pad, tgt, a.static_flags, a.Sbar, a.transposed,
+        ea1_epilogue<<<eg, pb, 0, st>>>(n, w.partial, n_pad, tgt, a.static_flags, a.Sbar, a.transposed,
                                         a.xbar, a.Jbar);
         ea2_mx<K><<<grid, UJ_THREADS, 0, st>>>(n, (const EA1Mx*)w.pack1, a.gam, tgt, a.J, a.static_flags,
                                                a.transposed, n_pad, (const EA2Mx*)w.pack2, box, w.partial);
     }
     sum_splits(w.partial, nsplit, NACC2, n, n_pad, st, launches);
-    ea2_epilogue<K><<<eg, pb, 0, st>>>(n, 1, w.partial, n_pad, tgt, a.static_flags, a.gam, a.sig, a.J,
-                                       a.transposed, mixed, a.xbar, a.gbar, a.sbar, a.Jbar);
+    ea2_epilogue<K><<<eg, pb, 0, st>>>(n, w.partial, n_pad, tgt, a.static_flags, a.gam, a.sig, a.J,
+                                       a.transposed, a.xbar, a.gbar, a.sbar, a.Jbar);
     *launches += 5;
     return cudaGetLastError();
 }

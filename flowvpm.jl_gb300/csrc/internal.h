@@ -47,7 +47,6 @@ constexpr int UJ_THREADS = 128;   // targets per block, one per thread
 constexpr int UJ_WARPS = UJ_THREADS / 32;
 constexpr int UJ_TILE = 128;      // sources staged in shared memory per tile
 constexpr int UJ_BLOCK = 64;      // sources summed in FP32 per inner block
-constexpr int UJ_FLUSH_TILES = 2; // tiles summed in FP32 before the FP64 add
 
 // Problem description handed from the ABI layer to the kernel launchers.
 struct UJArgs {

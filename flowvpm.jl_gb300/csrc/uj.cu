@@ -23,7 +23,7 @@
 //    warp evaluates those 4 pairs with dx = (x_t,hi - x_s,hi) + (x_t,lo - x_s,lo)
 //    and the full regular form of the kernel (vpm_math.cuh).
 // Sums run in FP32 over blocks of UJ_BLOCK sources, then in an FP32 mid-level
-// sum over UJ_FLUSH_TILES tiles, then in FP64.  In tiles with near sources the
+// sum over MID_BLOCKS of those, then in FP64.  In tiles with near sources the
 // FP32 blocks are of 8: a target's largest terms stand in one or two tiles of the
 // curve and often add with one sign (ring of 1,000, J: error 1.7e-7 with blocks of
 // 64, 0.8e-7 so, for 2 % of the time; 1.6e-7 in the caller's order).

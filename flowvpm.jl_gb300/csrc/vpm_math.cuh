@@ -31,7 +31,6 @@ constexpr double C1 = 0.063493635934240969;   // 1/(2*pi)^1.5
 constexpr double C2 = 0.79788456080286541;    // sqrt(2/pi)
 constexpr double C3 = 0.23873241463784300;    // 3/(4*pi)
 constexpr double C4 = 0.079577471545947673;   // 1/(4*pi)
-constexpr double INV_SQRT2 = 0.70710678118654752;
 
 enum : int { K_SING = 0, K_GAUS = 1, K_GAUSERF = 2, K_WNKLMNS = 3 };
 
