@@ -246,8 +246,8 @@ constexpr int ESTR_FLUSH_TILES = 24;     // evaluated warp tiles between FP64 ad
 // instruction and 16-byte reads of four sources' coordinates a pair takes 18 issue slots; one
 // source at a time from 64-byte records took 24 and 80 % of the shared-memory rate (every lane
 // reads every source, and the records' copies and conversions met bank conflicts).  Rings of
-// 200,000: 3.77 -> 3.08 ms; jet of 100,000, Winckelmans (no reach): 9.70 -> 8.69 ms (3.01 and
-// 8.55 before the test for coarse offsets).
+// 200,000: 3.77 -> 3.15 ms; jet of 100,000, Winckelmans (no reach): 9.70 -> 8.69 ms (2.98 and
+// 8.49 before the choice for coarse offsets).
 // With DZ (the weight difference of the dynamic procedure's test filter,
 // dynamic.cu) each weight zeta~(r, sigma_s) is replaced by
 // zeta~(r, alpha sigma_s) - zeta~(r, sigma_s) = zeta~(r, sigma_s) (ratio - 1),
@@ -365,7 +365,8 @@ estr_mixed_kernel(int64_t nt, const TgtPos* __restrict__ tgt, const double* __re
         }
         __syncwarp();
         if (beyond != 0xffffffffu) {
-            // (two loops: with the choice inside one loop the dense fields took 15 % longer)
+            // (two loops cost dense fields, which take the second, 5 %; the choice inside one loop cost them 15,
+            // a call for the first 5, and a pass of its own after the others 18)
             auto sources = [&](auto two_parts) {
 #pragma unroll 1
                 for (int sub = 0; sub < EWT; sub += ESTR_SUB) {

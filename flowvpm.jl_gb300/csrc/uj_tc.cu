@@ -42,11 +42,11 @@
 // reads.
 //
 // Bound: issue slots.  A far pair takes 10.5 instructions (packed f32x2 r^2 and weights, one
-// MUFU, the f16 splits) plus 4 for its share of a tile's set-up, waits and recombination,
-// against 40.4 in uj_mixed_kernel; 66 % of the issue slots are used (4 warps a scheduler, the
-// TMEM's limit), the tensor pipe 17 %.  Measured, whole calls, Gaussian-erf: N = 2^20 1360 ->
-// 735 ms, 262,144 102.8 -> 52.0, 65,536 7.83 -> 4.00, rings of 200,000 57.8 -> 39.5, ring of
-// 32,000 2.40 -> 1.52; Winckelmans 50,001 4.61 -> 2.66.  Tried: packed pairs split back to
+// MUFU, the f16 splits) plus 4.5 for its share of a tile's set-up, waits and recombination; all
+// classes together 19.0 at 262,144, against 40.4 in uj_mixed_kernel.  68 % of the issue slots are
+// used (4 warps a scheduler, the TMEM's limit), the tensor pipe 14 %.  Measured, whole calls,
+// Gaussian-erf: N = 2^20 1360 -> 758 ms, 262,144 102.8 -> 53.4, 65,536 7.83 -> 4.12, rings of
+// 200,000 57.8 -> 41.4, ring of 32,000 2.40 -> 1.62; Winckelmans 50,001 4.61 -> 2.77.  Tried: packed pairs split back to
 // scalar FP32 13 % slower, f16 remainders by conversion instead of the mixed-precision
 // subtraction 11 %, three blocks a SM 6 %, two A buffers of 16 sources (twice the barriers)
 // 16 %.
