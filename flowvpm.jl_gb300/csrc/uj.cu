@@ -65,8 +65,9 @@ int uj_num_splits(int64_t nt, int64_t ns, int num_sms, int precision, int per_sm
 
 // The tile kernels (uj_tc.cu) take a set on itself from 10,240 particles.  Below, most tiles of
 // 64 are near ones (4,099 random particles: 73 % of the pairs) and the tile pack is pure cost.
-// With uj_mixed_kernel / with tiles, us: random 6,500 269 / 275, 8,192 307 / 293, 10,000 378 / 360,
-// 12,000 450 / 424; ring of 8,000 291 / 305, of 12,000 445 / 431; Winckelmans 8,192 287 / 290.
+// With uj_mixed_kernel / with tiles, us: random 8,192 306 / 299, 10,240 382 / 390, 12,000 454 / 435,
+// 14,000 542 / 495; rings of 8,192 300 / 304, of 10,240 372 / 387, of 12,000 439 / 431; Winckelmans
+// 8,192 288 / 287, 10,240 373 / 364; jet of 10,240 408 / 429, of 12,000 477 / 472.
 bool uj_takes_tiles(const UJArgs& a) { return a.self && a.precision == 1 && a.ns >= 10240; }
 
 size_t uj_partial_bytes(int64_t nt, int nsplit, int components)
