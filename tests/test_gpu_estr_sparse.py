@@ -47,6 +47,18 @@ def test_close_pairs(ctx, n, kernel):
         assert (err <= lim).all(), f"seed {seed}: {float((err / lim).max()):.2f}"
 
 
+@pytest.mark.parametrize("kernel", [2, 3])
+@pytest.mark.parametrize("n", [4099, 12_000])
+def test_close_pairs_beside_a_far_particle(ctx, n, kernel):
+    x, g, sig, J = sparse(n, 1, outlier=1e3)
+    S = [torch.zeros(n, 3, device="cuda", dtype=torch.float64) for _ in range(2)]
+    for precision in (0, 1):
+        ctx.estr_dev(x, J, x, g, sig, J, S[precision], kernel, precision)
+    err = (S[1] - S[0]).norm(dim=1)
+    lim = bound(x, g, sig, J, kernel) + 1e-13 * S[0].norm()
+    assert (err <= lim).all(), f"{float((err / lim).max()):.2f}"
+
+
 @pytest.mark.parametrize("kernel", [1, 2, 3])
 @pytest.mark.parametrize("n", [33, 700, 1630, 4099])
 def test_close_pairs_adjoint(ctx, n, kernel):
